@@ -6,34 +6,30 @@
 // (PEGen_RayTracing_CircularHole/PESysMatGen.cu:951-1364), with a different execution plan:
 //
 //  * a block owns one crystal d and a 4x4x2 brick of voxels (work items handed out by an
-//    atomic counter over a persistent grid); one warp per matrix element; the 32 lanes
-//    take 32 consecutive sub-elements per round, 32 rounds;
-//  * candidate culling runs in three stages.  (1) Block: a conservative superset of the
-//    reference's cone test (:1105-1186) for every voxel of the brick, from the brick's
-//    centre and radius, is compacted into shared memory in the reference's object order.
-//    (2) Warp: the reference cone test itself, with the reference's float formula, on the
-//    superset; a passing object is kept only if its direction-slope rectangle (dx/dy,
-//    dz/dy seen from the voxel) overlaps the one of crystal d.  (3) Lane: an object whose
-//    rectangle does not contain the sub-element ray's slope is skipped.  A skipped object
-//    has an exactly-zero chord in the reference, and adding 0 or fma(mu, 0, x) leaves a
-//    float unchanged, so no stage changes any float result;
-//  * when an element has more kept objects than one shared-memory chunk holds, the warp
-//    walks them chunk by chunk for every round, in the same order, so the attenuation
-//    sums keep the reference's order;
+//    atomic counter over a persistent grid); one warp per matrix element;
+//  * the block builds a conservative superset of the reference's cone test (:1105-1186) for
+//    every voxel of the brick, from the brick's centre and radius, in the reference's object
+//    order.  Each warp keeps the objects of its element that pass the reference cone test and
+//    whose direction-slope rectangle (dx/dy, dz/dy seen from the voxel) overlaps the one of
+//    crystal d, and 32 rays at a time take those that can meet their slopes.  A skipped object
+//    has an exactly-zero chord in the reference, and adding 0 or fma(mu, 0, x) leaves a float
+//    unchanged, so no filter changes any float result;
 //  * the plate-bypass penalty (:1240-1254) is skipped for rays whose slope lies inside the
 //    plate's "through both faces" rectangle, where the chord is >= T >= 0.2 mm;
 //  * sub-elements whose plate penalty fired contribute exp(-(>=1e5)) = 0 and stop early
-//    (only when every attenuation coefficient is non-negative);
-//  * the element sum is one float chain in the reference's sub-element order
-//    (SYSMAT_MODE_REFERENCE, the reference's atomicAdd sequence at :1359) or an FP64
-//    accumulation (SYSMAT_MODE_PRECISE); lane 0 writes dst[d][v].
+//    (only when every attenuation coefficient is non-negative).
 //
-// Two more instances share the execution plan: the FP64 mode (SYSMAT_MODE_FP64,
-// pe_fp64.cuh: the element program in double, culling in float) and the sampled form
-// (pe_element_sampled: crystal divisions and voxel source points as parameters).
+// The element itself: pe_ref.cuh for the float modes SYSMAT_MODE_REFERENCE (one float chain in
+// the reference's sub-element order, its atomicAdd sequence at :1359) and SYSMAT_MODE_PRECISE
+// (the same contributions summed in FP64); pe_fp64.cuh (SYSMAT_MODE_FP64: the element program
+// in double, culling in float); pe_local.cuh (SYSMAT_MODE_LOCAL); pe_element_sampled (crystal
+// divisions and voxel source points as parameters); pe_adjoint.cuh (projections, gradient).
+#include <type_traits>
+
 #include "chord64.cuh"
 #include "geom.cuh"
 #include "pe.cuh"
+#include "rounding.cuh"
 
 namespace sysmat {
 
@@ -47,13 +43,25 @@ constexpr int kRound = 64;              // per-warp round buffer
 constexpr float kSlopeMargin = 2e-4f;   // slope units; >> FP32 position error / depth
 constexpr float kMinDepth = 1.0f;       // mm; slope rectangles need objects this far behind
 
+// Per-element constants shared by the lanes of a warp.
+struct Elem {
+    float xI, yI, zI;            // voxel centre (rotated)
+    float xIs, yIs, zIs;         // voxel in crystal d's frame
+    float xd, yd, zd, w, t, h;   // crystal d
+    float cosr, sinr;
+    float mu_t, mu_pe, imu_t;    // and RN(1 / mu_t)
+    float ux, uy, uz, crit_self; // reference cone test (:1110-1116)
+    float4 rd;                   // slope rectangle of crystal d
+    bool filt;
+};
+
 struct WarpSmem {
     // kept objects of the element (reference cone test + bundle filter), reference order
     float4 rect[kChunk];
     int id[kChunk];                      // holes: hole index; crystals: n_holes + crystal
     // the current round's objects (kept objects whose rectangle meets the round's rays),
     // with their geometry, so the walk reads contiguous shared memory:
-    //   hole:    A = (x, z, R, mu),   B = (y1, y2, -, -)
+    //   hole:    A = (x, z, R, mu),   B = (y1, y2, voxel x - x, voxel z - z)
     //   crystal: A = (x, y, z, mu),   B = (cos(-rot), sin(-rot), w, t),
     //            C = (h, voxel x, y, z in the crystal's frame)
     float4 rr[kRound], ra[kRound], rb[kRound], rc[kRound];
@@ -65,12 +73,16 @@ struct WarpSmem {
     };
 };
 
-struct BlockSmem {
-    float4 sdata[kSuperCap];             // holes: x, (y1+y2)/2, z, crit; crystals: x, y, z, diag
-    int sid[kSuperCap];
+// The objects that may pass the cone test for some voxel of a block's brick, in the reference's
+// order, and the block's work item.
+struct Superset {
+    unsigned short sid[kSuperCap];       // holes, then n_holes + crystal (at most 8877 + 6666 ids)
     int warp_cnt[kWarps];
     int s_count;                         // superset size; -1 = superset overflowed, use all
     long long item;
+};
+
+struct BlockSmem : Superset {
     WarpSmem w[kWarps];
 };
 
@@ -147,18 +159,6 @@ __device__ __forceinline__ int layer_of_hole(const DevGeom& g, int h)
     return m;
 }
 
-// Per-element constants shared by the lanes of a warp.
-struct Elem {
-    float xI, yI, zI;            // voxel centre (rotated)
-    float xIs, yIs, zIs;         // voxel in crystal d's frame
-    float xd, yd, zd, w, t, h;   // crystal d
-    float cosr, sinr;
-    float mu_t, mu_pe;
-    float ux, uy, uz, crit_self; // reference cone test (:1110-1116)
-    float4 rd;                   // slope rectangle of crystal d
-    bool filt;
-};
-
 // Reference cone test of object i against element e (:1120-1184), then the bundle filter.
 // Returns true if the object is kept; rect receives its slope rectangle.
 __device__ __forceinline__ bool keep_object(const DevGeom& g, const Elem& e, int i, float4 od,
@@ -209,8 +209,7 @@ __device__ int build_chunk(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, 
         int id = 0;
         if (j < n_src) {
             id = from_super ? bs.sid[j] : j;
-            const float4 od = from_super ? bs.sdata[j] : object_data(g, j);
-            keep = keep_object(g, e, id, od, d, rect);
+            keep = keep_object(g, e, id, object_data(g, id), d, rect);
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
@@ -250,12 +249,14 @@ __device__ __forceinline__ void close_layers(const DevGeom& g, Walk& s, int upto
 // Terms of the reference cylinder chord (PESysMatGen.cu:688-799) that depend only on the
 // ray (voxel -> sub-element) and on the cap planes y1, y2.  Hoisting them out of the
 // per-hole evaluation keeps every float identical: each is the same operation on the same
-// operands as in the per-hole formula.
+// operands as in the per-hole formula, and the divisions that share a divisor (tio, ky, kk)
+// go through its correctly rounded reciprocal (div_by: the quotient IEEE division gives).
 struct RayCyl {
     float xi, yi, zi, tio, kx, ky, kz, rx, rz, kk;
+    float iky, ikk;              // RN(1 / ky), RN(1 / kk)
     float y1, y2;                // cap planes the cached terms below belong to
-    bool degenerate;             // |y1 - y2| < 0.001
     float ta, tb, xl, xr, zl, zr;
+    float full;                  // chord of a ray inside the hole at both caps
 };
 
 __device__ __forceinline__ void ray_cyl_init(RayCyl& c, float xi, float yi, float zi, float xo, float yo,
@@ -263,13 +264,21 @@ __device__ __forceinline__ void ray_cyl_init(RayCyl& c, float xi, float yi, floa
 {
     const float dx = xo - xi, dy = yo - yi, dz = zo - zi;
     c.xi = xi; c.yi = yi; c.zi = zi;
-    c.tio = sqrtf(dx * dx + dy * dy + dz * dz);
-    c.kx = dx / c.tio;
-    c.ky = dy / c.tio;
-    c.kz = dz / c.tio;
-    c.rx = c.kx / c.ky;
-    c.rz = c.kz / c.ky;
+    c.tio = sqrt_mid(dx * dx + dy * dy + dz * dz);
+    const float itio = rcp_rn(c.tio);
+    c.kx = div_by(dx, c.tio, itio);
+    c.ky = div_by(dy, c.tio, itio);
+    c.kz = div_by(dz, c.tio, itio);
+    c.iky = rcp_rn(c.ky);
+    if (fabsf(c.ky) >= kMinDivisor) {
+        c.rx = div_by(c.kx, c.ky, c.iky);
+        c.rz = div_by(c.kz, c.ky, c.iky);
+    } else {                     // a ray along the plates
+        c.rx = c.kx / c.ky;
+        c.rz = c.kz / c.ky;
+    }
     c.kk = c.kx * c.kx + c.kz * c.kz;
+    c.ikk = rcp_rn(c.kk);
     c.y1 = NAN;                  // no cap planes cached yet (NaN never compares equal)
     c.y2 = NAN;
 }
@@ -279,40 +288,45 @@ __device__ __forceinline__ void ray_cyl_caps(RayCyl& c, float y1, float y2)
     if (y1 == c.y1 && y2 == c.y2) return;
     c.y1 = y1;
     c.y2 = y2;
-    c.degenerate = fabsf(y1 - y2) < 0.001f;
     c.xl = c.xi + c.rx * (y1 - c.yi);
     c.xr = c.xi + c.rx * (y2 - c.yi);
     c.zl = c.zi + c.rz * (y1 - c.yi);
     c.zr = c.zi + c.rz * (y2 - c.yi);
-    c.ta = (y1 - c.yi) / c.ky;
-    c.tb = (y2 - c.yi) / c.ky;
+    if (fabsf(c.ky) >= kMinDivisor) {
+        c.ta = div_by(y1 - c.yi, c.ky, c.iky);
+        c.tb = div_by(y2 - c.yi, c.ky, c.iky);
+    } else {
+        c.ta = (y1 - c.yi) / c.ky;
+        c.tb = (y2 - c.yi) / c.ky;
+    }
+    c.full = fabsf(c.tb - c.ta);
+    if (c.ta <= 0.0001f || c.tb <= 0.0001f || c.ta >= c.tio || c.tb >= c.tio) c.full = 0.0f;
+    // closer than 0.001: the reference returns 0; with both cap parameters 0 every case below does
+    if (fabsf(y1 - y2) < 0.001f) c.ta = c.tb = c.full = 0.0f;
 }
 
-// Cylinder chord of hole (xc, zc, r) with cap planes already cached in c.
-__device__ __forceinline__ float ray_cyl_chord(const RayCyl& c, float xc, float zc, float r)
+// Cylinder chord of hole (xc, zc, r), (ox, oz) = voxel - centre, with cap planes already
+// cached in c.  Straight-line: the reference's four cap/side cases are selects, so a warp
+// whose lanes meet different cases runs the code once, and two entries interleave (the four
+// returns of the branching form each cost a divergent pass).
+__device__ __forceinline__ float ray_cyl_chord(const RayCyl& c, float xc, float zc, float r, float ox, float oz)
 {
-    if (c.degenerate) return 0.0f;
     const bool fl = (c.xl - xc) * (c.xl - xc) + (c.zl - zc) * (c.zl - zc) <= r * r;
     const bool fr = (c.xr - xc) * (c.xr - xc) + (c.zr - zc) * (c.zr - zc) <= r * r;
-    if (fl && fr) {
-        if (c.ta <= 0.0001f || c.tb <= 0.0001f) return 0.0f;
-        if (c.ta >= c.tio || c.tb >= c.tio) return 0.0f;
-        return fabsf(c.tb - c.ta);
-    }
-    const float ox = c.xi - xc, oz = c.zi - zc;
     const float disc = c.kk * r * r - (c.kx * oz - c.kz * ox) * (c.kx * oz - c.kz * ox);
-    if (disc <= 0.00001f) return 0.0f;
-    const float t1 = (-(c.kx * ox + c.kz * oz) - sqrtf(disc)) / c.kk;
-    const float t2 = (-(c.kx * ox + c.kz * oz) + sqrtf(disc)) / c.kk;
-    float ea, eb;
-    if (!fl && !fr) {
-        if (!(t1 >= c.ta && t2 <= c.tb)) return 0.0f;
-        ea = t1; eb = t2;
-    } else if (fl) { ea = c.ta; eb = t2; }
-    else           { ea = t1; eb = c.tb; }
-    if (eb <= 0.0001f || ea <= 0.0001f) return 0.0f;
-    if (eb >= c.tio || ea >= c.tio) return 0.0f;
-    return eb - ea;
+    const bool meets = disc > 0.00001f;
+    const float sd = sqrt_mid(meets ? disc : 1.0f);
+    const float t1 = div_by(-(c.kx * ox + c.kz * oz) - sd, c.kk, c.ikk);
+    const float t2 = div_by(-(c.kx * ox + c.kz * oz) + sd, c.kk, c.ikk);
+    const float ea = fl ? c.ta : t1, eb = fr ? c.tb : t2;
+    const bool ok = meets && (fl || fr || (t1 >= c.ta && t2 <= c.tb)) &&
+                    !(eb <= 0.0001f || ea <= 0.0001f || eb >= c.tio || ea >= c.tio);
+    return (fl && fr) ? c.full : (ok ? eb - ea : 0.0f);
+}
+
+__device__ __forceinline__ float ray_cyl_chord(const RayCyl& c, float xc, float zc, float r)
+{
+    return ray_cyl_chord(c, xc, zc, r, c.xi - xc, c.zi - zc);
 }
 
 // Slope-space shadow of a y-aligned object (hole cylinder, or crystal in the disk around its
@@ -326,7 +340,7 @@ struct Capsule {
 
 __device__ __forceinline__ Capsule capsule_of(float xo, float zo, float y0, float y1, float R, const Elem& e)
 {
-    const float r0 = __frcp_rn(y0 - e.yI), r1 = __frcp_rn(y1 - e.yI);
+    const float r0 = rcp_approx(y0 - e.yI), r1 = rcp_approx(y1 - e.yI);
     Capsule c;
     c.ax = (xo - e.xI) * r0;
     c.az = (zo - e.zI) * r0;
@@ -425,7 +439,7 @@ __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const 
                 const float4 hb = __ldg(&g.hole.b[id]);
                 ws.rr[pos] = rect;
                 ws.ra[pos] = make_float4(ha.x, ha.w, hb.x, hb.y);
-                ws.rb[pos] = make_float4(ha.y, ha.z, 0.0f, 0.0f);
+                ws.rb[pos] = make_float4(ha.y, ha.z, e.xI - ha.x, e.zI - ha.w);
                 if constexpr (ELL) {        // rho_x, rho_z, cos, sin; a batch may mix in circular systems
                     ws.rc[pos] = g.hole_shape ? __ldg(&g.hole_shape[id]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 }
@@ -461,62 +475,75 @@ __device__ __forceinline__ bool hole_in_reach(const WarpSmem& ws, int j, float s
 
 // Walk round-buffer entries [0, nr) for one sub-element ray (voxel -> (xD, yD, zD)); holes
 // occupy [0, nh) and crystals [nh, nr), both in the reference's object order; the layer
-// terms are added when the walk leaves a layer.
+// terms are added when the walk leaves a layer.  Called by the whole warp: a lane without a
+// ray passes live = false and takes part with no entry, so every branch on an entry is
+// uniform.  Holes go two at a time when they share layer and cap planes (independent
+// straight-line chords: the serial chain of one chord leaves issue slots idle); a lane that an
+// entry does not concern adds an exact zero.
 template <bool ELL>
 __device__ __forceinline__ void walk_round(const DevGeom& g, const WarpSmem& ws, int nh, int nr,
                                            float xD, float yD, float zD, float sa_a, float sa_b,
-                                           float cosang, RayCyl& rc, Walk& s)
+                                           float cosang, bool live, RayCyl& rc, Walk& s)
 {
-    // the next entry's layer and rectangle are loaded one iteration ahead (shared-memory
-    // latency off the dependency chain: 4-5 % on the reference mode, same results)
-    int m_next = nh > 0 ? ws.rl[0] : 0;
-    float4 r_next = nh > 0 ? ws.rr[0] : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j < nh; ++j) {
-        const int m = m_next;
-        const float4 R = r_next;
-        if (j + 1 < nh) {
-            m_next = ws.rl[j + 1];
-            r_next = ws.rr[j + 1];
-        }
-        if (m != s.lay) close_layers(g, s, m, cosang);
-        if (!in_rect(R, sa_a, sa_b)) continue;
+    for (int j = 0; j < nh;) {
+        const int m = ws.rl[j];
         const float4 A = ws.ra[j];
         const float4 B = ws.rb[j];
-        float tmp;
+        if (m != s.lay) close_layers(g, s, m, cosang);
+        const bool in = live && in_rect(ws.rr[j], sa_a, sa_b);
         if constexpr (ELL) {
-            const float4 S = ws.rc[j];
+            ++j;
+            if (!__any_sync(0xffffffffu, in)) continue;
+            const float4 S = ws.rc[j - 1];
+            float tmp = 0.0f;
             if (S.x > 0.0f) {                                    // elliptical hole
-                tmp = ell_chord(rc.xi, rc.yi, rc.zi, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w);
+                if (in) tmp = ell_chord(rc.xi, rc.yi, rc.zi, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w);
             } else {
                 ray_cyl_caps(rc, B.x, B.y);
-                tmp = ray_cyl_chord(rc, A.x, A.y, A.z);
+                if (in) tmp = ray_cyl_chord(rc, A.x, A.y, A.z, B.z, B.w);
             }
+            s.len = s.len + tmp;                                 // :1276-1278
+            s.att = s.att + A.w * tmp;
+            s.hole_hits += (tmp != 0.0f);
+            s.hole_evals += in;
         } else {
+            const int k = j + 1 < nh ? j + 1 : j;
+            const float4 A2 = ws.ra[k];
+            const float4 B2 = ws.rb[k];
+            const bool pair = k > j && ws.rl[k] == m && B2.x == B.x && B2.y == B.y;
+            const bool in2 = pair && live && in_rect(ws.rr[k], sa_a, sa_b);
+            j = pair ? j + 2 : j + 1;
+            if (!__any_sync(0xffffffffu, in || in2)) continue;
             ray_cyl_caps(rc, B.x, B.y);
-            tmp = ray_cyl_chord(rc, A.x, A.y, A.z);
+            float tmp = ray_cyl_chord(rc, A.x, A.y, A.z, B.z, B.w);
+            float tmp2 = ray_cyl_chord(rc, A2.x, A2.y, A2.z, B2.z, B2.w);
+            tmp = in ? tmp : 0.0f;
+            tmp2 = in2 ? tmp2 : 0.0f;
+            s.len = s.len + tmp;                                 // :1276-1278
+            s.att = s.att + A.w * tmp;
+            s.len = s.len + tmp2;
+            s.att = s.att + A2.w * tmp2;
+            s.hole_hits += (tmp != 0.0f) + (tmp2 != 0.0f);
+            s.hole_evals += in + in2;
         }
-        s.len = s.len + tmp;                                     // :1276-1278
-        s.att = s.att + A.w * tmp;
-        s.hole_hits += (tmp != 0.0f);
-        ++s.hole_evals;
     }
     if (nr <= nh) return;
     if (s.lay < g.n_layers) close_layers(g, s, g.n_layers, cosang);
-    float4 c_next = ws.rr[nh];
     for (int j = nh; j < nr; ++j) {
-        const float4 R = c_next;
-        if (j + 1 < nr) c_next = ws.rr[j + 1];
-        if (!in_rect(R, sa_a, sa_b)) continue;
+        const bool in = live && in_rect(ws.rr[j], sa_a, sa_b);
+        if (!__any_sync(0xffffffffu, in)) continue;
         const float4 A = ws.ra[j];
         const float4 B = ws.rb[j];
         const float4 C = ws.rc[j];
         float xb, yb, zb;                                        // :1318-1320
         to_crystal_frame(A.x, A.y, A.z, B.x, B.y, xD, yD, zD, xb, yb, zb);
-        const float la = box_chord(C.y, C.z, C.w, xb, yb, zb, -0.5f * B.z, -0.5f * B.w, -0.5f * C.x,
-                                   0.5f * B.z, 0.5f * B.w, 0.5f * C.x);
+        float la = 0.0f;
+        if (in)
+            la = box_chord(C.y, C.z, C.w, xb, yb, zb, -0.5f * B.z, -0.5f * B.w, -0.5f * C.x, 0.5f * B.z, 0.5f * B.w,
+                           0.5f * C.x);
         s.att = s.att + la * A.w;
         s.cry_hits += (la != 0.0f);
-        ++s.cry_evals;
+        s.cry_evals += in;
     }
 }
 
@@ -559,16 +586,22 @@ __device__ __forceinline__ SubElem sub_element(const Elem& e, int s)
     return sub_element_at(e, (s >> 4) & 7, s & 15, s >> 7, 8.0f, 16.0f, 8.0f);
 }
 
+// box_chord of the segment voxel -> sub-element through a plate, out of line: few rays need it.
+static __device__ __noinline__ float plate_chord(float xi, float yi, float zi, float xo, float yo, float zo,
+                                                 float x1, float y1, float z1, float x2, float y2, float z2)
+{
+    return box_chord(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2);
+}
+
 // Plate penalty (:1240-1254); true if any layer fired.
-__device__ __forceinline__ bool plate_penalty(const DevGeom& g, const WarpSmem& ws, const Elem& e,
-                                              const SubElem& q, float& att)
+__device__ __forceinline__ bool plate_penalty(const DevGeom& g, const float4* plate_inner, const Elem& e, float xD,
+                                              float yD, float zD, float sa_a, float sa_b, float& att)
 {
     bool blocked = false;
     for (int m = 0; m < g.n_layers; ++m) {
-        if (in_rect(ws.inner[m], q.sa_a, q.sa_b)) continue;
-        const LayerInfo& Ly = g.layer[m];
-        const float tl = box_chord(e.xI, e.yI, e.zI, q.xD, q.yD, q.zD, Ly.x1, Ly.y1, Ly.z1, Ly.x2,
-                                   Ly.y2, Ly.z2);
+        if (in_rect(plate_inner[m], sa_a, sa_b)) continue;
+        const LayerInfo& L = g.layer[m];
+        const float tl = plate_chord(e.xI, e.yI, e.zI, xD, yD, zD, L.x1, L.y1, L.z1, L.x2, L.y2, L.z2);
         if (tl < 0.1f) { att = att + 100000.0f; blocked = true; }
     }
     return blocked;
@@ -609,15 +642,10 @@ __device__ __forceinline__ float finish_sub_element_at(const Elem& e, const SubE
     return eff * sa * absf;
 }
 
-__device__ __forceinline__ float finish_sub_element(const Elem& e, const SubElem& q, float att)
-{
-    return finish_sub_element_at(e, q, att, 8.0f, 16.0f, 8.0f);
-}
-
 // Per-element set-up shared by the lanes of a warp: voxel centre, crystal d, reference cone
 // constants, slope rectangle and the plate "through both faces" rectangles.  False when the
 // crystal's attenuation is too low for the reference to compute the element (it is 0).
-__device__ __forceinline__ bool init_element(const DevGeom& g, WarpSmem& ws, int d, long long v, float cr,
+__device__ __forceinline__ bool init_element(const DevGeom& g, float4* plate_inner, int d, long long v, float cr,
                                              float sr, int lane, Elem& e, float fx = 0.5f, float fy = 0.5f,
                                              float fz = 0.5f)
 {
@@ -631,7 +659,11 @@ __device__ __forceinline__ bool init_element(const DevGeom& g, WarpSmem& ws, int
     e.mu_t = M.x; e.mu_pe = M.y;
     e.cosr = T.x; e.sinr = T.y;
     if (!(e.mu_t > 0.01f)) return false;                   // :1107, :1194
-    to_crystal_frame(e.xd, e.yd, e.zd, T.z, T.w, e.xI, e.yI, e.zI, e.xIs, e.yIs, e.zIs);
+    e.imu_t = rcp_rn(e.mu_t);
+    const float vx = e.xI - e.xd, vz = e.zI - e.zd;        // :1066-1068, to_crystal_frame
+    e.xIs = __fmaf_rn(vx, T.z, -__fmul_rn(vz, T.w));
+    e.yIs = e.yI - e.yd;
+    e.zIs = __fmaf_rn(vx, T.w, __fmul_rn(vz, T.z));
     const float dist = sqrtf((e.yd - e.yI) * (e.yd - e.yI) + (e.xd - e.xI) * (e.xd - e.xI) +
                              (e.zd - e.zI) * (e.zd - e.zI));
     e.crit_self = S.w / dist / 2.0f;
@@ -653,7 +685,7 @@ __device__ __forceinline__ bool init_element(const DevGeom& g, WarpSmem& ws, int
             inner.z = fmaxf((Ly.z1 - e.zI) * r0, (Ly.z1 - e.zI) * r1) + kSlopeMargin;
             inner.w = fminf((Ly.z2 - e.zI) * r0, (Ly.z2 - e.zI) * r1) - kSlopeMargin;
         }
-        ws.inner[lane] = inner;
+        plate_inner[lane] = inner;
     }
 
     return true;
@@ -692,7 +724,7 @@ __device__ __forceinline__ bool walk_sub_element(const DevGeom& g, const BlockSm
 {
     RayCyl rc;
     ray_cyl_init(rc, e.xI, e.yI, e.zI, q.xD, q.yD, q.zD);
-    const bool blocked = plate_penalty(g, ws, e, q, s.att);
+    const bool blocked = plate_penalty(g, ws.inner, e, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, s.att);
     const bool skip = dead || (blocked && g.nonneg_mu);
     // slope box of the rays that still need the walk in this round
     float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
@@ -719,7 +751,7 @@ __device__ __forceinline__ bool walk_sub_element(const DevGeom& g, const BlockSm
             int next = kl.count, nh = 0;
             const int nr = fill_round<ELL>(g, ws, e, k, kl.count, box, 0, lane, &next, &nh);
             if constexpr (COUNT) n_sub_entries += nr;
-            if (!skip) walk_round<ELL>(g, ws, nh, nr, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, q.cosang, rc, s);
+            walk_round<ELL>(g, ws, nh, nr, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, q.cosang, !skip, rc, s);
             __syncwarp();
             k = next;
         }
@@ -729,125 +761,7 @@ __device__ __forceinline__ bool walk_sub_element(const DevGeom& g, const BlockSm
     return skip;
 }
 
-template <int MODE, bool COUNT, bool ELL = false>
-__device__ double pe_element(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, int d,
-                             long long v, float cr, float sr, int lane,
-                             unsigned long long* counters)
-{
-    Elem e;
-    if (!init_element(g, ws, d, v, cr, sr, lane, e)) return 0.0;
-    const bool from_super = bs.s_count >= 0;
-    const int n_src = from_super ? bs.s_count : g.n_holes + g.n_det;
-    int count = 0;
-    int cursor = build_chunk(g, bs, ws, e, d, 0, n_src, from_super, lane, &count);
-    const bool single = cursor >= n_src;
-
-    float chain = 0.0f;
-    double dacc = 0.0;
-    int n_hole_hits = 0, n_cry_hits = 0, n_blocked = 0, n_hole_evals = 0, n_cry_evals = 0;
-    long long n_sub_entries = 0;
-    // Round r covers sub-elements iz in {2p, 2p+1}, all 8 ix, iy in {2u, 2u+1} (p = r/8,
-    // u = r%8): a compact patch of the crystal, so a small slope box.  The 8 rounds of one p
-    // cover the reference indices s = 256p .. 256p+255, summed in index order after them.
-    for (int r = 0; r < 32; ++r) {
-        const int sidx = ((r >> 3) * 2 + (lane >> 4)) * 128 + ((lane >> 1) & 7) * 16 + (r & 7) * 2 +
-                         (lane & 1);
-        const SubElem q = sub_element(e, sidx);
-        Walk s{0.0f, 0.0f, 0, 0, 0, 0, 0};
-        RayCyl rc;
-        ray_cyl_init(rc, e.xI, e.yI, e.zI, q.xD, q.yD, q.zD);
-        const bool blocked = plate_penalty(g, ws, e, q, s.att);
-        const bool skip = blocked && g.nonneg_mu;
-        // slope box of the rays that still need the walk in this round
-        float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
-                                 skip ? INFINITY : q.sa_b, skip ? -INFINITY : q.sa_b);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, off));
-            box.y = fmaxf(box.y, __shfl_xor_sync(0xffffffffu, box.y, off));
-            box.z = fminf(box.z, __shfl_xor_sync(0xffffffffu, box.z, off));
-            box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, off));
-        }
-        // walk this round's objects: kept entries meeting the round box, copied with their
-        // geometry into the round buffer; an overfull round is walked in pieces (the walk
-        // state of each lane carries over, so the attenuation order is unchanged)
-        int cur = 0;
-        bool first_chunk = true;
-        while (true) {
-            if (!single && !first_chunk) {
-                cur = build_chunk(g, bs, ws, e, d, cur, n_src, from_super, lane, &count);
-            } else if (!single) {
-                if (r > 0) cur = build_chunk(g, bs, ws, e, d, 0, n_src, from_super, lane, &count);
-                else cur = cursor;
-            }
-            first_chunk = false;
-            int k = 0;
-            while (k < count) {
-                int next = count, nh = 0;
-                const int nr = fill_round<ELL>(g, ws, e, k, count, box, 0, lane, &next, &nh);
-                if constexpr (COUNT) n_sub_entries += nr;
-                if (!skip) walk_round<ELL>(g, ws, nh, nr, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, q.cosang, rc, s);
-                __syncwarp();
-                k = next;
-            }
-            if (single || cur >= n_src) break;
-        }
-        float contrib = 0.0f;
-        if (!skip) {
-            if (s.lay < g.n_layers) close_layers(g, s, g.n_layers, q.cosang);
-            contrib = finish_sub_element(e, q, s.att);
-        }
-        if constexpr (COUNT) {
-            n_hole_hits += s.hole_hits;
-            n_cry_hits += s.cry_hits;
-            n_hole_evals += s.hole_evals;
-            n_cry_evals += s.cry_evals;
-            n_blocked += skip;
-        }
-        if constexpr (MODE == 0) {
-            ws.chain[sidx & 255] = contrib;
-            if ((r & 7) == 7) {
-                __syncwarp();
-#pragma unroll 16
-                for (int k = 0; k < 256; ++k) chain = chain + ws.chain[k];
-                __syncwarp();
-            }
-        } else {
-            dacc += (double)contrib;
-        }
-    }
-    if constexpr (COUNT) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            n_hole_hits += __shfl_xor_sync(0xffffffffu, n_hole_hits, off);
-            n_cry_hits += __shfl_xor_sync(0xffffffffu, n_cry_hits, off);
-            n_blocked += __shfl_xor_sync(0xffffffffu, n_blocked, off);
-            n_hole_evals += __shfl_xor_sync(0xffffffffu, n_hole_evals, off);
-            n_cry_evals += __shfl_xor_sync(0xffffffffu, n_cry_evals, off);
-        }
-        if (lane == 0) {
-            atomicAdd(&counters[0], 1024ull);
-            atomicAdd(&counters[1], (unsigned long long)n_hole_hits);
-            atomicAdd(&counters[2], (unsigned long long)n_cry_hits);
-            atomicAdd(&counters[3], 1ull);
-            atomicAdd(&counters[4], (unsigned long long)n_blocked);
-            atomicAdd(&counters[5], single ? 0ull : 1ull);                 // chunked elements
-            atomicAdd(&counters[6], (unsigned long long)count);            // kept objects (last chunk)
-            atomicAdd(&counters[7], (unsigned long long)n_sub_entries);    // round sub-list entries
-            atomicAdd(&counters[8], bs.s_count < 0 ? 1ull : 0ull);         // superset overflow
-            atomicAdd(&counters[9], (unsigned long long)(bs.s_count < 0 ? 0 : bs.s_count));
-            atomicAdd(&counters[10], (unsigned long long)n_hole_evals);
-            atomicAdd(&counters[11], (unsigned long long)n_cry_evals);
-        }
-    }
-    if constexpr (MODE == 0) {
-        return chain;
-    } else {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
-        return dacc;
-    }
-}
+#include "pe_ref.cuh"
 
 // Element of the sampled form: the mean over the voxel's sx x sy x sz source points (centres of
 // a grid over the voxel) of the reference's element with crystal d divided into nx x ny x nz
@@ -869,7 +783,7 @@ __device__ double pe_element_sampled(const DevGeom& g, const BlockSmem& bs, Warp
         const int jx = p % sm.sx, jy = (p / sm.sx) % sm.sy, jz = p / (sm.sx * sm.sy);
         __syncwarp();                     // the previous point's lists are no longer read
         Elem e;
-        if (!init_element(g, ws, d, v, cr, sr, lane, e, ((float)jx + 0.5f) / (float)sm.sx,
+        if (!init_element(g, ws.inner, d, v, cr, sr, lane, e, ((float)jx + 0.5f) / (float)sm.sx,
                           ((float)jy + 0.5f) / (float)sm.sy, ((float)jz + 0.5f) / (float)sm.sz))
             return 0.0;                   // the crystal's mu does not depend on the point
         KeptList kl = start_kept_list(g, bs, ws, e, d, lane);
@@ -896,8 +810,7 @@ __device__ double pe_element_sampled(const DevGeom& g, const BlockSmem& bs, Warp
 // (cx, cy, cz): keep object o when |u_o - u_d| <= (rho + r_o)/(L_o - rho)
 // + (rho + r_d)/(L_d - rho) + 1e-4 at the centre (each direction moves by at most
 // rho/(L - rho) in chord length, each angular radius r/L grows to at most r/(L - rho)).
-__device__ void build_superset(const DevGeom& g, BlockSmem& bs, int d, float cx, float cy, float cz,
-                               float rho)
+__device__ void build_superset(const DevGeom& g, Superset& bs, int d, float cx, float cy, float cz, float rho)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float4 P = __ldg(&g.cry.pos[d]);
@@ -911,9 +824,8 @@ __device__ void build_superset(const DevGeom& g, BlockSmem& bs, int d, float cx,
     for (int base = 0; base < N; base += kThreads) {
         const int i = base + threadIdx.x;
         bool keep = false;
-        float4 od = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < N && !(i >= g.n_holes && i - g.n_holes == d)) {
-            od = object_data(g, i);
+            const float4 od = object_data(g, i);
             const float ro = (i < g.n_holes) ? od.w : 0.5f * od.w;
             const float Lo = sqrtf((od.x - cx) * (od.x - cx) + (od.y - cy) * (od.y - cy) +
                                    (od.z - cz) * (od.z - cz));
@@ -937,8 +849,7 @@ __device__ void build_superset(const DevGeom& g, BlockSmem& bs, int d, float cx,
         }
         const int pos = off + __popc(m & ((1u << lane) - 1u));
         if (keep && pos < kSuperCap) {
-            bs.sdata[pos] = od;
-            bs.sid[pos] = i;
+            bs.sid[pos] = (unsigned short)i;
         }
         running += tot;
         __syncthreads();
@@ -956,18 +867,30 @@ struct BrickOut {
     int det_count;
 };
 
+// Shared memory and blocks per SM of each kernel instance (pe_ref.cuh for the float modes 0, 1).
+template <int MODE, bool SAMPLED>
+struct Shape {
+    static constexpr bool ref = MODE <= 1 && !SAMPLED;
+    static constexpr int blocks = ref ? kRefBlocks : 2;
+    using Smem = typename std::conditional<ref, RefSmem, BlockSmem>::type;
+};
+__device__ __forceinline__ Superset& superset_of(RefSmem& sm) { return sm.sup; }
+__device__ __forceinline__ Superset& superset_of(BlockSmem& sm) { return sm; }
+
 // One work item: crystal det_begin + di against one voxel brick of bx x by x bz voxels (brick
 // (gx, gy, gz) of the block's grid starting at z-plane iz0).  The block builds the cone
 // superset of the brick, then its warps take the brick's voxels in turn.
 // SAMPLED: elements of the sampled form `smp` (source points anywhere in the voxels: the
 // superset radius grows by half a voxel diagonal).
 template <int MODE, bool COUNT, bool ELL = false, bool SAMPLED = false>
-__device__ __forceinline__ void pe_brick(const DevGeom& g, BlockSmem& bs, WarpSmem& ws, int lane, int wid,
+__device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, SAMPLED>::Smem& sm, int lane, int wid,
                                          const BrickOut& O, int di, int gx, int gy, int gz, int iz0, int iz1,
                                          int bx, int by, int bz, float cr, float sr,
                                          unsigned long long* counters, const Sampling* smp = nullptr,
                                          float rotation = 0.0f)
 {
+    constexpr bool REF = Shape<MODE, SAMPLED>::ref;
+    Superset& sup = superset_of(sm);
     const int x0 = gx * bx, y0 = gy * by, z0 = iz0 + gz * bz;
     const int x1 = min(x0 + bx, g.nx) - 1, y1 = min(y0 + by, g.ny) - 1, z1 = min(z0 + bz, iz1 + 1) - 1;
     const int d = O.det_begin + di;
@@ -979,36 +902,44 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, BlockSmem& bs, WarpSm
     float rho = 0.5f * sqrtf((bxx - ax) * (bxx - ax) + (byy - ay) * (byy - ay) +
                              (bzz - az) * (bzz - az)) + 1e-3f;
     if constexpr (SAMPLED) rho += 0.5f * sqrtf(g.wx * g.wx + g.wy * g.wy + g.wz * g.wz);
-    build_superset(g, bs, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho);
+    build_superset(g, sup, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho);
     const int n_slots = bx * by * bz;
     for (int slot = wid; slot < n_slots; slot += kWarps) {
         const int ox = slot % bx, oy = (slot / bx) % by, oz = slot / (bx * by);
         const int ix = x0 + ox, iy = y0 + oy, iz = z0 + oz;
-        if (ix >= g.nx || iy >= g.ny || iz > z1) continue;
         const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
-        if (v < O.vox_begin || v > O.vlast) continue;
-        float val;
-        if constexpr (MODE == 3) {
-            float* so = nullptr;
-            if (SAMPLED && O.sub_out)
-                so = O.sub_out + ((v - O.vox_begin) * O.det_count + di) * (long long)(smp->nx * smp->ny * smp->nz);
-            val = (float)pe_element_local<ELL, SAMPLED>(g, bs, ws, d, v, cr, sr, rotation, lane, smp, so);
-        } else if constexpr (SAMPLED) val = (float)pe_element_sampled<ELL>(g, bs, ws, d, v, cr, sr, lane, *smp);
-        else if constexpr (MODE == 2) val = (float)pe_element64(g, bs, ws, d, v, cr, sr, rotation, lane);
-        else val = (float)pe_element<MODE, COUNT, ELL>(g, bs, ws, d, v, cr, sr, lane, counters);
-        if (lane == 0) O.out[(long long)di * O.ld + (v - O.vox_begin)] = val;
-        __syncwarp();
+        if (ix < g.nx && iy < g.ny && iz <= z1 && v >= O.vox_begin && v <= O.vlast) {
+            float val;
+            if constexpr (REF) {
+                val = (float)pe_element_ref<MODE, COUNT, ELL>(g, sup, sm.w[wid], d, v, cr, sr, lane, counters);
+            } else {
+                WarpSmem& ws = sm.w[wid];
+                if constexpr (MODE == 3) {
+                    float* so = nullptr;
+                    if (SAMPLED && O.sub_out)
+                        so = O.sub_out + ((v - O.vox_begin) * O.det_count + di) * (long long)(smp->nx * smp->ny * smp->nz);
+                    val = (float)pe_element_local<ELL, SAMPLED>(g, sm, ws, d, v, cr, sr, rotation, lane, smp, so);
+                } else if constexpr (SAMPLED) {
+                    val = (float)pe_element_sampled<ELL>(g, sm, ws, d, v, cr, sr, lane, *smp);
+                } else {
+                    val = (float)pe_element64(g, sm, ws, d, v, cr, sr, rotation, lane);
+                }
+            }
+            if (lane == 0) O.out[(long long)di * O.ld + (v - O.vox_begin)] = val;
+            __syncwarp();
+        }
     }
     __syncthreads();
 }
 
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
-__global__ void __launch_bounds__(kThreads, 2) pe_kernel(DevGeom g, PeLaunch L)
+__global__ void __launch_bounds__(kThreads, Shape<MODE, SAMPLED>::blocks)
+pe_kernel(DevGeom g, PeLaunch L)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BlockSmem& bs = *reinterpret_cast<BlockSmem*>(smem_raw);
+    auto& sm = *reinterpret_cast<typename Shape<MODE, SAMPLED>::Smem*>(smem_raw);
+    Superset& bs = superset_of(sm);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpSmem& ws = bs.w[wid];
     const float ang = L.rotation * g.angle_step;           // :1006
     const float cr = cosf(ang), sr = sinf(ang);
     const long long nxy = (long long)g.nx * g.ny;
@@ -1031,15 +962,16 @@ __global__ void __launch_bounds__(kThreads, 2) pe_kernel(DevGeom g, PeLaunch L)
         const int gz = (int)(b / ((long long)nbx * nby));
         const int rem = (int)(b - (long long)gz * nbx * nby);
         const int gy = rem / nbx, gx = rem - gy * nbx;
-        pe_brick<MODE, COUNT, ELL, SAMPLED>(g, bs, ws, lane, wid, O, di, gx, gy, gz, iz0, iz1, bx, by, bz, cr, sr,
+        pe_brick<MODE, COUNT, ELL, SAMPLED>(g, sm, lane, wid, O, di, gx, gy, gz, iz0, iz1, bx, by, bz, cr, sr,
                                             L.counters, &L.smp, L.rotation);
     }
 }
 
 // Shared memory of the batched kernel: the block's working set plus the geometry of the
 // task in hand (copied in when the block moves to a task of another geometry).
+template <int MODE>
 struct BatchSmem {
-    BlockSmem bs;
+    typename Shape<MODE, false>::Smem bs;
     DevGeom g;
     int task;
 };
@@ -1048,13 +980,12 @@ struct BatchSmem {
 // tasks, taken from one work counter; a block finds its item's task by binary search over
 // the tasks' first item numbers.
 template <int MODE, bool ELL>
-__global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
+__global__ void __launch_bounds__(kThreads, Shape<MODE, false>::blocks) pe_batch_kernel(BatchLaunch B)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BatchSmem& sm = *reinterpret_cast<BatchSmem*>(smem_raw);
-    BlockSmem& bs = sm.bs;
+    BatchSmem<MODE>& sm = *reinterpret_cast<BatchSmem<MODE>*>(smem_raw);
+    Superset& bs = superset_of(sm.bs);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpSmem& ws = bs.w[wid];
     int cur_geom = -1;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1090,7 +1021,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
         const int rem = (int)(b - (long long)gz * T.nbx * T.nby);
         const int gy = rem / T.nbx, gx = rem - gy * T.nbx;
         const BrickOut O{T.out, T.ld, T.vox_begin, T.vox_begin + T.vox_count - 1, T.det_begin, nullptr, T.det_count};
-        pe_brick<MODE, false, ELL>(g, bs, ws, lane, wid, O, di, gx, gy, gz, T.iz0, T.iz1, B.bx, B.by, B.bz, cr,
+        pe_brick<MODE, false, ELL>(g, sm.bs, lane, wid, O, di, gx, gy, gz, T.iz0, T.iz1, B.bx, B.by, B.bz, cr,
                                    sr, nullptr, nullptr, T.rotation);
     }
 }
@@ -1102,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
 static int launch_mode(const DevGeom& g, const PeLaunch& L, int num_sms, cudaStream_t stream)
 {
-    const int smem = (int)sizeof(BlockSmem);
+    const int smem = (int)sizeof(typename Shape<MODE, SAMPLED>::Smem);
     static unsigned long long configured = 0;   // one bit per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -1124,7 +1055,7 @@ static int launch_mode(const DevGeom& g, const PeLaunch& L, int num_sms, cudaStr
 template <int KIND, bool ELL>
 static int launch_adjoint_kind(const DevGeom& g, const AdjLaunch& L, int num_sms, cudaStream_t stream)
 {
-    const int smem = (int)sizeof(AdjSmem);
+    const int smem = (int)sizeof(AdjSmem<KIND>);
     static unsigned long long configured = 0;   // one bit per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -1158,7 +1089,7 @@ int launch_pe_adjoint(const DevGeom& g, const AdjLaunch& L, int kind, int num_sm
 template <int MODE, bool ELL>
 static int configure_batch_mode(int* per_sm)
 {
-    const int smem = (int)sizeof(BatchSmem);
+    const int smem = (int)sizeof(BatchSmem<MODE>);
     static unsigned long long configured = 0;   // one bit per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -1188,22 +1119,19 @@ int configure_pe_batch(int mode, bool ell, int* blocks_per_sm)
     return mode == 0 ? configure_batch_mode<0, false>(blocks_per_sm) : configure_batch_mode<1, false>(blocks_per_sm);
 }
 
+template <int MODE, bool ELL>
+static void launch_batch_mode(const BatchLaunch& B, int grid, cudaStream_t stream)
+{
+    pe_batch_kernel<MODE, ELL><<<grid, kThreads, (int)sizeof(BatchSmem<MODE>), stream>>>(B);
+}
+
 int launch_pe_batch(const BatchLaunch& B, int mode, bool ell, int grid, cudaStream_t stream)
 {
     if (B.n_tasks < 1 || B.total_items < 1) return 0;
-    const int smem = (int)sizeof(BatchSmem);
-    if (mode == 2) {                              // FP64: shapes read at run time
-        pe_batch_kernel<2, false><<<grid, kThreads, smem, stream>>>(B);
-    } else if (mode == 3) {
-        if (ell) pe_batch_kernel<3, true><<<grid, kThreads, smem, stream>>>(B);
-        else pe_batch_kernel<3, false><<<grid, kThreads, smem, stream>>>(B);
-    } else if (ell) {
-        if (mode == 0) pe_batch_kernel<0, true><<<grid, kThreads, smem, stream>>>(B);
-        else pe_batch_kernel<1, true><<<grid, kThreads, smem, stream>>>(B);
-    } else {
-        if (mode == 0) pe_batch_kernel<0, false><<<grid, kThreads, smem, stream>>>(B);
-        else pe_batch_kernel<1, false><<<grid, kThreads, smem, stream>>>(B);
-    }
+    if (mode == 2) launch_batch_mode<2, false>(B, grid, stream);   // FP64: shapes read at run time
+    else if (mode == 3) ell ? launch_batch_mode<3, true>(B, grid, stream) : launch_batch_mode<3, false>(B, grid, stream);
+    else if (mode == 0) ell ? launch_batch_mode<0, true>(B, grid, stream) : launch_batch_mode<0, false>(B, grid, stream);
+    else ell ? launch_batch_mode<1, true>(B, grid, stream) : launch_batch_mode<1, false>(B, grid, stream);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -239,7 +239,7 @@ __device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSme
 #pragma unroll
     for (int i = 0; i <= kThetaN; ++i) acc[i] = 0.0;
     Elem e;
-    if (!init_element(g, ws, d, v, cr, sr, lane, e)) return;
+    if (!init_element(g, ws.inner, d, v, cr, sr, lane, e)) return;
     const bool from_super = bs.s_count >= 0;
     const int n_src = from_super ? bs.s_count : g.n_holes + g.n_det;
     int count = 0;
@@ -258,7 +258,7 @@ __device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSme
         for (int i = 0; i < kThetaN; ++i) s.da[i] = 0.0f;
         RayCyl rc;
         ray_cyl_init(rc, e.xI, e.yI, e.zI, q.xD, q.yD, q.zD);
-        const bool blocked = plate_penalty(g, ws, e, q, s.att);
+        const bool blocked = plate_penalty(g, ws.inner, e, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, s.att);
         const bool skip = blocked && g.nonneg_mu;
         float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
                                  skip ? INFINITY : q.sa_b, skip ? -INFINITY : q.sa_b);
@@ -303,9 +303,14 @@ __device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSme
         for (int off = 16; off > 0; off >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
 }
 
+// Projections run the reference-order element (pe_ref.cuh), the gradient its own.
+template <int KIND>
+using AdjShape = Shape<KIND == 1 ? 2 : 1, false>;
+
+template <int KIND>
 struct AdjSmem {
-    BlockSmem bs;
-    double acc[kWarps][kThetaN + 1];
+    typename AdjShape<KIND>::Smem bs;
+    double acc[KIND == 1 ? kWarps : 1][kThetaN + 1];
     int any;
 };
 
@@ -314,13 +319,12 @@ struct AdjSmem {
 // KIND 2: q[v] += sum_d A[d,v] u[d - det_begin] (back projection; x is not read).
 // Elements of zero weight are skipped, and so are bricks whose voxels all have x = 0.
 template <int KIND, bool ELL>
-__global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjLaunch L)
+__global__ void __launch_bounds__(kThreads, AdjShape<KIND>::blocks) pe_adjoint_kernel(DevGeom g, AdjLaunch L)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    AdjSmem& sm = *reinterpret_cast<AdjSmem*>(smem_raw);
-    BlockSmem& bs = sm.bs;
+    AdjSmem<KIND>& sm = *reinterpret_cast<AdjSmem<KIND>*>(smem_raw);
+    Superset& bs = superset_of(sm.bs);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpSmem& ws = bs.w[wid];
     if (KIND == 1 && lane <= kThetaN) sm.acc[wid][lane] = 0.0;
     const float ang = L.rotation * g.angle_step;           // :1006
     const float cr = cosf(ang), sr = sinf(ang);
@@ -368,14 +372,14 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
                 const float xv = KIND == 2 ? 1.0f : L.x[v];
                 if (xv == 0.0f || ud == 0.0f) continue;
                 if constexpr (KIND == 0) {
-                    const double val = pe_element<1, false, ELL>(g, bs, ws, d, v, cr, sr, lane, nullptr);
+                    const double val = pe_element_ref<1, false, ELL>(g, bs, sm.bs.w[wid], d, v, cr, sr, lane, nullptr);
                     if (lane == 0) atomicAdd(&L.p[di], val * (double)xv);
                 } else if constexpr (KIND == 2) {
-                    const double val = pe_element<1, false, ELL>(g, bs, ws, d, v, cr, sr, lane, nullptr);
+                    const double val = pe_element_ref<1, false, ELL>(g, bs, sm.bs.w[wid], d, v, cr, sr, lane, nullptr);
                     if (lane == 0) atomicAdd(&L.q[v], val * (double)ud);
                 } else {
                     double acc[kThetaN + 1];
-                    pe_element_grad<ELL>(g, bs, ws, d, v, cr, sr, lane, acc);
+                    pe_element_grad<ELL>(g, sm.bs, sm.bs.w[wid], d, v, cr, sr, lane, acc);
                     const double wgt = (double)ud * (double)xv;
                     if (lane == 0)
 #pragma unroll

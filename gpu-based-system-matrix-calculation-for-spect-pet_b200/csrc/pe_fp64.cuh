@@ -251,7 +251,7 @@ __device__ double pe_element64(const DevGeom& g, const BlockSmem& bs, WarpSmem& 
                                float sr, float rotation, int lane)
 {
     Elem e;
-    if (!init_element(g, ws, d, v, cr, sr, lane, e)) return 0.0;   // mu_t <= 0.01 (:1107, :1194)
+    if (!init_element(g, ws.inner, d, v, cr, sr, lane, e)) return 0.0;   // mu_t <= 0.01 (:1107, :1194)
     // warp-uniform constants in the warp's shared slot (registers would spill)
     static_assert(sizeof(Elem64) <= sizeof(ws.e64), "Elem64 exceeds its shared-memory slot");
     Elem64& E = *reinterpret_cast<Elem64*>(ws.e64);

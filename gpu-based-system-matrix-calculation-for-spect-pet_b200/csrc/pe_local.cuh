@@ -494,7 +494,7 @@ __device__ double pe_element_local(const DevGeom& g, const BlockSmem& bs, WarpSm
         const double fzd = ((double)jz + 0.5) / (double)szn;
         __syncwarp();                                    // the previous point's ElemL and plate rectangles are done
         Elem e;
-        if (!init_element(g, ws, d, v, cr, sr, lane, e, (float)fxd, (float)fyd, (float)fzd)) {   // mu_t <= 0.01
+        if (!init_element(g, ws.inner, d, v, cr, sr, lane, e, (float)fxd, (float)fyd, (float)fzd)) {   // mu_t <= 0.01
             if (sub_out) {                                                                     // (:1107, :1194)
                 for (int i = lane; i < n_sub; i += 32) sub_out[i] = 0.0f;
             }

@@ -1,0 +1,62 @@
+"""The phased element kernel (csrc/pe_ref.cuh) where its branches change: holes that share layer,
+caps and radius or not, crystals only, kept lists that fill one record array or several.  Against the
+oracle's FP32 twin, with the tolerance of the seeded systems in test_gpu_pe.py (the twin rounds as
+gcc contracts, the kernel as the reference's own build does)."""
+import numpy as np
+import pytest
+
+from conftest import geometry, oracle, rel_err, sysmat
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(layers, crystals, rotated=False, size=(1.7, 5.0, 1.3)):
+    cb = geometry._CollimatorBuilder()
+    for m, holes in enumerate(layers):
+        cb.add_layer(24.0, 4.0, 24.0, 4.5 * m, 1.1, 0.9, 0.2, holes)
+    rng = np.random.default_rng(2)
+    rots = rng.uniform(0, 6.28, len(crystals)) if rotated else None
+    det = geometry._detector(crystals, size, rotations=rots)
+    img = geometry._image((7, 5, 3), (1.9, 2.1, 2.3), 40.0, shift=(0.13, -0.21, 0.17))
+    return geometry.Geometry("phases", cb.build(), det, img, geometry._physics())
+
+
+def _grid(n, pitch, y):
+    return geometry._crystal_grid(n, n, pitch, y)
+
+
+def _holes(n, pitch, radius, spread=0.0):
+    rng = np.random.default_rng(1)
+    return [(x, z, radius + spread * rng.random()) for x, z, _ in geometry._square_holes(n, pitch, radius)]
+
+
+SYSTEMS = {
+    # name: (system, whether an element's kept list needs several chunks)
+    "even": (lambda: _system([_holes(7, 2.0, 0.6)], _grid(4, 1.8, 9.0)), False),
+    "uneven radii": (lambda: _system([_holes(7, 2.0, 0.4, 0.4)], _grid(4, 1.8, 9.0), True), False),
+    "two layers": (lambda: _system([_holes(7, 2.0, 0.6), _holes(9, 1.6, 0.5)], _grid(4, 1.8, 14.0)), False),
+    "no holes": (lambda: _system([[]], _grid(4, 1.8, 9.0)), False),
+    "no collimator": (lambda: _system([], _grid(5, 1.8, 9.0), True), False),
+    "dense holes": (lambda: _system([_holes(31, 0.4, 0.15)], _grid(2, 8.5, 9.0), size=(8.0, 5.0, 8.0)), True),
+    "dense layers": (lambda: _system([_holes(21, 0.5, 0.15, 0.05)] * 3, _grid(3, 4.5, 18.5), size=(4.0, 5.0, 4.0)), True),
+}
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+@pytest.mark.parametrize("mode", ["reference", "precise"])
+def test_phases_match_oracle(gpu, name, mode):
+    make, chunked = SYSTEMS[name]
+    geo = make()
+    ctx = sysmat.Context(geo)
+    out = gpu.empty((ctx.n_det, ctx.n_vox), dtype=gpu.float32, device="cuda")
+    counts = ctx.pe_work(out)
+    assert (counts["chunked"] > 0) == chunked, counts
+    if mode == "precise":
+        ctx.pe(out, mode=sysmat.MODE_PRECISE)
+    gpu.cuda.synchronize()
+    a = out.cpu().numpy()
+    r = rel_err(a, oracle.pe(geo, prec=32))
+    assert a.max() > 0
+    assert np.median(r) < 1e-6
+    assert np.mean(r > 3e-5) <= 0.005
+    assert r.max() < 1e-3
