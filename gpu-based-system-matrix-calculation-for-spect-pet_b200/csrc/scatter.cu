@@ -28,6 +28,7 @@
 
 #include <cub/cub.cuh>
 
+#include "rounding.cuh"
 #include "scatter.cuh"
 
 namespace sysmat {
@@ -97,59 +98,47 @@ __device__ __forceinline__ DetPoint det_point(float4 P, float4 S, float4 T)
     return q;
 }
 
-// ---- relationship bitmaps, one thread per 32-bit word (no atomics) ----
+// ---- relationship bitmaps (no atomics) ----
+//
+// A bit asks whether crystal k lies in the angular cone of a segment i-j, seen from one end: that
+// |u_k - u_j| <= c_k + c_j for the unit directions u and angular radii c of k and j seen from i.
+// Directions and radii belong to (i, k) alone, so a block takes one i, forms them for every
+// crystal once in shared memory (Seen), and each bit costs two shared loads, a distance and a
+// compare; a warp's ballot is the output word.  Per bit the former kernels recomputed both
+// directions with six divisions and four roots: the two bitmaps of configuration 3 (1.6e9 bits)
+// took 36.6 ms, and take 6.0 ms (bound by issue; the 201 MB written take 0.03 ms).
 
-__global__ void bitmap_crystal_kernel(const float* __restrict__ det, int n, long long words,
-                                      uint32_t* __restrict__ out)
+constexpr int kBitmapThreads = 256;
+
+// A crystal seen from a point: unit direction and angular radius (scatter.cu:1476-1500, :1975-1996).
+__device__ __forceinline__ float4 seen_from(float xi, float yi, float zi, const float* __restrict__ pk, float rk)
 {
-    const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= words) return;
-    const long long total_pairs = (long long)n * (n + 1) / 2;
-    long long bit = w * 32;
-    long long pair = bit / n;
-    int a = (int)(bit - pair * n);
-    // row i of pair index p = i*n - i(i+1)/2 + j (i <= j)
-    double disc = (2.0 * n + 1.0) * (2.0 * n + 1.0) - 8.0 * (double)pair;
-    long long i = (long long)floor(((2.0 * n + 1.0) - sqrt(disc > 0 ? disc : 0)) / 2.0);
-    if (i < 0) i = 0;
-    while (i > 0 && i * n - i * (i - 1) / 2 > pair) --i;
-    while ((i + 1) * n - (i + 1) * i / 2 <= pair) ++i;
-    long long j = pair - (i * n - i * (i + 1) / 2);
-    uint32_t word = 0;
-    for (int b = 0; b < 32; ++b) {
-        if (pair >= total_pairs) break;
-        const int ii = (int)i, jj = (int)j, k = a;
-        if (ii < jj && k != ii && k != jj) {
-            // scatter.cu:1465-1534
-            const float* pi = det + 12 * ii;
-            const float* pj = det + 12 * jj;
-            const float* pk = det + 12 * k;
-            const float ri = sqrtf(pi[4] * pi[4] + pi[6] * pi[6] + pi[5] * pi[5]) / 2.0f;
-            const float rj = sqrtf(pj[4] * pj[4] + pj[6] * pj[6] + pj[5] * pj[5]) / 2.0f;
-            const float lij = dist3(pi[1], pi[2], pi[3], pj[1], pj[2], pj[3]);
-            const float cij = ri / lij, cji = rj / lij;
-            const float rk = sqrtf(pk[4] * pk[4] + pk[6] * pk[6] + pk[5] * pk[5]) / 2.0f;
-            const float lik = dist3(pk[1], pk[2], pk[3], pi[1], pi[2], pi[3]);
-            const float cki = rk / lik;
-            const float ljk = dist3(pk[1], pk[2], pk[3], pj[1], pj[2], pj[3]);
-            const float ckj = rk / ljk;
-            const float d_i = dist3((pk[1] - pi[1]) / lik, (pk[2] - pi[2]) / lik, (pk[3] - pi[3]) / lik,
-                                    (pj[1] - pi[1]) / lij, (pj[2] - pi[2]) / lij, (pj[3] - pi[3]) / lij);
-            bool hit = d_i <= cki + cji;
-            if (!hit) {
-                const float d_j = dist3((pk[1] - pj[1]) / ljk, (pk[2] - pj[2]) / ljk, (pk[3] - pj[3]) / ljk,
-                                        (pi[1] - pj[1]) / lij, (pi[2] - pj[2]) / lij, (pi[3] - pj[3]) / lij);
-                hit = d_j <= ckj + cij;
-            }
-            if (hit) word |= 1u << b;
-        }
-        if (++a == n) {
-            a = 0;
-            ++pair;
-            if (++j == n) { ++i; j = i; }
-        }
-    }
-    out[w] = word;
+    const float l = dist3(pk[1], pk[2], pk[3], xi, yi, zi);
+    return make_float4((pk[1] - xi) / l, (pk[2] - yi) / l, (pk[3] - zi) / l, rk / l);
+}
+
+__device__ __forceinline__ float crystal_radius(const float* __restrict__ p)
+{
+    return sqrtf(p[4] * p[4] + p[6] * p[6] + p[5] * p[5]) / 2.0f;
+}
+
+// |u_k - u_j| <= c_k + c_j.  The root is the IEEE one (its argument is 0, where the root is too,
+// or well above sqrt_mid's lower bound: differences of unit vectors are multiples of 2^-26 or so).
+__device__ __forceinline__ bool cone_meets(const float4& k, const float4& j)
+{
+    const float dx = k.x - j.x, dy = k.y - j.y, dz = k.z - j.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const float d = d2 == 0.0f ? 0.0f : sqrt_mid(d2);
+    return d <= k.w + j.w;
+}
+
+// Whether crystal k may attenuate the path between crystals i and j, i < j (:1465-1534).
+__device__ __forceinline__ bool crystal_related(const float* __restrict__ det, int i, int j, int k)
+{
+    const float *pi = det + 12 * i, *pj = det + 12 * j, *pk = det + 12 * k;
+    const float ri = crystal_radius(pi), rj = crystal_radius(pj), rk = crystal_radius(pk);
+    return cone_meets(seen_from(pi[1], pi[2], pi[3], pk, rk), seen_from(pi[1], pi[2], pi[3], pj, rj)) ||
+           cone_meets(seen_from(pj[1], pj[2], pj[3], pk, rk), seen_from(pj[1], pj[2], pj[3], pi, ri));
 }
 
 // Whether crystal k may attenuate the path from hole i (raw parameters hr) to crystal j:
@@ -158,35 +147,119 @@ __global__ void bitmap_crystal_kernel(const float* __restrict__ det, int n, long
 __device__ __forceinline__ bool collimator_related(const float* __restrict__ det, float4 hr, int j, int k)
 {
     const float xi = hr.x, yi = (hr.y + hr.z) / 2.0f, zi = hr.w;
-    const float* pj = det + 12 * j;
-    const float* pk = det + 12 * k;
-    const float rj = sqrtf(pj[4] * pj[4] + pj[6] * pj[6] + pj[5] * pj[5]) / 2.0f;
-    const float lij = dist3(xi, yi, zi, pj[1], pj[2], pj[3]);
-    const float cji = rj / lij;
-    const float rk = sqrtf(pk[4] * pk[4] + pk[6] * pk[6] + pk[5] * pk[5]) / 2.0f;
-    const float lik = dist3(pk[1], pk[2], pk[3], xi, yi, zi);
-    const float cki = rk / lik;
-    const float dd = dist3((pk[1] - xi) / lik, (pk[2] - yi) / lik, (pk[3] - zi) / lik,
-                           (pj[1] - xi) / lij, (pj[2] - yi) / lij, (pj[3] - zi) / lij);
-    return dd <= cki + cji;
+    const float *pj = det + 12 * j, *pk = det + 12 * k;
+    return cone_meets(seen_from(xi, yi, zi, pk, crystal_radius(pk)), seen_from(xi, yi, zi, pj, crystal_radius(pj)));
 }
 
-__global__ void bitmap_collimator_kernel(const float* __restrict__ det, const float4* __restrict__ hraw,
-                                         int n, int nh, long long words, uint32_t* __restrict__ out)
+// First pair of row i (pairs (i, j), i <= j < n).
+__host__ __device__ __forceinline__ long long pair_row(long long n, long long i) { return i * n - i * (i - 1) / 2; }
+
+// The bit of the crystal bitmap at flat index `bit` (pair index (i n - i (i+1) / 2 + j), then k).
+__device__ bool crystal_bit(const float* __restrict__ det, int n, long long bit)
 {
-    const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= words) return;
-    const long long total = (long long)nh * n * n;
-    long long bit = w * 32;
-    uint32_t word = 0;
-    for (int b = 0; b < 32 && bit < total; ++b, ++bit) {
-        const int k = (int)(bit % n);
-        const long long ij = bit / n;
-        const int j = (int)(ij % n);
-        const int i = (int)(ij / n);
-        if (collimator_related(det, __ldg(&hraw[i]), j, k)) word |= 1u << b;
+    const long long pair = bit / n;
+    const int k = (int)(bit - pair * n);
+    const double disc = (2.0 * n + 1.0) * (2.0 * n + 1.0) - 8.0 * (double)pair;
+    long long i = (long long)floor(((2.0 * n + 1.0) - sqrt(disc > 0 ? disc : 0)) / 2.0);
+    if (i < 0) i = 0;
+    while (i > 0 && pair_row(n, i) > pair) --i;
+    while (pair_row(n, i + 1) <= pair) ++i;
+    const int ii = (int)i, jj = (int)(pair - pair_row(n, i) + i);
+    return ii < jj && k != ii && k != jj && crystal_related(det, ii, jj, k);
+}
+
+// Block (i, part of row i): the words whose first bit belongs to pairs (i, i .. n-1).
+__global__ void __launch_bounds__(kBitmapThreads) bitmap_crystal_kernel(const float* __restrict__ det, int n,
+                                                                        long long bits, uint32_t* __restrict__ out)
+{
+    extern __shared__ float4 seen[];                       // every crystal seen from crystal i, then radii
+    float* radius = reinterpret_cast<float*>(seen + n);
+    const int i = blockIdx.x, lane = threadIdx.x & 31;
+    const float* pi = det + 12 * i;
+    const float xi = pi[1], yi = pi[2], zi = pi[3];
+    for (int k = threadIdx.x; k < n; k += kBitmapThreads) {
+        const float rk = crystal_radius(det + 12 * k);
+        radius[k] = rk;
+        seen[k] = seen_from(xi, yi, zi, det + 12 * k, rk);
     }
-    out[w] = word;
+    __syncthreads();
+    const float ri = radius[i];
+    const long long b0 = pair_row(n, i) * n, b1 = pair_row(n, i + 1) * n;
+    const int step = 32 * (kBitmapThreads / 32) * gridDim.y;
+    const int step_j = step / n, step_k = step - step_j * n;
+    long long w = (b0 + 31) / 32 + blockIdx.y * (kBitmapThreads / 32) + (threadIdx.x >> 5);
+    const int off = (int)(w * 32 + lane - b0);             // a row holds at most n^2 < 2^31 bits
+    int j = off / n, k = off - j * n;
+    for (; w * 32 < b1; w += step / 32) {
+        const long long bit = w * 32 + lane;
+        bool hit = false;
+        if (bit < b1) {
+            const int jj = i + j;
+            if (j > 0 && k != i && k != jj) {
+                hit = cone_meets(seen[k], seen[jj]);
+                if (!hit) {                                 // seen from the other end
+                    const float* pj = det + 12 * jj;
+                    const float xj = __ldg(&pj[1]), yj = __ldg(&pj[2]), zj = __ldg(&pj[3]);
+                    const float* pk = det + 12 * k;
+                    const float dx = __ldg(&pk[1]) - xj, dy = __ldg(&pk[2]) - yj, dz = __ldg(&pk[3]) - zj;
+                    const float l2 = dx * dx + dy * dy + dz * dz;
+                    const float l = sqrtf(l2), rl = rcp_rn(l);
+                    const float4 u = make_float4(div_by(dx, l, rl), div_by(dy, l, rl), div_by(dz, l, rl),
+                                                 div_by(radius[k], l, rl));
+                    hit = cone_meets(u, seen_from(xj, yj, zj, pi, ri));
+                }
+            }
+        } else if (bit < bits) {                            // the word's tail in the next rows
+            hit = crystal_bit(det, n, bit);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) out[w] = m;
+        k += step_k;
+        j += step_j;
+        if (k >= n) {
+            k -= n;
+            ++j;
+        }
+    }
+}
+
+// Block (hole i, part of its bits): the words whose first bit belongs to hole i (bit
+// (i n + j) n + k).
+__global__ void __launch_bounds__(kBitmapThreads) bitmap_collimator_kernel(const float* __restrict__ det,
+                                                                           const float4* __restrict__ hraw, int n,
+                                                                           long long bits, uint32_t* __restrict__ out)
+{
+    extern __shared__ float4 seen[];                       // every crystal seen from the hole
+    const int i = blockIdx.x, lane = threadIdx.x & 31;
+    const float4 hr = __ldg(&hraw[i]);
+    const float xi = hr.x, yi = (hr.y + hr.z) / 2.0f, zi = hr.w;
+    for (int k = threadIdx.x; k < n; k += kBitmapThreads)
+        seen[k] = seen_from(xi, yi, zi, det + 12 * k, crystal_radius(det + 12 * k));
+    __syncthreads();
+    const long long nn = (long long)n * n, b0 = i * nn, b1 = b0 + nn;
+    const int step = 32 * (kBitmapThreads / 32) * gridDim.y;
+    const int step_j = step / n, step_k = step - step_j * n;
+    long long w = (b0 + 31) / 32 + blockIdx.y * (kBitmapThreads / 32) + (threadIdx.x >> 5);
+    const int off = (int)(w * 32 + lane - b0);
+    int j = off / n, k = off - j * n;
+    for (; w * 32 < b1; w += step / 32) {
+        const long long bit = w * 32 + lane;
+        bool hit = false;
+        if (bit < b1) {
+            hit = cone_meets(seen[k], seen[j]);
+        } else if (bit < bits) {                            // the word's tail in the next holes
+            const long long ij = bit / n;
+            hit = collimator_related(det, __ldg(&hraw[ij / n]), (int)(ij % n), (int)(bit - ij * n));
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) out[w] = m;
+        k += step_k;
+        j += step_j;
+        if (k >= n) {
+            k -= n;
+            ++j;
+        }
+    }
 }
 
 // ---- pair tables ----
@@ -718,22 +791,40 @@ long long bitmap_collimator_words(int n, int nh0)
     return ((long long)n * n * nh0 + 31) / 32;
 }
 
+// Blocks per row or hole: enough for several waves over the SMs, no more than there are words.
+static unsigned bitmap_parts(long long rows, long long words)
+{
+    const long long want = (8 * 148 + rows - 1) / rows, most = words / rows / (kBitmapThreads / 32) + 1;
+    return (unsigned)std::max(1LL, std::min(want, most));
+}
+
+template <class K>
+static int bitmap_smem(K kernel, size_t bytes)
+{
+    if (bytes <= 48 * 1024) return 0;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess ? 0 : -1;
+}
+
 int launch_bitmap_crystal(const DevGeom& g, uint32_t* words, cudaStream_t s)
 {
-    const long long nw = bitmap_crystal_words(g.n_det);
+    const long long nw = bitmap_crystal_words(g.n_det), n = g.n_det;
     if (nw == 0) return 0;
-    const long long blocks = (nw + 255) / 256;
-    bitmap_crystal_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.raw_det, g.n_det, nw, words);
+    const size_t smem = (sizeof(float4) + sizeof(float)) * (size_t)n;   // at most 6666 crystals: 133 KB
+    if (bitmap_smem(bitmap_crystal_kernel, smem)) return -1;
+    const dim3 grid((unsigned)n, bitmap_parts(n, nw));
+    bitmap_crystal_kernel<<<grid, kBitmapThreads, smem, s>>>(g.raw_det, g.n_det, n * (n + 1) / 2 * n, words);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_bitmap_collimator(const DevGeom& g, uint32_t* words, cudaStream_t s)
 {
-    const long long nw = bitmap_collimator_words(g.n_det, g.n_holes0);
+    const long long nw = bitmap_collimator_words(g.n_det, g.n_holes0), n = g.n_det;
     if (nw == 0) return 0;
-    const long long blocks = (nw + 255) / 256;
-    bitmap_collimator_kernel<<<(unsigned)blocks, 256, 0, s>>>(g.raw_det, g.hole.raw, g.n_det,
-                                                              g.n_holes0, nw, words);
+    const size_t smem = sizeof(float4) * (size_t)n;
+    if (bitmap_smem(bitmap_collimator_kernel, smem)) return -1;
+    const dim3 grid((unsigned)g.n_holes0, bitmap_parts(g.n_holes0, nw));
+    bitmap_collimator_kernel<<<grid, kBitmapThreads, smem, s>>>(g.raw_det, g.hole.raw, g.n_det, n * n * g.n_holes0,
+                                                                words);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
