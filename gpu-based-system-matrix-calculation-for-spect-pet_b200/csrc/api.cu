@@ -539,7 +539,7 @@ int scatter_setup(sysmat_ctx* ctx, int parts, int hole_model, float rotation, co
     L.att_offsets = ctx->att_offsets;
     L.out = d_out;
     if (!ctx->d_kn_tab || ctx->kn_e0 != ph.e0) {     // (re)build the FP64 Klein-Nishina table
-        std::vector<double> tab(3 * (size_t)(kKnTable + 1));
+        std::vector<double> tab(kKnDoubles);
         kn_table_build((double)ph.e0, tab.data());
         if (!ctx->d_kn_tab &&
             cudaMalloc(&ctx->d_kn_tab, sizeof(double) * tab.size()) != cudaSuccess) {

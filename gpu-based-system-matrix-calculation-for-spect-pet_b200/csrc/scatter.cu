@@ -14,12 +14,17 @@
 //    detector sub-division (the crystal box and the sub-element box are the same floats), so
 //    it is not evaluated;
 //  * the Klein-Nishina angular ratio is the reference's left Riemann sum with
-//    n = (int)((theta_max - theta_min) / 0.01f) + 1 terms (:980-993, :1338).  It is
-//    evaluated through the Euler-Maclaurin identity
+//    n = (int)((theta_max - theta_min) / 0.01f) + 1 terms (:980-993, :1338), evaluated through the
+//    Euler-Maclaurin identity
 //      sum_{i=0..n} F(a + i h) h = int_a^b F + h/2 (F(a) + F(b)) + h^2/12 (F'(b) - F'(a)) + O(h^4)
-//    with an 8-point Gauss-Legendre integral, instead of n+1 cos/sin evaluations; theta_min,
+//    from two FP64 tables of cubics (scatter.cuh), instead of n+1 cos/sin evaluations; theta_min,
 //    theta_max and n are computed with the reference's float formulas, so the step count
 //    matches.  The normalisation over [0, pi] is a host FP64 sum;
+//  * per item, the corner cosines of the theta range are formed only for the corners that can be
+//    extreme, the theta_min chord only for rays that pass near the crystal, and divisions share
+//    correctly rounded reciprocals.  Configuration 3, 768 voxels: 39.5 -> 27.6 ms (all eight
+//    corners, every chord and three table interpolations per end before; bound by issue, 62 % of
+//    the slots, 465 warp instructions per item);
 //  * one thread per matrix element (d, v); a block shares d, so pair records are staged in
 //    shared memory and attenuator lists are broadcast loads; each element sums its items in
 //    FP64 (the reference adds float items with atomicAdd in an unspecified order).
@@ -36,47 +41,28 @@ namespace sysmat {
 namespace {
 
 constexpr int kItemThreads = kScatterBlockVoxels;
-constexpr int kPairChunk = 512;
+constexpr int kPairChunk = 256;
 
 // ---- reference helper formulas (scatter.cu:961-1038) ----
 
-// Clamped cosine of the scattering angle at a between the directions s -> a and a -> d.
-__device__ __forceinline__ float cone_cosine(float xs, float ys, float zs, float xa, float ya, float za,
-                                             float xd, float yd, float zd)
+// Scattering angle at the point a between the directions s -> a and a -> d; mb = |a -> d|, the
+// pair's distance (the same float).
+__device__ __forceinline__ float cone_angle(float xs, float ys, float zs, float xa, float ya, float za,
+                                            float xd, float yd, float zd, float mb)
 {
     const float a0 = xa - xs, a1 = ya - ys, a2 = za - zs;
     const float b0 = xd - xa, b1 = yd - ya, b2 = zd - za;
     const float dot = b0 * a0 + b1 * a1 + b2 * a2;
-    const float ma = sqrtf(a0 * a0 + a1 * a1 + a2 * a2);
-    const float mb = sqrtf(b0 * b0 + b1 * b1 + b2 * b2);
-    float c = dot / (ma * mb);
+    const float ma = sqrt_mid(a0 * a0 + a1 * a1 + a2 * a2);
+    float c = div_rn(dot, ma * mb);
     if (c > 1.0f) c = 1.0f;
     if (c < -1.0f) c = -1.0f;
-    return c;
-}
-
-__device__ __forceinline__ float cone_angle(float xs, float ys, float zs, float xa, float ya, float za,
-                                            float xd, float yd, float zd)
-{
-    return acosf(cone_cosine(xs, ys, zs, xa, ya, za, xd, yd, zd));
+    return acosf(c);
 }
 
 __device__ __forceinline__ float dist3(float x1, float y1, float z1, float x2, float y2, float z2)
 {
     return sqrtf((x1 - x2) * (x1 - x2) + (y1 - y2) * (y1 - y2) + (z1 - z2) * (z1 - z2));
-}
-
-// Reference Riemann sum with n + 1 terms from a, step 0.01f, in FP64 from the table:
-//   sum = G(b) - G(a) + h/2 (F(a) + F(b)) + h^2/12 (F'(b) - F'(a)),  b = a + n h
-// (G, F and F' from kn_tab_eval, scatter.cuh).
-__device__ __forceinline__ double kn_sum_tab(float a, int n, const double* __restrict__ tab)
-{
-    const double h = (double)0.01f;
-    const double ad = (double)a, bd = ad + (double)n * h;
-    double Ga, Fa, Pa, Gb, Fb, Pb;
-    kn_tab_eval(tab, ad, Ga, Fa, Pa);
-    kn_tab_eval(tab, bd, Gb, Fb, Pb);
-    return (Gb - Ga) + 0.5 * h * (Fa + Fb) + (h * h / 12.0) * (Pb - Pa);
 }
 
 // Crystal d's single sub-element centre (1x1x1 division, :1242-1252) in its own frame and
@@ -548,76 +534,155 @@ struct ElemConst {
     float mu_pe, mu_c, eres;
     float lo, hi;
     float rdet;
-    float ux1, ux2, uy1, uy2, uz1, uz2;
 };
 
-// One (d, v, s) item; w_s is the interaction weight (PE * muC/muPE or hole solid angle *
-// muC/mu of layer 0).  Returns the float the reference would atomically add.
-template <bool NATIVE>
-__device__ float scatter_item(const ElemConst& e, const PairRec& pr, const PairNative& pn,
-                              const AttEntry* __restrict__ att,
-                              float xs, float ys, float zs, float w_s, float e0, float integ,
-                              const double* __restrict__ kn_tab)
+// A staged pair: its record and what else belongs to the pair alone, formed once per block: the
+// angular half width of d seen from the scatter point, and 1 / |corner - scatter point| for d's
+// eight corners (approximate: they only select corners).
+struct StagedPair {
+    PairRec r;
+    float half_width;
+    float rcorner[8];
+    float slack;                // bound of the selection's error per unit of the summed terms
+};
+
+// Corner c of d (bit 0: x, bit 1: y, bit 2: z) minus the scatter point, in d's frame
+// (the faces of the single detector unit, (0 / 1 - 0.5) w and (1 / 1 - 0.5) w, :1305-1320).
+__device__ __forceinline__ void corner_offset(const ElemConst& e, const PairRec& pr, int c, float& bx, float& by, float& bz)
 {
-    const float cone = cone_angle(e.xI, e.yI, e.zI, xs, ys, zs, e.q.xD, e.q.yD, e.q.zD);
+    bx = ((c & 1) ? 0.5f * e.w : -0.5f * e.w) - pr.xss;
+    by = ((c & 2) ? 0.5f * e.t : -0.5f * e.t) - pr.yss;
+    bz = ((c & 4) ? 0.5f * e.h : -0.5f * e.h) - pr.zss;
+}
+
+__device__ __forceinline__ StagedPair stage_pair(const ElemConst& e, const PairRec& pr)
+{
+    StagedPair p;
+    p.r = pr;
+    p.half_width = e.rdet / 2.0f / pr.lsd;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        float bx, by, bz;
+        corner_offset(e, pr, c, bx, by, bz);
+        p.rcorner[c] = rsqrtf(bx * bx + by * by + bz * bz);
+    }
+    float far = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) far = fmaxf(far, p.rcorner[c]);
+    p.slack = 2e-6f * far;
+    return p;
+}
+
+// One (d, v, s) item; (xs, ys, zs) the scatter point, w_s the interaction weight (PE * muC/muPE
+// or hole solid angle * muC/mu of layer 0).  Returns the float the reference would atomically add.
+template <bool NATIVE>
+__device__ float scatter_item(const ElemConst& e, const StagedPair& sp, const PairNative& pn,
+                              const AttEntry* __restrict__ att, float xs, float ys, float zs, float w_s, float e0,
+                              float re0, float integ, const double* __restrict__ kn_tab)
+{
+    const PairRec& pr = sp.r;
+    const float cone = cone_angle(e.xI, e.yI, e.zI, xs, ys, zs, e.q.xD, e.q.yD, e.q.zD, pr.lsd);
     const float es = e0 / (1.0f + (e0 / 511.0f) * (1.0f - cosf(cone)));     // :1016-1023
-    const float res = e.eres * sqrtf(es / e0);
-    if ((es * (1 + 2 * res / 2.35482f)) <= e.lo || (es * (1 - 2 * res / 2.35482f)) >= e.hi)
-        return 0.0f;                                                         // :1263-1269
-    const float pwin = window_prob(es, res, e.lo, e.hi);
+    const float res = e.eres * sqrt_mid(div_by(es, e0, re0));
+    constexpr float kFwhm = 2.35482f, kRFwhm = 1.0f / 2.35482f;
+    const float fw = div_by(res, kFwhm, kRFwhm);           // 2 * res / 2.35482f is its double
+    if ((es * (1 + 2 * fw)) <= e.lo || (es * (1 - 2 * fw)) >= e.hi) return 0.0f;   // :1263-1269
+    const float rs = rcp_rn(es);
+    // energy-window probability (calculategaussianIntegral, :1025-1038)
+    const float s2 = (float)((double)(fw * es) * 1.4142135623730951), rs2 = rcp_rn(s2);
+    float z1 = div_by(e.lo - es, s2, rs2), z2 = div_by(e.hi - es, s2, rs2);
+    if (!(s2 >= kMinDivisor)) {                            // no energy spread
+        z1 = (e.lo - es) / s2;
+        z2 = (e.hi - es) / s2;
+    }
+    const float pwin = 0.5f * (erff(z2) - erff(z1));
     const float sc = sinf(cone);
     float phi;
     if (pr.lsd * sc * 2.0f <= e.rdet) phi = (float)(2.0f * 3.14159265358979323846);
     else {
-        const float arg = e.rdet / 2.0f / pr.lsd / sc;
+        const float arg = div_rn(sp.half_width, sc);
         phi = 4.0f * asinf((arg <= 1.0f) ? arg : 1.0f);
     }
-    // theta range over the 8 corners of the (single) detector unit (:1305-1335)
-    const float dis = dist3(pr.xss, pr.yss, pr.zss, e.xIs, e.yIs, e.zIs);
-    const float xt = pr.xss + 1000.0f * (pr.xss - e.xIs) / dis;
-    const float yt = pr.yss + 1000.0f * (pr.yss - e.yIs) / dis;
-    const float zt = pr.zss + 1000.0f * (pr.zss - e.zIs) / dis;
-    const float lthr = box_chord(e.xIs, e.yIs, e.zIs, xt, yt, zt, e.ux1, e.uy1, e.uz1, e.ux2, e.uy2, e.uz2);
-    // The reference takes the extremes of the 8 corner angles acos(c_k); acos decreases, so
-    // they are acos(max c_k) and acos(min c_k): two arc cosines instead of eight (the same
-    // floats wherever acosf is monotone, which holds to within an ulp at ties).
-    float cmin = 2.0f, cmax = -2.0f;
+    // theta range over the 8 corners of the (single) detector unit (:1305-1335).  The reference
+    // takes the extremes of the 8 corner angles acos(c_k); acos decreases, so they are
+    // acos(max c_k) and acos(min c_k).  c_k = dot_k / (|a| |b_k|) rounds each quotient; approximate
+    // cosines (error below a quarter of the slack) select the corners that can be extreme, usually
+    // two or three, and only those quotients are formed.
+    const float ax = pr.xss - e.xIs, ay = pr.yss - e.yIs, az = pr.zss - e.zIs;
+    const float ma = sqrt_mid(ax * ax + ay * ay + az * az);
+    float tmin, tmax;
+    {
+        const float hw = 0.5f * e.w, ht = 0.5f * e.t, hh = 0.5f * e.h;
+        const float x0 = ax * (-hw - pr.xss), x1 = ax * (hw - pr.xss);
+        const float y0 = ay * (-ht - pr.yss), y1 = ay * (ht - pr.yss);
+        const float z0 = az * (-hh - pr.zss), z1 = az * (hh - pr.zss);
+        float c[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const int cx = c & 1, cy = (c >> 1) & 1, cz = c >> 2;
-        const float ck = cone_cosine(e.xIs, e.yIs, e.zIs, pr.xss, pr.yss, pr.zss, cx ? e.ux2 : e.ux1,
-                                     cy ? e.uy2 : e.uy1, cz ? e.uz2 : e.uz1);
-        cmin = fminf(cmin, ck);
-        cmax = fmaxf(cmax, ck);
+        for (int k = 0; k < 8; ++k)
+            c[k] = (((k & 1) ? x1 : x0) + ((k & 2) ? y1 : y0) + ((k & 4) ? z1 : z0)) * sp.rcorner[k];
+        float top = c[0], low = c[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            top = fmaxf(top, c[k]);
+            low = fminf(low, c[k]);
+        }
+        const float slack = (fabsf(x0) + fabsf(x1) + fabsf(y0) + fabsf(y1) + fabsf(z0) + fabsf(z1)) * sp.slack;
+        unsigned can = 0u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (c[k] >= top - slack || c[k] <= low + slack) can |= 1u << k;
+        float cmin = 2.0f, cmax = -2.0f;
+        while (can) {
+            const int k = __ffs(can) - 1;
+            can &= can - 1u;
+            float bx, by, bz;
+            corner_offset(e, pr, k, bx, by, bz);
+            const float dot = bx * ax + by * ay + bz * az;
+            const float mb = sqrt_mid(bx * bx + by * by + bz * bz);
+            float ck = div_rn(dot, ma * mb);
+            if (ck > 1.0f) ck = 1.0f;
+            if (ck < -1.0f) ck = -1.0f;
+            cmin = fminf(cmin, ck);
+            cmax = fmaxf(cmax, ck);
+        }
+        tmin = acosf(cmax);
+        tmax = acosf(cmin);
     }
-    float tmin = acosf(cmax), tmax = acosf(cmin);
-    if (lthr > 0.001f) tmin = 0.0f;
+    // a ray from the voxel through the scatter point that crosses d has theta_min = 0.  It passes
+    // d's centre at lsd sin(cone), so beyond d's circumscribed radius there is no chord to form.
+    if (pr.lsd * sc <= 1.001f * e.rdet + 0.01f) {
+        const float rdis = rcp_rn(ma);                     // |voxel - point| in d's frame (:1314)
+        const float xt = pr.xss + div_by(1000.0f * ax, ma, rdis);
+        const float yt = pr.yss + div_by(1000.0f * ay, ma, rdis);
+        const float zt = pr.zss + div_by(1000.0f * az, ma, rdis);
+        const float lthr = box_chord(e.xIs, e.yIs, e.zIs, xt, yt, zt, -0.5f * e.w, -0.5f * e.t, -0.5f * e.h, 0.5f * e.w,
+                                     0.5f * e.t, 0.5f * e.h);
+        if (lthr > 0.001f) tmin = 0.0f;
+    }
     const int n = (int)((tmax - tmin) / 0.01f);
-    const float ratio = (float)kn_sum_tab(tmin, n, kn_tab) / integ;
-    // attenuation by the flagged crystals at the scattered energy (:1369-1396)
-    // the scaled coefficient depends only on the attenuator's (mu_pe, mu_c) and E': it is
-    // recomputed only when those change along the list (same operands, same float)
+    const double ta = (double)tmin, tb = ta + (double)n * (double)0.01f;
+    const float ratio = (float)(kn_tab_eval(kn_tab, kKnU, tb) - kn_tab_eval(kn_tab, kKnV, ta)) / integ;
+    // attenuation by the flagged crystals at the scattered energy (:1369-1396): the scaled
+    // coefficient depends only on (mu_pe, mu_c) and E', so it is formed again only when they differ
+    // from the last ones used, starting from d's own (same operands, same float)
+    auto scaled_pe = [&](float mu) {                       // mu e0 e0 e0 / es / es / es
+        return div_by(div_by(div_by(mu * e0 * e0 * e0, es, rs), es, rs), es, rs);
+    };
+    const float mpe_s = scaled_pe(e.mu_pe);                // :1411-1417
+    const float mt_s = mpe_s + div_by(e.mu_c * e0, es, rs);
     float a_sum = 0.0f;
-    float c_pe = NAN, c_c = NAN, mt = 0.0f;
+    float c_pe = e.mu_pe, c_c = e.mu_c, mt = mt_s;
     for (int k = 0; k < pr.att_count; ++k) {
         const AttEntry ae = att[pr.att_begin + k];
         if (!(ae.mu_pe == c_pe && ae.mu_c == c_c)) {
             c_pe = ae.mu_pe;
             c_c = ae.mu_c;
-            const float mpe = ae.mu_pe * e0 * e0 * e0 / es / es / es;
-            const float mc = ae.mu_c * e0 / es;
-            mt = mpe + mc;
+            mt = scaled_pe(ae.mu_pe) + div_by(ae.mu_c * e0, es, rs);
         }
         a_sum = a_sum + ae.len * mt;
     }
-    if (NATIVE && (pn.w_pe != 0.0f || pn.w_c != 0.0f)) {  // native model: tungsten at E'
-        const float mpe_w = pn.w_pe * e0 * e0 * e0 / es / es / es;
-        const float mc_w = pn.w_c * e0 / es;
-        a_sum = a_sum + (mpe_w + mc_w);
-    }
-    const float mpe_s = e.mu_pe * e0 * e0 * e0 / es / es / es;              // :1411-1417
-    const float mc_s = e.mu_c * e0 / es;
-    const float mt_s = mpe_s + mc_s;
+    if (NATIVE && (pn.w_pe != 0.0f || pn.w_c != 0.0f))     // native model: tungsten at E'
+        a_sum = a_sum + (scaled_pe(pn.w_pe) + div_by(pn.w_c * e0, es, rs));
     const double c = (double)(w_s * phi / 2.0f) * (1.0 / 3.14159265358979323846) * (double)ratio *
                      (double)pwin * (double)expf(-a_sum) *
                      (double)(1.0f - expf(-pr.labs * mt_s)) * (double)mpe_s / (double)mt_s;
@@ -628,7 +693,7 @@ __device__ float scatter_item(const ElemConst& e, const PairRec& pr, const PairN
 // (t = threadIdx.x).  sp, spn: the block's pair staging buffers in shared memory.
 template <bool NATIVE>
 __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhysics& ph, const ScatterLaunch& L,
-                                             int di, long long vblock, PairRec* sp, PairNative* spn)
+                                             int di, long long vblock, StagedPair* sp, PairNative* spn)
 {
     const int d = L.det_begin + di;
     const long long vi = vblock * kItemThreads + threadIdx.x;
@@ -654,9 +719,7 @@ __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhys
     }
     e.rdet = sqrtf(e.w * e.w / (float)1 / (float)1 + e.h * e.h / (float)1 / (float)1 +
                    e.t * e.t / (float)1 / (float)1) / 2.0f;
-    e.ux1 = ((float)0 / (float)1 - 0.5f) * e.w; e.ux2 = (((float)0 + 1.0f) / (float)1 - 0.5f) * e.w;
-    e.uy1 = ((float)0 / (float)1 - 0.5f) * e.t; e.uy2 = (((float)0 + 1.0f) / (float)1 - 0.5f) * e.t;
-    e.uz1 = ((float)0 / (float)1 - 0.5f) * e.h; e.uz2 = (((float)0 + 1.0f) / (float)1 - 0.5f) * e.h;
+    const float re0 = rcp_rn(ph.e0);
 
     double acc_c = 0.0, acc_h = 0.0;
     const int s_begin = (L.parts & 1) ? 0 : g.n_det;
@@ -667,15 +730,15 @@ __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhys
         const int cnt = min(kPairChunk, s_end - s0);
         __syncthreads();
         for (int k = threadIdx.x; k < cnt; k += kItemThreads) {
-            sp[k] = prow[s0 + k];
+            sp[k] = stage_pair(e, prow[s0 + k]);
             if constexpr (NATIVE) spn[k] = L.native[(long long)d * ns + s0 + k];
         }
         __syncthreads();
         if (!run || !active) continue;
         for (int k = 0; k < cnt; ++k) {
             const int s = s0 + k;
-            const PairRec& pr = sp[k];
-            if (!pr.valid) continue;
+            const StagedPair& pr = sp[k];
+            if (!pr.r.valid) continue;
             float xs, ys, zs, w_s;
             const bool crystal = s < g.n_det;
             if (crystal) {
@@ -705,7 +768,7 @@ __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhys
             }
             // one call site keeps a single copy of the item code
             const double c = (double)scatter_item<NATIVE>(e, pr, spn[NATIVE ? k : 0], att_row, xs, ys, zs, w_s,
-                                                          ph.e0, ph.integ, L.kn_tab);
+                                                          ph.e0, re0, ph.integ, L.kn_tab);
             if (crystal) acc_c += c;
             else acc_h += c;
         }
@@ -722,7 +785,7 @@ template <bool NATIVE>
 __global__ void __launch_bounds__(kItemThreads)
 scatter_kernel(DevGeom g, ScatterPhysics ph, ScatterLaunch L)
 {
-    __shared__ PairRec sp[kPairChunk];
+    __shared__ StagedPair sp[kPairChunk];
     __shared__ PairNative spn[NATIVE ? kPairChunk : 1];
     scatter_rows<NATIVE>(g, ph, L, blockIdx.y, blockIdx.x, sp, spn);
 }
@@ -733,7 +796,7 @@ scatter_kernel(DevGeom g, ScatterPhysics ph, ScatterLaunch L)
 // item runs scatter_rows, so every element equals the single launch's bit for bit.
 __global__ void __launch_bounds__(kItemThreads) scatter_batch_kernel(ScatterBatchLaunch B)
 {
-    __shared__ PairRec sp[kPairChunk];
+    __shared__ StagedPair sp[kPairChunk];
     __shared__ PairNative spn[kPairChunk];
     __shared__ DevGeom sg;
     __shared__ ScatterTask st;
@@ -943,9 +1006,11 @@ static double kn_shape_sin_prime(double th, double alpha)
 void kn_table_build(double e0, double* tab)
 {
     const int N = kKnTable;
-    const double alpha = e0 / 511.0, hc = 3.14159265358979323846 / N;
+    const double alpha = e0 / 511.0, hc = 3.14159265358979323846 / N, h = (double)0.01f;
     static const double xg[4] = {0.1834346424956498, 0.5255324099163290, 0.7966664774136267, 0.9602898564975363};
     static const double wg[4] = {0.3626837833783620, 0.3137066458778873, 0.2223810344533745, 0.1012285362903763};
+    struct Node { double y[3], d[3]; };                    // G, U, V and their derivatives
+    Node prev{};
     double G = 0.0;
     for (int i = 0; i <= N; ++i) {
         const double th = i * hc;
@@ -956,10 +1021,21 @@ void kn_table_build(double e0, double* tab)
                 acc += wg[k] * (kn_shape_sin(mid - half * xg[k], alpha) + kn_shape_sin(mid + half * xg[k], alpha));
             G += half * acc;
         }
-        tab[i] = G;
-        tab[(N + 1) + i] = kn_shape_sin(th, alpha);
-        tab[2 * (N + 1) + i] = kn_shape_sin_prime(th, alpha);
+        const double F = kn_shape_sin(th, alpha), P = kn_shape_sin_prime(th, alpha), eps = 1e-4;
+        const double Q = (kn_shape_sin_prime(th + eps, alpha) - kn_shape_sin_prime(th - eps, alpha)) / (2.0 * eps);
+        const Node now{{G, G + 0.5 * h * F + h * h / 12.0 * P, G - 0.5 * h * F + h * h / 12.0 * P},
+                       {F, F + 0.5 * h * P + h * h / 12.0 * Q, F - 0.5 * h * P + h * h / 12.0 * Q}};
+        for (int q = 0; q < 3 && i > 0; ++q) {             // the cell's cubic Hermite polynomial
+            double* c = tab + 4 * N * q + 4 * (i - 1);
+            const double dy = now.y[q] - prev.y[q], d0 = hc * prev.d[q], d1 = hc * now.d[q];
+            c[0] = prev.y[q];
+            c[1] = d0;
+            c[2] = 3.0 * dy - 2.0 * d0 - d1;
+            c[3] = d0 + d1 - 2.0 * dy;
+        }
+        prev = now;
     }
+    tab[kKnTotal] = G;
 }
 
 double kn_normalisation(double e0)

@@ -74,44 +74,28 @@ struct ScatterLaunch {
     float* out;
 };
 
-// FP64 table of the Klein-Nishina shape on [0, pi]: nodes theta_i = i * pi / kKnTable;
-// [0 .. N] integral from 0, [N+1 .. 2N+1] F = KN(theta) sin(theta), [2N+2 .. 3N+2] dF/dtheta.
+// FP64 tables of the Klein-Nishina integral on [0, pi], cubic Hermite polynomials on kKnTable
+// cells: for cell i, four coefficients in t = theta / cell - i.  G: integral of F = KN(theta)
+// sin(theta) from 0.  U and V: the ends of the reference's Riemann sum with step h = 0.01f,
+//   sum_{i=0..n} F(a + i h) h = U(a + n h) - V(a) + O(h^4),
+//   U = G + h/2 F + h^2/12 F',  V = G - h/2 F + h^2/12 F'   (Euler-Maclaurin),
+// so a sum costs two cubics instead of the six interpolations of G, F and F' at both ends.
+// Then the total G(pi).
 constexpr int kKnTable = 4096;
-void kn_table_build(double e0, double* host_tab);   // host buffer of 3 * (kKnTable + 1) doubles
+constexpr int kKnG = 0, kKnU = 4 * kKnTable, kKnV = 8 * kKnTable, kKnTotal = 12 * kKnTable;
+constexpr int kKnDoubles = 12 * kKnTable + 1;
+void kn_table_build(double e0, double* host_tab);   // host buffer of kKnDoubles doubles
 
-// The Klein-Nishina table at angle th: G (integral from 0) and F by cubic Hermite
-// interpolation (error ~1e-14), F' linearly.
-__device__ __forceinline__ void kn_tab_eval(const double* __restrict__ tab, double th, double& G,
-                                            double& F, double& Fp)
+// Table function `which` (kKnG, kKnU or kKnV) at angle th (interpolation error ~1e-14).
+__device__ __forceinline__ double kn_tab_eval(const double* __restrict__ tab, int which, double th)
 {
-    const double hc = 3.14159265358979323846 / kKnTable;
-    double x = th * (kKnTable / 3.14159265358979323846);   // cell coordinate (no double division)
+    const double x = th * (kKnTable / 3.14159265358979323846);   // cell coordinate
     int i = (int)x;
     i = i < 0 ? 0 : (i > kKnTable - 1 ? kKnTable - 1 : i);
     const double t = x - (double)i;
-    const double t2 = t * t, t3 = t2 * t;
-    const double h00 = 2.0 * t3 - 3.0 * t2 + 1.0, h10 = t3 - 2.0 * t2 + t;
-    const double h01 = -2.0 * t3 + 3.0 * t2, h11 = t3 - t2;
-    const double* Gt = tab;
-    const double* Ft = tab + (kKnTable + 1);
-    const double* Pt = tab + 2 * (kKnTable + 1);
-    const double g0 = __ldg(&Gt[i]), g1 = __ldg(&Gt[i + 1]);
-    const double f0 = __ldg(&Ft[i]), f1 = __ldg(&Ft[i + 1]);
-    const double p0 = __ldg(&Pt[i]), p1 = __ldg(&Pt[i + 1]);
-    G = h00 * g0 + h10 * hc * f0 + h01 * g1 + h11 * hc * f1;
-    F = h00 * f0 + h10 * hc * p0 + h01 * f1 + h11 * hc * p1;
-    Fp = (1.0 - t) * p0 + t * p1;
-}
-
-// Energy-window probability of a Gaussian of resolution res (FWHM fraction) at energy e
-// (calculategaussianIntegral, ScatterGen_RayTracing_CircularHole/scatter.cu:1025-1038).
-__device__ __forceinline__ float window_prob(float e, float res, float lo, float hi)
-{
-    const float sigma = res / 2.35482f * e;
-    const float s2 = (float)((double)sigma * 1.4142135623730951);   // sigma * sqrt(2.0)
-    const float z1 = (lo - e) / s2;
-    const float z2 = (hi - e) / s2;
-    return 0.5f * (erff(z2) - erff(z1));
+    const double2* c = reinterpret_cast<const double2*>(tab + which) + 2 * i;
+    const double2 lo = __ldg(&c[0]), hi = __ldg(&c[1]);
+    return lo.x + t * (lo.y + t * (hi.x + t * hi.y));
 }
 
 // Word counts of the reference bitmap layouts (scatter.cu:2053-2056, :2234-2237).

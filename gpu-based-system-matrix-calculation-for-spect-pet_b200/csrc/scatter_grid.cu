@@ -526,9 +526,7 @@ __device__ bool point_terms(const DevGeom& g, const GridGeom& G, int d, const do
 
 __device__ __forceinline__ double kn_integral(const double* __restrict__ tab, double th)
 {
-    double G, F, P;
-    kn_tab_eval(tab, th, G, F, P);
-    return G;
+    return kn_tab_eval(tab, kKnG, th);
 }
 
 constexpr int kTerms = 8;
@@ -786,7 +784,7 @@ extern "C" SYSMAT_API int sysmat_scatter_grid(sysmat_ctx* ctx, int parts, float 
 
     // Klein-Nishina table at the photopeak (shared with sysmat_scatter)
     if (!ctx->d_kn_tab || ctx->kn_e0 != P[7]) {
-        std::vector<double> tab(3 * (size_t)(kKnTable + 1));
+        std::vector<double> tab(kKnDoubles);
         kn_table_build((double)P[7], tab.data());
         if (!ctx->d_kn_tab && cudaMalloc(&ctx->d_kn_tab, sizeof(double) * tab.size()) != cudaSuccess) {
             ctx->d_kn_tab = nullptr;
@@ -797,7 +795,7 @@ extern "C" SYSMAT_API int sysmat_scatter_grid(sysmat_ctx* ctx, int parts, float 
         ctx->kn_e0 = P[7];
     }
     double kn_total = 0.0;
-    CUDA_TRY(cudaMemcpy(&kn_total, ctx->d_kn_tab + kKnTable, sizeof(double), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&kn_total, ctx->d_kn_tab + kKnTotal, sizeof(double), cudaMemcpyDeviceToHost));
 
     // scratch: weights of one pass of voxels, the photoelectric block, the FP64 sums
     const int nv_max = (int)(vox_count < kGridMaxVox ? vox_count : kGridMaxVox);
