@@ -763,46 +763,6 @@ __device__ __forceinline__ bool walk_sub_element(const DevGeom& g, const BlockSm
 
 #include "pe_ref.cuh"
 
-// Element of the sampled form: the mean over the voxel's sx x sy x sz source points (centres of
-// a grid over the voxel) of the reference's element with crystal d divided into nx x ny x nz
-// sub-elements (x, depth, z), every contribution summed in FP64.  Each source point has its
-// own cone test and kept list; its sub-elements are taken 32 at a time in (z, depth, x) order,
-// x fastest, so a round is a compact patch of the crystal.  With 8 x 16 x 8 and 1 x 1 x 1 it
-// runs pe_element<1>'s float program, summed in another order (a separately compiled
-// instance: the compiler may contract the position expressions differently, in the last bit).
-template <bool ELL>
-__device__ double pe_element_sampled(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, int d, long long v,
-                                     float cr, float sr, int lane, const Sampling& sm)
-{
-    const int n_sub = sm.nx * sm.ny * sm.nz, nxy = sm.nx * sm.ny;
-    const int n_pts = sm.sx * sm.sy * sm.sz;
-    const float fx = (float)sm.nx, fy = (float)sm.ny, fz = (float)sm.nz;
-    double dacc = 0.0;
-    long long unused = 0;
-    for (int p = 0; p < n_pts; ++p) {
-        const int jx = p % sm.sx, jy = (p / sm.sx) % sm.sy, jz = p / (sm.sx * sm.sy);
-        __syncwarp();                     // the previous point's lists are no longer read
-        Elem e;
-        if (!init_element(g, ws.inner, d, v, cr, sr, lane, e, ((float)jx + 0.5f) / (float)sm.sx,
-                          ((float)jy + 0.5f) / (float)sm.sy, ((float)jz + 0.5f) / (float)sm.sz))
-            return 0.0;                   // the crystal's mu does not depend on the point
-        KeptList kl = start_kept_list(g, bs, ws, e, d, lane);
-        for (int base = 0; base < n_sub; base += 32) {
-            const int sidx = min(base + lane, n_sub - 1);
-            const int iz = sidx / nxy, rem = sidx - iz * nxy;
-            const int iy = rem / sm.nx, ix = rem - iy * sm.nx;
-            const SubElem q = sub_element_at(e, ix, iy, iz, fx, fy, fz);
-            Walk s{0.0f, 0.0f, 0, 0, 0, 0, 0};
-            const bool skip = walk_sub_element<false, ELL>(g, bs, ws, e, d, q, base + lane >= n_sub, base == 0,
-                                                           kl, lane, s, unused);
-            if (!skip) dacc += (double)finish_sub_element_at(e, q, s.att, fx, fy, fz);
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
-    return dacc / (double)n_pts;
-}
-
 #include "pe_fp64.cuh"
 #include "pe_local.cuh"
 
@@ -870,7 +830,7 @@ struct BrickOut {
 // Shared memory and blocks per SM of each kernel instance (pe_ref.cuh for the float modes 0, 1).
 template <int MODE, bool SAMPLED>
 struct Shape {
-    static constexpr bool ref = MODE <= 1 && !SAMPLED;
+    static constexpr bool ref = MODE <= 1;
     static constexpr int blocks = ref ? kRefBlocks : 2;
     using Smem = typename std::conditional<ref, RefSmem, BlockSmem>::type;
 };
@@ -889,7 +849,6 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, 
                                          unsigned long long* counters, const Sampling* smp = nullptr,
                                          float rotation = 0.0f)
 {
-    constexpr bool REF = Shape<MODE, SAMPLED>::ref;
     Superset& sup = superset_of(sm);
     const int x0 = gx * bx, y0 = gy * by, z0 = iz0 + gz * bz;
     const int x1 = min(x0 + bx, g.nx) - 1, y1 = min(y0 + by, g.ny) - 1, z1 = min(z0 + bz, iz1 + 1) - 1;
@@ -910,20 +869,17 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, 
         const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
         if (ix < g.nx && iy < g.ny && iz <= z1 && v >= O.vox_begin && v <= O.vlast) {
             float val;
-            if constexpr (REF) {
+            if constexpr (MODE <= 1 && SAMPLED) {
+                val = (float)pe_element_sampled<ELL>(g, sup, sm.w[wid], d, v, cr, sr, lane, *smp);
+            } else if constexpr (MODE <= 1) {
                 val = (float)pe_element_ref<MODE, COUNT, ELL>(g, sup, sm.w[wid], d, v, cr, sr, lane, counters);
+            } else if constexpr (MODE == 3) {
+                float* so = nullptr;
+                if (SAMPLED && O.sub_out)
+                    so = O.sub_out + ((v - O.vox_begin) * O.det_count + di) * (long long)(smp->nx * smp->ny * smp->nz);
+                val = (float)pe_element_local<ELL, SAMPLED>(g, sm, sm.w[wid], d, v, cr, sr, rotation, lane, smp, so);
             } else {
-                WarpSmem& ws = sm.w[wid];
-                if constexpr (MODE == 3) {
-                    float* so = nullptr;
-                    if (SAMPLED && O.sub_out)
-                        so = O.sub_out + ((v - O.vox_begin) * O.det_count + di) * (long long)(smp->nx * smp->ny * smp->nz);
-                    val = (float)pe_element_local<ELL, SAMPLED>(g, sm, ws, d, v, cr, sr, rotation, lane, smp, so);
-                } else if constexpr (SAMPLED) {
-                    val = (float)pe_element_sampled<ELL>(g, sm, ws, d, v, cr, sr, lane, *smp);
-                } else {
-                    val = (float)pe_element64(g, sm, ws, d, v, cr, sr, rotation, lane);
-                }
+                val = (float)pe_element64(g, sm, sm.w[wid], d, v, cr, sr, rotation, lane);
             }
             if (lane == 0) O.out[(long long)di * O.ld + (v - O.vox_begin)] = val;
             __syncwarp();

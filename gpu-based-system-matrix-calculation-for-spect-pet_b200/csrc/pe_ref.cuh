@@ -1,8 +1,9 @@
-// The reference-order photoelectric element (8 x 16 x 8 sub-elements, voxel centre; the float
-// program of PESysMatGen.cu:951-1364), included by pe.cu inside its anonymous namespace.
+// The photoelectric element in the reference's float program (PESysMatGen.cu:951-1364), with its
+// own 8 x 16 x 8 sub-elements and voxel centre (pe_element_ref) or any division and source points
+// (pe_element_sampled), included by pe.cu inside its anonymous namespace.
 //
 // One warp per element, in phases that each loop over rounds (a round: 32 rays, one per lane, to
-// a compact patch of 4 z x 4 x x 2 depth sub-elements):
+// a compact patch of sub-elements; the reference division: 4 z x 4 x x 2 depth):
 //   1. kept objects: a cheap slope filter, then the reference cone test on what is left; each
 //      kept object's geometry goes into the warp's record array (build_kept);
 //   2. masks: which kept objects meet which round's slope box (round_masks; one lane per object,
@@ -29,6 +30,7 @@ constexpr int kRefBlocks = 2;            // blocks of kWarps warps per SM
 constexpr int kPassRounds = 16;          // rounds per pass: half of an element
 constexpr int kUnits = 192;              // record units of 32 B: a hole takes one, a crystal two
 constexpr int kMaskWords = kUnits / 32;
+constexpr int kNear = 512;               // sampled form: objects near the bundle of any source point
 
 struct RefWarp {
     // kept objects in the reference's order.  Hole i at rec[2 i]: (x, z, voxel - x, voxel - z),
@@ -42,6 +44,7 @@ struct RefWarp {
     float att[kPassRounds * 32];         // [round][lane]: attenuation outside crystal d, then contribution
     float len[256];                      // hole length of the open layer (elements kept in several chunks)
     int cand[64];                        // build_kept: source positions awaiting the cone test
+    unsigned short near[kNear];          // sampled form: objects near the ray bundle of any source point
     float4 inner[kMaxLayers];            // plate "through both faces" slope rectangles
     Elem elem;
     // per sub-element index along x (0..7), depth (8..23), z (24..31): its centre, centre - voxel,
@@ -61,25 +64,69 @@ struct Kept {
     bool even;
 };
 
-// Sub-element indices of this lane in round r.
-__device__ __forceinline__ void round_indices(int r, int lane, int& ix, int& iy, int& iz)
+// How a crystal is divided: this lane's sub-element in a round, sub-element centres, and the
+// table rows (centre, centre - voxel, lower face - voxel, upper face - voxel) of an index
+// (:1207-1217).  The products are rounded before the sums, as the reference's build rounds them.
+__device__ __forceinline__ float sub_centre(int i, float f, float size)
 {
-    ix = 4 * ((r >> 3) & 1) + ((lane >> 1) & 3);
-    iy = 2 * (r & 7) + (lane & 1);
-    iz = 4 * (r >> 4) + (lane >> 3);
+    return __fadd_rn(-size / 2.0f, __fmul_rn(((float)i + 0.5f) / f, size));
 }
 
-// Lane l's entry of the sub-element table (:1207-1217 and the sub-element's faces).
-__device__ __forceinline__ float4 sub_entry(const Elem& e, int lane)
+__device__ __forceinline__ float4 sub_row(int i, float f, float size, float p)
 {
-    const int i = lane < 8 ? lane : (lane < 24 ? lane - 8 : lane - 24);
-    const float f = lane >= 8 && lane < 24 ? 16.0f : 8.0f;
-    const float size = lane < 8 ? e.w : (lane < 24 ? e.t : e.h);
-    const float p = lane < 8 ? e.xIs : (lane < 24 ? e.yIs : e.zIs);
-    const float c = __fadd_rn(-size / 2.0f, __fmul_rn(((float)i + 0.5f) / f, size));
+    const float c = sub_centre(i, f, size);
     const float u1 = ((float)i / f - 0.5f) * size, u2 = (((float)i + 1.0f) / f - 0.5f) * size;
     return make_float4(c, c - p, u1 - p, u2 - p);
 }
+
+// The reference's 8 x 16 x 8, rows kept in ws.sub.
+struct RefDivision {
+    static constexpr float fx = 8.0f, fy = 16.0f, fz = 8.0f;
+    __device__ __forceinline__ void indices(int r, int lane, int& ix, int& iy, int& iz) const
+    {
+        ix = 4 * ((r >> 3) & 1) + ((lane >> 1) & 3);
+        iy = 2 * (r & 7) + (lane & 1);
+        iz = 4 * (r >> 4) + (lane >> 3);
+    }
+    __device__ __forceinline__ bool dead(int, int) const { return false; }
+    __device__ __forceinline__ float3 centre(const RefWarp& ws, int ix, int iy, int iz) const
+    {
+        return make_float3(ws.sub[ix].x, ws.sub[8 + iy].x, ws.sub[24 + iz].x);
+    }
+    __device__ __forceinline__ float4 row_x(const RefWarp& ws, int i) const { return ws.sub[i]; }
+    __device__ __forceinline__ float4 row_y(const RefWarp& ws, int i) const { return ws.sub[8 + i]; }
+    __device__ __forceinline__ float4 row_z(const RefWarp& ws, int i) const { return ws.sub[24 + i]; }
+    // lane l's table row: x (l < 8), depth (l < 24), z
+    __device__ __forceinline__ static float4 entry(const Elem& e, int lane)
+    {
+        const int i = lane < 8 ? lane : (lane < 24 ? lane - 8 : lane - 24);
+        return sub_row(i, lane >= 8 && lane < 24 ? fy : fx, lane < 8 ? e.w : (lane < 24 ? e.t : e.h),
+                       lane < 8 ? e.xIs : (lane < 24 ? e.yIs : e.zIs));
+    }
+};
+
+// nx x ny x nz (x, depth, z), 32 to a round in (z, depth, x) order, x fastest, from sub-element
+// `base`; lanes past the end repeat the last one and are dead.
+struct AnyDivision {
+    int nx, ny, n_sub, base;
+    float fx, fy, fz;
+    __device__ __forceinline__ void indices(int r, int lane, int& ix, int& iy, int& iz) const
+    {
+        const int s = min(base + 32 * r + lane, n_sub - 1), nxy = nx * ny;
+        iz = s / nxy;
+        const int rem = s - iz * nxy;
+        iy = rem / nx;
+        ix = rem - iy * nx;
+    }
+    __device__ __forceinline__ bool dead(int r, int lane) const { return base + 32 * r + lane >= n_sub; }
+    __device__ __forceinline__ float3 centre(const RefWarp& ws, int ix, int iy, int iz) const
+    {
+        return make_float3(sub_centre(ix, fx, ws.elem.w), sub_centre(iy, fy, ws.elem.t), sub_centre(iz, fz, ws.elem.h));
+    }
+    __device__ __forceinline__ float4 row_x(const RefWarp& ws, int i) const { return sub_row(i, fx, ws.elem.w, ws.elem.xIs); }
+    __device__ __forceinline__ float4 row_y(const RefWarp& ws, int i) const { return sub_row(i, fy, ws.elem.t, ws.elem.yIs); }
+    __device__ __forceinline__ float4 row_z(const RefWarp& ws, int i) const { return sub_row(i, fz, ws.elem.h, ws.elem.zIs); }
+};
 
 // World position of the sub-element with centre (xDs, yDs, zDs) in crystal d's frame.
 __device__ __forceinline__ void ray_end(const Elem& e, float xDs, float yDs, float zDs, float& xD, float& yD, float& zD)
@@ -95,9 +142,11 @@ __device__ __forceinline__ float norm2(float x, float y, float z)
     return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
 }
 
-// Whether object i may meet the slope rectangle of crystal d (approximate reciprocals, within
-// the rectangles' margins); objects close to the voxel always may.
-__device__ __forceinline__ bool near_bundle(const DevGeom& g, const Elem& e, int i)
+// Whether object i may meet the slope rectangle rd of crystal d (approximate reciprocals, within
+// the rectangles' margins), seen from any source within (spread, spread, spread_z) of the
+// element's; objects close to the source always may.
+__device__ __forceinline__ bool near_bundle(const DevGeom& g, const Elem& e, const float4& rd, int i, float spread = 0.0f,
+                                            float spread_z = 0.0f)
 {
     float x0, x1, z0, z1, y0, y1;
     if (i < g.n_holes) {
@@ -111,13 +160,13 @@ __device__ __forceinline__ bool near_bundle(const DevGeom& g, const Elem& e, int
         const float hx = 0.5f * (s.x * fabsf(t.x) + s.z * fabsf(t.y)), hz = 0.5f * (s.x * fabsf(t.y) + s.z * fabsf(t.x));
         x0 = p.x - hx, x1 = p.x + hx, z0 = p.z - hz, z1 = p.z + hz, y0 = p.y - 0.5f * s.y, y1 = p.y + 0.5f * s.y;
     }
-    y0 -= e.yI;
-    y1 -= e.yI;
+    y0 -= e.yI + spread;
+    y1 -= e.yI - spread;
     if (!(y0 >= kMinDepth) || !(y1 >= kMinDepth)) return true;
     const float r0 = rcp_approx(y0), r1 = rcp_approx(y1);
-    x0 -= e.xI, x1 -= e.xI, z0 -= e.zI, z1 -= e.zI;
-    return fminf(x0 * r0, x0 * r1) - kSlopeMargin <= e.rd.y && fmaxf(x1 * r0, x1 * r1) + kSlopeMargin >= e.rd.x &&
-           fminf(z0 * r0, z0 * r1) - kSlopeMargin <= e.rd.w && fmaxf(z1 * r0, z1 * r1) + kSlopeMargin >= e.rd.z;
+    x0 -= e.xI + spread, x1 -= e.xI - spread, z0 -= e.zI + spread_z, z1 -= e.zI - spread_z;
+    return fminf(x0 * r0, x0 * r1) - kSlopeMargin <= rd.y && fmaxf(x1 * r0, x1 * r1) + kSlopeMargin >= rd.x &&
+           fminf(z0 * r0, z0 * r1) - kSlopeMargin <= rd.w && fmaxf(z1 * r0, z1 * r1) + kSlopeMargin >= rd.z;
 }
 
 // Reference cone test of object i (:1120-1184).
@@ -132,13 +181,13 @@ __device__ __forceinline__ bool in_cone(const DevGeom& g, const Elem& e, int i)
            crit + e.crit_self;
 }
 
-// Kept objects of the element from source positions [cursor, n_src) (the block's superset, or
-// all objects), in order.  The slope filter leaves a few percent of the superset, so what
+// Kept objects of the element from source positions [cursor, n_src) of the ids src (the block's
+// superset, say; nullptr: all objects), in order.  The slope filter leaves a few percent of the superset, so what
 // passes it is queued and the cone test (two square roots and four divisions) runs on full
 // groups of 32.  Stops before a group that would overflow the records; returns the position to
 // go on from.
-__device__ __forceinline__ int build_kept(const DevGeom& g, const Superset& sup, RefWarp& ws, const Elem& e, int d,
-                                          int cursor, int n_src, bool from_super, int lane, Kept& kept)
+__device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short* src, RefWarp& ws, const Elem& e,
+                                          int d, int cursor, int n_src, int lane, Kept& kept)
 {
     const unsigned below = (1u << lane) - 1u;
     int n = 0, nh = 0, units = 0, queued = 0;
@@ -149,8 +198,8 @@ __device__ __forceinline__ int build_kept(const DevGeom& g, const Superset& sup,
             const int j = cursor + lane;
             bool maybe = false;
             if (j < n_src) {
-                const int id = from_super ? sup.sid[j] : j;
-                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e, id));
+                const int id = src ? src[j] : j;
+                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e, e.rd, id));
             }
             const unsigned m = __ballot_sync(0xffffffffu, maybe);
             if (maybe) ws.cand[queued + __popc(m & below)] = j;
@@ -163,7 +212,7 @@ __device__ __forceinline__ int build_kept(const DevGeom& g, const Superset& sup,
         int id = 0;
         bool keep = false;
         if (lane < take) {
-            id = from_super ? sup.sid[ws.cand[lane]] : ws.cand[lane];
+            id = src ? src[ws.cand[lane]] : ws.cand[lane];
             keep = in_cone(g, e, id);
         }
         const bool hole = id < g.n_holes;
@@ -402,16 +451,17 @@ __device__ __forceinline__ void close_layers_ref(const DevGeom& g, Walk& s, int 
 // misses a hole adds an exact zero.  EVEN (all kept holes alike, the usual collimator): the cap
 // terms are formed once per ray, and holes go two at a time (independent chords: the serial
 // chain of one leaves issue slots idle).
-template <bool COUNT, bool ELL, bool EVEN>
-__device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, int nh, int r0, int r1, bool first, int lay0,
+template <bool COUNT, bool ELL, bool EVEN, class Div>
+__device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int r0, int r1, bool first, int lay0,
                                            int lay1, bool carry, int lane, int& n_hits, int& n_evals, int& n_blocked)
 {
     const Elem& e = ws.elem;
     for (int r = r0; r < r1; ++r) {
         int ix, iy, iz;
-        round_indices(r, lane, ix, iy, iz);
+        dv.indices(r, lane, ix, iy, iz);
+        const float3 q = dv.centre(ws, ix, iy, iz);
         float xD, yD, zD;
-        ray_end(e, ws.sub[ix].x, ws.sub[8 + iy].x, ws.sub[24 + iz].x, xD, yD, zD);
+        ray_end(e, q.x, q.y, q.z, xD, yD, zD);
         HoleRay c;
         hole_ray_init(c, xD - e.xI, yD - e.yI, zD - e.zI);
         Walk s{0.0f, 0.0f, lay0, 0, 0, 0, 0};
@@ -419,6 +469,7 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, int nh
         if (first) {
             const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;             // open rectangles: slope 0
             skip = plate_penalty(g, ws.inner, e, xD, yD, zD, (xD - e.xI) * rdy, (zD - e.zI) * rdy, s.att) && g.nonneg_mu;
+            skip = skip || dv.dead(r, lane);
         } else {
             s.att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
             s.len = ws.len[(r & 7) * 32 + lane];
@@ -510,8 +561,8 @@ __device__ __forceinline__ float crystal_chord(float xa, float ya, float za, flo
 
 // Other crystals along the rays of rounds [r0, r1): kept entries [nh, count), added to ws.att in
 // the reference's order (:1290-1325).
-template <bool COUNT>
-__device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, int nh, int count, int r0, int r1, int lane,
+template <bool COUNT, class Div>
+__device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int count, int r0, int r1, int lane,
                                               int& n_hits, int& n_evals)
 {
     const Elem& e = ws.elem;
@@ -519,9 +570,10 @@ __device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, int
         Entries it(ws, r, nh, count);
         if (!it.more()) continue;
         int ix, iy, iz;
-        round_indices(r, lane, ix, iy, iz);
+        dv.indices(r, lane, ix, iy, iz);
+        const float3 q = dv.centre(ws, ix, iy, iz);
         float xD, yD, zD;
-        ray_end(e, ws.sub[ix].x, ws.sub[8 + iy].x, ws.sub[24 + iz].x, xD, yD, zD);
+        ray_end(e, q.x, q.y, q.z, xD, yD, zD);
         const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;
         const float sa_a = (xD - e.xI) * rdy, sa_b = (zD - e.zI) * rdy;
         float att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
@@ -555,11 +607,12 @@ __device__ __forceinline__ float inside_length(float tmin, float tmax, float tio
 // slow cases): inside = the crystal and the sub-element boxes to the sub-element's centre,
 // otherwise the sub-element box along the extended ray to (xo, yo, zo).
 static __device__ __noinline__ float2 finish_parallel(float xi, float yi, float zi, float xo, float yo, float zo, float w,
-                                                      float t, float h, int ix, int iy, int iz, int inside)
+                                                      float t, float h, int ix, int iy, int iz, float fx, float fy,
+                                                      float fz, int inside)
 {
-    const float ux1 = ((float)ix / 8.0f - 0.5f) * w, ux2 = (((float)ix + 1.0f) / 8.0f - 0.5f) * w;
-    const float uy1 = ((float)iy / 16.0f - 0.5f) * t, uy2 = (((float)iy + 1.0f) / 16.0f - 0.5f) * t;
-    const float uz1 = ((float)iz / 8.0f - 0.5f) * h, uz2 = (((float)iz + 1.0f) / 8.0f - 0.5f) * h;
+    const float ux1 = ((float)ix / fx - 0.5f) * w, ux2 = (((float)ix + 1.0f) / fx - 0.5f) * w;
+    const float uy1 = ((float)iy / fy - 0.5f) * t, uy2 = (((float)iy + 1.0f) / fy - 0.5f) * t;
+    const float uz1 = ((float)iz / fz - 0.5f) * h, uz2 = (((float)iz + 1.0f) / fz - 0.5f) * h;
     float2 l = make_float2(0.0f, 0.0f);
     if (!inside) {
         l.x = box_chord_parallel(xi, yi, zi, xo, yo, zo, ux1, uy1, uz1, ux2, uy2, uz2, 0);
@@ -572,14 +625,15 @@ static __device__ __noinline__ float2 finish_parallel(float xi, float yi, float 
 
 // Contribution of sub-element (ix, iy, iz), given the attenuation outside crystal d: self
 // attenuation, absorption and solid angle (:1223-1231, :1329-1357).
-__device__ __forceinline__ float finish_ray(const RefWarp& ws, int ix, int iy, int iz, float att)
+template <class Div>
+__device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, int ix, int iy, int iz, float att)
 {
     const Elem& e = ws.elem;
-    const float4 X = ws.sub[ix], Y = ws.sub[8 + iy], Z = ws.sub[24 + iz];
+    const float4 X = dv.row_x(ws, ix), Y = dv.row_y(ws, iy), Z = dv.row_z(ws, iz);
     const float w = e.w, t = e.t, h = e.h;
     float l1, l2;
     if (fabsf(X.y) < kEps || fabsf(Y.y) < kEps || fabsf(Z.y) < kEps) {
-        const float2 l = finish_parallel(e.xIs, e.yIs, e.zIs, X.x, Y.x, Z.x, w, t, h, ix, iy, iz, 1);
+        const float2 l = finish_parallel(e.xIs, e.yIs, e.zIs, X.x, Y.x, Z.x, w, t, h, ix, iy, iz, dv.fx, dv.fy, dv.fz, 1);
         l1 = l.x;
         l2 = l.y;
     } else {
@@ -613,7 +667,7 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, int ix, int iy, i
     const float dx = xt - e.xIs, dy = yt - e.yIs, dz = zt - e.zIs;
     float labs;
     if (fabsf(dx) < kEps || fabsf(dy) < kEps || fabsf(dz) < kEps) {
-        labs = finish_parallel(e.xIs, e.yIs, e.zIs, xt, yt, zt, w, t, h, ix, iy, iz, 0).x;
+        labs = finish_parallel(e.xIs, e.yIs, e.zIs, xt, yt, zt, w, t, h, ix, iy, iz, dv.fx, dv.fy, dv.fz, 0).x;
     } else {
         const float tio = sqrt_mid(norm2(dy, dx, dz));
         const float rx = div_rn(tio, dx), ry = div_rn(tio, dy), rz = div_rn(tio, dz);
@@ -632,7 +686,7 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, int ix, int iy, i
     // is the largest of the three rounded values; the reciprocal in place of the reference's
     // divisions rounds identically except in double-rounding ties)
     const double rq = 1.0 / ((4.0 * 3.14159265358979323846) * (double)dsq * (double)sq);
-    const float ax = t * h / 8.0f / 16.0f, az = w * t / 8.0f / 16.0f, ay = w * h / 8.0f / 8.0f;
+    const float ax = t * h / dv.fz / dv.fy, az = w * t / dv.fx / dv.fy, ay = w * h / dv.fx / dv.fz;
     const double px = (double)ax * (double)fabsf((xD - e.xI) * e.cosr - (zD - e.zI) * e.sinr);
     const double pz = (double)az * (double)fabsf((xD - e.xI) * e.sinr + (zD - e.zI) * e.cosr);
     const double py = (double)ay * (double)fabsf(yD - e.yI);
@@ -641,27 +695,69 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, int ix, int iy, i
     return eff * sa * absf;
 }
 
+// Work counts of one lane (COUNT instances).
+struct Counts {
+    int hole_hits = 0, cry_hits = 0, blocked = 0, hole_evals = 0, cry_evals = 0;
+    long long entries = 0;
+};
+
+// Attenuation outside crystal d of the rays of rounds [r0, r1), into ws.att.  single: the kept
+// objects k are the element's and ws.mask holds the rounds'; otherwise the list is taken in
+// chunks, each ray's open-layer length carried in ws.len.
+template <bool COUNT, bool ELL, class Div>
+__device__ __forceinline__ void attenuation_pass(const DevGeom& g, RefWarp& ws, const Div& dv, const unsigned short* src,
+                                                 int n_src, int d, bool single, int r0, int r1, int lane, int cursor,
+                                                 Kept& k, Counts& n)
+{
+    const Elem& e = ws.elem;
+    int lay = 0;
+    for (bool first = true;; first = false) {
+        if (!single) {
+            cursor = build_kept(g, src, ws, e, d, first ? 0 : cursor, n_src, lane, k);
+            round_masks(ws, e, k, r0, r1, lane);
+        }
+        const bool last = cursor >= n_src;
+        // this chunk ends the holes when crystals follow or no object does
+        const int lay1 = last || k.nh < k.count ? g.n_layers : (k.nh > 0 ? layer_of_hole(g, ws.id[k.nh - 1]) : lay);
+        if (!ELL && k.even)
+            walk_holes<COUNT, ELL, true>(g, ws, dv, k.nh, r0, r1, first, lay, lay1, !single, lane, n.hole_hits,
+                                         n.hole_evals, n.blocked);
+        else
+            walk_holes<COUNT, ELL, false>(g, ws, dv, k.nh, r0, r1, first, lay, lay1, !single, lane, n.hole_hits,
+                                          n.hole_evals, n.blocked);
+        lay = lay1;
+        if (k.nh < k.count)
+            walk_crystals<COUNT>(g, ws, dv, k.nh, k.count, r0, r1, lane, n.cry_hits, n.cry_evals);
+        if constexpr (COUNT) {
+            for (int r = r0; r < r1; ++r)
+                for (int w = 0; w * 32 < k.count; ++w) n.entries += __popc(ws.mask[w][r]);
+        }
+        __syncwarp();
+        if (last) break;
+    }
+}
+
 // Element (d, v): the reference's float chain over sub-elements in its order (MODE 0) or an FP64
 // sum (MODE 1).
 template <int MODE, bool COUNT, bool ELL>
 __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp& ws, int d, long long v, float cr,
                                  float sr, int lane, unsigned long long* counters)
 {
-    const bool from_super = sup.s_count >= 0;
-    const int n_src = from_super ? sup.s_count : g.n_holes + g.n_det;
+    const unsigned short* src = sup.s_count >= 0 ? sup.sid : nullptr;
+    const int n_src = src ? sup.s_count : g.n_holes + g.n_det;
+    const RefDivision dv;
     int cursor;
     Kept k;
     {
         Elem el;
         if (!init_element(g, ws.inner, d, v, cr, sr, lane, el)) return 0.0;
         if (lane == 0) ws.elem = el;
-        ws.sub[lane] = sub_entry(el, lane);
-        cursor = build_kept(g, sup, ws, el, d, 0, n_src, from_super, lane, k);   // ends in a __syncwarp
+        ws.sub[lane] = RefDivision::entry(el, lane);
+        cursor = build_kept(g, src, ws, el, d, 0, n_src, lane, k);   // ends in a __syncwarp
     }
     const Elem& e = ws.elem;
     round_boxes(ws, e, lane);
-    int n_hole_hits = 0, n_cry_hits = 0, n_blocked = 0, n_hole_evals = 0, n_cry_evals = 0;
-    long long n_entries = 0;
+    Counts n;
     const bool single = cursor >= n_src;
     if (single) round_masks(ws, e, k, 0, 32, lane);
     // an element kept in several chunks goes a quarter at a time, so that the rays' open-layer
@@ -671,37 +767,13 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
     double dacc = 0.0;
     for (int q0 = 0; q0 < 32; q0 += kPassRounds) {
         for (int r0 = q0; r0 < q0 + kPassRounds; r0 += per) {
-            int lay = 0;
-            for (bool first = true;; first = false) {
-                if (!single) {
-                    cursor = build_kept(g, sup, ws, e, d, first ? 0 : cursor, n_src, from_super, lane, k);
-                    round_masks(ws, e, k, r0, r0 + per, lane);
-                }
-                const bool last = cursor >= n_src;
-                // this chunk ends the holes when crystals follow or no object does
-                const int lay1 = last || k.nh < k.count ? g.n_layers : (k.nh > 0 ? layer_of_hole(g, ws.id[k.nh - 1]) : lay);
-                if (!ELL && k.even)
-                    walk_holes<COUNT, ELL, true>(g, ws, k.nh, r0, r0 + per, first, lay, lay1, !single, lane, n_hole_hits,
-                                                 n_hole_evals, n_blocked);
-                else
-                    walk_holes<COUNT, ELL, false>(g, ws, k.nh, r0, r0 + per, first, lay, lay1, !single, lane,
-                                                  n_hole_hits, n_hole_evals, n_blocked);
-                lay = lay1;
-                if (k.nh < k.count)
-                    walk_crystals<COUNT>(g, ws, k.nh, k.count, r0, r0 + per, lane, n_cry_hits, n_cry_evals);
-                if constexpr (COUNT) {
-                    for (int r = r0; r < r0 + per; ++r)
-                        for (int w = 0; w * 32 < k.count; ++w) n_entries += __popc(ws.mask[w][r]);
-                }
-                __syncwarp();
-                if (last) break;
-            }
+            attenuation_pass<COUNT, ELL>(g, ws, dv, src, n_src, d, single, r0, r0 + per, lane, cursor, k, n);
         }
         for (int r = q0; r < q0 + kPassRounds; ++r) {
             int ix, iy, iz;
-            round_indices(r, lane, ix, iy, iz);
+            dv.indices(r, lane, ix, iy, iz);
             const float att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
-            const float c = isinf(att) ? 0.0f : finish_ray(ws, ix, iy, iz, att);
+            const float c = isinf(att) ? 0.0f : finish_ray(ws, dv, ix, iy, iz, att);
             if constexpr (MODE == 0) ws.att[(r & (kPassRounds - 1)) * 32 + lane] = c;
             else dacc += (double)c;
         }
@@ -722,25 +794,25 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
     if constexpr (COUNT) {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
-            n_hole_hits += __shfl_xor_sync(0xffffffffu, n_hole_hits, off);
-            n_cry_hits += __shfl_xor_sync(0xffffffffu, n_cry_hits, off);
-            n_blocked += __shfl_xor_sync(0xffffffffu, n_blocked, off);
-            n_hole_evals += __shfl_xor_sync(0xffffffffu, n_hole_evals, off);
-            n_cry_evals += __shfl_xor_sync(0xffffffffu, n_cry_evals, off);
+            n.hole_hits += __shfl_xor_sync(0xffffffffu, n.hole_hits, off);
+            n.cry_hits += __shfl_xor_sync(0xffffffffu, n.cry_hits, off);
+            n.blocked += __shfl_xor_sync(0xffffffffu, n.blocked, off);
+            n.hole_evals += __shfl_xor_sync(0xffffffffu, n.hole_evals, off);
+            n.cry_evals += __shfl_xor_sync(0xffffffffu, n.cry_evals, off);
         }
         if (lane == 0) {
             atomicAdd(&counters[0], 1024ull);
-            atomicAdd(&counters[1], (unsigned long long)n_hole_hits);
-            atomicAdd(&counters[2], (unsigned long long)n_cry_hits);
+            atomicAdd(&counters[1], (unsigned long long)n.hole_hits);
+            atomicAdd(&counters[2], (unsigned long long)n.cry_hits);
             atomicAdd(&counters[3], 1ull);
-            atomicAdd(&counters[4], (unsigned long long)n_blocked);
+            atomicAdd(&counters[4], (unsigned long long)n.blocked);
             atomicAdd(&counters[5], single ? 0ull : 1ull);                 // chunked elements
             atomicAdd(&counters[6], (unsigned long long)k.count);          // kept objects (last chunk)
-            atomicAdd(&counters[7], (unsigned long long)n_entries);        // entries over all rounds
+            atomicAdd(&counters[7], (unsigned long long)n.entries);        // entries over all rounds
             atomicAdd(&counters[8], sup.s_count < 0 ? 1ull : 0ull);        // superset overflow
             atomicAdd(&counters[9], (unsigned long long)(sup.s_count < 0 ? 0 : sup.s_count));
-            atomicAdd(&counters[10], (unsigned long long)n_hole_evals);
-            atomicAdd(&counters[11], (unsigned long long)n_cry_evals);
+            atomicAdd(&counters[10], (unsigned long long)n.hole_evals);
+            atomicAdd(&counters[11], (unsigned long long)n.cry_evals);
         }
     }
     if constexpr (MODE == 0) {
@@ -750,4 +822,122 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
         for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
         return dacc;
     }
+}
+
+__device__ __forceinline__ float warp_min(float x)
+{
+    float y;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float warp_max(float x)
+{
+    float y;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// ws.box and ws.reach of the first n rounds, from the rays themselves.
+template <class Div>
+__device__ __forceinline__ void ray_boxes(RefWarp& ws, const Div& dv, int n, int lane)
+{
+    const Elem& e = ws.elem;
+    for (int r = 0; r < n; ++r) {
+        int ix, iy, iz;
+        dv.indices(r, lane, ix, iy, iz);
+        const float3 q = dv.centre(ws, ix, iy, iz);
+        float x, y, z;
+        ray_end(e, q.x, q.y, q.z, x, y, z);
+        const float rdy = e.filt ? rcp_approx(y - e.yI) : 0.0f;
+        const float a = (x - e.xI) * rdy, b = (z - e.zI) * rdy;
+        const float4 box = make_float4(warp_min(a), warp_max(a), warp_min(b), warp_max(b));
+        if (lane == 0) {
+            const float px = fmaxf(fabsf(box.x), fabsf(box.y)), pz = fmaxf(fabsf(box.z), fabsf(box.w));
+            ws.box[r] = box;
+            ws.reach[r] = sqrtf(px * px + pz * pz);
+        }
+    }
+    __syncwarp();
+}
+
+// Element of the sampled form: the mean over the voxel's sx x sy x sz source points (centres of
+// a grid over the voxel) of the reference's element with crystal d divided into nx x ny x nz
+// sub-elements (x, depth, z), every contribution summed in FP64.  Each source point has its own
+// cone test and kept objects, drawn from one list per voxel of the objects near the ray bundle of
+// any source point (a few percent of the block's superset).  With 8 x 16 x 8 and 1 x 1 x 1 it runs
+// pe_element_ref<1>'s float program, summed in another order.
+template <bool ELL>
+__device__ double pe_element_sampled(const DevGeom& g, const Superset& sup, RefWarp& ws, int d, long long v, float cr,
+                                     float sr, int lane, const Sampling& sm)
+{
+    const int n_pts = sm.sx * sm.sy * sm.sz;
+    AnyDivision dv{sm.nx, sm.ny, sm.nx * sm.ny * sm.nz, 0, (float)sm.nx, (float)sm.ny, (float)sm.nz};
+    const int n_rounds = (dv.n_sub + 31) / 32;
+    const unsigned short* src = sup.s_count >= 0 ? sup.sid : nullptr;
+    int n_src = src ? sup.s_count : g.n_holes + g.n_det;
+    double dacc = 0.0;
+    if (src && n_pts > 1) {               // the voxel's list
+        Elem el;
+        if (!init_element(g, ws.inner, d, v, cr, sr, lane, el)) return 0.0;
+        const float hx = 0.5f * (fabsf(g.wx) + fabsf(g.wy)), hz = 0.5f * fabsf(g.wz);
+        // slope rectangle of crystal d's bounding cylinder from any source point
+        const float r = 0.5f * sqrtf(el.w * el.w + el.h * el.h) + hx, rz = 0.5f * sqrtf(el.w * el.w + el.h * el.h) + hz;
+        const float y0 = el.yd - 0.5f * el.t - el.yI - hx, y1 = el.yd + 0.5f * el.t - el.yI + hx;
+        if (y0 >= kMinDepth) {
+            const float r0 = 1.0f / y0, r1 = 1.0f / y1, x = el.xd - el.xI, z = el.zd - el.zI;
+            const float4 rd = make_float4(fminf((x - r) * r0, (x - r) * r1) - kSlopeMargin,
+                                          fmaxf((x + r) * r0, (x + r) * r1) + kSlopeMargin,
+                                          fminf((z - rz) * r0, (z - rz) * r1) - kSlopeMargin,
+                                          fmaxf((z + rz) * r0, (z + rz) * r1) + kSlopeMargin);
+            int n = 0;
+            for (int base = 0; base < n_src && n <= kNear; base += 32) {
+                const int j = base + lane;
+                const int id = j < n_src ? src[j] : 0;
+                const bool maybe = j < n_src && near_bundle(g, el, rd, id, hx, hz);
+                const unsigned m = __ballot_sync(0xffffffffu, maybe);
+                const int pos = n + __popc(m & ((1u << lane) - 1u));
+                if (maybe && pos < kNear) ws.near[pos] = (unsigned short)id;
+                n += __popc(m);
+            }
+            if (n <= kNear) {             // otherwise every source point filters the superset
+                src = ws.near;
+                n_src = n;
+            }
+        }
+    }
+    for (int p = 0; p < n_pts; ++p) {
+        const int jx = p % sm.sx, jy = (p / sm.sx) % sm.sy, jz = p / (sm.sx * sm.sy);
+        __syncwarp();                     // the previous point's records are no longer read
+        int cursor;
+        Kept k;
+        {
+            Elem el;
+            if (!init_element(g, ws.inner, d, v, cr, sr, lane, el, ((float)jx + 0.5f) / (float)sm.sx,
+                              ((float)jy + 0.5f) / (float)sm.sy, ((float)jz + 0.5f) / (float)sm.sz))
+                return 0.0;               // the crystal's mu does not depend on the point
+            if (lane == 0) ws.elem = el;
+            cursor = build_kept(g, src, ws, el, d, 0, n_src, lane, k);   // ends in a __syncwarp
+        }
+        const bool single = cursor >= n_src;
+        const int per = single ? kPassRounds : 8;
+        Counts unused;
+        for (int q0 = 0; q0 < n_rounds; q0 += per) {
+            const int n = min(per, n_rounds - q0);
+            dv.base = 32 * q0;
+            ray_boxes(ws, dv, n, lane);
+            if (single) round_masks(ws, ws.elem, k, 0, n, lane);
+            attenuation_pass<false, ELL>(g, ws, dv, src, n_src, d, single, 0, n, lane, cursor, k, unused);
+            for (int r = 0; r < n; ++r) {
+                int ix, iy, iz;
+                dv.indices(r, lane, ix, iy, iz);
+                const float att = ws.att[r * 32 + lane];
+                if (!isinf(att)) dacc += (double)finish_ray(ws, dv, ix, iy, iz, att);
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
+    return dacc / (double)n_pts;
 }
