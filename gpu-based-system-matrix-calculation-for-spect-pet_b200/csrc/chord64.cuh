@@ -125,68 +125,43 @@ __device__ __forceinline__ double box_chord_inside64(double xi, double yi, doubl
     return tmax - tmin;
 }
 
-// Terms of the cylinder chord (:688-799) that depend only on the ray (the ray's start point
-// is passed to each call: it is shared by a warp's rays and kept outside this per-lane state).
-struct RayCyl64 {
-    double tio, kx, kz, rx, rz, kk, ikk, iky;
-};
-
-__device__ __forceinline__ void ray_cyl64_init(RayCyl64& c, double xi, double yi, double zi, double xo, double yo,
-                                               double zo)
+// Out of line, for rays along an axis and other rare cases of the phases' loops.
+static __device__ __noinline__ double box_full64_call(double xi, double yi, double zi, double xo, double yo, double zo,
+                                                      double x1, double y1, double z1, double x2, double y2, double z2)
 {
-    const double dx = xo - xi, dy = yo - yi, dz = zo - zi;
-    c.tio = sqrt(dx * dx + dy * dy + dz * dz);
-    const double it = 1.0 / c.tio;
-    c.kx = dx * it;
-    const double ky = dy * it;
-    c.kz = dz * it;
-    c.iky = 1.0 / ky;
-    c.rx = c.kx * c.iky;
-    c.rz = c.kz * c.iky;
-    c.kk = c.kx * c.kx + c.kz * c.kz;
-    c.ikk = 1.0 / c.kk;
+    return box_chord64(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2);
 }
 
-// Chord through the y-parallel cylinder (x - xc)^2 + (z - zc)^2 <= r^2, y in [y1, y2].
-// The reference picks one of four entry/exit pairs from the cap tests fl, fr and then checks
-// the pair against the cap planes (:730-791).  Where fl, fr and the side crossings t1, t2
-// agree, every pair is the overlap [max(t1, ta), min(t2, tb)] of the side and cap intervals;
-// at a tie (the ray crossing a cap plane exactly on the rim) the cap test and the side
-// crossing are decided by independent roundings and the reference's pair can drop the
-// whole chord.  This form takes the overlap, which is continuous there, and keeps the
-// reference's thresholds.
-__device__ __forceinline__ double ray_cyl64_chord(const RayCyl64& c, double xi, double yi, double zi, double xc,
-                                                  double y1, double y2, double zc, double r)
+static __device__ __noinline__ double box_chord64_call(double xi, double yi, double zi, double xo, double yo, double zo,
+                                                       double w, double t, double h)
 {
-    if (fabs(y1 - y2) < 0.001) return 0.0;
-    const double xl = xi + c.rx * (y1 - yi), xr = xi + c.rx * (y2 - yi);
-    const double zl = zi + c.rz * (y1 - yi), zr = zi + c.rz * (y2 - yi);
-    const double ta = (y1 - yi) * c.iky, tb = (y2 - yi) * c.iky;
-    const bool fl = (xl - xc) * (xl - xc) + (zl - zc) * (zl - zc) <= r * r;
-    const bool fr = (xr - xc) * (xr - xc) + (zr - zc) * (zr - zc) <= r * r;
-    if (fl && fr) {
-        if (ta <= 0.0001 || tb <= 0.0001) return 0.0;
-        if (ta >= c.tio || tb >= c.tio) return 0.0;
-        return fabs(tb - ta);
-    }
-    const double ox = xi - xc, oz = zi - zc;
-    const double cr = c.kx * oz - c.kz * ox;
-    const double disc = c.kk * r * r - cr * cr;
-    if (disc <= 0.00001) return 0.0;
-    const double b = -(c.kx * ox + c.kz * oz), sd = sqrt(disc);
-    const double t1 = (b - sd) * c.ikk, t2 = (b + sd) * c.ikk;
-    const double ea = t1 > ta ? t1 : ta, eb = t2 < tb ? t2 : tb;
-    if (!(eb > ea)) return 0.0;                             // side crossings outside the caps
-    if (eb <= 0.0001 || ea <= 0.0001) return 0.0;
-    if (eb >= c.tio || ea >= c.tio) return 0.0;
-    return eb - ea;
+    return box_chord64(xi, yi, zi, xo, yo, zo, -0.5 * w, -0.5 * t, -0.5 * h, 0.5 * w, 0.5 * t, 0.5 * h);
 }
+
+static __device__ __noinline__ double box_inside64_call(double xi, double yi, double zi, double xo, double yo, double zo,
+                                                        double x1, double y1, double z1, double x2, double y2, double z2)
+{
+    return box_chord_inside64(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2);
+}
+
+static __device__ __noinline__ double plate_chord64(double xi, double yi, double zi, double xo, double yo, double zo,
+                                                    const double* Ly)
+{
+    return box_chord64(xi, yi, zi, xo, yo, zo, Ly[0], Ly[2], Ly[4], Ly[1], Ly[3], Ly[5]);
+}
+
+// The cylinder chord (:688-799) in double (Mode64::hole, pe_fp64.cuh) takes the overlap [max(t1,
+// ta), min(t2, tb)] of the side and cap intervals.  The reference picks one of four entry/exit pairs
+// from the cap tests fl, fr and then checks the pair against the cap planes (:730-791).  Where fl,
+// fr and the side crossings t1, t2 agree, every pair is that overlap; at a tie (the ray crossing a
+// cap plane exactly on the rim) the cap test and the side crossing are decided by independent
+// roundings and the reference's pair can drop the whole chord.  The overlap is continuous there;
+// the reference's thresholds are kept.
 
 // Elliptical cylinder ((x' - xc)/rx)^2 + ((z' - zc)/rz)^2 <= 1, y in [y1, y2], with the
 // segment's points rotated by theta about the axis first (PESysMatGen.cu:801-947, defined but
 // not called by the reference kernels); ct, st = cos(theta), sin(theta).  The expressions are
-// the reference's in double; the ending takes the overlap of the side and cap intervals, as
-// ray_cyl64_chord does.
+// the reference's in double; the ending takes the overlap of the side and cap intervals.
 __device__ __forceinline__ double ell_chord64(double xi, double yi, double zi, double xo, double yo, double zo,
                                               double xc, double y1, double y2, double zc, double rx, double rz,
                                               double ct, double st)
@@ -221,6 +196,13 @@ __device__ __forceinline__ double ell_chord64(double xi, double yi, double zi, d
     if (eb <= 0.0001 || ea <= 0.0001) return 0.0;
     if (eb >= tio || ea >= tio) return 0.0;
     return eb - ea;
+}
+
+static __device__ __noinline__ double ell_chord64_call(double xi, double yi, double zi, double xo, double yo, double zo,
+                                                       double xc, double y1, double y2, double zc, double rx, double rz,
+                                                       double ct, double st)
+{
+    return ell_chord64(xi, yi, zi, xo, yo, zo, xc, y1, y2, zc, rx, rz, ct, st);
 }
 
 }  // namespace sysmat

@@ -225,27 +225,6 @@ __device__ int build_chunk(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, 
     return cursor < n_src ? cursor : n_src;
 }
 
-// Attenuation walk state of one lane (one sub-element).
-struct Walk {
-    float att;      // accumulated mu * L
-    float len;      // hole chord sum of the current layer
-    int lay;        // current layer
-    int hole_hits;  // non-zero hole chords (work counters only)
-    int cry_hits;   // non-zero crystal chords (work counters only)
-    int hole_evals; // hole chords evaluated (work counters only)
-    int cry_evals;  // crystal chords evaluated (work counters only)
-};
-
-__device__ __forceinline__ void close_layers(const DevGeom& g, Walk& s, int upto, float cosang)
-{
-    while (s.lay < upto) {                                    // :1281-1284
-        const float lcol = g.layer[s.lay].thickness / cosang;
-        if ((lcol - s.len) >= 0.00001f) s.att = s.att + g.layer[s.lay].mu_total * (lcol - s.len);
-        s.len = 0.0f;
-        ++s.lay;
-    }
-}
-
 // Terms of the reference cylinder chord (PESysMatGen.cu:688-799) that depend only on the
 // ray (voxel -> sub-element) and on the cap planes y1, y2.  Hoisting them out of the
 // per-hole evaluation keeps every float identical: each is the same operation on the same
@@ -369,27 +348,11 @@ __device__ __forceinline__ bool capsule_meets_box(float xo, float zo, float y0, 
     return capsule_meets_box(capsule_of(xo, zo, y0, y1, R, e), box);
 }
 
-// Lane test of a hole entry of the round buffer: is the ray's slope (sa, sb) within the
-// hole's capsule?  c = (c(y0), c(y1) - c(y0)), rho2 = radius^2 (infinite for an entry without
-// a capsule: the hole is closer than kMinDepth to the voxel), inv_len2 = 1/|c(y1) - c(y0)|^2
-// (0 for a degenerate segment).
-__device__ __forceinline__ bool in_capsule(const float4& c, float rho2, float inv_len2, float sa, float sb)
-{
-    const float px = sa - c.x, pz = sb - c.y;
-    const float t = fminf(fmaxf((px * c.z + pz * c.w) * inv_len2, 0.0f), 1.0f);
-    const float ex = px - t * c.z, ez = pz - t * c.w;
-    return ex * ex + ez * ez <= rho2;
-}
-
 // Copy kept entries [k0, k1) whose rectangle and capsule meet the round's slope box into
 // the round buffer from position n, with their geometry (one entry per lane); returns the
 // new count.  Stops before the buffer could overflow; *next receives the first entry not
-// examined.  IDS: store each entry's object id (as the bits of ra.x) instead of its float
-// geometry, for walks that read their own geometry tables (FP64 mode), and a hole entry's
-// capsule in place of its rectangle for the lanes' test (hole_in_reach).  The float walks
-// test the rectangle: the warp runs an entry's chord whenever any lane needs it, and the
-// tighter lane test measured slower there (its cost without fewer warp-level evaluations).
-template <bool ELL, bool IDS = false>
+// examined.
+template <bool ELL>
 __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const Elem& e, int k0, int k1,
                                           float4 box, int n, int lane, int* next, int* nh)
 {
@@ -399,9 +362,6 @@ __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const 
         bool keep = false;
         int id = 0;
         float4 rect;
-        // hole entries carry their capsule for the lanes' test (none: every slope passes)
-        float4 cap = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float rho2 = INFINITY, inv_len2 = 0.0f;
         if (kk < k1) {
             rect = ws.rect[kk];
             keep = rects_overlap(rect, box);
@@ -411,10 +371,6 @@ __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const 
                     const float4 ha = __ldg(&g.hole.a[id]);
                     const Capsule c = capsule_of(ha.x, ha.w, ha.y, ha.z, __ldg(&g.hole.b[id].x), e);
                     keep = capsule_meets_box(c, box);
-                    cap = make_float4(c.ax, c.az, c.dx, c.dz);
-                    rho2 = c.rho * c.rho;
-                    const float l2 = c.dx * c.dx + c.dz * c.dz;
-                    inv_len2 = l2 > 1e-30f ? __frcp_rn(l2) : 0.0f;
                 } else {
                     const int o = id - g.n_holes;
                     const float4 po = __ldg(&g.cry.pos[o]);
@@ -429,12 +385,7 @@ __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const 
         *nh += __popc(__ballot_sync(0xffffffffu, keep && id < g.n_holes));
         if (keep) {
             const int pos = n + __popc(m & ((1u << lane) - 1u));
-            if constexpr (IDS) {
-                ws.rr[pos] = id < g.n_holes ? cap : rect;
-                ws.rb[pos] = make_float4(0.0f, 0.0f, rho2, inv_len2);
-                ws.ra[pos].x = __int_as_float(id);
-                ws.rl[pos] = id < g.n_holes ? layer_of_hole(g, id) : g.n_layers;
-            } else if (id < g.n_holes) {
+            if (id < g.n_holes) {
                 const float4 ha = __ldg(&g.hole.a[id]);
                 const float4 hb = __ldg(&g.hole.b[id]);
                 ws.rr[pos] = rect;
@@ -464,87 +415,6 @@ __device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const 
     __syncwarp();
     *next = k < k1 ? k : k1;
     return n;
-}
-
-// Lane test of round-buffer hole entry j of a fill_round<…, IDS> buffer (see in_capsule).
-__device__ __forceinline__ bool hole_in_reach(const WarpSmem& ws, int j, float sa, float sb)
-{
-    const float4 b = ws.rb[j];
-    return in_capsule(ws.rr[j], b.z, b.w, sa, sb);
-}
-
-// Walk round-buffer entries [0, nr) for one sub-element ray (voxel -> (xD, yD, zD)); holes
-// occupy [0, nh) and crystals [nh, nr), both in the reference's object order; the layer
-// terms are added when the walk leaves a layer.  Called by the whole warp: a lane without a
-// ray passes live = false and takes part with no entry, so every branch on an entry is
-// uniform.  Holes go two at a time when they share layer and cap planes (independent
-// straight-line chords: the serial chain of one chord leaves issue slots idle); a lane that an
-// entry does not concern adds an exact zero.
-template <bool ELL>
-__device__ __forceinline__ void walk_round(const DevGeom& g, const WarpSmem& ws, int nh, int nr,
-                                           float xD, float yD, float zD, float sa_a, float sa_b,
-                                           float cosang, bool live, RayCyl& rc, Walk& s)
-{
-    for (int j = 0; j < nh;) {
-        const int m = ws.rl[j];
-        const float4 A = ws.ra[j];
-        const float4 B = ws.rb[j];
-        if (m != s.lay) close_layers(g, s, m, cosang);
-        const bool in = live && in_rect(ws.rr[j], sa_a, sa_b);
-        if constexpr (ELL) {
-            ++j;
-            if (!__any_sync(0xffffffffu, in)) continue;
-            const float4 S = ws.rc[j - 1];
-            float tmp = 0.0f;
-            if (S.x > 0.0f) {                                    // elliptical hole
-                if (in) tmp = ell_chord(rc.xi, rc.yi, rc.zi, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w);
-            } else {
-                ray_cyl_caps(rc, B.x, B.y);
-                if (in) tmp = ray_cyl_chord(rc, A.x, A.y, A.z, B.z, B.w);
-            }
-            s.len = s.len + tmp;                                 // :1276-1278
-            s.att = s.att + A.w * tmp;
-            s.hole_hits += (tmp != 0.0f);
-            s.hole_evals += in;
-        } else {
-            const int k = j + 1 < nh ? j + 1 : j;
-            const float4 A2 = ws.ra[k];
-            const float4 B2 = ws.rb[k];
-            const bool pair = k > j && ws.rl[k] == m && B2.x == B.x && B2.y == B.y;
-            const bool in2 = pair && live && in_rect(ws.rr[k], sa_a, sa_b);
-            j = pair ? j + 2 : j + 1;
-            if (!__any_sync(0xffffffffu, in || in2)) continue;
-            ray_cyl_caps(rc, B.x, B.y);
-            float tmp = ray_cyl_chord(rc, A.x, A.y, A.z, B.z, B.w);
-            float tmp2 = ray_cyl_chord(rc, A2.x, A2.y, A2.z, B2.z, B2.w);
-            tmp = in ? tmp : 0.0f;
-            tmp2 = in2 ? tmp2 : 0.0f;
-            s.len = s.len + tmp;                                 // :1276-1278
-            s.att = s.att + A.w * tmp;
-            s.len = s.len + tmp2;
-            s.att = s.att + A2.w * tmp2;
-            s.hole_hits += (tmp != 0.0f) + (tmp2 != 0.0f);
-            s.hole_evals += in + in2;
-        }
-    }
-    if (nr <= nh) return;
-    if (s.lay < g.n_layers) close_layers(g, s, g.n_layers, cosang);
-    for (int j = nh; j < nr; ++j) {
-        const bool in = live && in_rect(ws.rr[j], sa_a, sa_b);
-        if (!__any_sync(0xffffffffu, in)) continue;
-        const float4 A = ws.ra[j];
-        const float4 B = ws.rb[j];
-        const float4 C = ws.rc[j];
-        float xb, yb, zb;                                        // :1318-1320
-        to_crystal_frame(A.x, A.y, A.z, B.x, B.y, xD, yD, zD, xb, yb, zb);
-        float la = 0.0f;
-        if (in)
-            la = box_chord(C.y, C.z, C.w, xb, yb, zb, -0.5f * B.z, -0.5f * B.w, -0.5f * C.x, 0.5f * B.z, 0.5f * B.w,
-                           0.5f * C.x);
-        s.att = s.att + la * A.w;
-        s.cry_hits += (la != 0.0f);
-        s.cry_evals += in;
-    }
 }
 
 struct SubElem {
@@ -607,41 +477,6 @@ __device__ __forceinline__ bool plate_penalty(const DevGeom& g, const float4* pl
     return blocked;
 }
 
-// Self attenuation, absorption and solid angle for a sub-element of an fx x fy x fz
-// division, given the attenuation accumulated outside crystal d (:1223-1231, :1329-1357).
-__device__ __forceinline__ float finish_sub_element_at(const Elem& e, const SubElem& q, float att, float fx,
-                                                       float fy, float fz)
-{
-    const float w = e.w, t = e.t, h = e.h;
-    const float ux1 = ((float)q.ix / fx - 0.5f) * w;
-    const float ux2 = (((float)q.ix + 1.0f) / fx - 0.5f) * w;
-    const float uy1 = ((float)q.iy / fy - 0.5f) * t;
-    const float uy2 = (((float)q.iy + 1.0f) / fy - 0.5f) * t;
-    const float uz1 = ((float)q.iz / fz - 0.5f) * h;
-    const float uz2 = (((float)q.iz + 1.0f) / fz - 0.5f) * h;
-    const float cbox[6] = {-w / 2.0f, -t / 2.0f, -h / 2.0f, w / 2.0f, t / 2.0f, h / 2.0f};
-    const float ubox[6] = {ux1, uy1, uz1, ux2, uy2, uz2};
-    float l1, l2;
-    box_chord_inside2(e.xIs, e.yIs, e.zIs, q.xDs, q.yDs, q.zDs, cbox, ubox, l1, l2);
-    att = att + (l1 - l2) * e.mu_t;
-    const float eff = 1.0f * expf(-att);
-    const float xt = q.xDs + 1000.0f * (q.xDs - e.xIs) / q.sq;
-    const float yt = q.yDs + 1000.0f * (q.yDs - e.yIs) / q.sq;
-    const float zt = q.zDs + 1000.0f * (q.zDs - e.zIs) / q.sq;
-    const float labs = box_chord(e.xIs, e.yIs, e.zIs, xt, yt, zt, ux1, uy1, uz1, ux2, uy2, uz2);
-    const float absf = (1.0f - expf(-labs * e.mu_t)) * e.mu_pe / e.mu_t;
-    // solid angle in double, as the reference's 4*M_PI promotion makes it; one shared
-    // reciprocal (the float results round identically except in double-rounding ties)
-    const double rq = 1.0 / ((4.0 * 3.14159265358979323846) * (double)q.dsq * (double)q.sq);
-    const float ax = t * h / fz / fy, az = w * t / fx / fy, ay = w * h / fx / fz;
-    const float sax = (float)((double)ax * (double)fabsf((q.xD - e.xI) * e.cosr - (q.zD - e.zI) * e.sinr) * rq);
-    const float saz = (float)((double)az * (double)fabsf((q.xD - e.xI) * e.sinr + (q.zD - e.zI) * e.cosr) * rq);
-    const float say = (float)((double)ay * (double)fabsf(q.yD - e.yI) * rq);
-    const float sxy = (sax >= say) ? sax : say;
-    const float sa = (sxy >= saz) ? sxy : saz;
-    return eff * sa * absf;
-}
-
 // Per-element set-up shared by the lanes of a warp: voxel centre, crystal d, reference cone
 // constants, slope rectangle and the plate "through both faces" rectangles.  False when the
 // crystal's attenuation is too low for the reference to compute the element (it is 0).
@@ -689,76 +524,6 @@ __device__ __forceinline__ bool init_element(const DevGeom& g, float4* plate_inn
     }
 
     return true;
-}
-
-// Kept-list state of one element (source point) of a warp: the first chunk's end, whether the
-// whole list fits one chunk, and the current chunk's entry count.
-struct KeptList {
-    int n_src, cursor, count;
-    bool from_super, single;
-};
-
-__device__ __forceinline__ KeptList start_kept_list(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws,
-                                                    const Elem& e, int d, int lane)
-{
-    KeptList k;
-    k.from_super = bs.s_count >= 0;
-    k.n_src = k.from_super ? bs.s_count : g.n_holes + g.n_det;
-    k.count = 0;
-    k.cursor = build_chunk(g, bs, ws, e, d, 0, k.n_src, k.from_super, lane, &k.count);
-    k.single = k.cursor >= k.n_src;
-    return k;
-}
-
-// Attenuation outside crystal d along the ray of sub-element q, into s: plate penalty, then
-// the kept objects that meet the round's slope box, walked in round buffers (an overfull
-// round in pieces: each lane's walk state carries over, so the attenuation order is kept).
-// Returns whether the lane skips the sub-element: `dead`, or blocked with every mu >= 0 (the
-// contribution is then exactly 0).  Used by the sampled form; pe_element keeps the same walk
-// inline (through this helper the reference-order kernel measured 1.5 % slower).
-template <bool COUNT, bool ELL>
-__device__ __forceinline__ bool walk_sub_element(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws,
-                                                 const Elem& e, int d, const SubElem& q, bool dead,
-                                                 bool first_round, KeptList& kl, int lane, Walk& s,
-                                                 long long& n_sub_entries)
-{
-    RayCyl rc;
-    ray_cyl_init(rc, e.xI, e.yI, e.zI, q.xD, q.yD, q.zD);
-    const bool blocked = plate_penalty(g, ws.inner, e, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, s.att);
-    const bool skip = dead || (blocked && g.nonneg_mu);
-    // slope box of the rays that still need the walk in this round
-    float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
-                             skip ? INFINITY : q.sa_b, skip ? -INFINITY : q.sa_b);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, off));
-        box.y = fmaxf(box.y, __shfl_xor_sync(0xffffffffu, box.y, off));
-        box.z = fminf(box.z, __shfl_xor_sync(0xffffffffu, box.z, off));
-        box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, off));
-    }
-    int cur = 0;
-    bool first_chunk = true;
-    while (true) {
-        if (!kl.single && !first_chunk) {
-            cur = build_chunk(g, bs, ws, e, d, cur, kl.n_src, kl.from_super, lane, &kl.count);
-        } else if (!kl.single) {
-            if (!first_round) cur = build_chunk(g, bs, ws, e, d, 0, kl.n_src, kl.from_super, lane, &kl.count);
-            else cur = kl.cursor;
-        }
-        first_chunk = false;
-        int k = 0;
-        while (k < kl.count) {
-            int next = kl.count, nh = 0;
-            const int nr = fill_round<ELL>(g, ws, e, k, kl.count, box, 0, lane, &next, &nh);
-            if constexpr (COUNT) n_sub_entries += nr;
-            walk_round<ELL>(g, ws, nh, nr, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, q.cosang, !skip, rc, s);
-            __syncwarp();
-            k = next;
-        }
-        if (kl.single || cur >= kl.n_src) break;
-    }
-    if (!skip && s.lay < g.n_layers) close_layers(g, s, g.n_layers, q.cosang);
-    return skip;
 }
 
 #include "pe_ref.cuh"
@@ -827,14 +592,12 @@ struct BrickOut {
     int det_count;
 };
 
-// Shared memory and blocks per SM of each kernel instance (pe_ref.cuh for the float modes 0, 1).
-template <int MODE, bool SAMPLED>
-struct Shape {
-    static constexpr bool ref = MODE <= 1;
-    static constexpr int blocks = ref ? kRefBlocks : 2;
-    using Smem = typename std::conditional<ref, RefSmem, BlockSmem>::type;
-};
-__device__ __forceinline__ Superset& superset_of(RefSmem& sm) { return sm.sup; }
+// Shared memory of each kernel instance; two blocks of kWarps warps per SM.
+template <int MODE, bool ELL> struct SmemOf { using type = RefSmem; };       // float modes 0, 1
+template <bool ELL> struct SmemOf<2, ELL> { using type = IdSmem<Mode64>; };
+template <bool ELL> struct SmemOf<3, ELL> { using type = IdSmem<ModeLocal<ELL>>; };
+template <class Smem>
+__device__ __forceinline__ Superset& superset_of(Smem& sm) { return sm.sup; }
 __device__ __forceinline__ Superset& superset_of(BlockSmem& sm) { return sm; }
 
 // One work item: crystal det_begin + di against one voxel brick of bx x by x bz voxels (brick
@@ -843,7 +606,7 @@ __device__ __forceinline__ Superset& superset_of(BlockSmem& sm) { return sm; }
 // SAMPLED: elements of the sampled form `smp` (source points anywhere in the voxels: the
 // superset radius grows by half a voxel diagonal).
 template <int MODE, bool COUNT, bool ELL = false, bool SAMPLED = false>
-__device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, SAMPLED>::Smem& sm, int lane, int wid,
+__device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE, ELL>::type& sm, int lane, int wid,
                                          const BrickOut& O, int di, int gx, int gy, int gz, int iz0, int iz1,
                                          int bx, int by, int bz, float cr, float sr,
                                          unsigned long long* counters, const Sampling* smp = nullptr,
@@ -877,9 +640,9 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, 
                 float* so = nullptr;
                 if (SAMPLED && O.sub_out)
                     so = O.sub_out + ((v - O.vox_begin) * O.det_count + di) * (long long)(smp->nx * smp->ny * smp->nz);
-                val = (float)pe_element_local<ELL, SAMPLED>(g, sm, sm.w[wid], d, v, cr, sr, rotation, lane, smp, so);
+                val = (float)pe_element_local<ELL, SAMPLED>(g, sup, sm.w[wid], d, v, cr, sr, rotation, lane, smp, so);
             } else {
-                val = (float)pe_element64(g, sm, sm.w[wid], d, v, cr, sr, rotation, lane);
+                val = (float)pe_element64(g, sup, sm.w[wid], d, v, cr, sr, rotation, lane);
             }
             if (lane == 0) O.out[(long long)di * O.ld + (v - O.vox_begin)] = val;
             __syncwarp();
@@ -889,11 +652,11 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename Shape<MODE, 
 }
 
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
-__global__ void __launch_bounds__(kThreads, Shape<MODE, SAMPLED>::blocks)
+__global__ void __launch_bounds__(kThreads, 2)
 pe_kernel(DevGeom g, PeLaunch L)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    auto& sm = *reinterpret_cast<typename Shape<MODE, SAMPLED>::Smem*>(smem_raw);
+    auto& sm = *reinterpret_cast<typename SmemOf<MODE, ELL>::type*>(smem_raw);
     Superset& bs = superset_of(sm);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float ang = L.rotation * g.angle_step;           // :1006
@@ -925,9 +688,9 @@ pe_kernel(DevGeom g, PeLaunch L)
 
 // Shared memory of the batched kernel: the block's working set plus the geometry of the
 // task in hand (copied in when the block moves to a task of another geometry).
-template <int MODE>
+template <int MODE, bool ELL>
 struct BatchSmem {
-    typename Shape<MODE, false>::Smem bs;
+    typename SmemOf<MODE, ELL>::type bs;
     DevGeom g;
     int task;
 };
@@ -936,10 +699,10 @@ struct BatchSmem {
 // tasks, taken from one work counter; a block finds its item's task by binary search over
 // the tasks' first item numbers.
 template <int MODE, bool ELL>
-__global__ void __launch_bounds__(kThreads, Shape<MODE, false>::blocks) pe_batch_kernel(BatchLaunch B)
+__global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BatchSmem<MODE>& sm = *reinterpret_cast<BatchSmem<MODE>*>(smem_raw);
+    BatchSmem<MODE, ELL>& sm = *reinterpret_cast<BatchSmem<MODE, ELL>*>(smem_raw);
     Superset& bs = superset_of(sm.bs);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int cur_geom = -1;
@@ -989,7 +752,7 @@ __global__ void __launch_bounds__(kThreads, Shape<MODE, false>::blocks) pe_batch
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
 static int launch_mode(const DevGeom& g, const PeLaunch& L, int num_sms, cudaStream_t stream)
 {
-    const int smem = (int)sizeof(typename Shape<MODE, SAMPLED>::Smem);
+    const int smem = (int)sizeof(typename SmemOf<MODE, ELL>::type);
     static unsigned long long configured = 0;   // one bit per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -1045,7 +808,7 @@ int launch_pe_adjoint(const DevGeom& g, const AdjLaunch& L, int kind, int num_sm
 template <int MODE, bool ELL>
 static int configure_batch_mode(int* per_sm)
 {
-    const int smem = (int)sizeof(BatchSmem<MODE>);
+    const int smem = (int)sizeof(BatchSmem<MODE, ELL>);
     static unsigned long long configured = 0;   // one bit per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -1078,7 +841,7 @@ int configure_pe_batch(int mode, bool ell, int* blocks_per_sm)
 template <int MODE, bool ELL>
 static void launch_batch_mode(const BatchLaunch& B, int grid, cudaStream_t stream)
 {
-    pe_batch_kernel<MODE, ELL><<<grid, kThreads, (int)sizeof(BatchSmem<MODE>), stream>>>(B);
+    pe_batch_kernel<MODE, ELL><<<grid, kThreads, (int)sizeof(BatchSmem<MODE, ELL>), stream>>>(B);
 }
 
 int launch_pe_batch(const BatchLaunch& B, int mode, bool ell, int grid, cudaStream_t stream)

@@ -305,11 +305,8 @@ __device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSme
 
 // Projections run the reference-order element (pe_ref.cuh), the gradient its own.
 template <int KIND>
-using AdjShape = Shape<KIND == 1 ? 2 : 1, false>;
-
-template <int KIND>
 struct AdjSmem {
-    typename AdjShape<KIND>::Smem bs;
+    typename std::conditional<KIND == 1, BlockSmem, RefSmem>::type bs;
     double acc[KIND == 1 ? kWarps : 1][kThetaN + 1];
     int any;
 };
@@ -319,7 +316,7 @@ struct AdjSmem {
 // KIND 2: q[v] += sum_d A[d,v] u[d - det_begin] (back projection; x is not read).
 // Elements of zero weight are skipped, and so are bricks whose voxels all have x = 0.
 template <int KIND, bool ELL>
-__global__ void __launch_bounds__(kThreads, AdjShape<KIND>::blocks) pe_adjoint_kernel(DevGeom g, AdjLaunch L)
+__global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjLaunch L)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     AdjSmem<KIND>& sm = *reinterpret_cast<AdjSmem<KIND>*>(smem_raw);

@@ -59,255 +59,274 @@ __device__ __forceinline__ void init_elem64(const DevGeom& g, int d, long long v
     E.uz = (E.zd - E.zI) / dist;
 }
 
-// Cone test of object i (:1120-1184) in double, then the float bundle filter.
-__device__ __forceinline__ bool keep_object64(const DevGeom& g, const Elem& e, const Elem64& E, int i, int d,
-                                              float4& rect)
-{
-    rect = open_rect();
-    double ox, oy, oz, crit;
-    if (i < g.n_holes) {
-        const D4 a = g.t64.hole_a[i], b = g.t64.hole_b[i];
-        ox = a.x; oy = b.z; oz = a.w;
-        crit = b.w;
-    } else {
-        const int o = i - g.n_holes;
-        if (o == d) return false;
-        const D4 P = g.t64.cry_pos[o], S = g.t64.cry_size[o];
-        ox = P.x; oy = P.y; oz = P.z;
-        crit = sqrt(S.x * S.x + S.z * S.z + S.y * S.y) / 2.0;
+#include "pe_ids.cuh"
+
+// The mode's phases (pe_ids.cuh).  Divisions become reciprocals (rcp64, sqrt64: Newton steps in
+// double from a float seed, an ulp or so): nothing here is matched to a float program bit for bit,
+// and the library's division and root each carry a range branch and a call into every loop.
+struct Mode64 {
+    struct Consts { Elem64 e64; };
+    using Warp = IdWarp<Mode64>;
+
+    struct Ray {
+        double xD, yD, zD;
+        double tio, kx, kz, ky, iky, rx, rz, kk, ikk;
+        double y1, y2, ta, tb, xl, xr, zl, zr, full;      // cap planes at hand
+        float sa_a, sa_b;
+    };
+    struct CryRay {
+        double xD, yD, zD;
+        float sa_a, sa_b;
+    };
+    struct State {
+        double att, len;
+        int lay;
+        __device__ __forceinline__ void begin() { att = 0.0; len = 0.0; }
+        __device__ __forceinline__ void resume(double a, double o) { att = a; len = o; }
+        __device__ __forceinline__ double open() const { return len; }
+    };
+
+    static constexpr int kUnitBytes = 0;                  // reads the double tables
+    static __device__ __forceinline__ void records(const DevGeom&, Warp&, int, int, int) {}
+
+    // Sub-element centre of the 8 x 16 x 8 division in crystal d's frame (:1207-1217).
+    static __device__ __forceinline__ void centre(const Elem64& E, int ix, int iy, int iz, double& xs, double& ys, double& zs)
+    {
+        xs = -E.w / 2.0 + ((double)ix + 0.5) / 8.0 * E.w;
+        zs = -E.h / 2.0 + ((double)iz + 0.5) / 8.0 * E.h;
+        ys = -E.t / 2.0 + ((double)iy + 0.5) / 16.0 * E.t;
     }
-    const double L = sqrt((E.xI - ox) * (E.xI - ox) + (E.yI - oy) * (E.yI - oy) + (E.zI - oz) * (E.zI - oz));
-    const double vx = (ox - E.xI) / L, vy = (oy - E.yI) / L, vz = (oz - E.zI) / L;
-    bool keep = sqrt((vz - E.uz) * (vz - E.uz) + (vy - E.uy) * (vy - E.uy) + (vx - E.ux) * (vx - E.ux)) <=
-                crit / L + E.crit_self;
-    if (keep && e.filt) {
-        if (i < g.n_holes) {
-            rect = hole_rect(__ldg(&g.hole.a[i]), __ldg(&g.hole.b[i].x), e.xI, e.yI, e.zI);
-        } else {
-            const int o = i - g.n_holes;
-            rect = crystal_rect(__ldg(&g.cry.pos[o]), __ldg(&g.cry.size[o]), __ldg(&g.cry.trig[o]), e.xI, e.yI,
-                                e.zI);
+    static __device__ __forceinline__ void end(const Elem64& E, int ix, int iy, int iz, double& xD, double& yD, double& zD)
+    {
+        double xs, ys, zs;
+        centre(E, ix, iy, iz, xs, ys, zs);
+        xD = E.xd + diff2(xs, E.cr, zs, E.sr);
+        zD = E.zd + sum2(xs, E.sr, zs, E.cr);
+        yD = E.yd + ys;
+    }
+    template <class Div>
+    static __device__ __forceinline__ Ray ray(const Warp& ws, const Div&, int ix, int iy, int iz)
+    {
+        const Elem64& E = ws.c.e64;
+        Ray q;
+        end(E, ix, iy, iz, q.xD, q.yD, q.zD);
+        const double dx = q.xD - E.xI, dy = q.yD - E.yI, dz = q.zD - E.zI;
+        q.tio = sqrt64(norm3(dx, dy, dz));
+        const double it = rcp64(q.tio);
+        q.kx = dx * it;
+        q.ky = dy * it;
+        q.kz = dz * it;
+        q.iky = fabs(q.ky) > 1e-30 ? rcp64(q.ky) : 1.0 / q.ky;
+        q.rx = q.kx * q.iky;
+        q.rz = q.kz * q.iky;
+        q.kk = sum2(q.kx, q.kx, q.kz, q.kz);
+        q.ikk = rcp64(q.kk);                              // NaN for an axial ray, whose discriminant is 0
+        q.y1 = NAN;                                       // never compares equal
+        const float rdy = ws.elem.filt ? rcp_approx((float)dy) : 0.0f;
+        q.sa_a = (float)dx * rdy;
+        q.sa_b = (float)dz * rdy;
+        return q;
+    }
+    template <class Div>
+    static __device__ __forceinline__ CryRay cry_ray(const Warp& ws, const Div&, int ix, int iy, int iz)
+    {
+        const Elem64& E = ws.c.e64;
+        CryRay q;
+        end(E, ix, iy, iz, q.xD, q.yD, q.zD);
+        const float rdy = ws.elem.filt ? rcp_approx((float)(q.yD - E.yI)) : 0.0f;
+        q.sa_a = (float)(q.xD - E.xI) * rdy;
+        q.sa_b = (float)(q.zD - E.zI) * rdy;
+        return q;
+    }
+    // Plate penalty (:1240-1254); the float "through both faces" rectangle skips rays whose chord
+    // is at least the plate thickness.
+    static __device__ __forceinline__ bool penalty(const DevGeom& g, const Warp& ws, const Ray& q, double& att)
+    {
+        bool blocked = false;
+        for (int m = 0; m < g.n_layers; ++m) {
+            if (in_rect(ws.inner[m], q.sa_a, q.sa_b)) continue;
+            const Elem64& E = ws.c.e64;
+            if (plate_chord64(E.xI, E.yI, E.zI, q.xD, q.yD, q.zD, g.t64.layer + kLayer64 * m) < (double)0.1f) {
+                att = att + 100000.0;
+                blocked = true;
+            }
         }
-        keep = rects_overlap(rect, e.rd);
+        return blocked;
     }
-    return keep;
-}
-
-// build_chunk with the double cone test.
-__device__ int build_chunk64(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, const Elem& e, const Elem64& E,
-                             int d, int cursor, int n_src, bool from_super, int lane, int* count)
-{
-    int n = 0;
-    while (cursor < n_src && n <= kChunk - 32) {
-        const int j = cursor + lane;
-        bool keep = false;
-        float4 rect;
-        int id = 0;
-        if (j < n_src) {
-            id = from_super ? bs.sid[j] : j;
-            keep = keep_object64(g, e, E, id, d, rect);
+    static __device__ __forceinline__ void close(const DevGeom& g, const Ray& q, State& s, int upto)
+    {
+        while (s.lay < upto) {                            // :1281-1284
+            const double* Ly = g.t64.layer + kLayer64 * s.lay;
+            const double lcol = Ly[6] * q.iky;            // cos(theta) is the direction's y component
+            if ((lcol - s.len) >= (double)0.00001f) s.att = s.att + Ly[7] * (lcol - s.len);
+            s.len = 0.0;
+            ++s.lay;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            const int pos = n + __popc(m & ((1u << lane) - 1u));
-            ws.rect[pos] = rect;
-            ws.id[pos] = id;
-        }
-        n += __popc(m);
-        cursor += 32;
     }
-    __syncwarp();
-    *count = n;
-    return cursor < n_src ? cursor : n_src;
-}
-
-// Sub-element (ix, iy, iz) of the 8 x 16 x 8 division in double (:1207-1221): its centre in
-// crystal d's frame, in world coordinates, and the ray's length and direction cosine.
-struct Sub64 {
-    int ix, iy, iz;
-    double xD, yD, zD, sq, cosang;
-};
-
-__device__ __forceinline__ void sub_local64(const Elem64& E, int ix, int iy, int iz, double& xDs, double& yDs,
-                                            double& zDs)
-{
-    xDs = -E.w / 2.0 + ((double)ix + 0.5) / 8.0 * E.w;
-    zDs = -E.h / 2.0 + ((double)iz + 0.5) / 8.0 * E.h;
-    yDs = -E.t / 2.0 + ((double)iy + 0.5) / 16.0 * E.t;
-}
-
-__device__ __forceinline__ Sub64 sub_element64(const Elem64& E, int ix, int iy, int iz)
-{
-    Sub64 q;
-    q.ix = ix; q.iy = iy; q.iz = iz;
-    double xDs, yDs, zDs;
-    sub_local64(E, ix, iy, iz, xDs, yDs, zDs);
-    q.xD = E.xd + (xDs * E.cr - zDs * E.sr);
-    q.zD = E.zd + (xDs * E.sr + zDs * E.cr);
-    q.yD = E.yd + yDs;
-    q.sq = sqrt((q.yD - E.yI) * (q.yD - E.yI) + (q.xD - E.xI) * (q.xD - E.xI) + (q.zD - E.zI) * (q.zD - E.zI));
-    q.cosang = (q.yD - E.yI) / q.sq;
-    return q;
-}
-
-struct Walk64 {
-    double att, len;
-    int lay;
-};
-
-__device__ __forceinline__ void close_layers64(const DevGeom& g, Walk64& s, int upto, double cosang)
-{
-    while (s.lay < upto) {                                    // :1281-1284
-        const double* Ly = g.t64.layer + kLayer64 * s.lay;
-        const double lcol = Ly[6] / cosang;
-        if ((lcol - s.len) >= (double)0.00001f) s.att = s.att + Ly[7] * (lcol - s.len);
-        s.len = 0.0;
-        ++s.lay;
-    }
-}
-
-// Plate penalty (:1240-1254) in double; the float "through both faces" rectangle skips rays
-// whose chord is at least the plate thickness.
-__device__ __forceinline__ bool plate_penalty64(const DevGeom& g, const WarpSmem& ws, const Elem64& E,
-                                                const Sub64& Q, float sa_a, float sa_b, double& att)
-{
-    bool blocked = false;
-    for (int m = 0; m < g.n_layers; ++m) {
-        if (in_rect(ws.inner[m], sa_a, sa_b)) continue;
-        const double* Ly = g.t64.layer + kLayer64 * m;
-        const double tl = box_chord64(E.xI, E.yI, E.zI, Q.xD, Q.yD, Q.zD, Ly[0], Ly[2], Ly[4], Ly[1], Ly[3], Ly[5]);
-        if (tl < (double)0.1f) { att = att + 100000.0; blocked = true; }
-    }
-    return blocked;
-}
-
-// Walk round-buffer entries [0, nr) (object ids: holes [0, nh), crystals [nh, nr)) for one
-// ray in double.
-__device__ __forceinline__ void walk_round64(const DevGeom& g, const WarpSmem& ws, int nh, int nr, const Elem64& E,
-                                             const Sub64& Q, float sa_a, float sa_b, RayCyl64& rc, Walk64& s)
-{
-    for (int j = 0; j < nh; ++j) {
-        const int m = ws.rl[j];
-        if (m != s.lay) close_layers64(g, s, m, Q.cosang);
-        if (!hole_in_reach(ws, j, sa_a, sa_b)) continue;
-        const int id = __float_as_int(ws.ra[j].x);
+    // The chord of ray_cyl64_chord (chord64.cuh) as selects.
+    static __device__ __forceinline__ void hole(const DevGeom& g, const Warp& ws, Ray& q, int, int id, State& s)
+    {
+        const Elem64& E = ws.c.e64;
         const D4 a = g.t64.hole_a[id], b = g.t64.hole_b[id];
         double tmp;
         const D4 S = g.t64.hole_shape ? g.t64.hole_shape[id] : D4{0.0, 0.0, 1.0, 0.0};
-        if (S.x > 0.0)                                          // elliptical hole
-            tmp = ell_chord64(E.xI, E.yI, E.zI, Q.xD, Q.yD, Q.zD, a.x, a.y, a.z, a.w, S.x, S.y, S.z, S.w);
-        else
-            tmp = ray_cyl64_chord(rc, E.xI, E.yI, E.zI, a.x, a.y, a.z, a.w, b.x);
-        s.len = s.len + tmp;                                   // :1276-1278
+        if (S.x > 0.0) {
+            tmp = ell_chord64_call(E.xI, E.yI, E.zI, q.xD, q.yD, q.zD, a.x, a.y, a.z, a.w, S.x, S.y, S.z, S.w);
+        } else {
+            if (!(a.y == q.y1 && a.z == q.y2)) {
+                q.y1 = a.y;
+                q.y2 = a.z;
+                const double u1 = a.y - E.yI, u2 = a.z - E.yI;
+                q.xl = E.xI + q.rx * u1;
+                q.xr = E.xI + q.rx * u2;
+                q.zl = E.zI + q.rz * u1;
+                q.zr = E.zI + q.rz * u2;
+                q.ta = u1 * q.iky;
+                q.tb = u2 * q.iky;
+                q.full = fabs(q.tb - q.ta);
+                if (q.ta <= 0.0001 || q.tb <= 0.0001 || q.ta >= q.tio || q.tb >= q.tio) q.full = 0.0;
+                if (fabs(a.y - a.z) < 0.001) q.ta = q.tb = q.full = 0.0;   // the chord is 0
+            }
+            const double r2 = b.x * b.x;
+            const double dxl = q.xl - a.x, dzl = q.zl - a.w, dxr = q.xr - a.x, dzr = q.zr - a.w;
+            const bool fl = sum2(dxl, dxl, dzl, dzl) <= r2, fr = sum2(dxr, dxr, dzr, dzr) <= r2;
+            const double ox = E.xI - a.x, oz = E.zI - a.w;
+            const double cr = diff2(q.kx, oz, q.kz, ox);
+            const double disc = diff2(q.kk, r2, cr, cr);
+            const bool meets = disc > 0.00001;
+            const double sd = sqrt64(meets ? disc : 1.0);
+            const double bb = -sum2(q.kx, ox, q.kz, oz);
+            const double t1 = (bb - sd) * q.ikk, t2 = (bb + sd) * q.ikk;
+            const double ea = t1 > q.ta ? t1 : q.ta, eb = t2 < q.tb ? t2 : q.tb;
+            const bool ok = meets && eb > ea && !(eb <= 0.0001 || ea <= 0.0001 || eb >= q.tio || ea >= q.tio);
+            tmp = (fl && fr) ? q.full : (ok ? eb - ea : 0.0);
+        }
+        s.len = s.len + tmp;                              // :1276-1278
         s.att = s.att + b.y * tmp;
     }
-    if (nr <= nh) return;
-    if (s.lay < g.n_layers) close_layers64(g, s, g.n_layers, Q.cosang);
-    for (int j = nh; j < nr; ++j) {                            // :1290-1325
-        if (!in_rect(ws.rr[j], sa_a, sa_b)) continue;
-        const int o = __float_as_int(ws.ra[j].x) - g.n_holes;
+    // mu times the chord in crystal o (:1290-1325), box_chord64 as selects.
+    static __device__ __forceinline__ double crystal(const DevGeom& g, const Warp& ws, const CryRay& q, int, int o)
+    {
+        const Elem64& E = ws.c.e64;
         const D4 P = g.t64.cry_pos[o], S = g.t64.cry_size[o], T = g.t64.cry_trig[o];
-        const double xa = (E.xI - P.x) * T.z - (E.zI - P.z) * T.w, ya = E.yI - P.y;
-        const double za = (E.xI - P.x) * T.w + (E.zI - P.z) * T.z;
-        const double xb = (Q.xD - P.x) * T.z - (Q.zD - P.z) * T.w, yb = Q.yD - P.y;
-        const double zb = (Q.xD - P.x) * T.w + (Q.zD - P.z) * T.z;
-        const double la = box_chord64(xa, ya, za, xb, yb, zb, -0.5 * S.x, -0.5 * S.y, -0.5 * S.z, 0.5 * S.x,
-                                      0.5 * S.y, 0.5 * S.z);
-        s.att = s.att + la * P.w;
+        const double xa = diff2(E.xI - P.x, T.z, E.zI - P.z, T.w), ya = E.yI - P.y;
+        const double za = sum2(E.xI - P.x, T.w, E.zI - P.z, T.z);
+        const double xb = diff2(q.xD - P.x, T.z, q.zD - P.z, T.w), yb = q.yD - P.y;
+        const double zb = sum2(q.xD - P.x, T.w, q.zD - P.z, T.z);
+        const double dx = xb - xa, dy = yb - ya, dz = zb - za;
+        if (fabs(dx) < kEps64 || fabs(dy) < kEps64 || fabs(dz) < kEps64)
+            return box_chord64_call(xa, ya, za, xb, yb, zb, S.x, S.y, S.z) * P.w;
+        const double tio = sqrt64(norm3(dx, dy, dz));
+        const double ix = tio * rcp64(dx), iy = tio * rcp64(dy), iz = tio * rcp64(dz);
+        double tmin, tmax;
+        clip_first(-0.5 * S.x - xa, 0.5 * S.x - xa, ix, tmin, tmax);
+        clip(-0.5 * S.y - ya, 0.5 * S.y - ya, iy, tmin, tmax);
+        clip(-0.5 * S.z - za, 0.5 * S.z - za, iz, tmin, tmax);
+        const bool out = (tmax - tmin) < kEps64 || tmin >= tio || tmax >= tio || tmin <= kEps64 || tmax <= kEps64;
+        return out ? 0.0 : (tmax - tmin) * P.w;
     }
-}
+    // Self attenuation, absorption and solid angle (:1223-1231, :1329-1357).  The extended ray of
+    // the absorption chord has the ray's own direction, so its slab crossings are the ray's.
+    static __device__ __forceinline__ double finish(const Warp& ws, int ix, int iy, int iz, double att)
+    {
+        const Elem64& E = ws.c.e64;
+        const double w = E.w, t = E.t, h = E.h;
+        double xs, ys, zs;
+        centre(E, ix, iy, iz, xs, ys, zs);
+        const double xD = E.xd + diff2(xs, E.cr, zs, E.sr) - E.xI, zD = E.zd + sum2(xs, E.sr, zs, E.cr) - E.zI;
+        const double yD = E.yd + ys - E.yI;
+        const double sq = sqrt64(norm3(xD, yD, zD)), isq = rcp64(sq);
+        const double ux1 = ((double)ix / 8.0 - 0.5) * w, ux2 = (((double)ix + 1.0) / 8.0 - 0.5) * w;
+        const double uy1 = ((double)iy / 16.0 - 0.5) * t, uy2 = (((double)iy + 1.0) / 16.0 - 0.5) * t;
+        const double uz1 = ((double)iz / 8.0 - 0.5) * h, uz2 = (((double)iz + 1.0) / 8.0 - 0.5) * h;
+        const double dx = xs - E.xIs, dy = ys - E.yIs, dz = zs - E.zIs;
+        double l1, l2, labs;
+        if (fabs(dx) < kEps64 || fabs(dy) < kEps64 || fabs(dz) < kEps64) {
+            l1 = box_inside64_call(E.xIs, E.yIs, E.zIs, xs, ys, zs, -w / 2.0, -t / 2.0, -h / 2.0, w / 2.0, t / 2.0, h / 2.0);
+            l2 = box_inside64_call(E.xIs, E.yIs, E.zIs, xs, ys, zs, ux1, uy1, uz1, ux2, uy2, uz2);
+            const double ext = 1000.0 * isq;
+            labs = box_full64_call(E.xIs, E.yIs, E.zIs, xs + dx * ext, ys + dy * ext, zs + dz * ext, ux1, uy1, uz1, ux2,
+                                   uy2, uz2);
+        } else {
+            const double tio = sqrt64(norm3(dx, dy, dz));
+            const double rx = tio * rcp64(dx), ry = tio * rcp64(dy), rz = tio * rcp64(dz);
+            double tmin, tmax;
+            clip_first(-w / 2.0 - E.xIs, w / 2.0 - E.xIs, rx, tmin, tmax);
+            clip(-t / 2.0 - E.yIs, t / 2.0 - E.yIs, ry, tmin, tmax);
+            clip(-h / 2.0 - E.zIs, h / 2.0 - E.zIs, rz, tmin, tmax);
+            l1 = inside(tmin, tmax, tio);
+            clip_first(ux1 - E.xIs, ux2 - E.xIs, rx, tmin, tmax);
+            clip(uy1 - E.yIs, uy2 - E.yIs, ry, tmin, tmax);
+            clip(uz1 - E.zIs, uz2 - E.zIs, rz, tmin, tmax);
+            l2 = inside(tmin, tmax, tio);
+            const double far = tio + 1000.0 * tio * isq;
+            const bool out = (tmax - tmin) < kEps64 || tmin >= far || tmax >= far || tmin <= kEps64 || tmax <= kEps64;
+            labs = out ? 0.0 : tmax - tmin;
+        }
+        att = att + (l1 - l2) * E.mu_t;
+        const double absf = -expm1(-labs * E.mu_t) * E.mu_pe * rcp64(E.mu_t);
+        const double rq = isq * isq * isq * (1.0 / (4.0 * 3.14159265358979323846));
+        const double sax = t * h / 8.0 / 16.0 * fabs(diff2(xD, E.cr, zD, E.sr));
+        const double saz = w * t / 8.0 / 16.0 * fabs(sum2(xD, E.sr, zD, E.cr));
+        const double say = w * h / 8.0 / 8.0 * fabs(yD);
+        const double sxy = (sax >= say) ? sax : say;
+        return exp(-att) * (((sxy >= saz) ? sxy : saz) * rq) * absf;
+    }
+    static __device__ __forceinline__ void clip_first(double lo, double hi, double inv, double& tmin, double& tmax)
+    {
+        const double u = lo * inv, v = hi * inv;
+        tmin = u < v ? u : v;
+        tmax = u < v ? v : u;
+    }
+    static __device__ __forceinline__ void clip(double lo, double hi, double inv, double& tmin, double& tmax)
+    {
+        double a, b;
+        clip_first(lo, hi, inv, a, b);
+        tmin = a > tmin ? a : tmin;
+        tmax = b < tmax ? b : tmax;
+    }
+    // box_chord_inside64's interval: the length from the box entry to the end point inside it.
+    static __device__ __forceinline__ double inside(double tmin, double tmax, double tio)
+    {
+        const bool out = (tmax - tmin) < kEps64 || tmin >= tio || tmax <= kEps64;
+        const double len = (tmax < tio ? tmax : tio) - (tmin > kEps64 ? tmin : 0.0);
+        return out ? 0.0 : len;
+    }
+};
 
-// Self attenuation, absorption and solid angle in double (:1223-1231, :1329-1357).
-__device__ __forceinline__ double finish64(const Elem64& E, const Sub64& Q, double att)
-{
-    const double w = E.w, t = E.t, h = E.h;
-    double xDs, yDs, zDs;
-    sub_local64(E, Q.ix, Q.iy, Q.iz, xDs, yDs, zDs);
-    const double ux1 = ((double)Q.ix / 8.0 - 0.5) * w, ux2 = (((double)Q.ix + 1.0) / 8.0 - 0.5) * w;
-    const double uy1 = ((double)Q.iy / 16.0 - 0.5) * t, uy2 = (((double)Q.iy + 1.0) / 16.0 - 0.5) * t;
-    const double uz1 = ((double)Q.iz / 8.0 - 0.5) * h, uz2 = (((double)Q.iz + 1.0) / 8.0 - 0.5) * h;
-    const double l1 = box_chord_inside64(E.xIs, E.yIs, E.zIs, xDs, yDs, zDs, -w / 2.0, -t / 2.0, -h / 2.0,
-                                         w / 2.0, t / 2.0, h / 2.0);
-    const double l2 = box_chord_inside64(E.xIs, E.yIs, E.zIs, xDs, yDs, zDs, ux1, uy1, uz1, ux2, uy2, uz2);
-    att = att + (l1 - l2) * E.mu_t;
-    const double eff = exp(-att);
-    const double xt = xDs + 1000.0 * (xDs - E.xIs) / Q.sq;
-    const double yt = yDs + 1000.0 * (yDs - E.yIs) / Q.sq;
-    const double zt = zDs + 1000.0 * (zDs - E.zIs) / Q.sq;
-    const double labs = box_chord64(E.xIs, E.yIs, E.zIs, xt, yt, zt, ux1, uy1, uz1, ux2, uy2, uz2);
-    const double absf = -expm1(-labs * E.mu_t) * E.mu_pe / E.mu_t;
-    const double rq = 1.0 / ((4.0 * 3.14159265358979323846) * (Q.sq * Q.sq) * Q.sq);
-    const double sax = t * h / 8.0 / 16.0 * fabs((Q.xD - E.xI) * E.cr - (Q.zD - E.zI) * E.sr) * rq;
-    const double saz = w * t / 8.0 / 16.0 * fabs((Q.xD - E.xI) * E.sr + (Q.zD - E.zI) * E.cr) * rq;
-    const double say = w * h / 8.0 / 8.0 * fabs(Q.yD - E.yI) * rq;
-    const double sxy = (sax >= say) ? sax : say;
-    const double sa = (sxy >= saz) ? sxy : saz;
-    return eff * sa * absf;
-}
-
-// Element in double.  Rounds, round boxes and chunking as pe_element; the float Elem and
-// SubElem drive the filters only.
-__device__ double pe_element64(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, int d, long long v, float cr,
+// Element in double.
+__device__ double pe_element64(const DevGeom& g, const Superset& sup, IdWarp<Mode64>& ws, int d, long long v, float cr,
                                float sr, float rotation, int lane)
 {
-    Elem e;
-    if (!init_element(g, ws.inner, d, v, cr, sr, lane, e)) return 0.0;   // mu_t <= 0.01 (:1107, :1194)
-    // warp-uniform constants in the warp's shared slot (registers would spill)
-    static_assert(sizeof(Elem64) <= sizeof(ws.e64), "Elem64 exceeds its shared-memory slot");
-    Elem64& E = *reinterpret_cast<Elem64*>(ws.e64);
-    if (lane == 0) init_elem64(g, d, v, rotation, E);
-    __syncwarp();
-    const bool from_super = bs.s_count >= 0;
-    const int n_src = from_super ? bs.s_count : g.n_holes + g.n_det;
-    int count = 0;
-    const int cursor = build_chunk64(g, bs, ws, e, E, d, 0, n_src, from_super, lane, &count);
+    const unsigned short* src = sup.s_count >= 0 ? sup.sid : nullptr;
+    const int n_src = src ? sup.s_count : g.n_holes + g.n_det;
+    int cursor, count, nh;
+    {
+        Elem el;
+        if (!init_element(g, ws.inner, d, v, cr, sr, lane, el)) return 0.0;   // mu_t <= 0.01 (:1107, :1194)
+        if (lane == 0) {
+            ws.elem = el;
+            init_elem64(g, d, v, rotation, ws.c.e64);
+        }
+        ws.sub[lane] = RefDivision::entry(el, lane);
+        __syncwarp();
+        cursor = build_ids(g, src, ws, el, ws.c.e64, d, 0, n_src, lane, count, nh);
+    }
     const bool single = cursor >= n_src;
     double dacc = 0.0;
-    for (int r = 0; r < 32; ++r) {
-        const int sidx = ((r >> 3) * 2 + (lane >> 4)) * 128 + ((lane >> 1) & 7) * 16 + (r & 7) * 2 + (lane & 1);
-        const SubElem q = sub_element(e, sidx);
-        const Sub64 Q = sub_element64(E, q.ix, q.iy, q.iz);
-        Walk64 s{0.0, 0.0, 0};
-        RayCyl64 rc;
-        ray_cyl64_init(rc, E.xI, E.yI, E.zI, Q.xD, Q.yD, Q.zD);
-        const bool blocked = plate_penalty64(g, ws, E, Q, q.sa_a, q.sa_b, s.att);
-        const bool skip = blocked && g.nonneg_mu;
-        float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
-                                 skip ? INFINITY : q.sa_b, skip ? -INFINITY : q.sa_b);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, off));
-            box.y = fmaxf(box.y, __shfl_xor_sync(0xffffffffu, box.y, off));
-            box.z = fminf(box.z, __shfl_xor_sync(0xffffffffu, box.z, off));
-            box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, off));
+    for (int q0 = 0; q0 < 32; q0 += kIdRounds) {
+        const RefDivisionAt dv(q0);
+        ray_boxes(ws, dv, kIdRounds, lane);
+        id_pass(g, ws, dv, src, n_src, d, single, kIdRounds, lane, cursor, count, nh);
+        for (int r = 0; r < kIdRounds; ++r) {
+            int ix, iy, iz;
+            dv.indices(r, lane, ix, iy, iz);
+            const double att = ws.att[r * 32 + lane];
+            if (!isinf(att)) dacc += Mode64::finish(ws, ix, iy, iz, att);
         }
-        int cur = 0;
-        bool first_chunk = true;
-        while (true) {
-            if (!single && !first_chunk) {
-                cur = build_chunk64(g, bs, ws, e, E, d, cur, n_src, from_super, lane, &count);
-            } else if (!single) {
-                if (r > 0) cur = build_chunk64(g, bs, ws, e, E, d, 0, n_src, from_super, lane, &count);
-                else cur = cursor;
-            }
-            first_chunk = false;
-            int k = 0;
-            while (k < count) {
-                int next = count, nh = 0;
-                const int nr = fill_round<false, true>(g, ws, e, k, count, box, 0, lane, &next, &nh);
-                if (!skip) walk_round64(g, ws, nh, nr, E, Q, q.sa_a, q.sa_b, rc, s);
-                __syncwarp();
-                k = next;
-            }
-            if (single || cur >= n_src) break;
-        }
-        if (!skip) {
-            if (s.lay < g.n_layers) close_layers64(g, s, g.n_layers, Q.cosang);
-            dacc += finish64(E, Q, s.att);
-        }
+        __syncwarp();
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
-    __syncwarp();                                    // E is rewritten by the warp's next element
     return dacc;
 }

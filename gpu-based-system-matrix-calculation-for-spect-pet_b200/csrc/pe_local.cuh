@@ -11,7 +11,7 @@
 // double and only small differences are rounded to float:
 //   - per element (lane 0, in the warp's shared slot): the voxel centre, crystal d's centre
 //     and the slopes of the central ray voxel -> centre, the plate boxes relative to the
-//     voxel; per kept object and round (fill_round_local): a hole's offset from the central
+//     voxel; per kept object (ModeLocal::records): a hole's offset from the central
 //     ray at its entry plane, its depth below the voxel and its length; a crystal's centre
 //     relative to crystal d's, in its own frame;
 //   - per ray, in float: the sub-element's offset from crystal d's centre, the slope
@@ -138,6 +138,21 @@ __device__ __forceinline__ float box_chord_near(const float P[3], const float q[
     return smax - smin;
 }
 
+static __device__ __noinline__ float box_chord_near_call(float Px, float Py, float Pz, float qx, float qy, float qz, float hx,
+                                                        float hy, float hz)
+{
+    const float P[3] = {Px, Py, Pz}, q[3] = {qx, qy, qz}, lo[3] = {-hx, -hy, -hz}, hi[3] = {hx, hy, hz};
+    return box_chord_near(P, q, lo, hi);
+}
+
+// Parameters where the line from p with direction cosine 1 / iu enters and leaves [-half, half].
+__device__ __forceinline__ void slab_ends(float p, float iu, float half, float& enter, float& leave)
+{
+    const float u = (half - p) * iu, v = (-half - p) * iu;
+    enter = fminf(u, v);
+    leave = fmaxf(u, v);
+}
+
 // Hole chord as a y-extent (see the file comment): the ray's offset from the hole axis at the
 // hole's entry plane is (u0, w0), its slopes are (rx, rz) per unit y (a = rx^2 + rz^2, ia =
 // 1/a), the hole spans [0, th] in y from that plane, dy below the voxel.  Cap/side cases and
@@ -151,34 +166,25 @@ __device__ __forceinline__ float hole_extent(double u0d, double w0d, double rxd,
                                              float r, float th, float dy, float sec, float tio, float ky,
                                              double tq = 1.0)
 {
-    if (fabsf(th) < kEps) return 0.0f;
-    const double u1d = u0d + rxd * (double)th, w1d = w0d + rzd * (double)th;
+    const double u1d = __fma_rn(rxd, (double)th, u0d), w1d = __fma_rn(rzd, (double)th, w0d);
     const double r2 = (double)r * (double)r;
-    const bool fl = u0d * u0d + w0d * w0d <= r2;
-    const bool fr = u1d * u1d + w1d * w1d <= r2;
-    if (fl && fr) {
-        const float ta = dy * sec, tb = (dy + th) * sec;
-        if (ta <= 0.0001f || tb <= 0.0001f) return 0.0f;
-        if (ta >= tio || tb >= tio) return 0.0f;
-        return th;
-    }
-    const double cross = u0d * rzd - w0d * rxd;
-    const double qd = ad * r2 - cross * cross;                 // b^2 - a c (Lagrange identity)
-    if ((double)(ky * ky) * tq * qd <= (double)0.00001f) return 0.0f;   // the reference's discriminant
-    const double bd = u0d * rxd + w0d * rzd;
-    const double sq = (double)sqrtf((float)qd);
+    const bool fl = sum2(u0d, u0d, w0d, w0d) <= r2;
+    const bool fr = sum2(u1d, u1d, w1d, w1d) <= r2;
+    const float ta = dy * sec, tb = (dy + th) * sec;
+    const float full = (ta <= 0.0001f || tb <= 0.0001f || ta >= tio || tb >= tio) ? 0.0f : th;
+    const double cross = diff2(u0d, rzd, w0d, rxd);
+    const double qd = diff2(ad, r2, cross, cross);                 // b^2 - a c (Lagrange identity)
+    const bool meets = (double)(ky * ky) * tq * qd > (double)0.00001f;   // the reference's discriminant
+    const double bd = sum2(u0d, rxd, w0d, rzd);
+    const double sq = (double)sqrt_mid(meets ? (float)qd : 1.0f);
     const double s1 = (-bd - sq) * iad, s2 = (-bd + sq) * iad;
-    double ea, eb;
-    if (!fl && !fr) {
-        if (!(s1 >= 0.0 && s2 <= (double)th)) return 0.0f;
-        ea = s1; eb = s2;
-    } else if (fl) { ea = 0.0; eb = s2; }
-    else           { ea = s1; eb = (double)th; }
+    const double ea = fl ? 0.0 : s1, eb = fr ? (double)th : s2;
     const float t1 = (dy + (float)ea) * sec, t2 = (dy + (float)eb) * sec;
-    if (t2 <= 0.0001f || t1 <= 0.0001f) return 0.0f;
-    if (t2 >= tio || t1 >= tio) return 0.0f;
-    if (!fl && !fr) return (float)(2.0 * sq * iad);
-    return (float)(eb - ea);
+    const bool ok = meets && (fl || fr || (s1 >= 0.0 && s2 <= (double)th)) &&
+                    !(t2 <= 0.0001f || t1 <= 0.0001f || t2 >= tio || t1 >= tio);
+    const float side = (float)((fl || fr) ? eb - ea : 2.0 * sq * iad);
+    const float len = (fl && fr) ? full : (ok ? side : 0.0f);
+    return fabsf(th) < kEps ? 0.0f : len;
 }
 
 // Elliptical hole (length_ellipticalcylinder_ray, PESysMatGen.cu:801-947, the y-parallel
@@ -192,93 +198,17 @@ __device__ __forceinline__ void to_unit_circle(double& u, double& w, double& rx,
                                                float& r, double& tq, float ex, float ez, float ct, float st)
 {
     const double c = (double)ct, s = (double)st, iex = 1.0 / (double)ex, iez = 1.0 / (double)ez;
-    const double p = (u * c + w * s) * iex, q = (-u * s + w * c) * iez;
-    const double al = (rx * c + rz * s) * iex, be = (-rx * s + rz * c) * iez;
+    const double p = sum2(u, c, w, s) * iex, q = diff2(w, c, u, s) * iez;
+    const double al = sum2(rx, c, rz, s) * iex, be = diff2(rz, c, rx, s) * iez;
     u = p;
     w = q;
     rx = al;
     rz = be;
-    a = al * al + be * be;
+    a = sum2(al, al, be, be);
     ia = 1.0 / a;
     r = 1.0f;
     const double e2 = (double)ex * (double)ex * (double)ez * (double)ez;
     tq = e2 * e2;
-}
-
-// Copy kept entries [k0, k1) whose rectangle and capsule meet the round's slope box into the
-// round buffer with their local geometry (one entry per lane):
-//   hole:    ra = (semi-axes rho_x, rho_z of an elliptical hole, 0 for a circle; radius; mu),
-//            rb = (y1 - yI, y2 - y1, offset of the central ray from the axis at y1: x as the two
-//            halves of a double), rc = (z the same way; cos, sin of the ellipse's angle)
-//   crystal: ra = (crystal d's centre minus this crystal's centre in its frame: x, y, z; mu),
-//            rb = (cos(-rot), sin(-rot), w, t), rc = (h, -, -, -)
-// Returns the new count; *next receives the first entry not examined.
-template <bool ELL>
-__device__ __forceinline__ int fill_round_local(const DevGeom& g, WarpSmem& ws, const Elem& e, const ElemL& L,
-                                                int k0, int k1, float4 box, int n, int lane, int* next, int* nh)
-{
-    int k = k0;
-    while (k < k1 && n <= kRound - 32) {
-        const int kk = k + lane;
-        bool keep = false;
-        int id = 0;
-        float4 rect;
-        if (kk < k1) {
-            rect = ws.rect[kk];
-            keep = rects_overlap(rect, box);
-            if (keep && !isinf(rect.x)) {
-                id = ws.id[kk];
-                if (id < g.n_holes) {
-                    const float4 ha = __ldg(&g.hole.a[id]);
-                    keep = capsule_meets_box(ha.x, ha.w, ha.y, ha.z, __ldg(&g.hole.b[id].x), e, box);
-                } else {
-                    const int o = id - g.n_holes;
-                    const float4 po = __ldg(&g.cry.pos[o]);
-                    const float4 so = __ldg(&g.cry.size[o]);
-                    keep = capsule_meets_box(po.x, po.z, po.y - 0.5f * so.y, po.y + 0.5f * so.y,
-                                             0.5f * sqrtf(so.x * so.x + so.z * so.z), e, box);
-                }
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) id = ws.id[kk];
-        *nh += __popc(__ballot_sync(0xffffffffu, keep && id < g.n_holes));
-        if (keep) {
-            const int pos = n + __popc(m & ((1u << lane) - 1u));
-            ws.rr[pos] = rect;
-            const Elem64& E = L.e64;
-            if (id < g.n_holes) {
-                const D4 a = g.t64.hole_a[id];
-                const float4 hb = __ldg(&g.hole.b[id]);
-                const double dy = a.y - E.yI;
-                const double hx = (E.xI - a.x) + L.rxc * dy, hz = (E.zI - a.w) + L.rzc * dy;
-                // elliptical: semi-axes and the cos, sin of the float angle in double, rounded once
-                const D4 S = (ELL && g.t64.hole_shape) ? g.t64.hole_shape[id] : D4{0.0, 0.0, 1.0, 0.0};
-                ws.ra[pos] = make_float4((float)S.x, (float)S.y, hb.x, hb.y);
-                // the offsets in double, as the bit patterns of two floats each
-                ws.rb[pos] = make_float4((float)dy, (float)(a.z - a.y), __int_as_float(__double2hiint(hx)),
-                                         __int_as_float(__double2loint(hx)));
-                ws.rc[pos] = make_float4(__int_as_float(__double2hiint(hz)), __int_as_float(__double2loint(hz)),
-                                         (float)S.z, (float)S.w);
-                ws.rl[pos] = layer_of_hole(g, id);
-            } else {
-                const int o = id - g.n_holes;
-                const D4 P = g.t64.cry_pos[o], T = g.t64.cry_trig[o];
-                const double ex = E.xd - P.x, ey = E.yd - P.y, ez = E.zd - P.z;
-                const float4 so = __ldg(&g.cry.size[o]);
-                ws.ra[pos] = make_float4((float)(ex * T.z - ez * T.w), (float)ey, (float)(ex * T.w + ez * T.z),
-                                         __ldg(&g.cry.mu[o].x));
-                ws.rb[pos] = make_float4((float)T.z, (float)T.w, so.x, so.y);
-                ws.rc[pos] = make_float4(so.z, 0.0f, 0.0f, 0.0f);
-                ws.rl[pos] = g.n_layers;
-            }
-        }
-        n += __popc(m);
-        k += 32;
-    }
-    __syncwarp();
-    *next = k < k1 ? k : k1;
-    return n;
 }
 
 // One ray of the local form: the sub-element's offset from crystal d's centre and the ray
@@ -287,7 +217,7 @@ struct RayL {
     float ox, oy, oz;            // sub-element centre minus crystal d's centre (world axes)
     float qx, qy, qz;            // sub-element centre minus the voxel
     float sq, sec, ky;           // ray length, 1 / cos, cos
-    float drx, drz, rx, rz;      // slope difference to the central ray, slopes
+    float rx, rz;                // slopes
     double dsec;                 // 1 / cos in double (septal lengths: heavily attenuated rays)
     double ddrx, ddrz;           // slope difference to the central ray, in double
     double drx_, drz_, da, dia;  // slopes in double, a = rx^2 + rz^2 and 1/a
@@ -296,116 +226,48 @@ struct RayL {
 __device__ __forceinline__ RayL ray_local(const ElemL& L, float xDs, float yDs, float zDs)
 {
     RayL r;
-    r.ox = xDs * L.cr - zDs * L.sr;
+    r.ox = diff2(xDs, L.cr, zDs, L.sr);
     r.oy = yDs;
-    r.oz = xDs * L.sr + zDs * L.cr;
+    r.oz = sum2(xDs, L.sr, zDs, L.cr);
     r.qx = L.fdx + r.ox;
     r.qy = L.fdy + r.oy;
     r.qz = L.fdz + r.oz;
-    r.sq = sqrtf(r.qy * r.qy + r.qx * r.qx + r.qz * r.qz);
+    r.sq = sqrt_mid(norm3(r.qx, r.qy, r.qz));
     r.ky = __fdividef(r.qy, r.sq);
     r.sec = __fdividef(r.sq, r.qy);
     const float den = __fdividef(1.0f, r.qy * L.fdy);
-    r.drx = (r.ox * L.fdy - L.fdx * r.oy) * den;
-    r.drz = (r.oz * L.fdy - L.fdz * r.oy) * den;
-    r.rx = L.frxc + r.drx;
-    r.rz = L.frzc + r.drz;
+    r.rx = __fmaf_rn(diff2(r.ox, L.fdy, L.fdx, r.oy), den, L.frxc);
+    r.rz = __fmaf_rn(diff2(r.oz, L.fdy, L.fdz, r.oy), den, L.frzc);
     const Elem64& E = L.e64;
     const double cx = E.xd - E.xI, cy = E.yd - E.yI, cz = E.zd - E.zI;   // voxel -> crystal d's centre
     const double dx = cx + (double)r.ox, dy = cy + (double)r.oy, dz = cz + (double)r.oz;
-    const double idy = 1.0 / dy;
-    r.dsec = sqrt(dx * dx + dy * dy + dz * dz) * idy;
+    const double idy = rcp64(dy);
+    r.dsec = sqrt64(norm3(dx, dy, dz)) * idy;
     const double f = idy * L.idyc;
-    r.ddrx = ((double)r.ox * cy - cx * (double)r.oy) * f;
-    r.ddrz = ((double)r.oz * cy - cz * (double)r.oy) * f;
+    r.ddrx = __dmul_rn(diff2((double)r.ox, cy, cx, (double)r.oy), f);
+    r.ddrz = __dmul_rn(diff2((double)r.oz, cy, cz, (double)r.oy), f);
     r.drx_ = L.rxc + r.ddrx;
     r.drz_ = L.rzc + r.ddrz;
-    r.da = r.drx_ * r.drx_ + r.drz_ * r.drz_;
-    r.dia = 1.0 / r.da;
+    r.da = sum2(r.drx_, r.drx_, r.drz_, r.drz_);
+    r.dia = rcp64(r.da);                       // NaN for the central axis, whose discriminant is below the threshold
     return r;
 }
 
-// The attenuation sum is kept in double: its float rounding (an ulp of ~50 for the rays that
-// cross the most tungsten) would alone move exp(-att) by ~1e-5.
-struct WalkL {
-    double att;     // accumulated mu * L
-    float ext;      // hole y-extents of the current layer
-    float hatt;     // mu-weighted hole y-extents of the current layer
-    int lay;
-};
-
-__device__ __forceinline__ void close_layers_local(const DevGeom& g, WalkL& s, int upto, double sec)
+// The three lengths of finish_local when the ray is parallel to an axis within eps.
+static __device__ __noinline__ float3 finish_lengths_parallel(float sq, float vx, float vy, float vz, float xDs, float yDs,
+                                                              float zDs, float w, float t, float h, float ux1, float uy1,
+                                                              float uz1, float ux2, float uy2, float uz2)
 {
-    while (s.lay < upto) {                                           // :1276-1284
-        const LayerInfo& Ly = g.layer[s.lay];
-        s.att = s.att + (double)s.hatt * sec;
-        const double sept = (double)(Ly.thickness - s.ext) * sec;
-        if (sept >= (double)0.00001f) s.att = s.att + (double)Ly.mu_total * sept;
-        s.ext = 0.0f;
-        s.hatt = 0.0f;
-        ++s.lay;
-    }
-}
-
-template <bool ELL>
-__device__ __forceinline__ void walk_round_local(const DevGeom& g, const WarpSmem& ws, int nh, int nr, const RayL& r,
-                                                 float sa_a, float sa_b, WalkL& s)
-{
-    for (int j = 0; j < nh; ++j) {
-        const int m = ws.rl[j];
-        if (m != s.lay) close_layers_local(g, s, m, r.dsec);
-        if (!in_rect(ws.rr[j], sa_a, sa_b)) continue;
-        const float4 A = ws.ra[j];
-        const float4 B = ws.rb[j];
-        const float4 Cc = ws.rc[j];
-        const double hx = __hiloint2double(__float_as_int(B.z), __float_as_int(B.w));
-        const double hz = __hiloint2double(__float_as_int(Cc.x), __float_as_int(Cc.y));
-        double u0 = hx + r.ddrx * (double)B.x, w0 = hz + r.ddrz * (double)B.x;
-        double rx = r.drx_, rz = r.drz_, a = r.da, ia = r.dia, tq = 1.0;
-        float rad = A.z;
-        if (ELL && A.x > 0.0f) to_unit_circle(u0, w0, rx, rz, a, ia, rad, tq, A.x, A.y, Cc.z, Cc.w);   // elliptical
-        const float ext = hole_extent(u0, w0, rx, rz, a, ia, rad, B.y, B.x, r.sec, r.sq, r.ky, tq);
-        s.ext = s.ext + ext;
-        s.hatt = s.hatt + A.w * ext;
-    }
-    if (nr <= nh) return;
-    if (s.lay < g.n_layers) close_layers_local(g, s, g.n_layers, r.dsec);
-    for (int j = nh; j < nr; ++j) {                                  // :1290-1325
-        if (!in_rect(ws.rr[j], sa_a, sa_b)) continue;
-        const float4 A = ws.ra[j];
-        const float4 B = ws.rb[j];
-        const float hh = ws.rc[j].x;
-        const float P[3] = {A.x + (r.ox * B.x - r.oz * B.y), A.y + r.oy, A.z + (r.ox * B.y + r.oz * B.x)};
-        const float q[3] = {r.qx * B.x - r.qz * B.y, r.qy, r.qx * B.y + r.qz * B.x};
-        const float lo[3] = {-0.5f * B.z, -0.5f * B.w, -0.5f * hh};
-        const float hi[3] = {0.5f * B.z, 0.5f * B.w, 0.5f * hh};
-        s.att = s.att + (double)(box_chord_near(P, q, lo, hi) * A.w);
-    }
-}
-
-// Self attenuation, absorption and solid angle of sub-element (ix, iy, iz) of the L.nx x L.ny
-// x L.nz division, from its centre (xDs, yDs, zDs) in crystal d's frame (:1223-1231,
-// :1329-1357).
-__device__ __forceinline__ float finish_local(const ElemL& L, const RayL& r, int ix, int iy, int iz, float xDs,
-                                              float yDs, float zDs, double att)
-{
-    const float w = L.w, t = L.t, h = L.h;
-    const float gx = L.rfx, gy = L.rfy, gz = L.rfz;
-    const float vq[3] = {r.qx * L.cmr - r.qz * L.smr, r.qy, r.qx * L.smr + r.qz * L.cmr};   // ray in d's frame
-    const float D3[3] = {xDs, yDs, zDs};
-    const float ulo[3] = {((float)ix * gx - 0.5f) * w, ((float)iy * gy - 0.5f) * t, ((float)iz * gz - 0.5f) * h};
-    const float uhi[3] = {(((float)ix + 1.0f) * gx - 0.5f) * w, (((float)iy + 1.0f) * gy - 0.5f) * t,
-                          (((float)iz + 1.0f) * gz - 0.5f) * h};
-    const float clo[3] = {-w / 2.0f, -t / 2.0f, -h / 2.0f}, chi[3] = {w / 2.0f, t / 2.0f, h / 2.0f};
-
     // crystal entry and sub-element entry, as distances back from the sub-element centre
     // (box_chord_inside, :321-324 and its parallel-axis cases); absorption: the full chord of
     // the extended ray through the sub-element (box_chord to 1000 mm past it, :1352-1357)
+    const float D3[3] = {xDs, yDs, zDs}, vq[3] = {vx, vy, vz}, ulo[3] = {ux1, uy1, uz1}, uhi[3] = {ux2, uy2, uz2};
+    const float clo[3] = {-w / 2.0f, -t / 2.0f, -h / 2.0f}, chi[3] = {w / 2.0f, t / 2.0f, h / 2.0f};
     float l1 = 0.0f, l2 = 0.0f;
     float b1 = INFINITY, b2 = INFINITY, f2 = INFINITY, fa = INFINITY, ba = INFINITY;
     const bool y_ok = fabsf(vq[1]) >= 0.001f;
     bool ok1 = y_ok, ok2 = y_ok, ok_abs = true;
-    const float ext = 1.0f + __fdividef(1000.0f, r.sq);
+    const float ext = 1.0f + __fdividef(1000.0f, sq);
     int npar_abs = 0, m_abs = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) npar_abs += fabsf(vq[a] * ext) < kEps;
@@ -414,7 +276,7 @@ __device__ __forceinline__ float finish_local(const ElemL& L, const RayL& r, int
         const float p0 = D3[a] - vq[a];                 // the voxel's coordinate
         const bool par_in = fabsf(vq[a]) < kEps;
         const bool par_abs = fabsf(vq[a] * ext) < kEps;
-        const float iv = __fdividef(r.sq, vq[a]);      // 1 / (direction cosine along a)
+        const float iv = __fdividef(sq, vq[a]);      // 1 / (direction cosine along a)
         float f, b;
         if (par_in) {
             if (p0 >= chi[a] || p0 <= clo[a]) ok1 = false;
@@ -441,17 +303,67 @@ __device__ __forceinline__ float finish_local(const ElemL& L, const RayL& r, int
     float labs = 0.0f;
     if (ok_abs && npar_abs < 3) labs = (npar_abs == 2) ? fabsf(uhi[m_abs] - ulo[m_abs]) : fa + ba;
     if (labs < kEps) labs = 0.0f;
-    att = att + (double)((l1 - l2) * L.mu_t);
+    return make_float3(l1, l2, labs);
+}
+
+// Self attenuation, absorption and solid angle of sub-element (ix, iy, iz) of the L.nx x L.ny
+// x L.nz division, from its centre (xDs, yDs, zDs) in crystal d's frame (:1223-1231,
+// :1329-1357).
+__device__ __forceinline__ float finish_local(const ElemL& L, int ix, int iy, int iz, float xDs, float yDs, float zDs,
+                                              double att)
+{
+    struct { float qx, qy, qz, sq; } r;                  // the ray's end minus the voxel, its length
+    r.qx = L.fdx + diff2(xDs, L.cr, zDs, L.sr);
+    r.qy = L.fdy + yDs;
+    r.qz = L.fdz + sum2(xDs, L.sr, zDs, L.cr);
+    const float qq = norm3(r.qx, r.qy, r.qz);
+    r.sq = sqrt_mid(qq);
+    const float w = L.w, t = L.t, h = L.h;
+    const float gx = L.rfx, gy = L.rfy, gz = L.rfz;
+    const float vq[3] = {diff2(r.qx, L.cmr, r.qz, L.smr), r.qy, sum2(r.qx, L.smr, r.qz, L.cmr)};   // ray in d's frame
+    const float D3[3] = {xDs, yDs, zDs};
+    const float ulo[3] = {__fmaf_rn((float)ix, gx, -0.5f) * w, __fmaf_rn((float)iy, gy, -0.5f) * t,
+                          __fmaf_rn((float)iz, gz, -0.5f) * h};
+    const float uhi[3] = {__fmaf_rn((float)ix + 1.0f, gx, -0.5f) * w, __fmaf_rn((float)iy + 1.0f, gy, -0.5f) * t,
+                          __fmaf_rn((float)iz + 1.0f, gz, -0.5f) * h};
+    const float clo[3] = {-w / 2.0f, -t / 2.0f, -h / 2.0f}, chi[3] = {w / 2.0f, t / 2.0f, h / 2.0f};
+
+    // crystal entry and sub-element entry, as distances back from the sub-element centre
+    // (box_chord_inside); absorption: the full chord of the extended ray through the sub-element
+    // (box_chord to 1000 mm past it, :1352-1357)
+    float l1, l2, labs;
+    if (fabsf(vq[0]) < kEps || fabsf(vq[1]) < kEps || fabsf(vq[2]) < kEps) {
+        const float3 l = finish_lengths_parallel(r.sq, vq[0], vq[1], vq[2], xDs, yDs, zDs, w, t, h, ulo[0], ulo[1], ulo[2],
+                                                 uhi[0], uhi[1], uhi[2]);
+        l1 = l.x, l2 = l.y, labs = l.z;
+    } else {
+        l1 = INFINITY;
+        l2 = INFINITY;
+        labs = INFINITY;                                 // forward part
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float iv = __fdividef(r.sq, vq[a]);    // 1 / (direction cosine along a)
+            float f, b;
+            slab_exit(D3[a], iv, clo[a], chi[a], f, b);
+            l1 = fminf(l1, b);
+            slab_exit(D3[a], iv, ulo[a], uhi[a], f, b);
+            l2 = fminf(l2, b);
+            labs = fminf(labs, f);
+        }
+        labs = labs + l2;
+        if (labs < kEps) labs = 0.0f;
+    }
+    att = att + (double)__fmul_rn(l1 - l2, L.mu_t);
     // exp(-att) = exp(-hi) exp(-lo), hi = att rounded to float: keeps expf's relative accuracy
     const float a_hi = (float)att, a_lo = (float)(att - (double)a_hi);
     const float eff = expf(-a_hi) * (1.0f - a_lo);
     const float absf = -expm1f(-labs * L.mu_t) * L.mu_pe / L.mu_t;
     // solid angle in double, as the reference's 4*M_PI promotion makes it
-    const double dsq = (double)(r.qy * r.qy + r.qx * r.qx + r.qz * r.qz);
-    const double rq = 1.0 / ((4.0 * 3.14159265358979323846) * dsq * (double)r.sq);
+    const double dsq = (double)qq;
+    const double rq = rcp64((4.0 * 3.14159265358979323846) * dsq * (double)r.sq);
     const float ax = t * h * gz * gy, az = w * t * gx * gy, ay = w * h * gx * gz;
-    const float sax = (float)((double)ax * (double)fabsf(r.qx * L.cr - r.qz * L.sr) * rq);
-    const float saz = (float)((double)az * (double)fabsf(r.qx * L.sr + r.qz * L.cr) * rq);
+    const float sax = (float)((double)ax * (double)fabsf(diff2(r.qx, L.cr, r.qz, L.sr)) * rq);
+    const float saz = (float)((double)az * (double)fabsf(sum2(r.qx, L.sr, r.qz, L.cr)) * rq);
     const float say = (float)((double)ay * (double)fabsf(r.qy) * rq);
     const float sxy = (sax >= say) ? sax : say;
     const float sa = (sxy >= saz) ? sxy : saz;
@@ -467,114 +379,228 @@ __device__ __forceinline__ void neumaier_add(float& s, float& c, float x)
     s = t;
 }
 
+// The mode's phases (pe_ids.cuh).
+template <bool ELL>
+struct ModeLocal {
+    using Consts = ElemL;
+    using Warp = IdWarp<ModeLocal<ELL>>;
+
+    struct Ray {
+        RayL r;
+        float sa_a, sa_b;
+    };
+    struct CryRay {
+        float ox, oy, oz, qx, qy, qz;
+        float sa_a, sa_b;
+    };
+    // The attenuation sum is kept in double: its float rounding (an ulp of ~50 for the rays that
+    // cross the most tungsten) would alone move exp(-att) by ~1e-5.
+    struct State {
+        double att;
+        float ext, hatt;             // hole y-extents of the open layer, plain and mu-weighted
+        int lay;
+        __device__ __forceinline__ void begin() { att = 0.0; ext = hatt = 0.0f; }
+        __device__ __forceinline__ void resume(double a, double o)
+        {
+            att = a;
+            ext = __int_as_float(__double2hiint(o));
+            hatt = __int_as_float(__double2loint(o));
+        }
+        __device__ __forceinline__ double open() const { return __hiloint2double(__float_as_int(ext), __float_as_int(hatt)); }
+    };
+
+    static __device__ __forceinline__ float3 centre(const ElemL& L, int ix, int iy, int iz)   // :1207-1217
+    {
+        return make_float3(__fmaf_rn(((float)ix + 0.5f) * L.rfx, L.w, -0.5f * L.w),
+                           __fmaf_rn(((float)iy + 0.5f) * L.rfy, L.t, -0.5f * L.t),
+                           __fmaf_rn(((float)iz + 0.5f) * L.rfz, L.h, -0.5f * L.h));
+    }
+    template <class Div>
+    static __device__ __forceinline__ Ray ray(const Warp& ws, const Div&, int ix, int iy, int iz)
+    {
+        const float3 c = centre(ws.c, ix, iy, iz);
+        Ray q;
+        q.r = ray_local(ws.c, c.x, c.y, c.z);
+        q.sa_a = ws.elem.filt ? q.r.rx : 0.0f;
+        q.sa_b = ws.elem.filt ? q.r.rz : 0.0f;
+        return q;
+    }
+    template <class Div>
+    static __device__ __forceinline__ CryRay cry_ray(const Warp& ws, const Div&, int ix, int iy, int iz)
+    {
+        const ElemL& L = ws.c;
+        const float3 c = centre(L, ix, iy, iz);
+        CryRay q;
+        q.ox = diff2(c.x, L.cr, c.z, L.sr);
+        q.oy = c.y;
+        q.oz = sum2(c.x, L.sr, c.z, L.cr);
+        q.qx = L.fdx + q.ox;
+        q.qy = L.fdy + q.oy;
+        q.qz = L.fdz + q.oz;
+        const float rdy = ws.elem.filt ? rcp_approx(q.qy) : 0.0f;
+        q.sa_a = q.qx * rdy;
+        q.sa_b = q.qz * rdy;
+        return q;
+    }
+    static __device__ __forceinline__ bool penalty(const DevGeom& g, const Warp& ws, const Ray& q, double& att)
+    {
+        bool blocked = false;                                              // :1240-1254
+        for (int m = 0; m < g.n_layers; ++m) {
+            if (in_rect(ws.inner[m], q.sa_a, q.sa_b)) continue;
+            const float* pb = ws.c.plate[m];
+            if (plate_chord(0.0f, 0.0f, 0.0f, q.r.qx, q.r.qy, q.r.qz, pb[0], pb[1], pb[2], pb[3], pb[4], pb[5]) < 0.1f) {
+                att = att + 100000.0;
+                blocked = true;
+            }
+        }
+        return blocked;
+    }
+    static __device__ __forceinline__ void close(const DevGeom& g, const Ray& q, State& s, int upto)
+    {
+        const double sec = q.r.dsec;
+        while (s.lay < upto) {                                             // :1276-1284
+            const LayerInfo& Ly = g.layer[s.lay];
+            s.att = __fma_rn((double)s.hatt, sec, s.att);
+            const double sept = (double)(Ly.thickness - s.ext) * sec;
+            if (sept >= (double)0.00001f) s.att = __fma_rn((double)Ly.mu_total, sept, s.att);
+            s.ext = 0.0f;
+            s.hatt = 0.0f;
+            ++s.lay;
+        }
+    }
+    // Kept hole j at unit j: its offset from the central ray at its entry plane (two doubles), its
+    // depth below the voxel, length, radius and mu.  Kept crystal at units 2 j - nh, + 1: crystal d's
+    // centre relative to its own in its frame, mu; cos(-rot), sin(-rot), w, t; h.
+    static constexpr int kUnitBytes = 32;
+    static __device__ __forceinline__ void records(const DevGeom& g, Warp& ws, int count, int nh, int lane)
+    {
+        const ElemL& L = ws.c;
+        for (int j = lane; j < count; j += 32) {
+            const int id = ws.id[j];
+            if (j < nh) {
+                const D4 a = g.t64.hole_a[id];
+                const float4 hb = __ldg(&g.hole.b[id]);
+                const double dy = a.y - L.e64.yI;
+                *reinterpret_cast<double2*>(&ws.rec[2 * j]) =
+                    make_double2(__fma_rn(L.rxc, dy, L.e64.xI - a.x), __fma_rn(L.rzc, dy, L.e64.zI - a.w));
+                ws.rec[2 * j + 1] = make_float4((float)dy, (float)(a.z - a.y), hb.x, hb.y);
+            } else {
+                const int o = id - g.n_holes, u = 2 * (2 * j - nh);
+                const D4 P = g.t64.cry_pos[o], T = g.t64.cry_trig[o];
+                const double ex = L.e64.xd - P.x, ey = L.e64.yd - P.y, ez = L.e64.zd - P.z;
+                const float4 so = __ldg(&g.cry.size[o]);
+                ws.rec[u] = make_float4((float)diff2(ex, T.z, ez, T.w), (float)ey, (float)sum2(ex, T.w, ez, T.z),
+                                        __ldg(&g.cry.mu[o].x));
+                ws.rec[u + 1] = make_float4((float)T.z, (float)T.w, so.x, so.y);
+                ws.rec[u + 2] = make_float4(so.z, 0.0f, 0.0f, 0.0f);
+            }
+        }
+    }
+    static __device__ __forceinline__ void hole(const DevGeom& g, const Warp& ws, const Ray& q, int j, int id, State& s)
+    {
+        const RayL& r = q.r;
+        const double2 off = *reinterpret_cast<const double2*>(&ws.rec[2 * j]);
+        const float4 B = ws.rec[2 * j + 1];
+        double u0 = __fma_rn(r.ddrx, (double)B.x, off.x), w0 = __fma_rn(r.ddrz, (double)B.x, off.y);
+        double rx = r.drx_, rz = r.drz_, da = r.da, ia = r.dia, tq = 1.0;
+        float rad = B.z;
+        if constexpr (ELL) {
+            const D4 S = g.t64.hole_shape ? g.t64.hole_shape[id] : D4{0.0, 0.0, 1.0, 0.0};
+            if (S.x > 0.0)
+                to_unit_circle(u0, w0, rx, rz, da, ia, rad, tq, (float)S.x, (float)S.y, (float)S.z, (float)S.w);
+        }
+        const float ext = hole_extent(u0, w0, rx, rz, da, ia, rad, B.y, B.x, r.sec, r.sq, r.ky, tq);
+        s.ext = s.ext + ext;
+        s.hatt = __fmaf_rn(B.w, ext, s.hatt);
+    }
+    // mu times the chord in a crystal (:1290-1325): box_chord_near as selects where no axis is parallel.
+    static __device__ __forceinline__ double crystal(const DevGeom&, const Warp& ws, const CryRay& q, int unit, int)
+    {
+        const float4 A = ws.rec[2 * unit], B = ws.rec[2 * unit + 1];
+        const float h = ws.rec[2 * unit + 2].x;
+        const float Px = A.x + diff2(q.ox, B.x, q.oz, B.y), Py = A.y + q.oy, Pz = A.z + sum2(q.ox, B.y, q.oz, B.x);
+        const float vx = diff2(q.qx, B.x, q.qz, B.y), vy = q.qy, vz = sum2(q.qx, B.y, q.qz, B.x);
+        float len;
+        if (fabsf(vx) < kEps || fabsf(vy) < kEps || fabsf(vz) < kEps) {
+            len = box_chord_near_call(Px, Py, Pz, vx, vy, vz, 0.5f * B.z, 0.5f * B.w, 0.5f * h);
+        } else {
+            const float tio = sqrt_mid(norm3(vx, vy, vz));
+            float smin, smax, a, b;                       // along P + s * (-v / tio)
+            slab_ends(Px, __fdividef(-tio, vx), 0.5f * B.z, smin, smax);
+            slab_ends(Py, __fdividef(-tio, vy), 0.5f * B.w, a, b);
+            smin = fmaxf(smin, a), smax = fminf(smax, b);
+            slab_ends(Pz, __fdividef(-tio, vz), 0.5f * h, a, b);
+            smin = fmaxf(smin, a), smax = fminf(smax, b);
+            // the reference's parameters from the voxel are t = tio - s
+            const bool out = !(smin <= smax) || (smax - smin) < kEps || smin <= 0.0f || smax >= tio - kEps;
+            len = out ? 0.0f : smax - smin;
+        }
+        return (double)(len * A.w);
+    }
+};
+
 // The element of the local form.  smp: the crystal division and the voxel's source points (the
 // element is the mean over the centres of an sx x sy x sz grid over the voxel, as in the
-// sampled form); nullptr = the reference's 8 x 16 x 8 division and the voxel centre.  The
-// reference division's rounds are the compact 2 z x 8 x x 2 depth patches of the
-// reference-order kernel; other divisions go 32 to a round in (z, depth, x) order, x fastest.
+// sampled form); nullptr = the reference's 8 x 16 x 8 division and the voxel centre.
 // sub_out (one source point only): each sub-element's contribution is also written there, at
 // index (iz * ny + iy) * nx + ix (the scatter grid's crystal-cell weights).
 template <bool ELL, bool SMP>
-__device__ double pe_element_local(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, int d, long long v, float cr,
-                                   float sr, float rotation, int lane, const Sampling* smp = nullptr,
+__device__ double pe_element_local(const DevGeom& g, const Superset& sup, IdWarp<ModeLocal<ELL>>& ws, int d, long long v,
+                                   float cr, float sr, float rotation, int lane, const Sampling* smp = nullptr,
                                    float* sub_out = nullptr)
 {
-    static_assert(sizeof(ElemL) <= sizeof(ws.chain), "ElemL exceeds its shared-memory slot");
-    ElemL& L = *reinterpret_cast<ElemL*>(ws.chain);
-    if constexpr (!SMP) smp = nullptr;               // the reference's sampling: constants below
+    const unsigned short* src = sup.s_count >= 0 ? sup.sid : nullptr;
+    const int n_src = src ? sup.s_count : g.n_holes + g.n_det;
     const int nx = SMP ? smp->nx : 8, ny = SMP ? smp->ny : 16, nz = SMP ? smp->nz : 8;
-    const int n_sub = nx * ny * nz, nxy = nx * ny;
+    const int n_sub = nx * ny * nz, n_rounds = (n_sub + 31) / 32;
     const int sxn = SMP ? smp->sx : 1, syn = SMP ? smp->sy : 1, szn = SMP ? smp->sz : 1;
     const int n_pts = sxn * syn * szn;
     float sum = 0.0f, comp = 0.0f;
-    for (int src = 0; src < n_pts; ++src) {
+    for (int p = 0; p < n_pts; ++p) {
         // source point at fractions ((j + 0.5) / n) of the voxel along x, y, z
-        const int jx = src % sxn, jy = (src / sxn) % syn, jz = src / (sxn * syn);
+        const int jx = p % sxn, jy = (p / sxn) % syn, jz = p / (sxn * syn);
         const double fxd = ((double)jx + 0.5) / (double)sxn, fyd = ((double)jy + 0.5) / (double)syn;
         const double fzd = ((double)jz + 0.5) / (double)szn;
-        __syncwarp();                                    // the previous point's ElemL and plate rectangles are done
-        Elem e;
-        if (!init_element(g, ws.inner, d, v, cr, sr, lane, e, (float)fxd, (float)fyd, (float)fzd)) {   // mu_t <= 0.01
-            if (sub_out) {                                                                     // (:1107, :1194)
-                for (int i = lane; i < n_sub; i += 32) sub_out[i] = 0.0f;
+        __syncwarp();                                    // the previous point's constants and lists are done
+        int cursor, count, nh;
+        {
+            Elem el;
+            if (!init_element(g, ws.inner, d, v, cr, sr, lane, el, (float)fxd, (float)fyd, (float)fzd)) {   // mu_t <= 0.01
+                if (sub_out) {                                                                     // (:1107, :1194)
+                    for (int i = lane; i < n_sub; i += 32) sub_out[i] = 0.0f;
+                }
+                return 0.0;
             }
-            return 0.0;
+            if (lane == 0) {
+                ws.elem = el;
+                init_elem_local(g, d, v, rotation, nx, ny, nz, ws.c, fxd, fyd, fzd);
+            }
+            if constexpr (!SMP) ws.sub[lane] = RefDivision::entry(el, lane);
+            __syncwarp();
+            cursor = build_ids(g, src, ws, el, ws.c.e64, d, 0, n_src, lane, count, nh);
         }
-        if (lane == 0) init_elem_local(g, d, v, rotation, nx, ny, nz, L, fxd, fyd, fzd);
-        __syncwarp();
-        const bool from_super = bs.s_count >= 0;
-        const int n_src = from_super ? bs.s_count : g.n_holes + g.n_det;
-        int count = 0;
-        const int cursor = build_chunk64(g, bs, ws, e, L.e64, d, 0, n_src, from_super, lane, &count);
         const bool single = cursor >= n_src;
-        const float gx = L.rfx, gy = L.rfy, gz = L.rfz;
-        for (int base = 0; base < n_sub; base += 32) {
-            const bool dead = base + lane >= n_sub;
-            int sidx, ix, iy, iz;
-            if constexpr (!SMP) {             // s = 128 iz + 16 ix + iy, as in pe_element's rounds
-                const int rr = base >> 5;
-                const int s = ((rr >> 3) * 2 + (lane >> 4)) * 128 + ((lane >> 1) & 7) * 16 + (rr & 7) * 2 + (lane & 1);
-                iz = s >> 7;
-                ix = (s >> 4) & 7;
-                iy = s & 15;
-                sidx = (iz * ny + iy) * nx + ix;
-            } else {
-                sidx = dead ? n_sub - 1 : base + lane;
-                iz = sidx / nxy;
-                const int rem = sidx - iz * nxy;
-                iy = rem / nx;
-                ix = rem - iy * nx;
-            }
-            const float xDs = -L.w / 2.0f + ((float)ix + 0.5f) * gx * L.w;       // :1207-1217
-            const float zDs = -L.h / 2.0f + ((float)iz + 0.5f) * gz * L.h;
-            const float yDs = -L.t / 2.0f + ((float)iy + 0.5f) * gy * L.t;
-            const RayL r = ray_local(L, xDs, yDs, zDs);
-            const float sa_a = e.filt ? r.rx : 0.0f, sa_b = e.filt ? r.rz : 0.0f;
-            WalkL s{0.0, 0.0f, 0.0f, 0};
-            bool blocked = false;
-            for (int m = 0; m < g.n_layers; ++m) {                             // plate penalty :1240-1254
-                if (in_rect(ws.inner[m], sa_a, sa_b)) continue;
-                const float* pb = L.plate[m];
-                const float tl = box_chord(0.0f, 0.0f, 0.0f, r.qx, r.qy, r.qz, pb[0], pb[1], pb[2], pb[3], pb[4], pb[5]);
-                if (tl < 0.1f) { s.att = s.att + 100000.0; blocked = true; }
-            }
-            const bool skip = dead || (blocked && g.nonneg_mu);
-            float4 box = make_float4(skip ? INFINITY : sa_a, skip ? -INFINITY : sa_a, skip ? INFINITY : sa_b,
-                                     skip ? -INFINITY : sa_b);
-    #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, off));
-                box.y = fmaxf(box.y, __shfl_xor_sync(0xffffffffu, box.y, off));
-                box.z = fminf(box.z, __shfl_xor_sync(0xffffffffu, box.z, off));
-                box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, off));
-            }
-            int cur = 0;
-            bool first_chunk = true;
-            while (true) {
-                if (!single && !first_chunk) {
-                    cur = build_chunk64(g, bs, ws, e, L.e64, d, cur, n_src, from_super, lane, &count);
-                } else if (!single) {
-                    if (base > 0) cur = build_chunk64(g, bs, ws, e, L.e64, d, 0, n_src, from_super, lane, &count);
-                    else cur = cursor;
+        for (int q0 = 0; q0 < n_rounds; q0 += kIdRounds) {
+            const int n = min(kIdRounds, n_rounds - q0);
+            auto pass = [&](const auto& dv) {
+                ray_boxes(ws, dv, n, lane);
+                id_pass(g, ws, dv, src, n_src, d, single, n, lane, cursor, count, nh);
+                for (int r = 0; r < n; ++r) {
+                    int ix, iy, iz;
+                    dv.indices(r, lane, ix, iy, iz);
+                    const double att = ws.att[r * 32 + lane];
+                    const float3 c = ModeLocal<ELL>::centre(ws.c, ix, iy, iz);
+                    float term = 0.0f;
+                    if (!isinf(att)) {
+                        term = finish_local(ws.c, ix, iy, iz, c.x, c.y, c.z, att);
+                        neumaier_add(sum, comp, term);
+                    }
+                    if (SMP && sub_out && !dv.dead(r, lane)) sub_out[(iz * ny + iy) * nx + ix] = term;
                 }
-                first_chunk = false;
-                int k = 0;
-                while (k < count) {
-                    int next = count, nh = 0;
-                    const int nr = fill_round_local<ELL>(g, ws, e, L, k, count, box, 0, lane, &next, &nh);
-                    if (!skip) walk_round_local<ELL>(g, ws, nh, nr, r, sa_a, sa_b, s);
-                    __syncwarp();
-                    k = next;
-                }
-                if (single || cur >= n_src) break;
-            }
-            float term = 0.0f;
-            if (!skip) {
-                if (s.lay < g.n_layers) close_layers_local(g, s, g.n_layers, r.dsec);
-                term = finish_local(L, r, ix, iy, iz, xDs, yDs, zDs, s.att);
-                neumaier_add(sum, comp, term);
-            }
-            if (sub_out && !dead) sub_out[sidx] = term;
+                __syncwarp();
+            };
+            if constexpr (SMP) pass(AnyDivision{nx, ny, n_sub, 32 * q0, (float)nx, (float)ny, (float)nz});
+            else pass(RefDivisionAt(q0));
         }
     }
     // warp sum of the (sum, compensation) pairs, compensated as well
@@ -585,6 +611,5 @@ __device__ double pe_element_local(const DevGeom& g, const BlockSmem& bs, WarpSm
         neumaier_add(sum, comp, os);
         comp += oc;
     }
-    __syncwarp();                                    // L is rewritten by the warp's next element
     return ((double)sum + (double)comp) / (double)n_pts;
 }

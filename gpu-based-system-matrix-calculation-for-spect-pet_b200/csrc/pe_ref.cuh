@@ -26,7 +26,6 @@
 // bit.  With them the distance to the sub-element (:1218-1219) and the length of the ray in the
 // cylinder chord (:696) are the same float, and cos(theta) is the direction's y component.
 
-constexpr int kRefBlocks = 2;            // blocks of kWarps warps per SM
 constexpr int kPassRounds = 16;          // rounds per pass: half of an element
 constexpr int kUnits = 192;              // record units of 32 B: a hole takes one, a crystal two
 constexpr int kMaskWords = kUnits / 32;
@@ -89,19 +88,33 @@ struct RefDivision {
         iz = 4 * (r >> 4) + (lane >> 3);
     }
     __device__ __forceinline__ bool dead(int, int) const { return false; }
-    __device__ __forceinline__ float3 centre(const RefWarp& ws, int ix, int iy, int iz) const
+    template <class W>
+    __device__ __forceinline__ float3 centre(const W& ws, int ix, int iy, int iz) const
     {
         return make_float3(ws.sub[ix].x, ws.sub[8 + iy].x, ws.sub[24 + iz].x);
     }
-    __device__ __forceinline__ float4 row_x(const RefWarp& ws, int i) const { return ws.sub[i]; }
-    __device__ __forceinline__ float4 row_y(const RefWarp& ws, int i) const { return ws.sub[8 + i]; }
-    __device__ __forceinline__ float4 row_z(const RefWarp& ws, int i) const { return ws.sub[24 + i]; }
+    template <class W>
+    __device__ __forceinline__ float4 row_x(const W& ws, int i) const { return ws.sub[i]; }
+    template <class W>
+    __device__ __forceinline__ float4 row_y(const W& ws, int i) const { return ws.sub[8 + i]; }
+    template <class W>
+    __device__ __forceinline__ float4 row_z(const W& ws, int i) const { return ws.sub[24 + i]; }
     // lane l's table row: x (l < 8), depth (l < 24), z
     __device__ __forceinline__ static float4 entry(const Elem& e, int lane)
     {
         const int i = lane < 8 ? lane : (lane < 24 ? lane - 8 : lane - 24);
         return sub_row(i, lane >= 8 && lane < 24 ? fy : fx, lane < 8 ? e.w : (lane < 24 ? e.t : e.h),
                        lane < 8 ? e.xIs : (lane < 24 ? e.yIs : e.zIs));
+    }
+};
+
+// The reference division from round `base`.
+struct RefDivisionAt : RefDivision {
+    int base;
+    __device__ __forceinline__ explicit RefDivisionAt(int b) : base(b) {}
+    __device__ __forceinline__ void indices(int r, int lane, int& ix, int& iy, int& iz) const
+    {
+        RefDivision::indices(base + r, lane, ix, iy, iz);
     }
 };
 
@@ -119,13 +132,17 @@ struct AnyDivision {
         ix = rem - iy * nx;
     }
     __device__ __forceinline__ bool dead(int r, int lane) const { return base + 32 * r + lane >= n_sub; }
-    __device__ __forceinline__ float3 centre(const RefWarp& ws, int ix, int iy, int iz) const
+    template <class W>
+    __device__ __forceinline__ float3 centre(const W& ws, int ix, int iy, int iz) const
     {
         return make_float3(sub_centre(ix, fx, ws.elem.w), sub_centre(iy, fy, ws.elem.t), sub_centre(iz, fz, ws.elem.h));
     }
-    __device__ __forceinline__ float4 row_x(const RefWarp& ws, int i) const { return sub_row(i, fx, ws.elem.w, ws.elem.xIs); }
-    __device__ __forceinline__ float4 row_y(const RefWarp& ws, int i) const { return sub_row(i, fy, ws.elem.t, ws.elem.yIs); }
-    __device__ __forceinline__ float4 row_z(const RefWarp& ws, int i) const { return sub_row(i, fz, ws.elem.h, ws.elem.zIs); }
+    template <class W>
+    __device__ __forceinline__ float4 row_x(const W& ws, int i) const { return sub_row(i, fx, ws.elem.w, ws.elem.xIs); }
+    template <class W>
+    __device__ __forceinline__ float4 row_y(const W& ws, int i) const { return sub_row(i, fy, ws.elem.t, ws.elem.yIs); }
+    template <class W>
+    __device__ __forceinline__ float4 row_z(const W& ws, int i) const { return sub_row(i, fz, ws.elem.h, ws.elem.zIs); }
 };
 
 // World position of the sub-element with centre (xDs, yDs, zDs) in crystal d's frame.
@@ -267,6 +284,43 @@ __device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short
     return cursor;
 }
 
+__device__ __forceinline__ float warp_min(float x)
+{
+    float y;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float warp_max(float x)
+{
+    float y;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// ws.box and ws.reach of the first n rounds, from the rays themselves.
+template <class W, class Div>
+__device__ __forceinline__ void ray_boxes(W& ws, const Div& dv, int n, int lane)
+{
+    const Elem& e = ws.elem;
+    for (int r = 0; r < n; ++r) {
+        int ix, iy, iz;
+        dv.indices(r, lane, ix, iy, iz);
+        const float3 q = dv.centre(ws, ix, iy, iz);
+        float x, y, z;
+        ray_end(e, q.x, q.y, q.z, x, y, z);
+        const float rdy = e.filt ? rcp_approx(y - e.yI) : 0.0f;
+        const float a = (x - e.xI) * rdy, b = (z - e.zI) * rdy;
+        const float4 box = make_float4(warp_min(a), warp_max(a), warp_min(b), warp_max(b));
+        if (lane == 0) {
+            const float px = fmaxf(fabsf(box.x), fabsf(box.y)), pz = fmaxf(fabsf(box.z), fabsf(box.w));
+            ws.box[r] = box;
+            ws.reach[r] = sqrtf(px * px + pz * pz);
+        }
+    }
+    __syncwarp();
+}
+
 // Slope boxes of the rounds (lane = round): the slopes of a box of points behind the voxel are
 // extreme at its corners.  All zero when the rectangles are open.
 __device__ __forceinline__ void round_boxes(RefWarp& ws, const Elem& e, int lane)
@@ -290,40 +344,59 @@ __device__ __forceinline__ void round_boxes(RefWarp& ws, const Elem& e, int lane
     __syncwarp();
 }
 
-// ws.mask for rounds [r0, r1).  A kept object stays for a round unless its slope rectangle misses
-// the round's box, or its shadow does: seen from the voxel, a y-aligned object with centre
-// offset C, footprint half axes a, b (a crystal) or radius R (a hole) meets a ray of slope p
-// only if |C x p| <= |a x p| + |b x p| + R |p|.  Objects close to the voxel (open rectangles)
-// always stay.
+// What a round's slope box is tested against: an object's slope rectangle and its shadow.  Seen
+// from the voxel, a y-aligned object with centre offset C, footprint half axes a, b (a crystal) or
+// radius R (a hole) meets a ray of slope p only if |C x p| <= |a x p| + |b x p| + R |p|.  Objects
+// close to the voxel (open rectangles) meet every box, a default Shadow none.
+struct Shadow {
+    float4 rect = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+    float cx = 0.0f, cz = 0.0f, ax = 0.0f, az = 0.0f, bx = 0.0f, bz = 0.0f, R = INFINITY;
+    float sx = 1e-3f, sz = 1e-3f;        // extents that scale the box's half widths and the margin
+
+    // a: x, y1, y2, z of the hole
+    __device__ __forceinline__ void hole(const Elem& e, float4 a, float r)
+    {
+        rect = e.filt ? hole_rect(a, r, e.xI, e.yI, e.zI) : open_rect();
+        if (isinf(rect.x)) return;
+        cx = e.xI - a.x, cz = e.zI - a.w, R = r * 1.0001f;
+        sx += fabsf(cx), sz += fabsf(cz);
+    }
+    // half axes (hw c, hw s) and (-hh s, hh c) of the crystal's footprint, its rectangle known
+    __device__ __forceinline__ void crystal(const Elem& e, float4 known, float x, float z, float hw, float hh, float c,
+                                            float s)
+    {
+        rect = known;
+        if (isinf(rect.x)) return;
+        cx = e.xI - x, cz = e.zI - z, R = 0.0f;
+        ax = hw * c, az = hw * s, bx = -hh * s, bz = hh * c;
+        sx += fabsf(cx) + fabsf(ax) + fabsf(bx), sz += fabsf(cz) + fabsf(az) + fabsf(bz);
+    }
+    __device__ __forceinline__ bool meets(const float4& box, float reach) const
+    {
+        const float mx = 0.5f * (box.x + box.y), mz = 0.5f * (box.z + box.w);
+        const float ex = 0.5f * (box.y - box.x) + kSlopeMargin, ez = 0.5f * (box.w - box.z) + kSlopeMargin;
+        const float far = fabsf(cx * mz - cz * mx) - fabsf(ax * mz - az * mx) - fabsf(bx * mz - bz * mx);
+        return rects_overlap(rect, box) && !(far > sx * ez + sz * ex + R * reach);
+    }
+};
+
+// ws.mask for rounds [r0, r1): the kept objects that meet each round's slope box.
 __device__ __forceinline__ void round_masks(RefWarp& ws, const Elem& e, const Kept& k, int r0, int r1, int lane)
 {
     for (int w = 0; w * 32 < k.count; ++w) {
         const int j = w * 32 + lane;
-        float4 rect = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);   // past the end: meets nothing
-        float cx = 0.0f, cz = 0.0f, ax = 0.0f, az = 0.0f, bx = 0.0f, bz = 0.0f, R = INFINITY;
+        Shadow s;
         if (j < k.nh) {
             const float4 A = ws.rec[2 * j], B = ws.rec[2 * j + 1];
-            rect = e.filt ? hole_rect(make_float4(A.x, B.x, B.y, A.y), B.z, e.xI, e.yI, e.zI) : open_rect();
-            if (!isinf(rect.x)) cx = A.z, cz = A.w, R = B.z * 1.0001f;
+            s.hole(e, make_float4(A.x, B.x, B.y, A.y), B.z);
         } else if (j < k.count) {
             const float4* r = &ws.rec[2 * k.nh + 4 * (j - k.nh)];
             const float4 A = r[0], B = r[1];
-            rect = r[3];
-            if (!isinf(rect.x)) {
-                const float hw = 0.5f * B.z, hh = 0.5f * r[2].x;
-                cx = e.xI - A.x, cz = e.zI - A.z, R = 0.0f;
-                ax = hw * B.x, az = -hw * B.y, bx = hh * B.y, bz = hh * B.x;
-            }
+            s.crystal(e, r[3], A.x, A.z, 0.5f * B.z, 0.5f * r[2].x, B.x, -B.y);
         }
-        const float sx = fabsf(cx) + fabsf(ax) + fabsf(bx) + 1e-3f, sz = fabsf(cz) + fabsf(az) + fabsf(bz) + 1e-3f;
         unsigned mine = 0u;
         for (int r = r0; r < r1; ++r) {
-            const float4 box = ws.box[r];
-            const float mx = 0.5f * (box.x + box.y), mz = 0.5f * (box.z + box.w);
-            const float ex = 0.5f * (box.y - box.x) + kSlopeMargin, ez = 0.5f * (box.w - box.z) + kSlopeMargin;
-            const float far = fabsf(cx * mz - cz * mx) - fabsf(ax * mz - az * mx) - fabsf(bx * mz - bz * mx);
-            const bool meets = rects_overlap(rect, box) && !(far > sx * ez + sz * ex + R * ws.reach[r]);
-            const unsigned m = __ballot_sync(0xffffffffu, meets);
+            const unsigned m = __ballot_sync(0xffffffffu, s.meets(ws.box[r], ws.reach[r]));
             if (lane == r) mine = m;
         }
         if (lane >= r0 && lane < r1) ws.mask[w][lane] = mine;
@@ -337,7 +410,8 @@ struct Entries {
     int r, w, w1, j0, j1;
     unsigned m;
 
-    __device__ __forceinline__ Entries(const RefWarp& ws, int r_, int j0_, int j1_) : mask(ws.mask), r(r_), j0(j0_), j1(j1_)
+    __device__ __forceinline__ Entries(const unsigned (*mask_)[32], int r_, int j0_, int j1_)
+        : mask(mask_), r(r_), j0(j0_), j1(j1_)
     {
         w = j0 >> 5;
         w1 = (j1 + 31) >> 5;
@@ -364,6 +438,12 @@ struct Entries {
         m &= m - 1u;
         return j;
     }
+};
+
+// Attenuation of one ray so far: accumulated mu L, and the open layer with its hole length.
+struct Walk {
+    float att, len;
+    int lay;
 };
 
 // A ray from the voxel in the walk over holes: the terms of the reference cylinder chord
@@ -464,7 +544,7 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const 
         ray_end(e, q.x, q.y, q.z, xD, yD, zD);
         HoleRay c;
         hole_ray_init(c, xD - e.xI, yD - e.yI, zD - e.zI);
-        Walk s{0.0f, 0.0f, lay0, 0, 0, 0, 0};
+        Walk s{0.0f, 0.0f, lay0};
         bool skip;
         if (first) {
             const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;             // open rectangles: slope 0
@@ -475,7 +555,7 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const 
             s.len = ws.len[(r & 7) * 32 + lane];
             skip = isinf(s.att);
         }
-        Entries it(ws, r, 0, nh);
+        Entries it(ws.mask, r, 0, nh);
         if (EVEN && it.more()) {
             const float4 B = ws.rec[1];
             const int m = layer_of_hole(g, ws.id[0]);
@@ -567,7 +647,7 @@ __device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, con
 {
     const Elem& e = ws.elem;
     for (int r = r0; r < r1; ++r) {
-        Entries it(ws, r, nh, count);
+        Entries it(ws.mask, r, nh, count);
         if (!it.more()) continue;
         int ix, iy, iz;
         dv.indices(r, lane, ix, iy, iz);
@@ -822,43 +902,6 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
         for (int off = 16; off > 0; off >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, off);
         return dacc;
     }
-}
-
-__device__ __forceinline__ float warp_min(float x)
-{
-    float y;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ float warp_max(float x)
-{
-    float y;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// ws.box and ws.reach of the first n rounds, from the rays themselves.
-template <class Div>
-__device__ __forceinline__ void ray_boxes(RefWarp& ws, const Div& dv, int n, int lane)
-{
-    const Elem& e = ws.elem;
-    for (int r = 0; r < n; ++r) {
-        int ix, iy, iz;
-        dv.indices(r, lane, ix, iy, iz);
-        const float3 q = dv.centre(ws, ix, iy, iz);
-        float x, y, z;
-        ray_end(e, q.x, q.y, q.z, x, y, z);
-        const float rdy = e.filt ? rcp_approx(y - e.yI) : 0.0f;
-        const float a = (x - e.xI) * rdy, b = (z - e.zI) * rdy;
-        const float4 box = make_float4(warp_min(a), warp_max(a), warp_min(b), warp_max(b));
-        if (lane == 0) {
-            const float px = fmaxf(fabsf(box.x), fabsf(box.y)), pz = fmaxf(fabsf(box.z), fabsf(box.w));
-            ws.box[r] = box;
-            ws.reach[r] = sqrtf(px * px + pz * pz);
-        }
-    }
-    __syncwarp();
 }
 
 // Element of the sampled form: the mean over the voxel's sx x sy x sz source points (centres of

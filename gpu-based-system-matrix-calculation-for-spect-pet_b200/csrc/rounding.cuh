@@ -54,4 +54,35 @@ __device__ __forceinline__ float sqrt_mid(float x)
     return __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(0.5f, y), g);
 }
 
+// a b + c d, a b - c d and x^2 + y^2 + z^2 with the fused product written out: which product of a
+// sum of two the compiler fuses depends on the code around it, so two kernels that inline the same
+// function can differ in the last bit.
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float diff2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ double sum2(double a, double b, double c, double d) { return __fma_rn(a, b, __dmul_rn(c, d)); }
+__device__ __forceinline__ double diff2(double a, double b, double c, double d) { return __fma_rn(a, b, -__dmul_rn(c, d)); }
+__device__ __forceinline__ float norm3(float x, float y, float z) { return __fmaf_rn(z, z, sum2(x, x, y, y)); }
+__device__ __forceinline__ double norm3(double x, double y, double z) { return __fma_rn(z, z, sum2(x, x, y, y)); }
+
+// Reciprocal and square root in double within about an ulp, from a float seed (relative error
+// 2^-22) by Newton's method: two steps square the error twice.  For arguments whose float value is
+// normal; no range branch.
+__device__ __forceinline__ double rcp64(double b)
+{
+    double y = (double)rcp_approx((float)b);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+
+__device__ __forceinline__ double sqrt64(double x)
+{
+    float f;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)x));
+    const double y = (double)f;
+    const double g = x * y, h = 0.5 * y;                  // sqrt(x), 1 / (2 sqrt(x)): coupled step
+    const double r = fma(-g, h, 0.5);
+    const double g1 = fma(g, r, g), h1 = fma(h, r, h);
+    return fma(fma(-g1, g1, x), h1, g1);
+}
+
 }  // namespace sysmat
