@@ -67,8 +67,6 @@ int upload_tasks(sysmat_batch_plan* p, const std::vector<sysmat_batch_item>& ite
     long long next = 0;
     for (const sysmat_batch_item& it : items) {
         const DevGeom& g = p->geoms[it.ctx];
-        const long long nxy = (long long)g.nx * g.ny;
-        const long long vlast = it.vox_begin + it.vox_count - 1;
         BatchTask k{};
         k.geom = it.ctx;
         k.rotation = it.rotation;
@@ -78,13 +76,9 @@ int upload_tasks(sysmat_batch_plan* p, const std::vector<sysmat_batch_item>& ite
         k.vox_count = it.vox_count;
         k.out = it.d_out;
         k.ld = it.ld;
-        k.iz0 = (int)(it.vox_begin / nxy);
-        k.iz1 = (int)(vlast / nxy);
-        k.nbx = (g.nx + bx - 1) / bx;
-        k.nby = (g.ny + by - 1) / by;
-        k.nbz = (k.iz1 - k.iz0 + 1 + bz - 1) / bz;
+        k.bricks = brick_grid(g, it.vox_begin, it.vox_count, bx, by, bz);
         k.item_begin = next;
-        next += (long long)k.nbx * k.nby * k.nbz * it.det_count;
+        next += (long long)k.bricks.nbx * k.bricks.nby * k.bricks.nbz * it.det_count;
         t.push_back(k);
     }
     if ((int)t.size() > p->task_capacity) return SYSMAT_ERR_CAPACITY;
@@ -94,9 +88,6 @@ int upload_tasks(sysmat_batch_plan* p, const std::vector<sysmat_batch_item>& ite
     p->launch.tasks = p->d_tasks;
     p->launch.n_tasks = (int)t.size();
     p->launch.total_items = next;
-    p->launch.bx = bx;
-    p->launch.by = by;
-    p->launch.bz = bz;
     p->launch.work_counter = p->d_counter;
     return SYSMAT_OK;
 }

@@ -80,6 +80,7 @@ struct Superset {
     int warp_cnt[kWarps];
     int s_count;                         // superset size; -1 = superset overflowed, use all
     long long item;
+    unsigned short slot[512];            // the brick's voxels that belong to the block
 };
 
 struct BlockSmem : Superset {
@@ -531,6 +532,26 @@ __device__ __forceinline__ bool init_element(const DevGeom& g, float4* plate_inn
 #include "pe_fp64.cuh"
 #include "pe_local.cuh"
 
+// Appends `value` of the threads with `in`, in thread order, to list[n ..] (capacity cap) and returns
+// how many there were.  All threads of the block call it.
+__device__ __forceinline__ int block_append(Superset& bs, bool in, unsigned short value, unsigned short* list, int n,
+                                            int cap, int lane, int wid)
+{
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) bs.warp_cnt[wid] = __popc(m);
+    __syncthreads();
+    int off = n, tot = 0;
+    for (int k = 0; k < kWarps; ++k) {
+        const int c = bs.warp_cnt[k];
+        if (k < wid) off += c;
+        tot += c;
+    }
+    const int pos = off + __popc(m & ((1u << lane) - 1u));
+    if (in && pos < cap) list[pos] = value;
+    __syncthreads();
+    return tot;
+}
+
 // Block superset of the reference cone test over all voxels within radius rho of
 // (cx, cy, cz): keep object o when |u_o - u_d| <= (rho + r_o)/(L_o - rho)
 // + (rho + r_d)/(L_d - rho) + 1e-4 at the centre (each direction moves by at most
@@ -563,21 +584,7 @@ __device__ void build_superset(const DevGeom& g, Superset& bs, int d, float cx, 
                 keep = sqrtf(dx * dx + dy * dy + dz * dz) <= thr;
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) bs.warp_cnt[wid] = __popc(m);
-        __syncthreads();
-        int off = running, tot = 0;
-        for (int k = 0; k < kWarps; ++k) {
-            const int c = bs.warp_cnt[k];
-            if (k < wid) off += c;
-            tot += c;
-        }
-        const int pos = off + __popc(m & ((1u << lane) - 1u));
-        if (keep && pos < kSuperCap) {
-            bs.sid[pos] = (unsigned short)i;
-        }
-        running += tot;
-        __syncthreads();
+        running += block_append(bs, keep, (unsigned short)i, bs.sid, running, kSuperCap, lane, wid);
     }
     if (threadIdx.x == 0) bs.s_count = (running <= kSuperCap) ? running : -1;
     __syncthreads();
@@ -600,22 +607,37 @@ template <class Smem>
 __device__ __forceinline__ Superset& superset_of(Smem& sm) { return sm.sup; }
 __device__ __forceinline__ Superset& superset_of(BlockSmem& sm) { return sm; }
 
-// One work item: crystal det_begin + di against one voxel brick of bx x by x bz voxels (brick
-// (gx, gy, gz) of the block's grid starting at z-plane iz0).  The block builds the cone
+// One work item: crystal det_begin + di against voxel brick b of the block's grid.  The block builds the cone
 // superset of the brick, then its warps take the brick's voxels in turn.
 // SAMPLED: elements of the sampled form `smp` (source points anywhere in the voxels: the
 // superset radius grows by half a voxel diagonal).
 template <int MODE, bool COUNT, bool ELL = false, bool SAMPLED = false>
 __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE, ELL>::type& sm, int lane, int wid,
-                                         const BrickOut& O, int di, int gx, int gy, int gz, int iz0, int iz1,
-                                         int bx, int by, int bz, float cr, float sr,
+                                         const BrickOut& O, int di, const BrickGrid& B, long long b, float cr,
+                                         float sr,
                                          unsigned long long* counters, const Sampling* smp = nullptr,
                                          float rotation = 0.0f)
 {
     Superset& sup = superset_of(sm);
-    const int x0 = gx * bx, y0 = gy * by, z0 = iz0 + gz * bz;
-    const int x1 = min(x0 + bx, g.nx) - 1, y1 = min(y0 + by, g.ny) - 1, z1 = min(z0 + bz, iz1 + 1) - 1;
+    const int gz = (int)(b / ((long long)B.nbx * B.nby));
+    const int rem = (int)(b - (long long)gz * B.nbx * B.nby);
+    const int gy = rem / B.nbx, gx = rem - gy * B.nbx;
+    const int bx = B.bx, by = B.by, bz = B.bz;
+    const int x0 = B.x0 + gx * bx, y0 = B.y0 + gy * by, z0 = B.z0 + gz * bz;
+    const int x1 = min(x0 + bx - 1, B.x1), y1 = min(y0 + by - 1, B.y1), z1 = min(z0 + bz - 1, B.z1);
     const int d = O.det_begin + di;
+    // the brick's voxels inside the block, so that a ragged block's warps share them evenly (and a
+    // brick without any builds no superset)
+    const int n_slots = bx * by * bz;
+    int n_active = 0;
+    for (int base = 0; base < n_slots; base += kThreads) {
+        const int slot = base + threadIdx.x;
+        const int ix = x0 + slot % bx, iy = y0 + (slot / bx) % by, iz = z0 + slot / (bx * by);
+        const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
+        const bool in = slot < n_slots && ix <= x1 && iy <= y1 && iz <= z1 && v >= O.vox_begin && v <= O.vlast;
+        n_active += block_append(sup, in, (unsigned short)slot, sup.slot, n_active, 512, lane, wid);
+    }
+    if (n_active == 0) return;
     // brick centre and radius from its extreme voxel centres (rotation about z keeps lengths)
     float ax, ay, az, bxx, byy, bzz;
     voxel_centre(g, x0 + g.nx * ((long long)y0 + g.ny * z0), 1.0f, 0.0f, ax, ay, az);
@@ -625,12 +647,11 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
                              (bzz - az) * (bzz - az)) + 1e-3f;
     if constexpr (SAMPLED) rho += 0.5f * sqrtf(g.wx * g.wx + g.wy * g.wy + g.wz * g.wz);
     build_superset(g, sup, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho);
-    const int n_slots = bx * by * bz;
-    for (int slot = wid; slot < n_slots; slot += kWarps) {
-        const int ox = slot % bx, oy = (slot / bx) % by, oz = slot / (bx * by);
-        const int ix = x0 + ox, iy = y0 + oy, iz = z0 + oz;
+    for (int i = wid; i < n_active; i += kWarps) {
+        const int slot = sup.slot[i];
+        const int ix = x0 + slot % bx, iy = y0 + (slot / bx) % by, iz = z0 + slot / (bx * by);
         const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
-        if (ix < g.nx && iy < g.ny && iz <= z1 && v >= O.vox_begin && v <= O.vlast) {
+        {
             float val;
             if constexpr (MODE <= 1 && SAMPLED) {
                 val = (float)pe_element_sampled<ELL>(g, sup, sm.w[wid], d, v, cr, sr, lane, *smp);
@@ -653,7 +674,7 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
 
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
 __global__ void __launch_bounds__(kThreads, 2)
-pe_kernel(DevGeom g, PeLaunch L)
+pe_kernel(DevGeom g, PeLaunch L, BrickGrid B)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<typename SmemOf<MODE, ELL>::type*>(smem_raw);
@@ -661,13 +682,8 @@ pe_kernel(DevGeom g, PeLaunch L)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float ang = L.rotation * g.angle_step;           // :1006
     const float cr = cosf(ang), sr = sinf(ang);
-    const long long nxy = (long long)g.nx * g.ny;
     const long long vlast = L.vox_begin + L.vox_count - 1;
-    const int iz0 = (int)(L.vox_begin / nxy), iz1 = (int)(vlast / nxy);
-    constexpr int bx = 4, by = 4, bz = 2;                 // voxel brick of one work item
-    const int nbx = (g.nx + bx - 1) / bx, nby = (g.ny + by - 1) / by;
-    const int nbz = (iz1 - iz0 + 1 + bz - 1) / bz;
-    const long long n_bricks = (long long)nbx * nby * nbz;
+    const long long n_bricks = (long long)B.nbx * B.nby * B.nbz;
     const long long total = n_bricks * L.det_count;
     const BrickOut O{L.out, L.ld, L.vox_begin, vlast, L.det_begin, L.sub_out, L.det_count};
     for (;;) {
@@ -678,11 +694,7 @@ pe_kernel(DevGeom g, PeLaunch L)
         if (item >= total) break;
         const int di = (int)(item / n_bricks);
         const long long b = item - (long long)di * n_bricks;
-        const int gz = (int)(b / ((long long)nbx * nby));
-        const int rem = (int)(b - (long long)gz * nbx * nby);
-        const int gy = rem / nbx, gx = rem - gy * nbx;
-        pe_brick<MODE, COUNT, ELL, SAMPLED>(g, sm, lane, wid, O, di, gx, gy, gz, iz0, iz1, bx, by, bz, cr, sr,
-                                            L.counters, &L.smp, L.rotation);
+        pe_brick<MODE, COUNT, ELL, SAMPLED>(g, sm, lane, wid, O, di, B, b, cr, sr, L.counters, &L.smp, L.rotation);
     }
 }
 
@@ -732,22 +744,32 @@ __global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
         const DevGeom& g = sm.g;
         const float ang = T.rotation * g.angle_step;       // :1006
         const float cr = cosf(ang), sr = sinf(ang);
-        const long long n_bricks = (long long)T.nbx * T.nby * T.nbz;
+        const long long n_bricks = (long long)T.bricks.nbx * T.bricks.nby * T.bricks.nbz;
         const long long local = item - T.item_begin;
         const int di = (int)(local / n_bricks);
         const long long b = local - (long long)di * n_bricks;
-        const int gz = (int)(b / ((long long)T.nbx * T.nby));
-        const int rem = (int)(b - (long long)gz * T.nbx * T.nby);
-        const int gy = rem / T.nbx, gx = rem - gy * T.nbx;
         const BrickOut O{T.out, T.ld, T.vox_begin, T.vox_begin + T.vox_count - 1, T.det_begin, nullptr, T.det_count};
-        pe_brick<MODE, false, ELL>(g, sm.bs, lane, wid, O, di, gx, gy, gz, T.iz0, T.iz1, B.bx, B.by, B.bz, cr,
-                                   sr, nullptr, nullptr, T.rotation);
+        pe_brick<MODE, false, ELL>(g, sm.bs, lane, wid, O, di, T.bricks, b, cr, sr, nullptr, nullptr, T.rotation);
     }
 }
 
 #include "pe_adjoint.cuh"
 
 }  // namespace
+
+// Brick of a block's work items: 16 voxels (two elements per warp share one superset; the superset of
+// a 32- or 64-voxel brick is larger and measured 2-11 % slower per element), 4 x 4 in a plane, or
+// as many rows as the block has.  Blocks of few elements take 8 or 4 voxels, so that every block of
+// the grid gets an item: a 36 x 128 matrix took 582 us in 32-voxel bricks, 328 in 16, 299 in 8.
+static BrickGrid choose_bricks(const DevGeom& g, const PeLaunch& L, int blocks)
+{
+    const BrickGrid all = brick_grid(g, L.vox_begin, L.vox_count, 1, 1, 1);
+    const int rows = all.y1 - all.y0 + 1;
+    const double elements = (double)L.det_count * (double)L.vox_count;
+    const int voxels = elements >= 32.0 * blocks ? 16 : (elements >= 4.0 * blocks ? 8 : 4);
+    const int by = rows >= 4 && voxels == 16 ? 4 : (rows >= 2 ? 2 : 1);
+    return brick_grid(g, L.vox_begin, L.vox_count, voxels / by, by, 1);
+}
 
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>
 static int launch_mode(const DevGeom& g, const PeLaunch& L, int num_sms, cudaStream_t stream)
@@ -767,7 +789,7 @@ static int launch_mode(const DevGeom& g, const PeLaunch& L, int num_sms, cudaStr
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pe_kernel<MODE, COUNT, ELL, SAMPLED>, kThreads, smem);
     if (per_sm < 1) per_sm = 1;
-    pe_kernel<MODE, COUNT, ELL, SAMPLED><<<num_sms * per_sm, kThreads, smem, stream>>>(g, L);
+    pe_kernel<MODE, COUNT, ELL, SAMPLED><<<num_sms * per_sm, kThreads, smem, stream>>>(g, L, choose_bricks(g, L, num_sms * per_sm));
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

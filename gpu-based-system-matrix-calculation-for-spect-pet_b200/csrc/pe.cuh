@@ -23,6 +23,33 @@ struct Sampling {
     int sx = 1, sy = 1, sz = 1;
 };
 
+// The bricks (work items) of a voxel block: bricks of bx x by x bz voxels over the voxel ranges that
+// the block touches, from (x0, y0, z0).
+struct BrickGrid {
+    int bx, by, bz;
+    int x0, y0, z0, x1, y1, z1;            // inclusive ranges
+    int nbx, nby, nbz;
+};
+
+// The grid of voxels [vox_begin, vox_begin + vox_count) in bricks of the given shape.
+inline BrickGrid brick_grid(const DevGeom& g, long long vox_begin, long long vox_count, int bx, int by, int bz)
+{
+    const long long nxy = (long long)g.nx * g.ny, last = vox_begin + vox_count - 1;
+    BrickGrid b{bx, by, bz, 0, 0, (int)(vox_begin / nxy), g.nx - 1, g.ny - 1, (int)(last / nxy), 0, 0, 0};
+    if (b.z0 == b.z1) {                    // within one plane: the rows it touches
+        b.y0 = (int)(vox_begin % nxy / g.nx);
+        b.y1 = (int)(last % nxy / g.nx);
+        if (b.y0 == b.y1) {                // within one row
+            b.x0 = (int)(vox_begin % g.nx);
+            b.x1 = (int)(last % g.nx);
+        }
+    }
+    b.nbx = (b.x1 - b.x0 + bx) / bx;
+    b.nby = (b.y1 - b.y0 + by) / by;
+    b.nbz = (b.z1 - b.z0 + bz) / bz;
+    return b;
+}
+
 struct PeLaunch {
     int det_begin, det_count;
     long long vox_begin, vox_count;
@@ -42,7 +69,7 @@ struct PeLaunch {
 };
 
 // One (geometry, rotation, detector x voxel block) task of a batched launch.  The host fills
-// the brick grid of the block (nbx x nby x nbz bricks over z-planes iz0..iz1) and the first
+// the brick grid of the block and the first
 // global item number of the task; items are (row, brick) pairs, row-major.
 struct BatchTask {
     int geom;                              // index into the launch's geometry array
@@ -52,7 +79,7 @@ struct BatchTask {
     float* out;
     long long ld;
     long long item_begin;
-    int nbx, nby, nbz, iz0, iz1;
+    BrickGrid bricks;
 };
 
 struct BatchLaunch {
@@ -60,7 +87,6 @@ struct BatchLaunch {
     const BatchTask* tasks;                // device array, item_begin ascending
     int n_tasks;
     long long total_items;
-    int bx, by, bz;
     unsigned long long* work_counter;      // zeroed before the launch
 };
 
