@@ -38,8 +38,6 @@ namespace {
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kSuperCap = 1024;         // block superset capacity (objects)
-constexpr int kChunk = 256;             // per-warp kept-object chunk
-constexpr int kRound = 64;              // per-warp round buffer
 constexpr float kSlopeMargin = 2e-4f;   // slope units; >> FP32 position error / depth
 constexpr float kMinDepth = 1.0f;       // mm; slope rectangles need objects this far behind
 
@@ -55,24 +53,6 @@ struct Elem {
     bool filt;
 };
 
-struct WarpSmem {
-    // kept objects of the element (reference cone test + bundle filter), reference order
-    float4 rect[kChunk];
-    int id[kChunk];                      // holes: hole index; crystals: n_holes + crystal
-    // the current round's objects (kept objects whose rectangle meets the round's rays),
-    // with their geometry, so the walk reads contiguous shared memory:
-    //   hole:    A = (x, z, R, mu),   B = (y1, y2, voxel x - x, voxel z - z)
-    //   crystal: A = (x, y, z, mu),   B = (cos(-rot), sin(-rot), w, t),
-    //            C = (h, voxel x, y, z in the crystal's frame)
-    float4 rr[kRound], ra[kRound], rb[kRound], rc[kRound];
-    int rl[kRound];                      // layer of a hole entry; n_layers for crystals
-    float4 inner[kMaxLayers];            // plate "through both faces" slope rectangle
-    union {
-        float chain[256];                // contributions of sub-elements 256p .. 256p+255
-        double e64[32];                  // FP64 mode: the element's constants (Elem64)
-    };
-};
-
 // The objects that may pass the cone test for some voxel of a block's brick, in the reference's
 // order, and the block's work item.
 struct Superset {
@@ -81,10 +61,6 @@ struct Superset {
     int s_count;                         // superset size; -1 = superset overflowed, use all
     long long item;
     unsigned short slot[512];            // the brick's voxels that belong to the block
-};
-
-struct BlockSmem : Superset {
-    WarpSmem w[kWarps];
 };
 
 __device__ __forceinline__ bool in_rect(const float4& r, float a, float b)
@@ -158,303 +134,6 @@ __device__ __forceinline__ int layer_of_hole(const DevGeom& g, int h)
     int m = 0;
     while (m + 1 < g.n_layers && h >= g.layer[m + 1].hole_begin) ++m;
     return m;
-}
-
-// Reference cone test of object i against element e (:1120-1184), then the bundle filter.
-// Returns true if the object is kept; rect receives its slope rectangle.
-__device__ __forceinline__ bool keep_object(const DevGeom& g, const Elem& e, int i, float4 od,
-                                            int d, float4& rect)
-{
-    rect = open_rect();
-    bool keep;
-    if (i < g.n_holes) {
-        const float L = sqrtf((e.xI - od.x) * (e.xI - od.x) + (e.yI - od.y) * (e.yI - od.y) +
-                              (e.zI - od.z) * (e.zI - od.z));
-        const float crit = od.w / L;
-        const float vx = (od.x - e.xI) / L, vy = (od.y - e.yI) / L, vz = (od.z - e.zI) / L;
-        keep = sqrtf((vz - e.uz) * (vz - e.uz) + (vy - e.uy) * (vy - e.uy) + (vx - e.ux) * (vx - e.ux)) <=
-               crit + e.crit_self;
-        if (keep && e.filt) {
-            rect = hole_rect(__ldg(&g.hole.a[i]), __ldg(&g.hole.b[i].x), e.xI, e.yI, e.zI);
-            keep = rects_overlap(rect, e.rd);
-        }
-    } else {
-        const int o = i - g.n_holes;
-        if (o == d) return false;
-        const float L = sqrtf((e.xI - od.x) * (e.xI - od.x) + (e.yI - od.y) * (e.yI - od.y) +
-                              (e.zI - od.z) * (e.zI - od.z));
-        const float crit = od.w / L / 2.0f;
-        const float vx = (od.x - e.xI) / L, vy = (od.y - e.yI) / L, vz = (od.z - e.zI) / L;
-        keep = sqrtf((vz - e.uz) * (vz - e.uz) + (vy - e.uy) * (vy - e.uy) + (vx - e.ux) * (vx - e.ux)) <=
-               crit + e.crit_self;
-        if (keep && e.filt) {
-            rect = crystal_rect(__ldg(&g.cry.pos[o]), __ldg(&g.cry.size[o]), __ldg(&g.cry.trig[o]),
-                                e.xI, e.yI, e.zI);
-            keep = rects_overlap(rect, e.rd);
-        }
-    }
-    return keep;
-}
-
-// Fill the warp's chunk with kept objects, scanning source positions [cursor, n_src).
-// Source = block superset (n_src = s_count) or all objects.  Returns the new cursor; the
-// chunk count goes to *count.  Stops early when the chunk could overflow.
-__device__ int build_chunk(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, const Elem& e,
-                           int d, int cursor, int n_src, bool from_super, int lane, int* count)
-{
-    int n = 0;
-    while (cursor < n_src && n <= kChunk - 32) {
-        const int j = cursor + lane;
-        bool keep = false;
-        float4 rect;
-        int id = 0;
-        if (j < n_src) {
-            id = from_super ? bs.sid[j] : j;
-            keep = keep_object(g, e, id, object_data(g, id), d, rect);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            const int pos = n + __popc(m & ((1u << lane) - 1u));
-            ws.rect[pos] = rect;
-            ws.id[pos] = id;
-        }
-        n += __popc(m);
-        cursor += 32;
-    }
-    __syncwarp();
-    *count = n;
-    return cursor < n_src ? cursor : n_src;
-}
-
-// Terms of the reference cylinder chord (PESysMatGen.cu:688-799) that depend only on the
-// ray (voxel -> sub-element) and on the cap planes y1, y2.  Hoisting them out of the
-// per-hole evaluation keeps every float identical: each is the same operation on the same
-// operands as in the per-hole formula, and the divisions that share a divisor (tio, ky, kk)
-// go through its correctly rounded reciprocal (div_by: the quotient IEEE division gives).
-struct RayCyl {
-    float xi, yi, zi, tio, kx, ky, kz, rx, rz, kk;
-    float iky, ikk;              // RN(1 / ky), RN(1 / kk)
-    float y1, y2;                // cap planes the cached terms below belong to
-    float ta, tb, xl, xr, zl, zr;
-    float full;                  // chord of a ray inside the hole at both caps
-};
-
-__device__ __forceinline__ void ray_cyl_init(RayCyl& c, float xi, float yi, float zi, float xo, float yo,
-                                             float zo)
-{
-    const float dx = xo - xi, dy = yo - yi, dz = zo - zi;
-    c.xi = xi; c.yi = yi; c.zi = zi;
-    c.tio = sqrt_mid(dx * dx + dy * dy + dz * dz);
-    const float itio = rcp_rn(c.tio);
-    c.kx = div_by(dx, c.tio, itio);
-    c.ky = div_by(dy, c.tio, itio);
-    c.kz = div_by(dz, c.tio, itio);
-    c.iky = rcp_rn(c.ky);
-    if (fabsf(c.ky) >= kMinDivisor) {
-        c.rx = div_by(c.kx, c.ky, c.iky);
-        c.rz = div_by(c.kz, c.ky, c.iky);
-    } else {                     // a ray along the plates
-        c.rx = c.kx / c.ky;
-        c.rz = c.kz / c.ky;
-    }
-    c.kk = c.kx * c.kx + c.kz * c.kz;
-    c.ikk = rcp_rn(c.kk);
-    c.y1 = NAN;                  // no cap planes cached yet (NaN never compares equal)
-    c.y2 = NAN;
-}
-
-__device__ __forceinline__ void ray_cyl_caps(RayCyl& c, float y1, float y2)
-{
-    if (y1 == c.y1 && y2 == c.y2) return;
-    c.y1 = y1;
-    c.y2 = y2;
-    c.xl = c.xi + c.rx * (y1 - c.yi);
-    c.xr = c.xi + c.rx * (y2 - c.yi);
-    c.zl = c.zi + c.rz * (y1 - c.yi);
-    c.zr = c.zi + c.rz * (y2 - c.yi);
-    if (fabsf(c.ky) >= kMinDivisor) {
-        c.ta = div_by(y1 - c.yi, c.ky, c.iky);
-        c.tb = div_by(y2 - c.yi, c.ky, c.iky);
-    } else {
-        c.ta = (y1 - c.yi) / c.ky;
-        c.tb = (y2 - c.yi) / c.ky;
-    }
-    c.full = fabsf(c.tb - c.ta);
-    if (c.ta <= 0.0001f || c.tb <= 0.0001f || c.ta >= c.tio || c.tb >= c.tio) c.full = 0.0f;
-    // closer than 0.001: the reference returns 0; with both cap parameters 0 every case below does
-    if (fabsf(y1 - y2) < 0.001f) c.ta = c.tb = c.full = 0.0f;
-}
-
-// Cylinder chord of hole (xc, zc, r), (ox, oz) = voxel - centre, with cap planes already
-// cached in c.  Straight-line: the reference's four cap/side cases are selects, so a warp
-// whose lanes meet different cases runs the code once, and two entries interleave (the four
-// returns of the branching form each cost a divergent pass).
-__device__ __forceinline__ float ray_cyl_chord(const RayCyl& c, float xc, float zc, float r, float ox, float oz)
-{
-    const bool fl = (c.xl - xc) * (c.xl - xc) + (c.zl - zc) * (c.zl - zc) <= r * r;
-    const bool fr = (c.xr - xc) * (c.xr - xc) + (c.zr - zc) * (c.zr - zc) <= r * r;
-    const float disc = c.kk * r * r - (c.kx * oz - c.kz * ox) * (c.kx * oz - c.kz * ox);
-    const bool meets = disc > 0.00001f;
-    const float sd = sqrt_mid(meets ? disc : 1.0f);
-    const float t1 = div_by(-(c.kx * ox + c.kz * oz) - sd, c.kk, c.ikk);
-    const float t2 = div_by(-(c.kx * ox + c.kz * oz) + sd, c.kk, c.ikk);
-    const float ea = fl ? c.ta : t1, eb = fr ? c.tb : t2;
-    const bool ok = meets && (fl || fr || (t1 >= c.ta && t2 <= c.tb)) &&
-                    !(eb <= 0.0001f || ea <= 0.0001f || eb >= c.tio || ea >= c.tio);
-    return (fl && fr) ? c.full : (ok ? eb - ea : 0.0f);
-}
-
-__device__ __forceinline__ float ray_cyl_chord(const RayCyl& c, float xc, float zc, float r)
-{
-    return ray_cyl_chord(c, xc, zc, r, c.xi - xc, c.zi - zc);
-}
-
-// Slope-space shadow of a y-aligned object (hole cylinder, or crystal in the disk around its
-// xz footprint) seen from the voxel: every line from the voxel that meets the object at a
-// depth y in [y0, y1] has slopes within rho(y) = R/(y - yI) of the point c(y) on the
-// segment c(y0) -> c(y1), so within rho(y0) of that segment (the capsule; its radius is
-// inflated by the slope margin).
-struct Capsule {
-    float ax, az, dx, dz, rho;    // c(y0), c(y1) - c(y0), radius
-};
-
-__device__ __forceinline__ Capsule capsule_of(float xo, float zo, float y0, float y1, float R, const Elem& e)
-{
-    const float r0 = rcp_approx(y0 - e.yI), r1 = rcp_approx(y1 - e.yI);
-    Capsule c;
-    c.ax = (xo - e.xI) * r0;
-    c.az = (zo - e.zI) * r0;
-    c.dx = (xo - e.xI) * r1 - c.ax;
-    c.dz = (zo - e.zI) * r1 - c.az;
-    c.rho = R * r0 * 1.0001f + kSlopeMargin;
-    return c;
-}
-
-// False only when the capsule is separated from the box along x, along z, or along the
-// segment's normal; decided without divisions.
-__device__ __forceinline__ bool capsule_meets_box(const Capsule& c, float4 box)
-{
-    const float bx = c.ax + c.dx, bz = c.az + c.dz, rho = c.rho;
-    if (fminf(c.ax, bx) - rho > box.y || fmaxf(c.ax, bx) + rho < box.x) return false;
-    if (fminf(c.az, bz) - rho > box.w || fmaxf(c.az, bz) + rho < box.z) return false;
-    const float mx = 0.5f * (box.x + box.y) - c.ax, mz = 0.5f * (box.z + box.w) - c.az;
-    const float sep = fabsf(c.dx * mz - c.dz * mx) - (fabsf(c.dz) * 0.5f * (box.y - box.x) +
-                                                      fabsf(c.dx) * 0.5f * (box.w - box.z));
-    return !(sep > 0.0f && sep * sep > rho * rho * (c.dx * c.dx + c.dz * c.dz));
-}
-
-__device__ __forceinline__ bool capsule_meets_box(float xo, float zo, float y0, float y1, float R,
-                                                  const Elem& e, float4 box)
-{
-    return capsule_meets_box(capsule_of(xo, zo, y0, y1, R, e), box);
-}
-
-// Copy kept entries [k0, k1) whose rectangle and capsule meet the round's slope box into
-// the round buffer from position n, with their geometry (one entry per lane); returns the
-// new count.  Stops before the buffer could overflow; *next receives the first entry not
-// examined.
-template <bool ELL>
-__device__ __forceinline__ int fill_round(const DevGeom& g, WarpSmem& ws, const Elem& e, int k0, int k1,
-                                          float4 box, int n, int lane, int* next, int* nh)
-{
-    int k = k0;
-    while (k < k1 && n <= kRound - 32) {
-        const int kk = k + lane;
-        bool keep = false;
-        int id = 0;
-        float4 rect;
-        if (kk < k1) {
-            rect = ws.rect[kk];
-            keep = rects_overlap(rect, box);
-            if (keep && !isinf(rect.x)) {                  // finite: object wholly behind the voxel
-                id = ws.id[kk];
-                if (id < g.n_holes) {
-                    const float4 ha = __ldg(&g.hole.a[id]);
-                    const Capsule c = capsule_of(ha.x, ha.w, ha.y, ha.z, __ldg(&g.hole.b[id].x), e);
-                    keep = capsule_meets_box(c, box);
-                } else {
-                    const int o = id - g.n_holes;
-                    const float4 po = __ldg(&g.cry.pos[o]);
-                    const float4 so = __ldg(&g.cry.size[o]);
-                    keep = capsule_meets_box(po.x, po.z, po.y - 0.5f * so.y, po.y + 0.5f * so.y,
-                                             0.5f * sqrtf(so.x * so.x + so.z * so.z), e, box);
-                }
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) id = ws.id[kk];
-        *nh += __popc(__ballot_sync(0xffffffffu, keep && id < g.n_holes));
-        if (keep) {
-            const int pos = n + __popc(m & ((1u << lane) - 1u));
-            if (id < g.n_holes) {
-                const float4 ha = __ldg(&g.hole.a[id]);
-                const float4 hb = __ldg(&g.hole.b[id]);
-                ws.rr[pos] = rect;
-                ws.ra[pos] = make_float4(ha.x, ha.w, hb.x, hb.y);
-                ws.rb[pos] = make_float4(ha.y, ha.z, e.xI - ha.x, e.zI - ha.w);
-                if constexpr (ELL) {        // rho_x, rho_z, cos, sin; a batch may mix in circular systems
-                    ws.rc[pos] = g.hole_shape ? __ldg(&g.hole_shape[id]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
-                ws.rl[pos] = layer_of_hole(g, id);
-            } else {
-                const int o = id - g.n_holes;
-                const float4 po = __ldg(&g.cry.pos[o]);
-                const float4 so = __ldg(&g.cry.size[o]);
-                const float4 to = __ldg(&g.cry.trig[o]);
-                float xa, ya, za;                                   // :1305-1307
-                to_crystal_frame(po.x, po.y, po.z, to.z, to.w, e.xI, e.yI, e.zI, xa, ya, za);
-                ws.rr[pos] = rect;
-                ws.ra[pos] = make_float4(po.x, po.y, po.z, __ldg(&g.cry.mu[o].x));
-                ws.rb[pos] = make_float4(to.z, to.w, so.x, so.y);
-                ws.rc[pos] = make_float4(so.z, xa, ya, za);
-                ws.rl[pos] = g.n_layers;
-            }
-        }
-        n += __popc(m);
-        k += 32;
-    }
-    __syncwarp();
-    *next = k < k1 ? k : k1;
-    return n;
-}
-
-struct SubElem {
-    int ix, iy, iz;
-    float xDs, yDs, zDs, xD, yD, zD, dsq, sq, cosang, sa_a, sa_b;
-};
-
-// Sub-element (ix, iy, iz) of a crystal divided into fx x fy x fz (x, depth, z) parts.
-__device__ __forceinline__ SubElem sub_element_at(const Elem& e, int ix, int iy, int iz, float fx, float fy,
-                                                  float fz)
-{
-    SubElem q;
-    q.iz = iz;
-    q.ix = ix;
-    q.iy = iy;
-    q.xDs = -e.w / 2.0f + ((float)q.ix + 0.5f) / fx * e.w;   // :1207-1217
-    q.zDs = -e.h / 2.0f + ((float)q.iz + 0.5f) / fz * e.h;
-    q.yDs = -e.t / 2.0f + ((float)q.iy + 0.5f) / fy * e.t;
-    q.xD = e.xd + (q.xDs * e.cosr - q.zDs * e.sinr);
-    q.zD = e.zd + (q.xDs * e.sinr + q.zDs * e.cosr);
-    q.yD = e.yd + q.yDs;
-    q.dsq = (q.yD - e.yI) * (q.yD - e.yI) + (q.xD - e.xI) * (q.xD - e.xI) + (q.zD - e.zI) * (q.zD - e.zI);
-    q.sq = sqrtf(q.dsq);
-    q.cosang = (q.yD - e.yI) / q.sq;
-    if (e.filt) {             // every sub-element lies >= kMinDepth behind the voxel
-        const float rdy = __frcp_rn(q.yD - e.yI);
-        q.sa_a = (q.xD - e.xI) * rdy;
-        q.sa_b = (q.zD - e.zI) * rdy;
-    } else {                  // all rectangles are open: any finite slope passes
-        q.sa_a = 0.0f;
-        q.sa_b = 0.0f;
-    }
-    return q;
-}
-
-// Reference sub-element s = 128 iz + 16 ix + iy of the 8 x 16 x 8 division.
-__device__ __forceinline__ SubElem sub_element(const Elem& e, int s)
-{
-    return sub_element_at(e, (s >> 4) & 7, s & 15, s >> 7, 8.0f, 16.0f, 8.0f);
 }
 
 // box_chord of the segment voxel -> sub-element through a plate, out of line: few rays need it.
@@ -603,9 +282,6 @@ struct BrickOut {
 template <int MODE, bool ELL> struct SmemOf { using type = RefSmem; };       // float modes 0, 1
 template <bool ELL> struct SmemOf<2, ELL> { using type = IdSmem<Mode64>; };
 template <bool ELL> struct SmemOf<3, ELL> { using type = IdSmem<ModeLocal<ELL>>; };
-template <class Smem>
-__device__ __forceinline__ Superset& superset_of(Smem& sm) { return sm.sup; }
-__device__ __forceinline__ Superset& superset_of(BlockSmem& sm) { return sm; }
 
 // One work item: crystal det_begin + di against voxel brick b of the block's grid.  The block builds the cone
 // superset of the brick, then its warps take the brick's voxels in turn.
@@ -618,7 +294,7 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
                                          unsigned long long* counters, const Sampling* smp = nullptr,
                                          float rotation = 0.0f)
 {
-    Superset& sup = superset_of(sm);
+    Superset& sup = sm.sup;
     const int gz = (int)(b / ((long long)B.nbx * B.nby));
     const int rem = (int)(b - (long long)gz * B.nbx * B.nby);
     const int gy = rem / B.nbx, gx = rem - gy * B.nbx;
@@ -678,7 +354,7 @@ pe_kernel(DevGeom g, PeLaunch L, BrickGrid B)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<typename SmemOf<MODE, ELL>::type*>(smem_raw);
-    Superset& bs = superset_of(sm);
+    Superset& bs = sm.sup;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float ang = L.rotation * g.angle_step;           // :1006
     const float cr = cosf(ang), sr = sinf(ang);
@@ -715,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_batch_kernel(BatchLaunch B)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchSmem<MODE, ELL>& sm = *reinterpret_cast<BatchSmem<MODE, ELL>*>(smem_raw);
-    Superset& bs = superset_of(sm.bs);
+    Superset& bs = sm.bs.sup;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int cur_geom = -1;
     for (;;) {

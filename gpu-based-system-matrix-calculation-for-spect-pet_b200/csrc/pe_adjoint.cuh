@@ -23,36 +23,26 @@
 
 constexpr int kThetaN = 7;
 
-// Partials of the chord of ray_cyl_chord (same case analysis) with respect to the hole radius
-// r, the centre (xc, zc) and a common shift dy of both cap planes.  Zero for a zero chord.
+// Partials of a hole's chord with respect to its radius r, its centre (x, z) and a common shift dy
+// of both cap planes (elliptical holes: dr is the partial of the frame angle).
 struct CylGrad {
     float dr, dx, dz, dy;
 };
 
-__device__ __forceinline__ float ray_cyl_chord_grad(const RayCyl& c, float xc, float zc, float r, CylGrad& gr)
+// Partials of hole_chord (same case analysis), zero for a zero chord L and for cap to cap: with
+// disc = kk r^2 - C^2, the side crossings are t1,2 = (-(kx ox + kz oz) -+ sqrt(disc)) / kk.
+__device__ __forceinline__ CylGrad hole_chord_grad(const HoleRay& c, const ChordParts& p, float L, float r)
 {
-    gr = CylGrad{0.0f, 0.0f, 0.0f, 0.0f};
-    const float L = ray_cyl_chord(c, xc, zc, r);
-    if (L == 0.0f) return L;
-    const bool fl = (c.xl - xc) * (c.xl - xc) + (c.zl - zc) * (c.zl - zc) <= r * r;
-    const bool fr = (c.xr - xc) * (c.xr - xc) + (c.zr - zc) * (c.zr - zc) <= r * r;
-    if (fl && fr) return L;                     // |tb - ta|: cap to cap, shift invariant
-    const float ox = c.xi - xc, oz = c.zi - zc;
-    const float C = c.kx * oz - c.kz * ox;     // cross term; disc = kk r^2 - C^2
-    const float sq = sqrtf(c.kk * r * r - C * C);
-    const float isq = 1.0f / sq, ikk = 1.0f / c.kk;
-    // side crossings t1,2 = (-(kx ox + kz oz) -+ sq) / kk
+    const float isq = rcp_rn(p.sd), C = p.cross;
     const float dsq_r = c.kk * r * isq, dsq_x = -C * c.kz * isq, dsq_z = C * c.kx * isq;
-    const float dt2_r = dsq_r * ikk, dt2_x = (c.kx + dsq_x) * ikk, dt2_z = (c.kz + dsq_z) * ikk;
-    const float dt1_r = -dsq_r * ikk, dt1_x = (c.kx - dsq_x) * ikk, dt1_z = (c.kz - dsq_z) * ikk;
-    if (!fl && !fr) {                           // side to side
-        gr = CylGrad{dt2_r - dt1_r, dt2_x - dt1_x, dt2_z - dt1_z, 0.0f};
-    } else if (fl) {                            // cap y1 to side: t2 - ta
-        gr = CylGrad{dt2_r, dt2_x, dt2_z, -1.0f / c.ky};
-    } else {                                    // side to cap y2: tb - t1
-        gr = CylGrad{-dt1_r, -dt1_x, -dt1_z, 1.0f / c.ky};
-    }
-    return L;
+    const float dt2_r = dsq_r * c.ikk, dt2_x = (c.kx + dsq_x) * c.ikk, dt2_z = (c.kz + dsq_z) * c.ikk;
+    const float dt1_r = -dsq_r * c.ikk, dt1_x = (c.kx - dsq_x) * c.ikk, dt1_z = (c.kz - dsq_z) * c.ikk;
+    // side to side t2 - t1; cap y1 to side t2 - ta (fl); side to cap y2 tb - t1 (fr)
+    const float a1 = p.fl ? 0.0f : 1.0f, a2 = p.fr ? 0.0f : 1.0f;
+    CylGrad g{a2 * dt2_r - a1 * dt1_r, a2 * dt2_x - a1 * dt1_x, a2 * dt2_z - a1 * dt1_z, 0.0f};
+    if (p.fl) g.dy = -c.iky;
+    if (p.fr) g.dy = c.iky;
+    return (L == 0.0f || (p.fl && p.fr)) ? CylGrad{0.0f, 0.0f, 0.0f, 0.0f} : g;
 }
 
 // Partials of the elliptical-cylinder chord (ell_chord, same case analysis) with respect to the
@@ -110,22 +100,51 @@ __device__ __forceinline__ float ell_chord_grad(float xi, float yi, float zi, fl
     return L;
 }
 
-// Walk state with the partials of att (index: theta order) and the current layer's sums of
-// hole-chord partials (radius, x, z, y, tilt).
+// The gradient's element runs the phases of pe_ref.cuh with each ray's partials kept beside its
+// attenuation (one loop with chords, partials and contributions in it held the kernel to its
+// instruction fetch, as there).
+constexpr int kGradRounds = 4;           // rounds per pass
+constexpr int kGradUnits = 128;
+constexpr int kGradRays = kGradRounds * 32;
+
+struct GradWarp {
+    static constexpr int units = kGradUnits;
+    float4 rec[2 * kGradUnits];          // as RefWarp
+    unsigned short id[kGradUnits];
+    unsigned mask[kGradUnits / 32][32];
+    float4 box[32];
+    float reach[32];
+    // [round][lane] of: attenuation outside crystal d (infinite: skipped) and its partials in theta order
+    float att[kGradRays], da[kThetaN][kGradRays];
+    float open[6][kGradRays];            // the open layer's length and partials (several chunks)
+    int cand[64];
+    float4 inner[kMaxLayers];
+    Elem elem;
+    float4 sub[32];
+};
+
+struct GradSmem {
+    Superset sup;
+    GradWarp w[kWarps];
+};
+
+// One ray's attenuation with its partials (index: theta order) and the open layer's sums of hole
+// chords and of their partials (radius, x, z, y, tilt).
 struct WalkGrad {
     float att, len;
     int lay;
-    float da[kThetaN];
+    float da[kThetaN];                   // da[1] belongs to the crystals
     float lr, lx, lz, ly, lp;
 };
 
-__device__ __forceinline__ void close_layers_grad(const DevGeom& g, WalkGrad& s, int upto, float cosang)
+__device__ __forceinline__ void close_layers_grad(const DevGeom& g, WalkGrad& s, int upto, const HoleRay& c)
 {
     while (s.lay < upto) {                                    // :1281-1284
         const float mu = g.layer[s.lay].mu_total;
-        const float lcol = g.layer[s.lay].thickness / cosang;
+        float lcol = div_by(g.layer[s.lay].thickness, c.ky, c.iky);
+        if (!c.steep) lcol = g.layer[s.lay].thickness / c.ky;
         if ((lcol - s.len) >= 0.00001f) {
-            s.att = s.att + mu * (lcol - s.len);
+            s.att = __fmaf_rn(mu, lcol - s.len, s.att);
             s.da[0] += lcol - s.len;
             s.da[2] -= mu * s.lr;
             s.da[3] -= mu * s.lx;
@@ -139,163 +158,169 @@ __device__ __forceinline__ void close_layers_grad(const DevGeom& g, WalkGrad& s,
     }
 }
 
-template <bool ELL>
-__device__ __forceinline__ void walk_round_grad(const DevGeom& g, const WarpSmem& ws, int nh, int nr, float xD,
-                                                float yD, float zD, float sa_a, float sa_b, float cosang,
-                                                RayCyl& rc, WalkGrad& s)
+// Attenuation outside crystal d and its partials, rounds [0, kGradRounds) of division dv.
+template <bool ELL, class Div>
+__device__ __forceinline__ void grad_pass(const DevGeom& g, GradWarp& ws, const Div& dv, const unsigned short* src, int n_src,
+                                          int d, bool single, int lane, int cursor, Kept& k)
 {
-    for (int j = 0; j < nh; ++j) {
-        const int m = ws.rl[j];
-        if (m != s.lay) close_layers_grad(g, s, m, cosang);
-        if (!in_rect(ws.rr[j], sa_a, sa_b)) continue;
-        const float4 A = ws.ra[j];               // x, z, R, mu of the hole
-        const float4 B = ws.rb[j];
-        CylGrad gr;
-        float tmp, dr = 0.0f, dth = 0.0f;        // radius and frame-angle partials
-        bool ell = false;
-        if constexpr (ELL) {
-            const float4 S = ws.rc[j];
-            if (S.x > 0.0f) {                    // elliptical hole: gr.dr holds the angle partial
-                tmp = ell_chord_grad(rc.xi, rc.yi, rc.zi, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w, gr);
-                dth = gr.dr;
-                ell = true;
+    const Elem& e = ws.elem;
+    int lay = 0;
+    for (bool first = true;; first = false) {
+        if (!single) cursor = build_kept(g, src, ws, e, d, first ? 0 : cursor, n_src, lane, k);
+        round_masks(ws, e, k, 0, kGradRounds, lane);
+        const bool last = single || cursor >= n_src;
+        const int lay1 = last || k.nh < k.count ? g.n_layers : (k.nh > 0 ? layer_of_hole(g, ws.id[k.nh - 1]) : lay);
+        for (int r = 0; r < kGradRounds; ++r) {                           // holes and layers
+            const int slot = r * 32 + lane;
+            int ix, iy, iz;
+            dv.indices(r, lane, ix, iy, iz);
+            const float3 q = dv.centre(ws, ix, iy, iz);
+            float xD, yD, zD;
+            ray_end(e, q.x, q.y, q.z, xD, yD, zD);
+            HoleRay c;
+            hole_ray_init(c, xD - e.xI, yD - e.yI, zD - e.zI);
+            WalkGrad s;
+            s.lay = lay;
+            bool skip;
+            if (first) {
+                s.att = s.len = 0.0f;
+                s.lr = s.lx = s.lz = s.ly = s.lp = 0.0f;
+#pragma unroll
+                for (int i = 0; i < kThetaN; ++i) s.da[i] = 0.0f;
+                const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;
+                skip = plate_penalty(g, ws.inner, e, xD, yD, zD, (xD - e.xI) * rdy, (zD - e.zI) * rdy, s.att) && g.nonneg_mu;
+            } else {
+                s.att = ws.att[slot];
+#pragma unroll
+                for (int i = 0; i < kThetaN; ++i) s.da[i] = ws.da[i][slot];
+                s.len = ws.open[0][slot], s.lr = ws.open[1][slot], s.lx = ws.open[2][slot];
+                s.lz = ws.open[3][slot], s.ly = ws.open[4][slot], s.lp = ws.open[5][slot];
+                skip = isinf(s.att);
+            }
+            float y1 = NAN, y2 = NAN;                     // cap planes at hand (NaN never compares equal)
+            Entries it(ws.mask, r, 0, k.nh);
+            while (it.more()) {
+                const int j = it.take();
+                const float4 A = ws.rec[2 * j], B = ws.rec[2 * j + 1];
+                const int id = ws.id[j], m = layer_of_hole(g, id);
+                if (m != s.lay) close_layers_grad(g, s, m, c);
+                float tmp = 0.0f, dr = 0.0f, dth = 0.0f;  // radius and frame-angle partials
+                CylGrad gr{0.0f, 0.0f, 0.0f, 0.0f};
+                float4 S = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if constexpr (ELL) {
+                    if (g.hole_shape) S = __ldg(&g.hole_shape[id]);
+                }
+                if (ELL && S.x > 0.0f) {                  // elliptical hole: gr.dr holds the angle partial
+                    if (!skip)
+                        tmp = ell_chord_grad(e.xI, e.yI, e.zI, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w, gr);
+                    dth = gr.dr;
+                } else {
+                    if (!(B.x == y1 && B.y == y2)) {
+                        y1 = B.x;
+                        y2 = B.y;
+                        hole_ray_caps(c, e, y1, y2);
+                    }
+                    ChordParts p;
+                    tmp = hole_chord(c, A, B.z, __fmul_rn(c.kk, B.z), __fmul_rn(B.z, B.z), &p);
+                    gr = hole_chord_grad(c, p, tmp, B.z);
+                    dr = gr.dr;
+                }
+                s.len = s.len + tmp;                                      // :1276-1278
+                s.att = __fmaf_rn(B.w, tmp, s.att);
+                const float dp = -A.y * gr.dx + A.x * gr.dz + dth;        // tilt about the y axis
+                s.lr += dr; s.lx += gr.dx; s.lz += gr.dz; s.ly += gr.dy; s.lp += dp;
+                if (B.w != 0.0f) {                                        // the hole's own medium
+                    s.da[2] += B.w * dr; s.da[3] += B.w * gr.dx; s.da[4] += B.w * gr.dy;
+                    s.da[5] += B.w * gr.dz; s.da[6] += B.w * dp;
+                }
+            }
+            if (s.lay < lay1) close_layers_grad(g, s, lay1, c);
+            ws.att[slot] = skip ? INFINITY : s.att;
+#pragma unroll
+            for (int i = 0; i < kThetaN; ++i) ws.da[i][slot] = s.da[i];
+            if (!single) {
+                ws.open[0][slot] = s.len, ws.open[1][slot] = s.lr, ws.open[2][slot] = s.lx;
+                ws.open[3][slot] = s.lz, ws.open[4][slot] = s.ly, ws.open[5][slot] = s.lp;
             }
         }
-        if (!ell) {
-            ray_cyl_caps(rc, B.x, B.y);
-            tmp = ray_cyl_chord_grad(rc, A.x, A.y, A.z, gr);
-            dr = gr.dr;
+        lay = lay1;
+        for (int r = 0; r < kGradRounds && k.nh < k.count; ++r) {         // other crystals (:1290-1325)
+            Entries it(ws.mask, r, k.nh, k.count);
+            if (!it.more()) continue;
+            const int slot = r * 32 + lane;
+            int ix, iy, iz;
+            dv.indices(r, lane, ix, iy, iz);
+            const float3 q = dv.centre(ws, ix, iy, iz);
+            float xD, yD, zD;
+            ray_end(e, q.x, q.y, q.z, xD, yD, zD);
+            const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;
+            const float sa_a = (xD - e.xI) * rdy, sa_b = (zD - e.zI) * rdy;
+            float att = ws.att[slot], da = ws.da[1][slot];
+            const bool skip = isinf(att);
+            do {
+                const float4* rec = &ws.rec[2 * k.nh + 4 * (it.take() - k.nh)];
+                const bool in = !skip && in_rect(rec[3], sa_a, sa_b);
+                if (!__any_sync(0xffffffffu, in)) continue;
+                float mu;
+                const float la = record_chord(rec, xD, yD, zD, in, mu);
+                att = __fmaf_rn(la, mu, att);
+                da += la;
+            } while (it.more());
+            ws.att[slot] = att;
+            ws.da[1][slot] = da;
         }
-        s.len = s.len + tmp;                                     // :1276-1278
-        s.att = s.att + A.w * tmp;
-        if (tmp != 0.0f) {
-            const float dp = -A.y * gr.dx + A.x * gr.dz + dth;   // tilt about the y axis
-            s.lr += dr; s.lx += gr.dx; s.lz += gr.dz; s.ly += gr.dy; s.lp += dp;
-            s.da[2] += A.w * dr; s.da[3] += A.w * gr.dx; s.da[4] += A.w * gr.dy;
-            s.da[5] += A.w * gr.dz; s.da[6] += A.w * dp;
-        }
+        __syncwarp();
+        if (last) break;
     }
-    if (nr <= nh) return;
-    if (s.lay < g.n_layers) close_layers_grad(g, s, g.n_layers, cosang);
-    for (int j = nh; j < nr; ++j) {
-        if (!in_rect(ws.rr[j], sa_a, sa_b)) continue;
-        const float4 A = ws.ra[j];
-        const float4 B = ws.rb[j];
-        const float4 C = ws.rc[j];
-        float xb, yb, zb;                                        // :1318-1320
-        to_crystal_frame(A.x, A.y, A.z, B.x, B.y, xD, yD, zD, xb, yb, zb);
-        const float la = box_chord(C.y, C.z, C.w, xb, yb, zb, -0.5f * B.z, -0.5f * B.w, -0.5f * C.x,
-                                   0.5f * B.z, 0.5f * B.w, 0.5f * C.x);
-        s.att = s.att + la * A.w;
-        s.da[1] += la;
-    }
-}
-
-// finish_sub_element with the partials of its contribution: dc[i] = d contrib / d theta_i.
-__device__ __forceinline__ float finish_sub_element_grad(const Elem& e, const SubElem& q, WalkGrad& s,
-                                                         float* dc)
-{
-    const float w = e.w, t = e.t, h = e.h;
-    const float ux1 = ((float)q.ix / 8.0f - 0.5f) * w;
-    const float ux2 = (((float)q.ix + 1.0f) / 8.0f - 0.5f) * w;
-    const float uy1 = ((float)q.iy / 16.0f - 0.5f) * t;
-    const float uy2 = (((float)q.iy + 1.0f) / 16.0f - 0.5f) * t;
-    const float uz1 = ((float)q.iz / 8.0f - 0.5f) * h;
-    const float uz2 = (((float)q.iz + 1.0f) / 8.0f - 0.5f) * h;
-    const float cbox[6] = {-w / 2.0f, -t / 2.0f, -h / 2.0f, w / 2.0f, t / 2.0f, h / 2.0f};
-    const float ubox[6] = {ux1, uy1, uz1, ux2, uy2, uz2};
-    float l1, l2;
-    box_chord_inside2(e.xIs, e.yIs, e.zIs, q.xDs, q.yDs, q.zDs, cbox, ubox, l1, l2);
-    const float att = s.att + (l1 - l2) * e.mu_t;
-    s.da[1] += l1 - l2;
-    const float eff = 1.0f * expf(-att);
-    const float xt = q.xDs + 1000.0f * (q.xDs - e.xIs) / q.sq;
-    const float yt = q.yDs + 1000.0f * (q.yDs - e.yIs) / q.sq;
-    const float zt = q.zDs + 1000.0f * (q.zDs - e.zIs) / q.sq;
-    const float labs = box_chord(e.xIs, e.yIs, e.zIs, xt, yt, zt, ux1, uy1, uz1, ux2, uy2, uz2);
-    const float ea = expf(-labs * e.mu_t);
-    const float absf = (1.0f - ea) * e.mu_pe / e.mu_t;
-    const float dabsf = labs * ea * e.mu_pe / e.mu_t - (1.0f - ea) * e.mu_pe / (e.mu_t * e.mu_t);
-    const double rq = 1.0 / ((4.0 * 3.14159265358979323846) * (double)q.dsq * (double)q.sq);
-    const float ax = t * h / 8.0f / 16.0f, az = w * t / 8.0f / 16.0f, ay = w * h / 8.0f / 8.0f;
-    const float sax = (float)((double)ax * (double)fabsf((q.xD - e.xI) * e.cosr - (q.zD - e.zI) * e.sinr) * rq);
-    const float saz = (float)((double)az * (double)fabsf((q.xD - e.xI) * e.sinr + (q.zD - e.zI) * e.cosr) * rq);
-    const float say = (float)((double)ay * (double)fabsf(q.yD - e.yI) * rq);
-    const float sxy = (sax >= say) ? sax : say;
-    const float sa = (sxy >= saz) ? sxy : saz;
-    const float base = eff * sa;
-#pragma unroll
-    for (int i = 0; i < kThetaN; ++i) dc[i] = -base * absf * s.da[i];
-    dc[1] += base * dabsf;
-    return base * absf;
 }
 
 // Value and theta-partials of element (d, v), summed over its sub-elements in double; every
 // lane returns the warp's totals in acc[0..7] (acc[kThetaN] = the value).
 template <bool ELL>
-__device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSmem& bs, WarpSmem& ws, int d, long long v,
-                                float cr, float sr, int lane, double* acc)
+__device__ __forceinline__ void pe_element_grad(const DevGeom& g, const Superset& sup, GradWarp& ws, int d, long long v,
+                                                float cr, float sr, int lane, double* acc)
 {
 #pragma unroll
     for (int i = 0; i <= kThetaN; ++i) acc[i] = 0.0;
-    Elem e;
-    if (!init_element(g, ws.inner, d, v, cr, sr, lane, e)) return;
-    const bool from_super = bs.s_count >= 0;
-    const int n_src = from_super ? bs.s_count : g.n_holes + g.n_det;
-    int count = 0;
-    const int cursor = build_chunk(g, bs, ws, e, d, 0, n_src, from_super, lane, &count);
+    const unsigned short* src = sup.s_count >= 0 ? sup.sid : nullptr;
+    const int n_src = src ? sup.s_count : g.n_holes + g.n_det;
+    int cursor;
+    Kept k;
+    {
+        Elem el;
+        if (!init_element(g, ws.inner, d, v, cr, sr, lane, el)) return;
+        if (lane == 0) ws.elem = el;
+        ws.sub[lane] = RefDivision::entry(el, lane);
+        cursor = build_kept(g, src, ws, el, d, 0, n_src, lane, k);   // ends in a __syncwarp
+    }
+    const Elem& e = ws.elem;
     const bool single = cursor >= n_src;
-    for (int r = 0; r < 32; ++r) {
-        const int sidx = ((r >> 3) * 2 + (lane >> 4)) * 128 + ((lane >> 1) & 7) * 16 + (r & 7) * 2 +
-                         (lane & 1);
-        const SubElem q = sub_element(e, sidx);
-        WalkGrad s;
-        s.att = 0.0f;
-        s.len = 0.0f;
-        s.lay = 0;
-        s.lr = s.lx = s.lz = s.ly = s.lp = 0.0f;
+    for (int q0 = 0; q0 < 32; q0 += kGradRounds) {
+        const RefDivisionAt dv(q0);
+        ray_boxes(ws, dv, kGradRounds, lane);
+        grad_pass<ELL>(g, ws, dv, src, n_src, d, single, lane, cursor, k);
+        for (int r = 0; r < kGradRounds; ++r) {
+            const int slot = r * 32 + lane;
+            const float outside = ws.att[slot];
+            if (isinf(outside)) continue;
+            int ix, iy, iz;
+            dv.indices(r, lane, ix, iy, iz);
+            const RayEnd q = ray_end_terms(ws, dv, ix, iy, iz);
+            const float eff = 1.0f * expf(-__fmaf_rn(q.self, e.mu_t, outside));
+            const float ea = expf(-q.labs * e.mu_t);
+            const float absf = div_by((1.0f - ea) * e.mu_pe, e.mu_t, e.imu_t);
+            const float dabsf = q.labs * ea * e.mu_pe / e.mu_t - (1.0f - ea) * e.mu_pe / (e.mu_t * e.mu_t);
+            const float base = eff * q.sa;
 #pragma unroll
-        for (int i = 0; i < kThetaN; ++i) s.da[i] = 0.0f;
-        RayCyl rc;
-        ray_cyl_init(rc, e.xI, e.yI, e.zI, q.xD, q.yD, q.zD);
-        const bool blocked = plate_penalty(g, ws.inner, e, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, s.att);
-        const bool skip = blocked && g.nonneg_mu;
-        float4 box = make_float4(skip ? INFINITY : q.sa_a, skip ? -INFINITY : q.sa_a,
-                                 skip ? INFINITY : q.sa_b, skip ? -INFINITY : q.sa_b);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, off));
-            box.y = fmaxf(box.y, __shfl_xor_sync(0xffffffffu, box.y, off));
-            box.z = fminf(box.z, __shfl_xor_sync(0xffffffffu, box.z, off));
-            box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, off));
-        }
-        int cur = 0;
-        bool first_chunk = true;
-        while (true) {
-            if (!single && !first_chunk) {
-                cur = build_chunk(g, bs, ws, e, d, cur, n_src, from_super, lane, &count);
-            } else if (!single) {
-                if (r > 0) cur = build_chunk(g, bs, ws, e, d, 0, n_src, from_super, lane, &count);
-                else cur = cursor;
+            for (int i = 0; i < kThetaN; ++i) {
+                const float da = ws.da[i][slot] + (i == 1 ? q.self : 0.0f);
+                float dc = -base * absf * da;
+                if (i == 1) dc += base * dabsf;
+                acc[i] += (double)dc;
             }
-            first_chunk = false;
-            int k = 0;
-            while (k < count) {
-                int next = count, nh = 0;
-                const int nr = fill_round<ELL>(g, ws, e, k, count, box, 0, lane, &next, &nh);
-                if (!skip) walk_round_grad<ELL>(g, ws, nh, nr, q.xD, q.yD, q.zD, q.sa_a, q.sa_b, q.cosang, rc, s);
-                __syncwarp();
-                k = next;
-            }
-            if (single || cur >= n_src) break;
+            acc[kThetaN] += (double)(base * absf);
         }
-        if (!skip) {
-            if (s.lay < g.n_layers) close_layers_grad(g, s, g.n_layers, q.cosang);
-            float dc[kThetaN];
-            acc[kThetaN] += (double)finish_sub_element_grad(e, q, s, dc);
-#pragma unroll
-            for (int i = 0; i < kThetaN; ++i) acc[i] += (double)dc[i];
-        }
+        __syncwarp();
     }
 #pragma unroll
     for (int i = 0; i <= kThetaN; ++i)
@@ -306,9 +331,8 @@ __device__ __forceinline__ void pe_element_grad(const DevGeom& g, const BlockSme
 // Projections run the reference-order element (pe_ref.cuh), the gradient its own.
 template <int KIND>
 struct AdjSmem {
-    typename std::conditional<KIND == 1, BlockSmem, RefSmem>::type bs;
+    typename std::conditional<KIND == 1, GradSmem, RefSmem>::type bs;
     double acc[KIND == 1 ? kWarps : 1][kThetaN + 1];
-    int any;
 };
 
 // KIND 0: p[d - det_begin] += sum_v A[d,v] x[v] (precise-mode elements).
@@ -320,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     AdjSmem<KIND>& sm = *reinterpret_cast<AdjSmem<KIND>*>(smem_raw);
-    Superset& bs = superset_of(sm.bs);
+    Superset& bs = sm.bs.sup;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (KIND == 1 && lane <= kThetaN) sm.acc[wid][lane] = 0.0;
     const float ang = L.rotation * g.angle_step;           // :1006
@@ -330,10 +354,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
     const long long total = n_bricks * L.det_count;
     const int n_slots = L.bx * L.by * L.bz;
     for (;;) {
-        if (threadIdx.x == 0) {
-            bs.item = (long long)atomicAdd(L.work_counter, 1ull);
-            sm.any = 0;
-        }
+        if (threadIdx.x == 0) bs.item = (long long)atomicAdd(L.work_counter, 1ull);
         __syncthreads();
         const long long item = bs.item;
         if (item >= total) break;
@@ -344,15 +365,16 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
         const int gy = rem / nbx, gx = rem - gy * nbx;
         const int x0 = gx * L.bx, y0 = gy * L.by, z0 = gz * L.bz;
         const float ud = KIND >= 1 ? L.u[di] : 1.0f;
-        // any voxel of the brick with a non-zero weight?
-        for (int slot = threadIdx.x; slot < n_slots; slot += kThreads) {
+        // the brick's voxels of non-zero weight, shared evenly by the warps
+        int n_active = 0;
+        for (int base = 0; base < n_slots; base += kThreads) {
+            const int slot = base + threadIdx.x;
             const int ix = x0 + slot % L.bx, iy = y0 + (slot / L.bx) % L.by, iz = z0 + slot / (L.bx * L.by);
-            if (ix < g.nx && iy < g.ny && iz < g.nz && ud != 0.0f &&
-                (KIND == 2 || L.x[ix + g.nx * ((long long)iy + (long long)g.ny * iz)] != 0.0f))
-                sm.any = 1;
+            const bool in = slot < n_slots && ix < g.nx && iy < g.ny && iz < g.nz && ud != 0.0f &&
+                            (KIND == 2 || L.x[ix + g.nx * ((long long)iy + (long long)g.ny * iz)] != 0.0f);
+            n_active += block_append(bs, in, (unsigned short)slot, bs.slot, n_active, 512, lane, wid);
         }
-        __syncthreads();
-        if (sm.any) {
+        if (n_active > 0) {
             const int x1 = min(x0 + L.bx, g.nx) - 1, y1 = min(y0 + L.by, g.ny) - 1, z1 = min(z0 + L.bz, g.nz) - 1;
             const int d = L.det_begin + di;
             float ax, ay, az, bxx, byy, bzz;
@@ -362,12 +384,11 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
             const float rho = 0.5f * sqrtf((bxx - ax) * (bxx - ax) + (byy - ay) * (byy - ay) +
                                            (bzz - az) * (bzz - az)) + 1e-3f;
             build_superset(g, bs, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho);
-            for (int slot = wid; slot < n_slots; slot += kWarps) {
+            for (int i = wid; i < n_active; i += kWarps) {
+                const int slot = bs.slot[i];
                 const int ix = x0 + slot % L.bx, iy = y0 + (slot / L.bx) % L.by, iz = z0 + slot / (L.bx * L.by);
-                if (ix >= g.nx || iy >= g.ny || iz >= g.nz) continue;
                 const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
                 const float xv = KIND == 2 ? 1.0f : L.x[v];
-                if (xv == 0.0f || ud == 0.0f) continue;
                 if constexpr (KIND == 0) {
                     const double val = pe_element_ref<1, false, ELL>(g, bs, sm.bs.w[wid], d, v, cr, sr, lane, nullptr);
                     if (lane == 0) atomicAdd(&L.p[di], val * (double)xv);
@@ -376,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
                     if (lane == 0) atomicAdd(&L.q[v], val * (double)ud);
                 } else {
                     double acc[kThetaN + 1];
-                    pe_element_grad<ELL>(g, sm.bs, sm.bs.w[wid], d, v, cr, sr, lane, acc);
+                    pe_element_grad<ELL>(g, bs, sm.bs.w[wid], d, v, cr, sr, lane, acc);
                     const double wgt = (double)ud * (double)xv;
                     if (lane == 0)
 #pragma unroll

@@ -28,16 +28,16 @@
 
 constexpr int kPassRounds = 16;          // rounds per pass: half of an element
 constexpr int kUnits = 192;              // record units of 32 B: a hole takes one, a crystal two
-constexpr int kMaskWords = kUnits / 32;
 constexpr int kNear = 512;               // sampled form: objects near the bundle of any source point
 
 struct RefWarp {
+    static constexpr int units = kUnits;
     // kept objects in the reference's order.  Hole i at rec[2 i]: (x, z, voxel - x, voxel - z),
     // (y1, y2, R, mu); crystal i (of those kept) at rec[2 nh + 4 i]: (x, y, z, mu), (cos(-rot),
     // sin(-rot), w, t), (h, voxel in its frame), slope rectangle
     float4 rec[2 * kUnits];
     unsigned short id[kUnits];           // hole ids
-    unsigned mask[kMaskWords][32];       // per round: the kept objects that meet its slope box
+    unsigned mask[kUnits / 32][32];      // per round: the kept objects that meet its slope box
     float4 box[32];                      // the rounds' slope boxes
     float reach[32];                     // and the largest slope length in each
     float att[kPassRounds * 32];         // [round][lane]: attenuation outside crystal d, then contribution
@@ -203,7 +203,8 @@ __device__ __forceinline__ bool in_cone(const DevGeom& g, const Elem& e, int i)
 // passes it is queued and the cone test (two square roots and four divisions) runs on full
 // groups of 32.  Stops before a group that would overflow the records; returns the position to
 // go on from.
-__device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short* src, RefWarp& ws, const Elem& e,
+template <class W>
+__device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short* src, W& ws, const Elem& e,
                                           int d, int cursor, int n_src, int lane, Kept& kept)
 {
     const unsigned below = (1u << lane) - 1u;
@@ -235,7 +236,7 @@ __device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short
         const bool hole = id < g.n_holes;
         const unsigned mh = __ballot_sync(0xffffffffu, keep && hole), mc = __ballot_sync(0xffffffffu, keep && !hole);
         const int need = __popc(mh) + 2 * __popc(mc);
-        if (units + need > kUnits) {
+        if (units + need > W::units) {
             cursor = ws.cand[0];
             break;
         }
@@ -381,7 +382,8 @@ struct Shadow {
 };
 
 // ws.mask for rounds [r0, r1): the kept objects that meet each round's slope box.
-__device__ __forceinline__ void round_masks(RefWarp& ws, const Elem& e, const Kept& k, int r0, int r1, int lane)
+template <class W>
+__device__ __forceinline__ void round_masks(W& ws, const Elem& e, const Kept& k, int r0, int r1, int lane)
 {
     for (int w = 0; w * 32 < k.count; ++w) {
         const int j = w * 32 + lane;
@@ -496,7 +498,13 @@ __device__ __forceinline__ void hole_ray_caps(HoleRay& c, const Elem& e, float y
 // Chord of hole A = (x, z, voxel - x, voxel - z) of radius r; kr = RN(kk r), r2 = RN(r^2).
 // Straight-line: the reference's four cap/side cases are selects (a warp whose lanes meet
 // different cases runs it once, and two holes interleave).
-__device__ __forceinline__ float hole_chord(const HoleRay& c, const float4& A, float r, float kr, float r2)
+struct ChordParts {
+    bool fl, fr;                 // inside the hole at the front and back cap
+    float cross, sd;             // the cross term and the root of the discriminant
+};
+
+__device__ __forceinline__ float hole_chord(const HoleRay& c, const float4& A, float r, float kr, float r2,
+                                            ChordParts* parts = nullptr)
 {
     const float dxl = c.xl - A.x, dzl = c.zl - A.y, dxr = c.xr - A.x, dzr = c.zr - A.y;
     const bool fl = __fmaf_rn(dzl, dzl, __fmul_rn(dxl, dxl)) <= r2;
@@ -510,6 +518,7 @@ __device__ __forceinline__ float hole_chord(const HoleRay& c, const float4& A, f
     const float ea = fl ? c.ta : t1, eb = fr ? c.tb : t2;
     const bool ok = meets && (fl || fr || (t1 >= c.ta && t2 <= c.tb)) &&
                     !(eb <= 0.0001f || ea <= 0.0001f || eb >= c.tio || ea >= c.tio);
+    if (parts) *parts = ChordParts{fl, fr, cross, sd};
     return (fl && fr) ? c.full : (ok ? eb - ea : 0.0f);
 }
 
@@ -639,6 +648,17 @@ __device__ __forceinline__ float crystal_chord(float xa, float ya, float za, flo
     return out ? 0.0f : tmax - tmin;
 }
 
+// Chord of the ray to (xD, yD, zD) in the crystal recorded at rec (0 for a lane it does not concern),
+// and the crystal's mu.
+__device__ __forceinline__ float record_chord(const float4* rec, float xD, float yD, float zD, bool in, float& mu)
+{
+    const float4 A = rec[0], B = rec[1], C = rec[2];
+    const float vx = xD - A.x, vz = zD - A.z;                             // :1318-1320
+    const float xb = __fmaf_rn(vx, B.x, -__fmul_rn(vz, B.y)), zb = __fmaf_rn(vz, B.x, __fmul_rn(vx, B.y));
+    mu = A.w;
+    return in ? crystal_chord(C.y, C.z, C.w, xb, yD - A.y, zb, B.z, B.w, C.x) : 0.0f;
+}
+
 // Other crystals along the rays of rounds [r0, r1): kept entries [nh, count), added to ws.att in
 // the reference's order (:1290-1325).
 template <bool COUNT, class Div>
@@ -662,12 +682,9 @@ __device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, con
             const float4* rec = &ws.rec[2 * nh + 4 * (it.take() - nh)];
             const bool in = !skip && in_rect(rec[3], sa_a, sa_b);
             if (!__any_sync(0xffffffffu, in)) continue;
-            const float4 A = rec[0], B = rec[1], C = rec[2];
-            const float vx = xD - A.x, vz = zD - A.z;                             // :1318-1320
-            const float xb = __fmaf_rn(vx, B.x, -__fmul_rn(vz, B.y)), zb = __fmaf_rn(vz, B.x, __fmul_rn(vx, B.y));
-            float la = 0.0f;
-            if (in) la = crystal_chord(C.y, C.z, C.w, xb, yD - A.y, zb, B.z, B.w, C.x);
-            att = __fmaf_rn(la, A.w, att);
+            float mu;
+            const float la = record_chord(rec, xD, yD, zD, in, mu);
+            att = __fmaf_rn(la, mu, att);
             if constexpr (COUNT) n_hits += (la != 0.0f), n_evals += in;
         } while (it.more());
         ws.att[(r & (kPassRounds - 1)) * 32 + lane] = att;
@@ -703,10 +720,14 @@ static __device__ __noinline__ float2 finish_parallel(float xi, float yi, float 
     return l;
 }
 
-// Contribution of sub-element (ix, iy, iz), given the attenuation outside crystal d: self
-// attenuation, absorption and solid angle (:1223-1231, :1329-1357).
-template <class Div>
-__device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, int ix, int iy, int iz, float att)
+// What crystal d makes of a ray to its sub-element (ix, iy, iz) (:1223-1231, :1329-1357): the length
+// of crystal d before the sub-element, the absorption chord and the solid angle.
+struct RayEnd {
+    float self, labs, sa;
+};
+
+template <class W, class Div>
+__device__ __forceinline__ RayEnd ray_end_terms(const W& ws, const Div& dv, int ix, int iy, int iz)
 {
     const Elem& e = ws.elem;
     const float4 X = dv.row_x(ws, ix), Y = dv.row_y(ws, iy), Z = dv.row_z(ws, iz);
@@ -734,8 +755,6 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, in
         tmin = fmaxf(tmin, fminf(a, b)), tmax = fminf(tmax, fmaxf(a, b));
         l2 = inside_length(tmin, tmax, tio);
     }
-    att = __fmaf_rn(l1 - l2, e.mu_t, att);
-    const float eff = 1.0f * expf(-att);
     float xD, yD, zD;
     ray_end(e, X.x, Y.x, Z.x, xD, yD, zD);
     const float dsq = norm2(xD - e.xI, yD - e.yI, zD - e.zI);
@@ -760,7 +779,6 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, in
         const bool out = (tmax - tmin) < kEps || tmin >= tio || tmax >= tio || tmin <= kEps || tmax <= kEps;
         labs = out ? 0.0f : tmax - tmin;
     }
-    const float absf = div_by((1.0f - expf(-labs * e.mu_t)) * e.mu_pe, e.mu_t, e.imu_t);
     // solid angle in double, as the reference's 4*M_PI promotion makes it: the largest of three
     // exact double products times one reciprocal, rounded once (rounding keeps the order, so this
     // is the largest of the three rounded values; the reciprocal in place of the reference's
@@ -772,7 +790,18 @@ __device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, in
     const double py = (double)ay * (double)fabsf(yD - e.yI);
     const double pm = px >= py ? (px >= pz ? px : pz) : (py >= pz ? py : pz);
     const float sa = (float)(pm * rq);
-    return eff * sa * absf;
+    return RayEnd{l1 - l2, labs, sa};
+}
+
+// Contribution of sub-element (ix, iy, iz), given the attenuation outside crystal d.
+template <class Div>
+__device__ __forceinline__ float finish_ray(const RefWarp& ws, const Div& dv, int ix, int iy, int iz, float att)
+{
+    const Elem& e = ws.elem;
+    const RayEnd q = ray_end_terms(ws, dv, ix, iy, iz);
+    const float eff = 1.0f * expf(-__fmaf_rn(q.self, e.mu_t, att));
+    const float absf = div_by((1.0f - expf(-q.labs * e.mu_t)) * e.mu_pe, e.mu_t, e.imu_t);
+    return eff * q.sa * absf;
 }
 
 // Work counts of one lane (COUNT instances).
