@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
             const float mx = 0.5f * (ax + bxx), my = 0.5f * (ay + byy), mz = 0.5f * (az + bzz);
             const float rho = 0.5f * sqrtf((bxx - ax) * (bxx - ax) + (byy - ay) * (byy - ay) +
                                            (bzz - az) * (bzz - az)) + 1e-3f;
-            build_superset(g, bs, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho);
+            build_superset(g, bs, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho, 0.5f * fabsf(bzz - az) + 1e-3f);
             for (int i = wid; i < n_active; i += kWarps) {
                 const int slot = bs.slot[i];
                 const int ix = x0 + slot % L.bx, iy = y0 + (slot / L.bx) % L.by, iz = z0 + slot / (L.bx * L.by);

@@ -73,7 +73,7 @@ __device__ __forceinline__ int build_ids(const DevGeom& g, const unsigned short*
             bool maybe = false;
             if (j < n_src) {
                 const int id = src ? src[j] : j;
-                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e, e.rd, id));
+                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e.xI, e.yI, e.zI, e.rd, id));
             }
             const unsigned m = __ballot_sync(0xffffffffu, maybe);
             if (maybe) ws.cand[queued + __popc(m & below)] = j;

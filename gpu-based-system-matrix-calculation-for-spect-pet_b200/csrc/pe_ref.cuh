@@ -56,6 +56,9 @@ struct RefSmem {
     RefWarp w[kWarps];
 };
 
+// Attenuation beyond which expf(-att) is 0: half the smallest float is exp(-103.97).
+constexpr float kDark = 104.5f;
+
 // What build_kept leaves: entries [0, nh) are holes, [nh, count) crystals; even: the holes share
 // layer, cap planes and radius.
 struct Kept {
@@ -160,10 +163,10 @@ __device__ __forceinline__ float norm2(float x, float y, float z)
 }
 
 // Whether object i may meet the slope rectangle rd of crystal d (approximate reciprocals, within
-// the rectangles' margins), seen from any source within (spread, spread, spread_z) of the
-// element's; objects close to the source always may.
-__device__ __forceinline__ bool near_bundle(const DevGeom& g, const Elem& e, const float4& rd, int i, float spread = 0.0f,
-                                            float spread_z = 0.0f)
+// the rectangles' margins), seen from any source within (spread, spread, spread_z) of (xs, ys, zs);
+// objects close to the source always may.
+__device__ __forceinline__ bool near_bundle(const DevGeom& g, float xs, float ys, float zs, const float4& rd, int i,
+                                            float spread = 0.0f, float spread_z = 0.0f)
 {
     float x0, x1, z0, z1, y0, y1;
     if (i < g.n_holes) {
@@ -177,13 +180,28 @@ __device__ __forceinline__ bool near_bundle(const DevGeom& g, const Elem& e, con
         const float hx = 0.5f * (s.x * fabsf(t.x) + s.z * fabsf(t.y)), hz = 0.5f * (s.x * fabsf(t.y) + s.z * fabsf(t.x));
         x0 = p.x - hx, x1 = p.x + hx, z0 = p.z - hz, z1 = p.z + hz, y0 = p.y - 0.5f * s.y, y1 = p.y + 0.5f * s.y;
     }
-    y0 -= e.yI + spread;
-    y1 -= e.yI - spread;
+    y0 -= ys + spread;
+    y1 -= ys - spread;
     if (!(y0 >= kMinDepth) || !(y1 >= kMinDepth)) return true;
     const float r0 = rcp_approx(y0), r1 = rcp_approx(y1);
-    x0 -= e.xI + spread, x1 -= e.xI - spread, z0 -= e.zI + spread_z, z1 -= e.zI - spread_z;
+    x0 -= xs + spread, x1 -= xs - spread, z0 -= zs + spread_z, z1 -= zs - spread_z;
     return fminf(x0 * r0, x0 * r1) - kSlopeMargin <= rd.y && fmaxf(x1 * r0, x1 * r1) + kSlopeMargin >= rd.x &&
            fminf(z0 * r0, z0 * r1) - kSlopeMargin <= rd.w && fmaxf(z1 * r0, z1 * r1) + kSlopeMargin >= rd.z;
+}
+
+// Slope rectangle of crystal d's bounding cylinder from any source within (spread, spread, spread_z)
+// of (xs, ys, zs); false when the crystal is too close to the sources for one.
+__device__ __forceinline__ bool bundle_rect(const DevGeom& g, int d, float xs, float ys, float zs, float spread,
+                                            float spread_z, float4& rd)
+{
+    const float4 P = __ldg(&g.cry.pos[d]), S = __ldg(&g.cry.size[d]);
+    const float foot = 0.5f * sqrtf(S.x * S.x + S.z * S.z), rx = foot + spread, rz = foot + spread_z;
+    const float y0 = P.y - 0.5f * S.y - ys - spread, y1 = P.y + 0.5f * S.y - ys + spread;
+    if (!(y0 >= kMinDepth)) return false;
+    const float r0 = 1.0f / y0, r1 = 1.0f / y1, x = P.x - xs, z = P.z - zs;
+    rd = make_float4(fminf((x - rx) * r0, (x - rx) * r1) - kSlopeMargin, fmaxf((x + rx) * r0, (x + rx) * r1) + kSlopeMargin,
+                     fminf((z - rz) * r0, (z - rz) * r1) - kSlopeMargin, fmaxf((z + rz) * r0, (z + rz) * r1) + kSlopeMargin);
+    return true;
 }
 
 // Reference cone test of object i (:1120-1184).
@@ -217,7 +235,7 @@ __device__ __forceinline__ int build_kept(const DevGeom& g, const unsigned short
             bool maybe = false;
             if (j < n_src) {
                 const int id = src ? src[j] : j;
-                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e, e.rd, id));
+                maybe = id - g.n_holes != d && (!e.filt || near_bundle(g, e.xI, e.yI, e.zI, e.rd, id));
             }
             const unsigned m = __ballot_sync(0xffffffffu, maybe);
             if (maybe) ws.cand[queued + __popc(m & below)] = j;
@@ -559,6 +577,7 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const 
             const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;             // open rectangles: slope 0
             skip = plate_penalty(g, ws.inner, e, xD, yD, zD, (xD - e.xI) * rdy, (zD - e.zI) * rdy, s.att) && g.nonneg_mu;
             skip = skip || dv.dead(r, lane);
+            if constexpr (COUNT) n_blocked += skip;
         } else {
             s.att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
             s.len = ws.len[(r & 7) * 32 + lane];
@@ -621,9 +640,10 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const 
             }
         }
         if (s.lay < lay1) close_layers_ref(g, s, lay1, c);
+        // past kDark the contribution is exactly 0 whatever follows (every mu >= 0): as if blocked
+        skip = skip || (s.att > kDark && g.nonneg_mu);
         ws.att[(r & (kPassRounds - 1)) * 32 + lane] = skip ? INFINITY : s.att;
         if (carry) ws.len[(r & 7) * 32 + lane] = s.len;
-        if constexpr (COUNT) n_blocked += first && skip;
     }
 }
 
@@ -953,20 +973,13 @@ __device__ double pe_element_sampled(const DevGeom& g, const Superset& sup, RefW
         Elem el;
         if (!init_element(g, ws.inner, d, v, cr, sr, lane, el)) return 0.0;
         const float hx = 0.5f * (fabsf(g.wx) + fabsf(g.wy)), hz = 0.5f * fabsf(g.wz);
-        // slope rectangle of crystal d's bounding cylinder from any source point
-        const float r = 0.5f * sqrtf(el.w * el.w + el.h * el.h) + hx, rz = 0.5f * sqrtf(el.w * el.w + el.h * el.h) + hz;
-        const float y0 = el.yd - 0.5f * el.t - el.yI - hx, y1 = el.yd + 0.5f * el.t - el.yI + hx;
-        if (y0 >= kMinDepth) {
-            const float r0 = 1.0f / y0, r1 = 1.0f / y1, x = el.xd - el.xI, z = el.zd - el.zI;
-            const float4 rd = make_float4(fminf((x - r) * r0, (x - r) * r1) - kSlopeMargin,
-                                          fmaxf((x + r) * r0, (x + r) * r1) + kSlopeMargin,
-                                          fminf((z - rz) * r0, (z - rz) * r1) - kSlopeMargin,
-                                          fmaxf((z + rz) * r0, (z + rz) * r1) + kSlopeMargin);
+        float4 rd;
+        if (bundle_rect(g, d, el.xI, el.yI, el.zI, hx, hz, rd)) {
             int n = 0;
             for (int base = 0; base < n_src && n <= kNear; base += 32) {
                 const int j = base + lane;
                 const int id = j < n_src ? src[j] : 0;
-                const bool maybe = j < n_src && near_bundle(g, el, rd, id, hx, hz);
+                const bool maybe = j < n_src && near_bundle(g, el.xI, el.yI, el.zI, rd, id, hx, hz);
                 const unsigned m = __ballot_sync(0xffffffffu, maybe);
                 const int pos = n + __popc(m & ((1u << lane) - 1u));
                 if (maybe && pos < kNear) ws.near[pos] = (unsigned short)id;
