@@ -353,11 +353,13 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
         spread_z += 0.5f * fabsf(g.wz);
     }
     build_superset(g, sup, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho, spread_z);
-    for (int i = wid; i < n_active; i += kWarps) {
-        const int slot = sup.slot[i];
-        const int ix = x0 + slot % bx, iy = y0 + (slot / bx) % by, iz = z0 + slot / (bx * by);
-        const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
-        {
+    // the block's warps start each element together: they then run the same phase's loop, which the
+    // schedulers' instruction caches hold, most of the time
+    for (int base = 0; base < n_active; base += kWarps) {
+        if (base + wid < n_active) {
+            const int slot = sup.slot[base + wid];
+            const int ix = x0 + slot % bx, iy = y0 + (slot / bx) % by, iz = z0 + slot / (bx * by);
+            const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
             float val;
             if constexpr (MODE <= 1 && SAMPLED) {
                 val = (float)pe_element_sampled<ELL>(g, sup, sm.w[wid], d, v, cr, sr, lane, *smp);
@@ -372,10 +374,9 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
                 val = (float)pe_element64(g, sup, sm.w[wid], d, v, cr, sr, rotation, lane);
             }
             if (lane == 0) O.out[(long long)di * O.ld + (v - O.vox_begin)] = val;
-            __syncwarp();
         }
+        __syncthreads();
     }
-    __syncthreads();
 }
 
 template <int MODE, bool COUNT, bool ELL, bool SAMPLED = false>

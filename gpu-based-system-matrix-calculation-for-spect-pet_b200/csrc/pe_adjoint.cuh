@@ -384,8 +384,10 @@ __global__ void __launch_bounds__(kThreads, 2) pe_adjoint_kernel(DevGeom g, AdjL
             const float rho = 0.5f * sqrtf((bxx - ax) * (bxx - ax) + (byy - ay) * (byy - ay) +
                                            (bzz - az) * (bzz - az)) + 1e-3f;
             build_superset(g, bs, d, mx * cr - my * sr, mx * sr + my * cr, mz, rho, 0.5f * fabsf(bzz - az) + 1e-3f);
-            for (int i = wid; i < n_active; i += kWarps) {
-                const int slot = bs.slot[i];
+            for (int first = 0; first < n_active; first += kWarps) {
+                if (first > 0) __syncthreads();            // elements start together (pe_brick)
+                if (first + wid >= n_active) continue;
+                const int slot = bs.slot[first + wid];
                 const int ix = x0 + slot % L.bx, iy = y0 + (slot / L.bx) % L.by, iz = z0 + slot / (L.bx * L.by);
                 const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
                 const float xv = KIND == 2 ? 1.0f : L.x[v];

@@ -84,6 +84,7 @@ __device__ __forceinline__ float4 sub_row(int i, float f, float size, float p)
 // The reference's 8 x 16 x 8, rows kept in ws.sub.
 struct RefDivision {
     static constexpr float fx = 8.0f, fy = 16.0f, fz = 8.0f;
+    static constexpr int rays = 2;       // rounds that the walks take at a time
     __device__ __forceinline__ void indices(int r, int lane, int& ix, int& iy, int& iz) const
     {
         ix = 4 * ((r >> 3) & 1) + ((lane >> 1) & 3);
@@ -124,6 +125,7 @@ struct RefDivisionAt : RefDivision {
 // nx x ny x nz (x, depth, z), 32 to a round in (z, depth, x) order, x fastest, from sub-element
 // `base`; lanes past the end repeat the last one and are dead.
 struct AnyDivision {
+    static constexpr int rays = 1;
     int nx, ny, n_sub, base;
     float fx, fy, fz;
     __device__ __forceinline__ void indices(int r, int lane, int& ix, int& iy, int& iz) const
@@ -424,14 +426,17 @@ __device__ __forceinline__ void round_masks(W& ws, const Elem& e, const Kept& k,
     __syncwarp();
 }
 
-// The set bits of round r's mask between entries [j0, j1), in order.
+// The set bits of the masks of rounds r and q (q = r: one round) between entries [j0, j1), in order.
 struct Entries {
     const unsigned (*mask)[32];
-    int r, w, w1, j0, j1;
+    int r, q, w, w1, j0, j1;
     unsigned m;
 
-    __device__ __forceinline__ Entries(const unsigned (*mask_)[32], int r_, int j0_, int j1_)
-        : mask(mask_), r(r_), j0(j0_), j1(j1_)
+    __device__ __forceinline__ Entries(const unsigned (*mask_)[32], int r_, int j0_, int j1_) : Entries(mask_, r_, r_, j0_, j1_)
+    {
+    }
+    __device__ __forceinline__ Entries(const unsigned (*mask_)[32], int r_, int q_, int j0_, int j1_)
+        : mask(mask_), r(r_), q(q_), j0(j0_), j1(j1_)
     {
         w = j0 >> 5;
         w1 = (j1 + 31) >> 5;
@@ -439,7 +444,7 @@ struct Entries {
     }
     __device__ __forceinline__ unsigned word() const
     {
-        unsigned x = mask[w][r];
+        unsigned x = mask[w][r] | mask[w][q];
         if (w == j0 >> 5) x &= 0xffffffffu << (j0 & 31);
         if (w == j1 >> 5) x &= (1u << (j1 & 31)) - 1u;
         return x;
@@ -551,62 +556,88 @@ __device__ __forceinline__ void close_layers_ref(const DevGeom& g, Walk& s, int 
     }
 }
 
-// Holes and layers along the rays of rounds [r0, r1).  first: the rays start here (plate
-// penalty, :1240-1254), otherwise they go on from ws.att / ws.len in layer lay0; at the end the
-// layers below lay1 are closed.  A ray that the plate penalty blocked (every mu >= 0) gets
-// infinite attenuation.  Every branch on an entry is uniform across the warp, and a ray that
-// misses a hole adds an exact zero.  EVEN (all kept holes alike, the usual collimator): the cap
-// terms are formed once per ray, and holes go two at a time (independent chords: the serial
-// chain of one leaves issue slots idle).
+// Holes and layers along the rays of rounds [r0, r1), Div::rays rounds at a time.  first: the rays
+// start here (plate penalty, :1240-1254), otherwise they go on from ws.att / ws.len in layer lay0;
+// at the end the layers below lay1 are closed.  A ray that the plate penalty blocked (every
+// mu >= 0) gets infinite attenuation.  Every branch on an entry is uniform across the warp, and a
+// ray that misses a hole adds an exact zero.  A lane always has two independent chords in hand
+// (the serial chain of one leaves issue slots idle): one hole for the rays of two rounds, or with
+// one round and EVEN two holes for its ray.  EVEN (all kept holes alike, the usual collimator): the
+// cap terms are formed once per ray.
 template <bool COUNT, bool ELL, bool EVEN, class Div>
-__device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int r0, int r1, bool first, int lay0,
-                                           int lay1, bool carry, int lane, int& n_hits, int& n_evals, int& n_blocked)
+__device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int r0, int r1, bool first,
+                                           int lay0, int lay1, bool carry, int lane, int& n_hits, int& n_evals,
+                                           int& n_blocked)
 {
+    constexpr int NR = Div::rays;
     const Elem& e = ws.elem;
-    for (int r = r0; r < r1; ++r) {
-        int ix, iy, iz;
-        dv.indices(r, lane, ix, iy, iz);
-        const float3 q = dv.centre(ws, ix, iy, iz);
-        float xD, yD, zD;
-        ray_end(e, q.x, q.y, q.z, xD, yD, zD);
-        HoleRay c;
-        hole_ray_init(c, xD - e.xI, yD - e.yI, zD - e.zI);
-        Walk s{0.0f, 0.0f, lay0};
-        bool skip;
-        if (first) {
-            const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;             // open rectangles: slope 0
-            skip = plate_penalty(g, ws.inner, e, xD, yD, zD, (xD - e.xI) * rdy, (zD - e.zI) * rdy, s.att) && g.nonneg_mu;
-            skip = skip || dv.dead(r, lane);
-            if constexpr (COUNT) n_blocked += skip;
-        } else {
-            s.att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
-            s.len = ws.len[(r & 7) * 32 + lane];
-            skip = isinf(s.att);
+    for (int r = r0; r < r1; r += NR) {
+        HoleRay c[NR];
+        Walk s[NR];
+        bool skip[NR];
+        float3 end[ELL ? NR : 1];
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            int ix, iy, iz;
+            dv.indices(r + n, lane, ix, iy, iz);
+            const float3 q = dv.centre(ws, ix, iy, iz);
+            float xD, yD, zD;
+            ray_end(e, q.x, q.y, q.z, xD, yD, zD);
+            if constexpr (ELL) end[n] = make_float3(xD, yD, zD);
+            hole_ray_init(c[n], xD - e.xI, yD - e.yI, zD - e.zI);
+            s[n] = Walk{0.0f, 0.0f, lay0};
+            if (first) {
+                const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;             // open rectangles: slope 0
+                skip[n] = plate_penalty(g, ws.inner, e, xD, yD, zD, (xD - e.xI) * rdy, (zD - e.zI) * rdy, s[n].att) &&
+                          g.nonneg_mu;
+                skip[n] = skip[n] || dv.dead(r + n, lane);
+                if constexpr (COUNT) n_blocked += skip[n];
+            } else {
+                s[n].att = ws.att[((r + n) & (kPassRounds - 1)) * 32 + lane];
+                s[n].len = ws.len[((r + n) & 7) * 32 + lane];
+                skip[n] = isinf(s[n].att);
+            }
         }
-        Entries it(ws.mask, r, 0, nh);
+        Entries it(ws.mask, r, r + NR - 1, 0, nh);
         if (EVEN && it.more()) {
             const float4 B = ws.rec[1];
             const int m = layer_of_hole(g, ws.id[0]);
-            if (m != s.lay) close_layers_ref(g, s, m, c);
-            hole_ray_caps(c, e, B.x, B.y);
-            const float kr = __fmul_rn(c.kk, B.z), r2 = __fmul_rn(B.z, B.z);
+            const float r2 = __fmul_rn(B.z, B.z);
+            float kr[NR];
+#pragma unroll
+            for (int n = 0; n < NR; ++n) {
+                if (m != s[n].lay) close_layers_ref(g, s[n], m, c[n]);
+                hole_ray_caps(c[n], e, B.x, B.y);
+                kr[n] = __fmul_rn(c[n].kk, B.z);
+            }
             do {
                 const int j = it.take();
                 const float4 A = ws.rec[2 * j];
                 const float mu = ws.rec[2 * j + 1].w;
-                const bool pair = it.m != 0u;
-                const int j2 = pair ? it.take() : j;
-                const float4 A2 = ws.rec[2 * j2];
-                const float mu2 = ws.rec[2 * j2 + 1].w;
-                const float tmp = hole_chord(c, A, B.z, kr, r2);
-                const float two = hole_chord(c, A2, B.z, kr, r2);
-                const float tmp2 = pair ? two : 0.0f;
-                s.len = s.len + tmp;                                              // :1276-1278
-                s.att = __fmaf_rn(mu, tmp, s.att);
-                s.len = s.len + tmp2;
-                s.att = __fmaf_rn(mu2, tmp2, s.att);
-                if constexpr (COUNT) {
-                    if (!skip) n_hits += (tmp != 0.0f) + (tmp2 != 0.0f), n_evals += 1 + pair;
+                if constexpr (NR == 2) {
+                    float tmp[NR];
+#pragma unroll
+                    for (int n = 0; n < NR; ++n) tmp[n] = hole_chord(c[n], A, B.z, kr[n], r2);
+#pragma unroll
+                    for (int n = 0; n < NR; ++n) {
+                        s[n].len = s[n].len + tmp[n];                             // :1276-1278
+                        s[n].att = __fmaf_rn(mu, tmp[n], s[n].att);
+                        if constexpr (COUNT) {
+                            if (!skip[n]) n_hits += tmp[n] != 0.0f, ++n_evals;
+                        }
+                    }
+                } else {
+                    const bool pair = it.m != 0u;
+                    const int j2 = pair ? it.take() : j;
+                    const float4 A2 = ws.rec[2 * j2];
+                    const float mu2 = ws.rec[2 * j2 + 1].w;
+                    const float tmp = hole_chord(c[0], A, B.z, kr[0], r2);
+                    const float two = hole_chord(c[0], A2, B.z, kr[0], r2);
+                    const float tmp2 = pair ? two : 0.0f;
+                    s[0].len = s[0].len + tmp;                                    // :1276-1278
+                    s[0].att = __fmaf_rn(mu, tmp, s[0].att);
+                    s[0].len = s[0].len + tmp2;
+                    s[0].att = __fmaf_rn(mu2, tmp2, s[0].att);
                 }
             } while (it.more());
         }
@@ -616,34 +647,44 @@ __device__ __forceinline__ void walk_holes(const DevGeom& g, RefWarp& ws, const 
                 const int j = it.take();
                 const float4 A = ws.rec[2 * j], B = ws.rec[2 * j + 1];
                 const int id = ws.id[j], m = layer_of_hole(g, id);
-                if (m != s.lay) close_layers_ref(g, s, m, c);
-                float tmp = 0.0f;
                 float4 S = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if constexpr (ELL) {
                     if (g.hole_shape) S = __ldg(&g.hole_shape[id]);
                 }
-                if (ELL && S.x > 0.0f) {                                          // elliptical hole
-                    if (!skip) tmp = ell_chord(e.xI, e.yI, e.zI, xD, yD, zD, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w);
-                } else {
-                    if (!(B.x == y1 && B.y == y2)) {
-                        y1 = B.x;
-                        y2 = B.y;
-                        hole_ray_caps(c, e, y1, y2);
-                    }
-                    tmp = hole_chord(c, A, B.z, __fmul_rn(c.kk, B.z), __fmul_rn(B.z, B.z));
+                const bool ell = ELL && S.x > 0.0f;
+                const bool caps = !ell && !(B.x == y1 && B.y == y2);
+                if (caps) {
+                    y1 = B.x;
+                    y2 = B.y;
                 }
-                s.len = s.len + tmp;                                              // :1276-1278
-                s.att = __fmaf_rn(B.w, tmp, s.att);
-                if constexpr (COUNT) {
-                    if (!skip) n_hits += (tmp != 0.0f), ++n_evals;
+#pragma unroll
+                for (int n = 0; n < NR; ++n) {
+                    if (m != s[n].lay) close_layers_ref(g, s[n], m, c[n]);
+                    float tmp = 0.0f;
+                    if (ell) {                                                    // elliptical hole
+                        const float3 q = end[ELL ? n : 0];
+                        if (!skip[n])
+                            tmp = ell_chord(e.xI, e.yI, e.zI, q.x, q.y, q.z, A.x, B.x, B.y, A.y, S.x, S.y, S.z, S.w);
+                    } else {
+                        if (caps) hole_ray_caps(c[n], e, y1, y2);
+                        tmp = hole_chord(c[n], A, B.z, __fmul_rn(c[n].kk, B.z), __fmul_rn(B.z, B.z));
+                    }
+                    s[n].len = s[n].len + tmp;                                    // :1276-1278
+                    s[n].att = __fmaf_rn(B.w, tmp, s[n].att);
+                    if constexpr (COUNT) {
+                        if (!skip[n]) n_hits += tmp != 0.0f, ++n_evals;
+                    }
                 }
             }
         }
-        if (s.lay < lay1) close_layers_ref(g, s, lay1, c);
-        // past kDark the contribution is exactly 0 whatever follows (every mu >= 0): as if blocked
-        skip = skip || (s.att > kDark && g.nonneg_mu);
-        ws.att[(r & (kPassRounds - 1)) * 32 + lane] = skip ? INFINITY : s.att;
-        if (carry) ws.len[(r & 7) * 32 + lane] = s.len;
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            if (s[n].lay < lay1) close_layers_ref(g, s[n], lay1, c[n]);
+            // past kDark the contribution is exactly 0 whatever follows (every mu >= 0): as if blocked
+            skip[n] = skip[n] || (s[n].att > kDark && g.nonneg_mu);
+            ws.att[((r + n) & (kPassRounds - 1)) * 32 + lane] = skip[n] ? INFINITY : s[n].att;
+            if (carry) ws.len[((r + n) & 7) * 32 + lane] = s[n].len;
+        }
     }
 }
 
@@ -679,35 +720,49 @@ __device__ __forceinline__ float record_chord(const float4* rec, float xD, float
     return in ? crystal_chord(C.y, C.z, C.w, xb, yD - A.y, zb, B.z, B.w, C.x) : 0.0f;
 }
 
-// Other crystals along the rays of rounds [r0, r1): kept entries [nh, count), added to ws.att in
-// the reference's order (:1290-1325).
+// Other crystals along the rays of rounds [r0, r1), Div::rays rounds at a time: kept entries [nh,
+// count), added to ws.att in the reference's order (:1290-1325).
 template <bool COUNT, class Div>
-__device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int count, int r0, int r1, int lane,
-                                              int& n_hits, int& n_evals)
+__device__ __forceinline__ void walk_crystals(const DevGeom& g, RefWarp& ws, const Div& dv, int nh, int count, int r0, int r1,
+                                              int lane, int& n_hits, int& n_evals)
 {
+    constexpr int NR = Div::rays;
     const Elem& e = ws.elem;
-    for (int r = r0; r < r1; ++r) {
-        Entries it(ws.mask, r, nh, count);
+    for (int r = r0; r < r1; r += NR) {
+        Entries it(ws.mask, r, r + NR - 1, nh, count);
         if (!it.more()) continue;
-        int ix, iy, iz;
-        dv.indices(r, lane, ix, iy, iz);
-        const float3 q = dv.centre(ws, ix, iy, iz);
-        float xD, yD, zD;
-        ray_end(e, q.x, q.y, q.z, xD, yD, zD);
-        const float rdy = e.filt ? rcp_approx(yD - e.yI) : 0.0f;
-        const float sa_a = (xD - e.xI) * rdy, sa_b = (zD - e.zI) * rdy;
-        float att = ws.att[(r & (kPassRounds - 1)) * 32 + lane];
-        const bool skip = isinf(att);
+        float xD[NR], yD[NR], zD[NR], sa_a[NR], sa_b[NR], att[NR];
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            int ix, iy, iz;
+            dv.indices(r + n, lane, ix, iy, iz);
+            const float3 q = dv.centre(ws, ix, iy, iz);
+            ray_end(e, q.x, q.y, q.z, xD[n], yD[n], zD[n]);
+            const float rdy = e.filt ? rcp_approx(yD[n] - e.yI) : 0.0f;
+            sa_a[n] = (xD[n] - e.xI) * rdy, sa_b[n] = (zD[n] - e.zI) * rdy;
+            att[n] = ws.att[((r + n) & (kPassRounds - 1)) * 32 + lane];
+        }
         do {
             const float4* rec = &ws.rec[2 * nh + 4 * (it.take() - nh)];
-            const bool in = !skip && in_rect(rec[3], sa_a, sa_b);
-            if (!__any_sync(0xffffffffu, in)) continue;
-            float mu;
-            const float la = record_chord(rec, xD, yD, zD, in, mu);
-            att = __fmaf_rn(la, mu, att);
-            if constexpr (COUNT) n_hits += (la != 0.0f), n_evals += in;
+            const float4 rect = rec[3];
+            bool in[NR], any = false;
+#pragma unroll
+            for (int n = 0; n < NR; ++n) {
+                in[n] = !isinf(att[n]) && in_rect(rect, sa_a[n], sa_b[n]);
+                any = any || in[n];
+            }
+            if (!__any_sync(0xffffffffu, any)) continue;
+            float la[NR], mu;
+#pragma unroll
+            for (int n = 0; n < NR; ++n) la[n] = record_chord(rec, xD[n], yD[n], zD[n], in[n], mu);
+#pragma unroll
+            for (int n = 0; n < NR; ++n) {
+                att[n] = __fmaf_rn(la[n], mu, att[n]);
+                if constexpr (COUNT) n_hits += (la[n] != 0.0f), n_evals += in[n];
+            }
         } while (it.more());
-        ws.att[(r & (kPassRounds - 1)) * 32 + lane] = att;
+#pragma unroll
+        for (int n = 0; n < NR; ++n) ws.att[((r + n) & (kPassRounds - 1)) * 32 + lane] = att[n];
     }
 }
 
