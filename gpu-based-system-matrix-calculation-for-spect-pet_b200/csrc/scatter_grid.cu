@@ -16,7 +16,7 @@
 //   1. crystal-cell weights: the local sampled photoelectric kernel writes every sub-element's
 //      contribution (pe_local.cuh) into Wc[voxel][crystal][cell];
 //   2. septal-cell weights: one thread per (voxel, septal cell), in double, into Ws;
-//   3. grid_sum_kernel: a block takes a tile of 64 detectors and a range of points; per chunk
+//   3. grid_sum_kernel: a block takes a tile of 32 detectors and a range of points; per chunk
 //      of 256 points it stages the weights of all the chunk's voxels in shared memory, and per
 //      detector it forms each point's detector-only terms in double once (position in the
 //      detector's frame, absorption chord, attenuation sums of the crystals, tungsten and hole
@@ -27,6 +27,7 @@
 // Calls are synchronous: the weights live in scratch allocated and freed by the call.
 #include <cmath>
 #include <cstdio>
+#include <algorithm>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -37,6 +38,7 @@
 #include "ctx.cuh"
 #include "geom.cuh"
 #include "pe.cuh"
+#include "rounding.cuh"
 #include "scatter.cuh"
 
 #define CUDA_TRY(expr)                                                                     \
@@ -56,8 +58,8 @@ namespace {
 constexpr int kGridThreads = 256;
 constexpr int kGridChunk = 256;          // points per chunk (one per thread)
 constexpr int kGridMaxVox = 48;          // voxels per pass
-constexpr int kGridDetTile = 64;         // detectors per block
-constexpr int kGridChunksPerBlock = 8;
+constexpr int kGridDetTile = 32;         // detectors per block
+constexpr int kGridChunksPerBlock = 8;   // chunks per block at most
 
 
 // Septal cells are numbered brick by brick (bricks of 8 x 4 x 8 cells, x fastest inside a brick
@@ -146,8 +148,8 @@ constexpr int kCandCry = 1024, kCandHole = 2048;
 struct Cands {
     int n_cry;
     int hole_off[kMaxLayers + 1];        // holes of layer m: hole[hole_off[m] .. hole_off[m+1]); -1 = all
-    int cry[kCandCry];
-    int hole[kCandHole];
+    unsigned short cry[kCandCry];        // at most 6666 crystals, 8877 holes
+    unsigned short hole[kCandHole];
     int warp_cnt[kGridThreads / 32];
     float lo[3], hi[3];                  // the chunk's bounding box
 };
@@ -155,7 +157,7 @@ struct Cands {
 // Ordered compaction over the block of the items i in [0, n) with keep(i) into list[off ..]
 // (capacity cap); returns the number kept, or -1 past the capacity.
 template <class F>
-__device__ int block_select(int n, F keep, int* list, int off, int cap, int* warp_cnt)
+__device__ int block_select(int n, F keep, unsigned short* list, int off, int cap, int* warp_cnt)
 {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     int total = 0;
@@ -172,7 +174,7 @@ __device__ int block_select(int n, F keep, int* list, int off, int cap, int* war
             all += c;
         }
         const int pos = total + before + __popc(m & ((1u << lane) - 1u));
-        if (k && pos < cap) list[off + pos] = i;
+        if (k && pos < cap) list[off + pos] = (unsigned short)i;
         total += all;
         __syncthreads();
     }
@@ -206,16 +208,29 @@ __device__ void chunk_candidates(const DevGeom& g, const GridGeom& G, Cands& C, 
                                   (C.hi[2] - C.lo[2]) * (C.hi[2] - C.lo[2])) + 2e-3f;
     const float ex = (float)E[0], ey = (float)E[1], ez = (float)E[2];
     const float gx = ex - cx, gy = ey - cy, gz = ez - cz;
-    const float gl2 = gx * gx + gy * gy + gz * gz;
     if (cry) {
+        // a crystal's box meets a path only where the path is at the box's depths, and there within its
+        // footprint's circle: the xz distance to that part of the segment, the points' extent added
+        const float bx = 0.5f * (C.hi[0] - C.lo[0]), by = 0.5f * (C.hi[1] - C.lo[1]) + 2e-3f, bz = 0.5f * (C.hi[2] - C.lo[2]);
+        const float rxz = sqrtf(bx * bx + bz * bz) + 2e-3f;
+        const float g2 = gx * gx + gz * gz, ig2 = g2 > 0.0f ? 1.0f / g2 : 0.0f;
+        const float igy = fabsf(gy) > 1e-3f ? 1.0f / gy : 0.0f;
         const int n = block_select(g.n_det, [&](int a) {
-            const float4 pa = __ldg(&g.cry.pos[a]);
-            const float ra = 0.5f * __ldg(&g.cry.size[a].w) + 1e-3f + rc;
-            const float hx = pa.x - cx, hy = pa.y - cy, hz = pa.z - cz;
-            float u = gl2 > 0.0f ? (hx * gx + hy * gy + hz * gz) / gl2 : 0.0f;
-            u = fminf(fmaxf(u, 0.0f), 1.0f);
-            const float qx = hx - u * gx, qy = hy - u * gy, qz = hz - u * gz;
-            return qx * qx + qy * qy + qz * qz <= ra * ra;
+            const float4 pa = __ldg(&g.cry.pos[a]), sa = __ldg(&g.cry.size[a]);
+            float u0 = 0.0f, u1 = 1.0f;
+            const float y0 = pa.y - 0.5f * sa.y - by - cy, y1 = pa.y + 0.5f * sa.y + by - cy;
+            if (igy != 0.0f) {
+                u0 = fmaxf(u0, fminf(y0 * igy, y1 * igy) - 1e-4f);
+                u1 = fminf(u1, fmaxf(y0 * igy, y1 * igy) + 1e-4f);
+                if (u0 > u1) return false;
+            } else if (y0 > fabsf(gy) || y1 < -fabsf(gy)) {
+                return false;
+            }
+            const float ra = 0.5f * sqrtf(sa.x * sa.x + sa.z * sa.z) + rxz;
+            const float hx = pa.x - cx, hz = pa.z - cz;
+            const float u = fminf(fmaxf((hx * gx + hz * gz) * ig2, u0), u1);
+            const float qx = hx - u * gx, qz = hz - u * gz;
+            return qx * qx + qz * qz <= ra * ra;
         }, C.cry, 0, kCandCry, C.warp_cnt);
         if (threadIdx.x == 0) C.n_cry = n;
     }
@@ -243,114 +258,197 @@ __device__ void chunk_candidates(const DevGeom& g, const GridGeom& G, Cands& C, 
     __syncthreads();
 }
 
-// Hole h's axis (x, z) is farther than r from the xz projection of segment a -> b (with a
-// small margin): the segment cannot meet the hole.
-__device__ __forceinline__ bool hole_far(double ax, double az, double bx, double bz, double hx, double hz, double r)
+// A segment A -> A + d with what its overlaps with boxes and cylinders share: reciprocals (rcp64;
+// a component below 1e-30 counts as 0 and has none), length, and the xz part a = dx^2 + dz^2.
+struct Seg64 {
+    double A[3], d[3], id[3];
+    double len, a, ia;
+};
+
+__device__ __forceinline__ Seg64 make_seg(const double A[3], const double B[3])
 {
-    const double ex = bx - ax, ez = bz - az;
-    const double l2 = ex * ex + ez * ez;
-    double t = l2 > 0.0 ? ((hx - ax) * ex + (hz - az) * ez) / l2 : 0.0;
-    t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
-    const double dx = ax + t * ex - hx, dz = az + t * ez - hz;
-    return dx * dx + dz * dz > (r + 1e-6) * (r + 1e-6);
+    Seg64 s;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double d = B[k] - A[k];
+        s.A[k] = A[k];
+        s.d[k] = fabs(d) < 1e-30 ? 0.0 : d;
+        s.id[k] = rcp64(s.d[k]);
+    }
+    s.a = s.d[0] * s.d[0] + s.d[2] * s.d[2];
+    s.ia = rcp64(s.a);
+    const double l2 = s.a + s.d[1] * s.d[1];
+    s.len = l2 > 0.0 ? sqrt64(l2) : 0.0;
+    return s;
 }
 
-// Length of segment A -> B inside the box [lo, hi]: the exact overlap of the segment's
-// parameter range with the three slabs.  The grid model's paths start or end inside the plate
-// or a crystal, where the reference's chords (full crossings between the two ends) do not apply.
-__device__ double seg_box64(const double A[3], const double B[3], const double lo[3], const double hi[3])
+// The part [t0, t1] of the segment's parameter range inside the slab [lo, hi] of one axis.
+__device__ __forceinline__ void seg_clip(double A, double d, double id, double lo, double hi, double& t0, double& t1)
+{
+    if (d == 0.0) {
+        if (A < lo || A > hi) t1 = -1.0;
+        return;
+    }
+    const double u = (lo - A) * id, v = (hi - A) * id;
+    const double e = u < v ? u : v, x = u < v ? v : u;
+    t0 = e > t0 ? e : t0;
+    t1 = x < t1 ? x : t1;
+}
+
+// Length of the segment inside the box [lo, hi]: the exact overlap of its parameter range with the
+// three slabs.  The grid model's paths start or end inside the plate or a crystal, where the
+// reference's chords (full crossings between the two ends) do not apply.
+__device__ __forceinline__ double seg_box64(const Seg64& s, const double lo[3], const double hi[3])
 {
     double t0 = 0.0, t1 = 1.0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const double d = B[a] - A[a];
-        if (d == 0.0) {
-            if (A[a] < lo[a] || A[a] > hi[a]) return 0.0;
-            continue;
-        }
-        double u = (lo[a] - A[a]) / d, v = (hi[a] - A[a]) / d;
-        if (u > v) { const double w = u; u = v; v = w; }
-        t0 = fmax(t0, u);
-        t1 = fmin(t1, v);
-    }
-    if (t1 <= t0) return 0.0;
-    return (t1 - t0) * sqrt((B[0] - A[0]) * (B[0] - A[0]) + (B[1] - A[1]) * (B[1] - A[1]) + (B[2] - A[2]) * (B[2] - A[2]));
+    for (int a = 0; a < 3; ++a) seg_clip(s.A[a], s.d[a], s.id[a], lo[a], hi[a], t0, t1);
+    return t1 <= t0 ? 0.0 : (t1 - t0) * s.len;
 }
 
-// Length of segment A -> B inside the y-parallel cylinder (x - xc)^2 + (z - zc)^2 <= r^2,
-// y in [y1, y2] (exact overlap).  S: an elliptical hole's (rho_x, rho_z, cos, sin) (S.x > 0), in
-// whose frame (u = dx cos + dz sin, w = -dx sin + dz cos, as the reference turns points),
-// divided by the semi-axes, the segment meets the unit circle over the same parameter range.
-__device__ double seg_cyl64(const double A[3], const double B[3], double xc, double zc, double y1, double y2, double r,
-                            const D4& S)
+// Length of the segment inside the y-parallel cylinder (x - xc)^2 + (z - zc)^2 <= r^2, y in [y1, y2]
+// (exact overlap).  E: an elliptical hole's (rho_x, rho_z, cos, sin) (E.x > 0), in whose frame
+// (u = dx cos + dz sin, w = -dx sin + dz cos, as the reference turns points), divided by the
+// semi-axes, the segment meets the unit circle over the same parameter range.
+__device__ __forceinline__ double seg_cyl64(const Seg64& s, double xc, double zc, double y1, double y2, double r,
+                                            const D4& E)
 {
     double t0 = 0.0, t1 = 1.0;
-    const double dy = B[1] - A[1];
-    if (dy == 0.0) {
-        if (A[1] < y1 || A[1] > y2) return 0.0;
-    } else {
-        double u = (y1 - A[1]) / dy, v = (y2 - A[1]) / dy;
-        if (u > v) { const double w = u; u = v; v = w; }
-        t0 = fmax(t0, u);
-        t1 = fmin(t1, v);
-    }
-    const double dx0 = B[0] - A[0], dz0 = B[2] - A[2];
-    double dx = dx0, dz = dz0, ox = A[0] - xc, oz = A[2] - zc;
-    if (S.x > 0.0) {
-        const double pdx = (dx * S.z + dz * S.w) / S.x, pdz = (-dx * S.w + dz * S.z) / S.y;
-        const double pox = (ox * S.z + oz * S.w) / S.x, poz = (-ox * S.w + oz * S.z) / S.y;
+    seg_clip(s.A[1], s.d[1], s.id[1], y1 < y2 ? y1 : y2, y1 < y2 ? y2 : y1, t0, t1);
+    double dx = s.d[0], dz = s.d[2], ox = s.A[0] - xc, oz = s.A[2] - zc, a = s.a, ia = s.ia;
+    if (E.x > 0.0) {
+        const double rx = 1.0 / E.x, rz = 1.0 / E.y;
+        const double pdx = (dx * E.z + dz * E.w) * rx, pdz = (-dx * E.w + dz * E.z) * rz;
+        const double pox = (ox * E.z + oz * E.w) * rx, poz = (-ox * E.w + oz * E.z) * rz;
         dx = pdx; dz = pdz; ox = pox; oz = poz;
         r = 1.0;
+        a = dx * dx + dz * dz;
+        ia = rcp64(a);
     }
-    const double a = dx * dx + dz * dz, b = ox * dx + oz * dz, c = ox * ox + oz * oz - r * r;
+    const double b = ox * dx + oz * dz, c = ox * ox + oz * oz - r * r;
     if (a == 0.0) {
         if (c > 0.0) return 0.0;
     } else {
         const double disc = b * b - a * c;
-        if (disc <= 0.0) return 0.0;
-        const double sq = sqrt(disc);
-        t0 = fmax(t0, (-b - sq) / a);
-        t1 = fmin(t1, (-b + sq) / a);
+        if (disc <= 1e-60) return 0.0;
+        const double sq = sqrt64(disc);
+        const double u = (-b - sq) * ia, v = (-b + sq) * ia;
+        t0 = u > t0 ? u : t0;
+        t1 = v < t1 ? v : t1;
     }
-    if (t1 <= t0) return 0.0;
-    return (t1 - t0) * sqrt(dx0 * dx0 + dz0 * dz0 + dy * dy);
+    return t1 <= t0 ? 0.0 : (t1 - t0) * s.len;
 }
 
-// Attenuation sums (mu_total, mu_pe, mu_C times length) of layer m along segment A -> B: its
-// length in the plate box minus its lengths in the layer's holes, with the layer's
-// coefficients, plus its lengths in the holes with the holes' own coefficients.
-__device__ void layer_path64(const DevGeom& g, const GridGeom& G, int m, const double A[3], const double B[3],
-                             double& wt, double& wpe, double& wc, const Cands* C = nullptr)
+// A warp's queue of (path, object) pairs that passed their lane's float test, each lane with one
+// path.  The paths of a warp cross different objects, so the overlap in double, run where the tests
+// are, would run once per object that any lane crosses; queued, 32 pairs at a time take a lane each
+// (paths read from their lanes by shuffles) and add to their path's sums in shared memory.
+constexpr int kPathSums = 4;
+
+struct PathSums {
+    int queue[kGridThreads / 32][64];    // lane | object << 5
+    double sum[kGridThreads][kPathSums];
+};
+
+struct PairQueue {
+    int* q;
+    int n;
+
+    // f(path, object, lane of the path), for the first `take` pairs
+    template <class F>
+    __device__ __forceinline__ void run(int take, int lane, const Seg64& own, F&& f)
+    {
+        __syncwarp();
+        const int code = lane < take ? q[lane] : lane;
+        const int src = code & 31;
+        Seg64 s;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s.A[k] = __shfl_sync(0xffffffffu, own.A[k], src);
+            s.d[k] = __shfl_sync(0xffffffffu, own.d[k], src);
+            s.id[k] = __shfl_sync(0xffffffffu, own.id[k], src);
+        }
+        s.len = __shfl_sync(0xffffffffu, own.len, src);
+        s.a = __shfl_sync(0xffffffffu, own.a, src);
+        s.ia = __shfl_sync(0xffffffffu, own.ia, src);
+        if (lane < take) f(s, code >> 5, src);
+        const int rest = n - take;
+        const int moved = lane < rest ? q[take + lane] : 0;
+        __syncwarp();
+        if (lane < rest) q[lane] = moved;
+        n = rest;
+    }
+    template <class F>
+    __device__ __forceinline__ void push(bool want, int object, int lane, const Seg64& own, F&& f)
+    {
+        const unsigned m = __ballot_sync(0xffffffffu, want);
+        if (m == 0u) return;
+        if (want) q[n + __popc(m & ((1u << lane) - 1u))] = lane | (object << 5);
+        n += __popc(m);
+        if (n >= 32) run(32, lane, own, f);
+    }
+    template <class F>
+    __device__ __forceinline__ void drain(int lane, const Seg64& own, F&& f)
+    {
+        if (n > 0) run(n, lane, own, f);
+        __syncwarp();
+    }
+};
+
+// Warp-collective: attenuation sums (mu_total, mu_pe, mu_C times length) of layer m along each lane's
+// segment (`on`: the lane has one): its length in the plate box minus its lengths in the layer's holes,
+// with the layer's coefficients, plus its lengths in the holes with the holes' own coefficients.
+__device__ void layer_path64(const DevGeom& g, const GridGeom& G, int m, const Seg64& s, bool on, double& wt, double& wpe,
+                             double& wc, const Cands& C, PathSums& ps)
 {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const double* Ly = g.t64.layer + kLayer64 * m;
     const double lo[3] = {Ly[0], Ly[2], Ly[4]}, hi[3] = {Ly[1], Ly[3], Ly[5]};
-    const double box = seg_box64(A, B, lo, hi);
-    if (box == 0.0) return;
+    const double box = on ? seg_box64(s, lo, hi) : 0.0;
+    if (!__any_sync(0xffffffffu, box != 0.0)) return;
     const GridLayer& L = G.layer[m];
-    // candidate holes of the chunk (in hole order), or every hole of the layer
-    const bool listed = C && C->hole_off[m] >= 0 && C->hole_off[m + 1] >= 0;
-    const int n = listed ? C->hole_off[m + 1] - C->hole_off[m] : L.hole_count;
-    double hsum = 0.0;
-    for (int q = 0; q < n; ++q) {
-        const int j = L.hole_begin + (listed ? C->hole[C->hole_off[m] + q] : q);
+#pragma unroll
+    for (int k = 0; k < kPathSums; ++k) ps.sum[t][k] = 0.0;
+    auto overlap = [&](const Seg64& q, int j, int src) {
         const D4 a = g.t64.hole_a[j];
-        const double r = g.t64.hole_b[j].x;
-        if (hole_far(A[0], A[2], B[0], B[2], a.x, a.w, r)) continue;
         const D4 S = g.t64.hole_shape ? g.t64.hole_shape[j] : D4{0.0, 0.0, 1.0, 0.0};
-        const double l = seg_cyl64(A, B, a.x, a.w, a.y, a.z, r, S);
-        if (l == 0.0) continue;
+        const double l = seg_cyl64(q, a.x, a.w, a.y, a.z, g.t64.hole_b[j].x, S);
+        if (l == 0.0) return;
         const float* hp = G.raw_col + 100 + 9 * j;
-        hsum += l;
-        wt += (double)__ldg(&hp[5]) * l;
-        wpe += (double)__ldg(&hp[6]) * l;
-        wc += (double)__ldg(&hp[7]) * l;
+        double* sum = ps.sum[32 * warp + src];
+        atomicAdd(&sum[0], l);
+        const float mt = __ldg(&hp[5]), mp = __ldg(&hp[6]), mc = __ldg(&hp[7]);
+        if (mt != 0.0f) atomicAdd(&sum[1], (double)mt * l);
+        if (mp != 0.0f) atomicAdd(&sum[2], (double)mp * l);
+        if (mc != 0.0f) atomicAdd(&sum[3], (double)mc * l);
+    };
+    // candidate holes of the chunk, or every hole of the layer; a float distance test (2 um of margin)
+    // takes out the holes that the segment passes by
+    const bool listed = C.hole_off[m] >= 0 && C.hole_off[m + 1] >= 0;
+    const int n = listed ? C.hole_off[m + 1] - C.hole_off[m] : L.hole_count;
+    const float fx = (float)s.A[0], fz = (float)s.A[2], dx = (float)s.d[0], dz = (float)s.d[2];
+    const float l2 = dx * dx + dz * dz, il2 = l2 > 0.0f ? rcp_approx(l2) : 0.0f;
+    PairQueue queue{ps.queue[warp], 0};
+    for (int q = 0; q < n; ++q) {
+        const int j = L.hole_begin + (listed ? C.hole[C.hole_off[m] + q] : q);
+        const float4 ha = __ldg(&g.hole.a[j]);
+        const float rm = __ldg(&g.hole.b[j].x) + 2e-3f;
+        const float hx = ha.x - fx, hz = ha.w - fz;
+        const float u = __saturatef((hx * dx + hz * dz) * il2);
+        const float ux = hx - u * dx, uz = hz - u * dz;
+        queue.push(box != 0.0 && ux * ux + uz * uz <= rm * rm, j, lane, s, overlap);
     }
-    const double lw = box - hsum;
+    queue.drain(lane, s, overlap);
+    wt += ps.sum[t][1];
+    wpe += ps.sum[t][2];
+    wc += ps.sum[t][3];
+    const double lw = box - ps.sum[t][0];
     if (lw > 0.0) {
         wt += (double)L.mu_t * lw;
         wpe += (double)L.mu_pe * lw;
         wc += (double)L.mu_c * lw;
     }
+    __syncwarp();
 }
 
 // Septal weight V / (4 pi r^2) exp(-A(v -> p)) mu_C for every (voxel, septal cell).
@@ -361,6 +459,7 @@ __global__ void __launch_bounds__(kGridThreads) septal_weight_kernel(DevGeom g, 
                                                                      float* __restrict__ ws)
 {
     __shared__ Cands C;
+    __shared__ PathSums sums;
     const int vi = blockIdx.y;
     const long long j = (long long)blockIdx.x * kGridThreads + threadIdx.x;
     const bool has = j < n_sep;
@@ -370,9 +469,10 @@ __global__ void __launch_bounds__(kGridThreads) septal_weight_kernel(DevGeom g, 
     voxel_centre64(g, vox_begin + vi, rotation, I3[0], I3[1], I3[2]);
     block_bounds(C, has, p);
     chunk_candidates(g, G, C, I3, false, true);
-    if (!has) return;
     double at = 0.0, ape = 0.0, ac = 0.0;
-    for (int mm = 0; mm < G.n_layers; ++mm) layer_path64(g, G, mm, I3, p, at, ape, ac, &C);
+    const Seg64 seg = make_seg(I3, p);
+    for (int mm = 0; mm < G.n_layers; ++mm) layer_path64(g, G, mm, seg, has, at, ape, ac, C, sums);
+    if (!has) return;
     const GridLayer& L = G.layer[m];
     const double r2 = (p[0] - I3[0]) * (p[0] - I3[0]) + (p[1] - I3[1]) * (p[1] - I3[1]) + (p[2] - I3[2]) * (p[2] - I3[2]);
     const double vcell = L.cx * L.cy * L.cz;
@@ -453,66 +553,93 @@ __device__ void grid_point(const DevGeom& g, const GridGeom& G, const GridSum& S
     }
 }
 
-// Detector-only terms of point p for detector d (double, rounded once): p in d's frame, the
-// absorption chord of the extended ray p -> d's centre in d, and the attenuation sums Lpe, Lc
-// of everything on the way (crystals other than d and the scattering crystal, and for septal
-// points the tungsten and hole media), over the chunk's candidate crystals and holes C.
-// Returns false when the point does not scatter into d.
-__device__ bool point_terms(const DevGeom& g, const GridGeom& G, int d, const double p[3], int k, int m, double conv,
-                            const Cands& C, float* out)
+// Warp-collective: detector-only terms of each lane's point p for detector d (double, rounded once):
+// p in d's frame, the absorption chord of the extended ray p -> d's centre in d, and the attenuation
+// sums Lpe, Lc of everything on the way (crystals other than d and the scattering crystal, and for
+// septal points the tungsten and hole media), over the chunk's candidate crystals and holes C.
+// Returns false when the lane has no point or it does not scatter into d.
+__device__ bool point_terms(const DevGeom& g, const GridGeom& G, int d, const double p[3], bool has, int k, int m,
+                            double conv, const Cands& C, PathSums& sums, bool any_sep, float* out)
 {
-    if (k == d) return false;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool on = has && k != d;
     const D4 Pd = g.t64.cry_pos[d], Zd = g.t64.cry_size[d], Td = g.t64.cry_trig[d];
     const double D3[3] = {Pd.x, Pd.y, Pd.z};                  // centre of the 1 x 1 x 1 division
-    const double ex = p[0] - Pd.x, ez = p[2] - Pd.z;
-    const double ps[3] = {ex * Td.z - ez * Td.w, p[1] - Pd.y, ex * Td.w + ez * Td.z};
-    const double lsd = sqrt(ps[0] * ps[0] + ps[1] * ps[1] + ps[2] * ps[2]);
-    // absorption: the ray p -> centre extended 1000 mm through d (scatter.cu:1420-1424)
-    const double labs = box_chord64(ps[0], ps[1], ps[2], -1000.0 * ps[0] / lsd, -1000.0 * ps[1] / lsd,
-                                    -1000.0 * ps[2] / lsd, -0.5 * Zd.x, -0.5 * Zd.y, -0.5 * Zd.z, 0.5 * Zd.x,
-                                    0.5 * Zd.y, 0.5 * Zd.z);
-    double lpe = 0.0, lc = 0.0;
-    // crystals on the way: bounding-sphere reject, then the reference box chord in double
-    const float fx = (float)p[0], fy = (float)p[1], fz = (float)p[2];
-    const float gx = (float)D3[0] - fx, gy = (float)D3[1] - fy, gz = (float)D3[2] - fz;
-    const float gl2 = gx * gx + gy * gy + gz * gz;
-    const int n_cry = C.n_cry >= 0 ? C.n_cry : g.n_det;
-    for (int q = 0; q < n_cry; ++q) {
-        const int a = C.n_cry >= 0 ? C.cry[q] : q;
-        if (a == d || a == k) continue;
-        const float4 pa = __ldg(&g.cry.pos[a]);
-        const float ra = 0.5f * __ldg(&g.cry.size[a].w) + 1e-3f;
-        const float hx = pa.x - fx, hy = pa.y - fy, hz = pa.z - fz;
-        float t = (hx * gx + hy * gy + hz * gz) / gl2;
-        t = fminf(fmaxf(t, 0.0f), 1.0f);
-        const float qx = hx - t * gx, qy = hy - t * gy, qz = hz - t * gz;
-        if (qx * qx + qy * qy + qz * qz > ra * ra) continue;
+    const Seg64 seg = make_seg(p, D3);
+    sums.sum[t][0] = 0.0;
+    sums.sum[t][1] = 0.0;
+    // crystals on the way: the separating axes of segment and box in float (2 um of margin) leave the
+    // crystals that the path crosses or nearly so; then the reference box chord in double (box_chord64;
+    // for an unrotated crystal the path's reciprocals serve it too)
+    auto chord = [&](const Seg64& q, int a, int src) {
         const D4 Pa = g.t64.cry_pos[a], Za = g.t64.cry_size[a], Ta = g.t64.cry_trig[a];
-        const double ax = p[0] - Pa.x, az = p[2] - Pa.z, bx = D3[0] - Pa.x, bz = D3[2] - Pa.z;
-        const double la = box_chord64(ax * Ta.z - az * Ta.w, p[1] - Pa.y, ax * Ta.w + az * Ta.z,
-                                      bx * Ta.z - bz * Ta.w, D3[1] - Pa.y, bx * Ta.w + bz * Ta.z, -0.5 * Za.x,
-                                      -0.5 * Za.y, -0.5 * Za.z, 0.5 * Za.x, 0.5 * Za.y, 0.5 * Za.z);
+        const double ax = q.A[0] - Pa.x, ay = q.A[1] - Pa.y, az = q.A[2] - Pa.z;
+        const bool slanted = fabs(q.d[0]) >= kEps64 && fabs(q.d[1]) >= kEps64 && fabs(q.d[2]) >= kEps64;
+        double la;
+        if (slanted && Ta.z == 1.0 && Ta.w == 0.0) {
+            double t0 = -1e30, t1 = 1e30;                     // box_chord64's parameters, in units of the path
+            seg_clip(ax, q.d[0], q.id[0], -0.5 * Za.x, 0.5 * Za.x, t0, t1);
+            seg_clip(ay, q.d[1], q.id[1], -0.5 * Za.y, 0.5 * Za.y, t0, t1);
+            seg_clip(az, q.d[2], q.id[2], -0.5 * Za.z, 0.5 * Za.z, t0, t1);
+            t0 *= q.len;
+            t1 *= q.len;
+            const bool out = (t1 - t0) < kEps64 || t0 >= q.len || t1 >= q.len || t0 <= kEps64 || t1 <= kEps64;
+            la = out ? 0.0 : t1 - t0;
+        } else {
+            const double bx = D3[0] - Pa.x, bz = D3[2] - Pa.z;
+            la = box_chord64_call(ax * Ta.z - az * Ta.w, ay, ax * Ta.w + az * Ta.z, bx * Ta.z - bz * Ta.w, D3[1] - Pa.y,
+                                  bx * Ta.w + bz * Ta.z, Za.x, Za.y, Za.z);
+        }
         if (la != 0.0) {
             const float4 mu = __ldg(&g.cry.mu[a]);
-            lpe += (double)mu.y * la;
-            lc += (double)mu.z * la;
+            atomicAdd(&sums.sum[32 * warp + src][0], (double)mu.y * la);
+            atomicAdd(&sums.sum[32 * warp + src][1], (double)mu.z * la);
         }
+    };
+    const float gx = 0.5f * (float)seg.d[0], gy = 0.5f * (float)seg.d[1], gz = 0.5f * (float)seg.d[2];
+    const float mx = (float)p[0] + gx, my = (float)p[1] + gy, mz = (float)p[2] + gz;   // the path's middle
+    const int n_cry = C.n_cry >= 0 ? C.n_cry : g.n_det;
+    PairQueue queue{sums.queue[warp], 0};
+    for (int q = 0; q < n_cry; ++q) {
+        const int a = C.n_cry >= 0 ? C.cry[q] : q;
+        if (a == d) continue;
+        const float4 pa = __ldg(&g.cry.pos[a]), sa = __ldg(&g.cry.size[a]), ta = __ldg(&g.cry.trig[a]);
+        const float cx = (mx - pa.x) * ta.z - (mz - pa.z) * ta.w, cy = my - pa.y;
+        const float cz = (mx - pa.x) * ta.w + (mz - pa.z) * ta.z;
+        const float ex = gx * ta.z - gz * ta.w, ez = gx * ta.w + gz * ta.z;
+        const float fx = fabsf(ex), fy = fabsf(gy), fz = fabsf(ez);
+        const float hx = 0.5f * sa.x + 2e-3f, hy = 0.5f * sa.y + 2e-3f, hz = 0.5f * sa.z + 2e-3f;
+        const bool apart = fabsf(cx) > hx + fx || fabsf(cy) > hy + fy || fabsf(cz) > hz + fz ||
+                           fabsf(cy * ez - cz * gy) > hy * fz + hz * fy + 1e-3f ||
+                           fabsf(cz * ex - cx * ez) > hz * fx + hx * fz + 1e-3f ||
+                           fabsf(cx * gy - cy * ex) > hx * fy + hy * fx + 1e-3f;
+        queue.push(on && a != k && !apart, a, lane, seg, chord);
     }
+    queue.drain(lane, seg, chord);
+    double lpe = sums.sum[t][0], lc = sums.sum[t][1];
+    __syncwarp();
+    if (any_sep) {                                            // tungsten and hole media on the way
+        double wt = 0.0;
+        for (int mm = 0; mm < G.n_layers; ++mm) layer_path64(g, G, mm, seg, on && m >= 0, wt, lpe, lc, C, sums);
+    }
+    if (!on) return false;
     if (k >= 0) {                                             // the rest of crystal k, from p to its exit
         const D4 Pk = g.t64.cry_pos[k], Zk = g.t64.cry_size[k], Tk = g.t64.cry_trig[k];
         const double ax = p[0] - Pk.x, az = p[2] - Pk.z, bx = D3[0] - Pk.x, bz = D3[2] - Pk.z;
         const double pa[3] = {ax * Tk.z - az * Tk.w, p[1] - Pk.y, ax * Tk.w + az * Tk.z};
         const double pb[3] = {bx * Tk.z - bz * Tk.w, D3[1] - Pk.y, bx * Tk.w + bz * Tk.z};
         const double lo[3] = {-0.5 * Zk.x, -0.5 * Zk.y, -0.5 * Zk.z}, hi[3] = {0.5 * Zk.x, 0.5 * Zk.y, 0.5 * Zk.z};
-        const double lk = seg_box64(pa, pb, lo, hi);
+        const double lk = seg_box64(make_seg(pa, pb), lo, hi);
         const float4 mu = __ldg(&g.cry.mu[k]);
         lpe += (double)mu.y * lk;
         lc += (double)mu.z * lk;
     }
-    if (m >= 0) {                                             // tungsten and hole media on the way
-        double wt = 0.0;
-        for (int mm = 0; mm < G.n_layers; ++mm) layer_path64(g, G, mm, p, D3, wt, lpe, lc, &C);
-    }
+    const double ex = p[0] - Pd.x, ez = p[2] - Pd.z;
+    const double ps[3] = {ex * Td.z - ez * Td.w, p[1] - Pd.y, ex * Td.w + ez * Td.z};
+    const double lsd = sqrt64(ps[0] * ps[0] + ps[1] * ps[1] + ps[2] * ps[2]), ext = -1000.0 * rcp64(lsd);
+    // absorption: the ray p -> centre extended 1000 mm through d (scatter.cu:1420-1424)
+    const double labs = box_full64_call(ps[0], ps[1], ps[2], ps[0] * ext, ps[1] * ext, ps[2] * ext, -0.5 * Zd.x,
+                                        -0.5 * Zd.y, -0.5 * Zd.z, 0.5 * Zd.x, 0.5 * Zd.y, 0.5 * Zd.z);
     out[0] = (float)ps[0];
     out[1] = (float)ps[1];
     out[2] = (float)ps[2];
@@ -531,33 +658,43 @@ __device__ __forceinline__ double kn_integral(const double* __restrict__ tab, do
 
 constexpr int kTerms = 8;
 
+// Shared memory of a block; the arrays over a pass's voxels follow it, sized by their number.
 struct GridSmem {
     Cands cand;                                 // the chunk's candidates for the current detector
-    double acc[kGridDetTile][kGridMaxVox];      // block sums per (detector, voxel)
-    float wt[kGridMaxVox][kGridChunk];          // the chunk's weights
+    PathSums sums;
     float terms[kTerms][kGridChunk];            // the chunk's detector-only terms
     float rlb[9][kGridChunk];                   // 1 / |corner c of d - p| (c < 8), 1 / |p - d|
-    float4 vox_s[kGridMaxVox];                  // voxels in the current detector's frame
 };
 
-__global__ void __launch_bounds__(kGridThreads) grid_sum_kernel(DevGeom g, GridGeom G, GridSum S)
+__host__ __device__ constexpr size_t grid_smem_bytes(int nv)
+{
+    return (sizeof(GridSmem) + 15) / 16 * 16 +
+           (size_t)nv * (sizeof(float4) + sizeof(double) * kGridDetTile + sizeof(float) * kGridChunk);
+}
+
+// Three blocks to an SM: a block's phases (candidates, terms in double, items) each leave issue slots
+// idle (38 % used with at most two at 128 registers), which other blocks fill.  Configuration 3 at 0.5 mm
+// cells, 64 detectors x 24 voxels: 38.3 ms with two blocks, 27.0 with three (80 registers, 176 B of
+// spills), 28.1 with four.
+__global__ void __launch_bounds__(kGridThreads, 3) grid_sum_kernel(DevGeom g, GridGeom G, GridSum S, int chunks_per_block)
 {
     extern __shared__ __align__(16) unsigned char grid_smem_raw[];
     GridSmem& sm = *reinterpret_cast<GridSmem*>(grid_smem_raw);
-    auto& wt = sm.wt;
+    // voxels in the current detector's frame; block sums [detector][voxel]; the chunk's weights [voxel][point]
+    float4* vox_s = reinterpret_cast<float4*>(grid_smem_raw + (sizeof(GridSmem) + 15) / 16 * 16);
+    double* acc = reinterpret_cast<double*>(vox_s + S.nv);
+    float* wt = reinterpret_cast<float*>(acc + kGridDetTile * S.nv);
     auto& terms = sm.terms;
-    auto& acc = sm.acc;
-    auto& vox_s = sm.vox_s;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int d0 = S.det_begin + blockIdx.y * kGridDetTile;
     const int nd = min(kGridDetTile, S.det_begin + S.det_count - d0);
-    for (int i = t; i < kGridDetTile * kGridMaxVox; i += kGridThreads) (&acc[0][0])[i] = 0.0;
+    for (int i = t; i < kGridDetTile * S.nv; i += kGridThreads) acc[i] = 0.0;
     const float e0 = S.e0;
     const double inv_kn_total = 1.0 / S.kn_total;
     const float ang = S.rotation * g.angle_step;
     const float crot = cosf(ang), srot = sinf(ang);
-    for (int ch = 0; ch < kGridChunksPerBlock; ++ch) {
-        const long long p0 = ((long long)blockIdx.x * kGridChunksPerBlock + ch) * kGridChunk;
+    for (int ch = 0; ch < chunks_per_block; ++ch) {
+        const long long p0 = ((long long)blockIdx.x * chunks_per_block + ch) * kGridChunk;
         if (p0 >= S.n_pts) break;
         const long long pidx = p0 + t;
         __syncthreads();
@@ -571,7 +708,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_sum_kernel(DevGeom g, GridG
             float w = 0.0f;
             if (pidx < S.n_cry_pts) w = S.wc[(long long)vi * S.n_cry_pts + pidx];
             else if (pidx < S.n_pts) w = S.ws[(long long)vi * S.n_sep + (pidx - S.n_cry_pts)];
-            wt[vi][t] = w;
+            wt[vi * kGridChunk + t] = w;
         }
         for (int dl = 0; dl < nd; ++dl) {
             const int d = d0 + dl;
@@ -582,7 +719,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_sum_kernel(DevGeom g, GridG
             const double E3[3] = {Pd.x, Pd.y, Pd.z};
             chunk_candidates(g, G, sm.cand, E3, true, any_sep);
             float tv[kTerms];
-            const bool ok = has && point_terms(g, G, d, pt, kc, mc, conv, sm.cand, tv);
+            const bool ok = point_terms(g, G, d, pt, has, kc, mc, conv, sm.cand, sm.sums, any_sep, tv);
             if (!ok) tv[7] = 0.0f;                              // zero weight factor: no contribution
 #pragma unroll
             for (int q = 0; q < kTerms; ++q) terms[q][t] = ok ? tv[q] : (q == 3 ? 1.0f : 0.0f);
@@ -613,7 +750,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_sum_kernel(DevGeom g, GridG
                 const float4 I = vox_s[vi];
                 double sum = 0.0;
                 for (int j = lane; j < kGridChunk; j += 32) {
-                    const float w = wt[vi][j] * terms[7][j];
+                    const float w = wt[vi * kGridChunk + j] * terms[7][j];
                     if (w == 0.0f) continue;
                     const float px = terms[0][j], py = terms[1][j], pz = terms[2][j], lsd = terms[3][j];
                     const float ax = px - I.x, ay = py - I.y, az = pz - I.z;      // v -> p
@@ -658,14 +795,14 @@ __global__ void __launch_bounds__(kGridThreads) grid_sum_kernel(DevGeom g, GridG
                 }
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-                if (lane == 0) acc[dl][vi] += sum;
+                if (lane == 0) acc[dl * S.nv + vi] += sum;
             }
         }
     }
     __syncthreads();
     for (int i = t; i < nd * S.nv; i += kGridThreads) {
         const int dl = i / S.nv, vi = i - dl * S.nv;
-        const double a = acc[dl][vi];
+        const double a = acc[dl * S.nv + vi];
         if (a != 0.0) atomicAdd(&S.acc[(long long)(d0 - S.det_begin + dl) * S.nv + vi], a);
     }
 }
@@ -824,7 +961,8 @@ extern "C" SYSMAT_API int sysmat_scatter_grid(sysmat_ctx* ctx, int parts, float 
     S.same_window = (int)std::floor(P[4] + 0.5f) > 0;
     S.kn_tab = ctx->d_kn_tab;
     S.kn_total = kn_total;
-    CUDA_TRY(cudaFuncSetAttribute(grid_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GridSmem)));
+    CUDA_TRY(cudaFuncSetAttribute(grid_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)grid_smem_bytes(kGridMaxVox)));
     for (long long vb = vox_begin; vb < vox_begin + vox_count; vb += kGridMaxVox) {
         const int nv = (int)((vox_begin + vox_count - vb) < kGridMaxVox ? (vox_begin + vox_count - vb) : kGridMaxVox);
         if (parts & 1) {                                          // crystal-cell weights
@@ -858,10 +996,12 @@ extern "C" SYSMAT_API int sysmat_scatter_grid(sysmat_ctx* ctx, int parts, float 
         S.vox_begin = vb;
         S.nv = nv;
         CUDA_TRY(cudaMemsetAsync(acc.p, 0, sizeof(double) * (size_t)nv * det_count, s));
-        const long long pblocks = (S.n_pts + (long long)kGridChunk * kGridChunksPerBlock - 1) /
-                                  ((long long)kGridChunk * kGridChunksPerBlock);
-        dim3 grid((unsigned)pblocks, (unsigned)((det_count + kGridDetTile - 1) / kGridDetTile));
-        grid_sum_kernel<<<grid, kGridThreads, sizeof(GridSmem), s>>>(g, G, S);
+        // chunks per block: fewer when the grid would not fill the GPU several times over
+        const long long chunks = (S.n_pts + kGridChunk - 1) / kGridChunk;
+        const long long tiles = (det_count + kGridDetTile - 1) / kGridDetTile;
+        const long long per = std::max(1LL, std::min((long long)kGridChunksPerBlock, chunks * tiles / (12LL * ctx->num_sms)));
+        const dim3 grid((unsigned)((chunks + per - 1) / per), (unsigned)tiles);
+        grid_sum_kernel<<<grid, kGridThreads, grid_smem_bytes(nv), s>>>(g, G, S, (int)per);
         if (cudaGetLastError() != cudaSuccess) return SYSMAT_ERR_CUDA;
         const long long n = (long long)nv * det_count;
         grid_store_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((const double*)acc.p, det_count, nv, d_out, ld,
