@@ -166,9 +166,10 @@ extern "C" SYSMAT_API int sysmat_create(sysmat_ctx** out, int device, const floa
     ctx->h_det.assign(pD, pD + kNDetector);
     if (pC) { ctx->h_col15 = pC[15]; ctx->h_col17 = pC[17]; }
     if (pP) ctx->h_phys.assign(pP, pP + kNPhysics);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { delete ctx; return SYSMAT_ERR_CUDA; }
-    ctx->num_sms = prop.multiProcessorCount;
+    if (cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        delete ctx;
+        return SYSMAT_ERR_CUDA;
+    }
 
     const int D = g.n_det, H = g.n_holes;
     const size_t n_tables = 4 * (size_t)D + 3 * (size_t)(H > 0 ? H : 1);
