@@ -12,15 +12,17 @@ namespace sysmat {
 // Device scratch owned by a context for the scatter path: per-(scatterer, detector) pair
 // records and the attenuator lists they index.
 struct ScatterScratch {
-    void* base = nullptr;
+    void* base = nullptr;        // counts, offsets, records
     size_t bytes = 0;
+    void* att = nullptr;         // attenuator lists
+    size_t att_bytes = 0;
 };
 
 inline void scatter_scratch_free(ScatterScratch& s)
 {
     if (s.base) cudaFree(s.base);
-    s.base = nullptr;
-    s.bytes = 0;
+    if (s.att) cudaFree(s.att);
+    s = ScatterScratch{};
 }
 
 // Pair record of scatterer s (crystal k = s, or hole h = s - D) and detector crystal d,
