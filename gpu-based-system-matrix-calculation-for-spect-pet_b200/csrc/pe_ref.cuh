@@ -16,10 +16,14 @@
 // on B200 with straight-line multiply-add loops: 0.93-0.98 issues per cycle up to there, 0.5-0.65
 // beyond).  One loop over rounds with the whole body in it (about 1300 instructions) ran at
 // that second rate whatever was shortened in it; every phase's loop fits the first.
+// The walks take two rounds at a time, for two independent chains per lane, and a block's warps start
+// each element together, which keeps the warps of a scheduler in the same phase.
 // Bound by instruction issue (DRAM moves a few MB per launch).  Crystals 1984..2015 x one plane of
 // configuration 2: 82.7e3 warp instructions per element at 58 % of the issue slots in one loop,
-// 52.7e3 at 66 % in phases, 36.9 -> 20.6 ms, every float the same.  Two blocks of 8 warps at 128
-// registers: three blocks at 80 issue at 70 % but need 11 % more instructions (spills).
+// 48.1e3 at 68 % now, 36.9 -> 18.1 ms, every float the same.  Two blocks of 8 warps at 128
+// registers: three blocks at 80 issue at 70 % but need 11 % more instructions (spills); one block
+// of 16 warps is 2 % slower, 40 % on matrices of few elements.  Forming the hole terms of a ray only
+// in rounds that have holes is 7 % slower (registers).
 //
 // The fused multiply-adds are written out: they are the ones that the compiler chose for the
 // reference's own expressions, and which product of a sum of two is fused changes the last
@@ -1012,7 +1016,8 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
 // a grid over the voxel) of the reference's element with crystal d divided into nx x ny x nz
 // sub-elements (x, depth, z), every contribution summed in FP64.  Each source point has its own
 // cone test and kept objects, drawn from one list per voxel of the objects near the ray bundle of
-// any source point (a few percent of the block's superset).  With 8 x 16 x 8 and 1 x 1 x 1 it runs
+// any source point (a few percent of the block's superset).  The configuration-2 sampling, 96
+// crystals x 4608 voxels: 38.0 -> 18.8 ms, bound by instruction issue.  With 8 x 16 x 8 and 1 x 1 x 1 it runs
 // pe_element_ref<1>'s float program, summed in another order.
 template <bool ELL>
 __device__ double pe_element_sampled(const DevGeom& g, const Superset& sup, RefWarp& ws, int d, long long v, float cr,
