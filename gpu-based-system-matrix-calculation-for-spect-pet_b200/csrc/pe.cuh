@@ -7,11 +7,6 @@
 
 namespace sysmat {
 
-// Per-element capacities of the shared-memory candidate lists (after cone culling and
-// the ray-bundle filter).  An element that exceeds them raises kStatusCapacity.
-constexpr int kPeEffCrystals = 96;
-constexpr int kPeEffHoles = 192;
-
 // Bits of the device status word.
 constexpr int kStatusCapacity = 1;
 
