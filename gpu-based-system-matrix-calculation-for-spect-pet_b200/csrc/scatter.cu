@@ -355,17 +355,16 @@ __device__ __forceinline__ bool may_meet(const DevGeom& g, int a, float xs, floa
              fabsf(mx * vz - mz * vx) > hx * az + hz * ax);
 }
 
-// Chord of the scatter point -> detector point segment inside attenuating crystal a
-// (scatter.cu:1377-1394).
-__device__ __forceinline__ float attenuator_chord(const DevGeom& g, int a, float xs, float ys, float zs,
-                                                  const DetPoint& q)
+// Chord of the scatter point -> detector point segment inside an attenuating crystal (tables pa, sa,
+// ta; scatter.cu:1377-1394).  Out of line: the kernel that counts a pair's chords and the one that
+// stores them then run the same instructions.  Inlined in each, the compiler may contract a sum of
+// products one way here and another way there, and a chord at a threshold is 0 in one of them only.
+static __device__ __noinline__ float attenuator_chord(float4 pa, float4 sa, float4 ta, float xs, float ys, float zs,
+                                                      float xD, float yD, float zD)
 {
-    const float4 pa = __ldg(&g.cry.pos[a]);
-    const float4 sa = __ldg(&g.cry.size[a]);
-    const float4 ta = __ldg(&g.cry.trig[a]);
     float xa, ya, za, xb, yb, zb;
     to_crystal_frame(pa.x, pa.y, pa.z, ta.z, ta.w, xs, ys, zs, xa, ya, za);
-    to_crystal_frame(pa.x, pa.y, pa.z, ta.z, ta.w, q.xD, q.yD, q.zD, xb, yb, zb);
+    to_crystal_frame(pa.x, pa.y, pa.z, ta.z, ta.w, xD, yD, zD, xb, yb, zb);
     return box_chord(xa, ya, za, xb, yb, zb, -0.5f * sa.x, -0.5f * sa.y, -0.5f * sa.z, 0.5f * sa.x,
                      0.5f * sa.y, 0.5f * sa.z);
 }
@@ -386,7 +385,9 @@ __device__ __forceinline__ void warp_attenuators(const DevGeom& g, const uint32_
     auto flush = [&](int cnt) {                            // the first cnt <= 32 of the queue
         const bool ok = lane < cnt;
         const int a = ok ? lists.queue[lane] : 0;
-        const float len = ok ? attenuator_chord(g, a, xs, ys, zs, q) : 0.0f;
+        const float len = ok ? attenuator_chord(__ldg(&g.cry.pos[a]), __ldg(&g.cry.size[a]), __ldg(&g.cry.trig[a]), xs,
+                                                ys, zs, q.xD, q.yD, q.zD)
+                             : 0.0f;
         f(a, len, ok);
     };
     for (int c0 = 0; c0 < n; c0 += kPairSpan) {
@@ -547,19 +548,22 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_fill_kernel(DevGeom g, i
             r.labs = box_chord(r.xss, r.yss, r.zss, xt, yt, zt, ux1, uy1, uz1, ux2, uy2, uz2);
             // row-relative start: a row holds at most ns * D entries, which fits an int
             r.att_begin = (int)(offsets[p] - offsets[(long long)d * ns]);
+            // never past the pair's own part of the list, whatever the bitmaps hold by now
             AttEntry* dst = att + offsets[p];
+            const int room = (int)(offsets[p + 1] - offsets[p]);
             int k = 0;
             warp_attenuators<NATIVE>(g, bm_cry, bm_col, s, d, xs, ys, zs, q, lane, lists[wid],
                                      [&](int a, float len, bool ok) {
                                          const bool nz = ok && len != 0.0f;
                                          const unsigned m = __ballot_sync(0xffffffffu, nz);
-                                         if (nz) {
+                                         const int at = k + __popc(m & ((1u << lane) - 1u));
+                                         if (nz && at < room) {
                                              const float4 mu = __ldg(&g.cry.mu[a]);
-                                             dst[k + __popc(m & ((1u << lane) - 1u))] = AttEntry{len, mu.y, mu.z};
+                                             dst[at] = AttEntry{len, mu.y, mu.z};
                                          }
                                          k += __popc(m);
                                      });
-            r.att_count = k;
+            r.att_count = min(k, room);
         }
         if (lane == 0) pairs[p] = r;
     }
