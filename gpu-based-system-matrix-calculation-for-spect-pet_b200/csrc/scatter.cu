@@ -926,21 +926,28 @@ static unsigned bitmap_parts(long long rows, long long words)
     return (unsigned)std::max(1LL, std::min(want, most));
 }
 
+// Opt-in above 48 KB of dynamic shared memory: the most crystals that a system can have, not this call's
+// number, since the limit belongs to the kernel and calls from several threads may set it in turn.
+constexpr int kMostCrystals = (kNDetector - 1) / 12;
+
 template <class K>
-static int bitmap_smem(K kernel, size_t bytes)
+static int bitmap_smem(K kernel, size_t per_crystal, int n)
 {
-    if (bytes <= 48 * 1024) return 0;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess ? 0 : -1;
+    if (per_crystal * n <= 48 * 1024) return 0;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(per_crystal * kMostCrystals)) ==
+                   cudaSuccess
+               ? 0
+               : -1;
 }
 
 int launch_bitmap_crystal(const DevGeom& g, uint32_t* words, cudaStream_t s)
 {
     const long long nw = bitmap_crystal_words(g.n_det), n = g.n_det;
     if (nw == 0) return 0;
-    const size_t smem = (sizeof(float4) + sizeof(float)) * (size_t)n;   // at most 6666 crystals: 133 KB
-    if (bitmap_smem(bitmap_crystal_kernel, smem)) return -1;
+    constexpr size_t per_crystal = sizeof(float4) + sizeof(float);   // at most 6666 crystals: 133 KB
+    if (bitmap_smem(bitmap_crystal_kernel, per_crystal, g.n_det)) return -1;
     const dim3 grid((unsigned)n, bitmap_parts(n, nw));
-    bitmap_crystal_kernel<<<grid, kBitmapThreads, smem, s>>>(g.raw_det, g.n_det, n * (n + 1) / 2 * n, words);
+    bitmap_crystal_kernel<<<grid, kBitmapThreads, per_crystal * n, s>>>(g.raw_det, g.n_det, n * (n + 1) / 2 * n, words);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -948,10 +955,10 @@ int launch_bitmap_collimator(const DevGeom& g, uint32_t* words, cudaStream_t s)
 {
     const long long nw = bitmap_collimator_words(g.n_det, g.n_holes0), n = g.n_det;
     if (nw == 0) return 0;
-    const size_t smem = sizeof(float4) * (size_t)n;
-    if (bitmap_smem(bitmap_collimator_kernel, smem)) return -1;
+    constexpr size_t per_crystal = sizeof(float4);
+    if (bitmap_smem(bitmap_collimator_kernel, per_crystal, g.n_det)) return -1;
     const dim3 grid((unsigned)g.n_holes0, bitmap_parts(g.n_holes0, nw));
-    bitmap_collimator_kernel<<<grid, kBitmapThreads, smem, s>>>(g.raw_det, g.hole.raw, g.n_det, n * n * g.n_holes0,
+    bitmap_collimator_kernel<<<grid, kBitmapThreads, per_crystal * n, s>>>(g.raw_det, g.hole.raw, g.n_det, n * n * g.n_holes0,
                                                                 words);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
