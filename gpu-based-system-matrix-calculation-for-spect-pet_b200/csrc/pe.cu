@@ -332,13 +332,22 @@ __device__ __forceinline__ void pe_brick(const DevGeom& g, typename SmemOf<MODE,
     // the brick's voxels inside the block, so that a ragged block's warps share them evenly (and a
     // brick without any builds no superset)
     const int n_slots = bx * by * bz;
-    int n_active = 0;
-    for (int base = 0; base < n_slots; base += kThreads) {
-        const int slot = base + threadIdx.x;
+    auto active = [&](int slot) {
         const int ix = x0 + slot % bx, iy = y0 + (slot / bx) % by, iz = z0 + slot / (bx * by);
         const long long v = ix + g.nx * ((long long)iy + (long long)g.ny * iz);
-        const bool in = slot < n_slots && ix <= x1 && iy <= y1 && iz <= z1 && v >= O.vox_begin && v <= O.vlast;
-        n_active += block_append(sup, in, (unsigned short)slot, sup.slot, n_active, 512, lane, wid);
+        return slot < n_slots && ix <= x1 && iy <= y1 && iz <= z1 && v >= O.vox_begin && v <= O.vlast;
+    };
+    int n_active = 0;
+    if (SAMPLED && n_slots <= 32) {        // every warp counts them; build_superset's barriers publish the list
+        const bool in = active(lane);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        n_active = __popc(m);
+        if (wid == 0 && in) sup.slot[__popc(m & ((1u << lane) - 1u))] = (unsigned short)lane;
+    } else {
+        for (int base = 0; base < n_slots; base += kThreads) {
+            const int slot = base + threadIdx.x;
+            n_active += block_append(sup, active(slot), (unsigned short)slot, sup.slot, n_active, 512, lane, wid);
+        }
     }
     if (n_active == 0) return;
     // brick centre and radius from its extreme voxel centres (rotation about z keeps lengths)

@@ -599,7 +599,7 @@ __device__ double pe_element_local(const DevGeom& g, const Superset& sup, IdWarp
                 }
                 __syncwarp();
             };
-            if constexpr (SMP) pass(AnyDivision{nx, ny, n_sub, 32 * q0, (float)nx, (float)ny, (float)nz});
+            if constexpr (SMP) pass(AnyDivision(nx, ny, nz, 32 * q0));
             else pass(RefDivisionAt(q0));
         }
     }
