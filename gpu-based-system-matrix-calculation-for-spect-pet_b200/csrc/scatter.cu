@@ -598,6 +598,7 @@ struct ElemConst {
     float w, t, h;
     float mu_pe, mu_c, eres;
     float lo, hi;
+    bool bounded;               // both bounds small enough for div_by
     float rdet;
 };
 
@@ -656,7 +657,7 @@ __device__ float scatter_item(const ElemConst& e, const StagedPair& sp, const Pa
     // energy-window probability (calculategaussianIntegral, :1025-1038)
     const float s2 = (float)((double)(fw * es) * 1.4142135623730951), rs2 = rcp_rn(s2);
     float z1 = div_by(e.lo - es, s2, rs2), z2 = div_by(e.hi - es, s2, rs2);
-    if (!(s2 >= kMinDivisor)) {                            // no energy spread
+    if (!(s2 >= kMinDivisor && e.bounded)) {               // no energy spread, or an open window
         z1 = (e.lo - es) / s2;
         z2 = (e.hi - es) / s2;
     }
@@ -782,6 +783,7 @@ __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhys
         e.lo = (1 - e.eres / 2.0f) * ph.e0;                                  // :1161-1162
         e.hi = (1 + e.eres / 2.0f) * ph.e0;
     }
+    e.bounded = fabsf(e.lo) <= 1e15f && fabsf(e.hi) <= 1e15f;
     e.rdet = sqrtf(e.w * e.w / (float)1 / (float)1 + e.h * e.h / (float)1 / (float)1 +
                    e.t * e.t / (float)1 / (float)1) / 2.0f;
     const float re0 = rcp_rn(ph.e0);
