@@ -599,7 +599,7 @@ struct ElemConst {
     float mu_pe, mu_c, eres;
     float lo, hi;
     bool bounded;               // both bounds small enough for div_by
-    float rdet;
+    float rdet, near2;          // circumscribed radius; its square with a margin
 };
 
 // A staged pair: its record and what else belongs to the pair alone, formed once per block: the
@@ -715,8 +715,11 @@ __device__ float scatter_item(const ElemConst& e, const StagedPair& sp, const Pa
         tmax = acosf(cmin);
     }
     // a ray from the voxel through the scatter point that crosses d has theta_min = 0.  It passes
-    // d's centre at lsd sin(cone), so beyond d's circumscribed radius there is no chord to form.
-    if (pr.lsd * sc <= 1.001f * e.rdet + 0.01f) {
+    // d's centre at lsd sin(cone), so beyond d's circumscribed radius there is no chord to form.  A float
+    // cosine of the cone is within nine units of 2^-24 of the exact one, and cosines that far apart have
+    // squared sines within 1.1e-6 of each other, whatever the angle: a tenth of a millimetre at 1 m.
+    const float pass = pr.lsd * sc;
+    if (pass * pass <= __fmaf_rn(1.2e-6f * pr.lsd, pr.lsd, e.near2)) {
         const float rdis = rcp_rn(ma);                     // |voxel - point| in d's frame (:1314)
         const float xt = pr.xss + div_by(1000.0f * ax, ma, rdis);
         const float yt = pr.yss + div_by(1000.0f * ay, ma, rdis);
@@ -786,6 +789,7 @@ __device__ __forceinline__ void scatter_rows(const DevGeom& g, const ScatterPhys
     e.bounded = fabsf(e.lo) <= 1e15f && fabsf(e.hi) <= 1e15f;
     e.rdet = sqrtf(e.w * e.w / (float)1 / (float)1 + e.h * e.h / (float)1 / (float)1 +
                    e.t * e.t / (float)1 / (float)1) / 2.0f;
+    e.near2 = (1.001f * e.rdet + 0.01f) * (1.001f * e.rdet + 0.01f);
     const float re0 = rcp_rn(ph.e0);
 
     double acc_c = 0.0, acc_h = 0.0;
