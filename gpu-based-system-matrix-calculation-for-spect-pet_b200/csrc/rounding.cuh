@@ -10,6 +10,7 @@
 namespace sysmat {
 
 constexpr float kMinDivisor = 1e-15f;   // div_by: smaller divisors take the IEEE division
+constexpr float kMinRoot = 0x1p-100f;   // sqrt_mid: the least argument
 
 // Correctly rounded a / b, given y = RN(1 / b): two residual corrections of a y.  The first
 // makes the quotient faithful, and by Markstein's theorem (P. Markstein, "Computation of

@@ -96,11 +96,14 @@ __device__ __forceinline__ DetPoint det_point(float4 P, float4 S, float4 T)
 
 constexpr int kBitmapThreads = 256;
 
+// Angular radius of a crystal at distance l, at least 2^-51.
+__device__ __forceinline__ float angular_radius(float r, float l) { return fmaxf(r / l, 0x1p-51f); }
+
 // A crystal seen from a point: unit direction and angular radius (scatter.cu:1476-1500, :1975-1996).
 __device__ __forceinline__ float4 seen_from(float xi, float yi, float zi, const float* __restrict__ pk, float rk)
 {
     const float l = dist3(pk[1], pk[2], pk[3], xi, yi, zi);
-    return make_float4((pk[1] - xi) / l, (pk[2] - yi) / l, (pk[3] - zi) / l, rk / l);
+    return make_float4((pk[1] - xi) / l, (pk[2] - yi) / l, (pk[3] - zi) / l, angular_radius(rk, l));
 }
 
 __device__ __forceinline__ float crystal_radius(const float* __restrict__ p)
@@ -108,14 +111,14 @@ __device__ __forceinline__ float crystal_radius(const float* __restrict__ p)
     return sqrtf(p[4] * p[4] + p[6] * p[6] + p[5] * p[5]) / 2.0f;
 }
 
-// |u_k - u_j| <= c_k + c_j.  The root is the IEEE one (its argument is 0, where the root is too,
-// or well above sqrt_mid's lower bound: differences of unit vectors are multiples of 2^-26 or so).
+// |u_k - u_j| <= c_k + c_j.  The root is the IEEE one from 2^-50 on; crystals that lie behind one another
+// but for offsets below 1e-15 of their distance count as that far apart, which angular_radius's least value
+// always covers.
 __device__ __forceinline__ bool cone_meets(const float4& k, const float4& j)
 {
     const float dx = k.x - j.x, dy = k.y - j.y, dz = k.z - j.z;
     const float d2 = dx * dx + dy * dy + dz * dz;
-    const float d = d2 == 0.0f ? 0.0f : sqrt_mid(d2);
-    return d <= k.w + j.w;
+    return sqrt_mid(d2 < kMinRoot ? kMinRoot : d2) <= k.w + j.w;   // false for a NaN (no direction)
 }
 
 // cone_meets of crystals k and i (centres, radii) seen from (x, y, z).  Approximate directions decide
@@ -134,7 +137,8 @@ __device__ __forceinline__ bool cone_meets_from(float x, float y, float z, float
     if (d2 < low * low) return true;
     if (d2 > top * top) return false;
     const float lk = dist3(xk, yk, zk, x, y, z), li = dist3(xi, yi, zi, x, y, z);
-    return cone_meets(make_float4(kx / lk, ky / lk, kz / lk, rk / lk), make_float4(jx / li, jy / li, jz / li, ri / li));
+    return cone_meets(make_float4(kx / lk, ky / lk, kz / lk, angular_radius(rk, lk)),
+                      make_float4(jx / li, jy / li, jz / li, angular_radius(ri, li)));
 }
 
 // Whether crystal k may attenuate the path between crystals i and j, i < j (:1465-1534).
