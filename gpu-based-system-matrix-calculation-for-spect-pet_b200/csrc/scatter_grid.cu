@@ -258,8 +258,13 @@ __device__ void chunk_candidates(const DevGeom& g, const GridGeom& G, Cands& C, 
     __syncthreads();
 }
 
-// A segment A -> A + d with what its overlaps with boxes and cylinders share: reciprocals (rcp64;
-// a component below 1e-30 counts as 0 and has none), length, and the xz part a = dx^2 + dz^2.
+// A segment A -> A + d with what its overlaps with boxes and cylinders share: reciprocals (rcp64; a
+// component below kLevel counts as 0 and has none), length, and the xz part a = dx^2 + dz^2.  With
+// components of 1e-12 mm and more, squares and the discriminants that they bound stay in the domain of
+// rcp64 and sqrt64, whose float seeds end at 1e-38.
+constexpr double kLevel = 1e-12;         // mm
+constexpr double kMinDisc = 1e-37;       // at most this: the path touches the cylinder at most, its chord is 0
+
 struct Seg64 {
     double A[3], d[3], id[3];
     double len, a, ia;
@@ -272,7 +277,7 @@ __device__ __forceinline__ Seg64 make_seg(const double A[3], const double B[3])
     for (int k = 0; k < 3; ++k) {
         const double d = B[k] - A[k];
         s.A[k] = A[k];
-        s.d[k] = fabs(d) < 1e-30 ? 0.0 : d;
+        s.d[k] = fabs(d) < kLevel ? 0.0 : d;
         s.id[k] = rcp64(s.d[k]);
     }
     s.a = s.d[0] * s.d[0] + s.d[2] * s.d[2];
@@ -330,7 +335,7 @@ __device__ __forceinline__ double seg_cyl64(const Seg64& s, double xc, double zc
         if (c > 0.0) return 0.0;
     } else {
         const double disc = b * b - a * c;
-        if (disc <= 1e-60) return 0.0;
+        if (disc <= kMinDisc) return 0.0;
         const double sq = sqrt64(disc);
         const double u = (-b - sq) * ia, v = (-b + sq) * ia;
         t0 = u > t0 ? u : t0;
