@@ -241,7 +241,7 @@ __device__ __forceinline__ RayL ray_local(const ElemL& L, float xDs, float yDs, 
     const Elem64& E = L.e64;
     const double cx = E.xd - E.xI, cy = E.yd - E.yI, cz = E.zd - E.zI;   // voxel -> crystal d's centre
     const double dx = cx + (double)r.ox, dy = cy + (double)r.oy, dz = cz + (double)r.oz;
-    const double idy = rcp64(dy);
+    const double idy = fabs(dy) > 1e-30 ? rcp64(dy) : 1.0 / dy;   // a ray level with the plates: infinite
     r.dsec = sqrt64(norm3(dx, dy, dz)) * idy;
     const double f = idy * L.idyc;
     r.ddrx = __dmul_rn(diff2((double)r.ox, cy, cx, (double)r.oy), f);
@@ -460,7 +460,7 @@ struct ModeLocal {
         const double sec = q.r.dsec;
         while (s.lay < upto) {                                             // :1276-1284
             const LayerInfo& Ly = g.layer[s.lay];
-            s.att = __fma_rn((double)s.hatt, sec, s.att);
+            if (s.hatt != 0.0f) s.att = __fma_rn((double)s.hatt, sec, s.att);
             const double sept = (double)(Ly.thickness - s.ext) * sec;
             if (sept >= (double)0.00001f) s.att = __fma_rn((double)Ly.mu_total, sept, s.att);
             s.ext = 0.0f;
