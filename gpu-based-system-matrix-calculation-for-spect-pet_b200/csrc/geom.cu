@@ -67,7 +67,7 @@ __global__ void ell_chords_kernel(const float* __restrict__ a, float* __restrict
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* p = a + 13 * (long long)i;
-    out[i] = ell_chord(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], p[11], cosf(p[12]),
+    out[i] = ell_chord<true>(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], p[11], cosf(p[12]),
                        sinf(p[12]));
 }
 

@@ -250,58 +250,73 @@ __device__ __forceinline__ float cyl_chord(float xi, float yi, float zi, float x
     return eb - ea;
 }
 
-// Chord through the y-parallel elliptical cylinder ((x'-xc)/rx)^2 + ((z'-zc)/rz)^2 <= 1,
-// y in [y1, y2], with the segment's points rotated by theta about the axis first
-// (PESysMatGen.cu:801-947, defined but not called by the reference kernels).  ct, st are
-// cos(theta), sin(theta) as the reference evaluates them; each expression is written as the
-// reference writes it, so nvcc contracts it the same way.
+// Elliptical-cylinder chord: the segment's points rotated by theta about the hole's axis, its
+// direction and its points on the cap planes y1, y2 (PESysMatGen.cu:801-860, defined but not called by
+// the reference kernels); ct, st are cos(theta), sin(theta) as the reference evaluates them.  The
+// cancelling sums below make the chord depend on which products are fused (by up to 7e-3 mm), so they
+// are written out: left to the compiler, they change with the code that the chord is inlined in.
+struct EllFrame {
+    float x_in, z_in, tio, kx, ky, kz, ta, tb;
+    bool fl, fr;                 // inside the hole at the caps
+};
+
+__device__ __forceinline__ EllFrame ell_frame(float x_in, float y_in, float z_in, float x_out, float y_out, float z_out,
+                                              float xc, float y1, float y2, float zc, float rx, float rz, float ct, float st)
+{
+    EllFrame f;
+    const float x_in_ = x_in - xc, z_in_ = z_in - zc, x_out_ = x_out - xc, z_out_ = z_out - zc;
+    f.x_in = __fmaf_rn(z_in_, st, __fmaf_rn(x_in_, ct, xc));
+    f.z_in = __fmaf_rn(z_in_, ct, __fmaf_rn(-x_in_, st, zc));
+    const float dx = __fmaf_rn(z_out_, st, __fmaf_rn(x_out_, ct, xc)) - f.x_in, dy = y_out - y_in;
+    const float dz = __fmaf_rn(z_out_, ct, __fmaf_rn(-x_out_, st, zc)) - f.z_in;
+    f.tio = sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
+    f.kx = dx / f.tio;
+    f.ky = dy / f.tio;
+    f.kz = dz / f.tio;
+    const float sx = f.kx / f.ky, sz = f.kz / f.ky;
+    const float xl = __fmaf_rn(sx, y1 - y_in, f.x_in) - xc, xr = __fmaf_rn(sx, y2 - y_in, f.x_in) - xc;
+    const float zl = __fmaf_rn(sz, y1 - y_in, f.z_in) - zc, zr = __fmaf_rn(sz, y2 - y_in, f.z_in) - zc;
+    f.ta = (y1 - y_in) / f.ky;
+    f.tb = (y2 - y_in) / f.ky;
+    f.fl = __fadd_rn(__fmul_rn(xl, xl) / rx / rx, __fmul_rn(zl, zl) / rz / rz) <= 1.0f;
+    f.fr = __fadd_rn(__fmul_rn(xr, xr) / rx / rx, __fmul_rn(zr, zr) / rz / rz) <= 1.0f;
+    return f;
+}
+
+// Chord through the y-parallel elliptical cylinder ((x'-xc)/rx)^2 + ((z'-zc)/rz)^2 <= 1, y in [y1, y2]
+// (PESysMatGen.cu:801-947).  REFERENCE: the fusions under which most chords equal the reference
+// function's own (93 % of 4000 measured; sysmat_ell_chords).  The elements' chord has the other product
+// of c fused, which 83 % do.
+template <bool REFERENCE = false>
 __device__ __forceinline__ float ell_chord(float x_in, float y_in, float z_in, float x_out, float y_out,
                                            float z_out, float xc, float y1, float y2, float zc, float rx,
                                            float rz, float ct, float st)
 {
-    const float x_in_ = x_in - xc;
-    const float z_in_ = z_in - zc;
-    const float x_out_ = x_out - xc;
-    const float z_out_ = z_out - zc;
-    x_in = xc + x_in_ * ct + z_in_ * st;
-    z_in = zc - x_in_ * st + z_in_ * ct;
-    x_out = xc + x_out_ * ct + z_out_ * st;
-    z_out = zc - x_out_ * st + z_out_ * ct;
     if (fabsf(y1 - y2) < 0.001f) return 0.0f;
-    const float tio = sqrtf((x_out - x_in) * (x_out - x_in) + (y_out - y_in) * (y_out - y_in) +
-                            (z_out - z_in) * (z_out - z_in));
-    const float kx = (x_out - x_in) / tio;
-    const float ky = (y_out - y_in) / tio;
-    const float kz = (z_out - z_in) / tio;
-    const float xl = x_in + kx / ky * (y1 - y_in);
-    const float xr = x_in + kx / ky * (y2 - y_in);
-    const float zl = z_in + kz / ky * (y1 - y_in);
-    const float zr = z_in + kz / ky * (y2 - y_in);
-    const float ta = (y1 - y_in) / ky;
-    const float tb = (y2 - y_in) / ky;
-    const bool fl = ((xl - xc) * (xl - xc) / rx / rx + (zl - zc) * (zl - zc) / rz / rz) <= 1.0f;
-    const bool fr = ((xr - xc) * (xr - xc) / rx / rx + (zr - zc) * (zr - zc) / rz / rz) <= 1.0f;
-    if (fr && fl) {
+    const EllFrame f = ell_frame(x_in, y_in, z_in, x_out, y_out, z_out, xc, y1, y2, zc, rx, rz, ct, st);
+    const float ta = f.ta, tb = f.tb, tio = f.tio;
+    if (f.fr && f.fl) {
         if (ta <= 0.0001f || tb <= 0.0001f) return 0.0f;
         if (ta >= tio || tb >= tio) return 0.0f;
         return fabsf(tb - ta);
     }
-    const float x_ = x_in - xc;
-    const float z_ = z_in - zc;
-    const float a = (kx * kx * rz * rz + kz * kz * rx * rx);
-    const float b = kx * x_ * rz * rz + kz * z_ * rx * rx;
-    const float c = rz * rz * x_ * x_ + rx * rx * z_ * z_ - rx * rx * rz * rz;
-    const float delta = (b * b - a * c);
+    const float x_ = f.x_in - xc, z_ = f.z_in - zc;
+    const float a = __fmaf_rn(__fmul_rn(__fmul_rn(f.kx, f.kx), rz), rz, __fmul_rn(__fmul_rn(__fmul_rn(f.kz, f.kz), rx), rx));
+    const float b = __fmaf_rn(__fmul_rn(__fmul_rn(f.kx, x_), rz), rz, __fmul_rn(__fmul_rn(__fmul_rn(f.kz, z_), rx), rx));
+    const float cx = __fmul_rn(__fmul_rn(rz, rz), x_), cz = __fmul_rn(__fmul_rn(rx, rx), z_);
+    const float c = __fmaf_rn(-__fmul_rn(__fmul_rn(rx, rx), rz), rz,
+                              REFERENCE ? __fmaf_rn(cx, x_, __fmul_rn(cz, z_)) : __fmaf_rn(cz, z_, __fmul_rn(cx, x_)));
+    const float delta = __fmaf_rn(b, b, -__fmul_rn(a, c));
     if (delta <= 0.00001f) return 0.0f;
     const float t1 = (-b - sqrtf(delta)) / a;
     const float t2 = (-b + sqrtf(delta)) / a;
-    if (!fr && !fl) {
+    if (!f.fr && !f.fl) {
         if (!((t1 >= ta) && (t2 <= tb))) return 0.0f;
         if (t2 <= 0.0001f || t1 <= 0.0001f) return 0.0f;
         if (t2 >= tio || t1 >= tio) return 0.0f;
         return t2 - t1;
     }
-    if (fl && !fr) {
+    if (f.fl && !f.fr) {
         if (t2 <= 0.0001f || ta <= 0.0001f) return 0.0f;
         if (t2 >= tio || ta >= tio) return 0.0f;
         return t2 - ta;

@@ -58,18 +58,11 @@ __device__ __forceinline__ float ell_chord_grad(float xi, float yi, float zi, fl
     gr = CylGrad{0.0f, 0.0f, 0.0f, 0.0f};
     const float L = ell_chord(xi, yi, zi, xo, yo, zo, xc, y1, y2, zc, rx, rz, ct, st);
     if (L == 0.0f) return L;
-    // the frame quantities of ell_chord, with its expressions (same case flags)
-    const float xi_ = xi - xc, zi_ = zi - zc, xo_ = xo - xc, zo_ = zo - zc;
-    const float xin = xc + xi_ * ct + zi_ * st, zin = zc - xi_ * st + zi_ * ct;
-    const float xout = xc + xo_ * ct + zo_ * st, zout = zc - xo_ * st + zo_ * ct;
-    const float tio = sqrtf((xout - xin) * (xout - xin) + (yo - yi) * (yo - yi) + (zout - zin) * (zout - zin));
-    const float kx = (xout - xin) / tio, ky = (yo - yi) / tio, kz = (zout - zin) / tio;
-    const float xl = xin + kx / ky * (y1 - yi), xr = xin + kx / ky * (y2 - yi);
-    const float zl = zin + kz / ky * (y1 - yi), zr = zin + kz / ky * (y2 - yi);
-    const bool fl = ((xl - xc) * (xl - xc) / rx / rx + (zl - zc) * (zl - zc) / rz / rz) <= 1.0f;
-    const bool fr = ((xr - xc) * (xr - xc) / rx / rx + (zr - zc) * (zr - zc) / rz / rz) <= 1.0f;
+    const EllFrame f = ell_frame(xi, yi, zi, xo, yo, zo, xc, y1, y2, zc, rx, rz, ct, st);   // same case flags
+    const float kx = f.kx, ky = f.ky, kz = f.kz;
+    const bool fl = f.fl, fr = f.fr;
     if (fl && fr) return L;                     // |tb - ta|: cap to cap, shift and turn invariant
-    const float u0 = xin - xc, w0 = zin - zc;
+    const float u0 = f.x_in - xc, w0 = f.z_in - zc;
     const float rx2 = rx * rx, rz2 = rz * rz;
     const float a = kx * kx * rz2 + kz * kz * rx2;
     const float b = kx * u0 * rz2 + kz * w0 * rx2;
