@@ -82,8 +82,9 @@ __device__ __forceinline__ float sub_centre(int i, float f, float rf, float size
 __device__ __forceinline__ float4 sub_row(int i, float f, float rf, float size, float p)
 {
     const float c = sub_centre(i, f, rf, size);
-    const float u1 = (div_by((float)i, f, rf) - 0.5f) * size, u2 = (div_by((float)i + 1.0f, f, rf) - 0.5f) * size;
-    return make_float4(c, c - p, u1 - p, u2 - p);
+    const float u1 = __fmul_rn(div_by((float)i, f, rf) - 0.5f, size);
+    const float u2 = __fmul_rn(div_by((float)i + 1.0f, f, rf) - 0.5f, size);
+    return make_float4(c, c - p, __fsub_rn(u1, p), __fsub_rn(u2, p));
 }
 
 // The reference's 8 x 16 x 8, rows kept in ws.sub.
