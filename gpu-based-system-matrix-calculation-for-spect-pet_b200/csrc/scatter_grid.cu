@@ -287,14 +287,20 @@ __device__ __forceinline__ Seg64 make_seg(const double A[3], const double B[3])
     return s;
 }
 
-// The part [t0, t1] of the segment's parameter range inside the slab [lo, hi] of one axis.
+// The part [t0, t1] of the segment's parameter range inside the slab [lo, hi] of one axis.  FACE: the
+// quotients get their residual, so that a segment that ends on a face has the parameter 1 there exactly.
+template <bool FACE = false>
 __device__ __forceinline__ void seg_clip(double A, double d, double id, double lo, double hi, double& t0, double& t1)
 {
     if (d == 0.0) {
         if (A < lo || A > hi) t1 = -1.0;
         return;
     }
-    const double u = (lo - A) * id, v = (hi - A) * id;
+    double u = (lo - A) * id, v = (hi - A) * id;
+    if constexpr (FACE) {
+        u = fma(fma(-d, u, lo - A), id, u);
+        v = fma(fma(-d, v, hi - A), id, v);
+    }
     const double e = u < v ? u : v, x = u < v ? v : u;
     t0 = e > t0 ? e : t0;
     t1 = x < t1 ? x : t1;
@@ -302,12 +308,14 @@ __device__ __forceinline__ void seg_clip(double A, double d, double id, double l
 
 // Length of the segment inside the box [lo, hi]: the exact overlap of its parameter range with the
 // three slabs.  The grid model's paths start or end inside the plate or a crystal, where the
-// reference's chords (full crossings between the two ends) do not apply.
+// reference's chords (full crossings between the two ends) do not apply.  Exactly 0 for a path that only
+// touches the box: a layer counts for the paths that are inside its plate somewhere, and its holes may
+// reach beyond it.
 __device__ __forceinline__ double seg_box64(const Seg64& s, const double lo[3], const double hi[3])
 {
     double t0 = 0.0, t1 = 1.0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) seg_clip(s.A[a], s.d[a], s.id[a], lo[a], hi[a], t0, t1);
+    for (int a = 0; a < 3; ++a) seg_clip<true>(s.A[a], s.d[a], s.id[a], lo[a], hi[a], t0, t1);
     return t1 <= t0 ? 0.0 : (t1 - t0) * s.len;
 }
 
