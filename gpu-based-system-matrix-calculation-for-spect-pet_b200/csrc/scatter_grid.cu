@@ -327,7 +327,7 @@ __device__ __forceinline__ double seg_cyl64(const Seg64& s, double xc, double zc
                                             const D4& E)
 {
     double t0 = 0.0, t1 = 1.0;
-    seg_clip(s.A[1], s.d[1], s.id[1], y1 < y2 ? y1 : y2, y1 < y2 ? y2 : y1, t0, t1);
+    seg_clip(s.A[1], s.d[1], s.id[1], y1, y2, t0, t1);      // a level segment is in no slab whose ends are exchanged
     double dx = s.d[0], dz = s.d[2], ox = s.A[0] - xc, oz = s.A[2] - zc, a = s.a, ia = s.ia;
     if (E.x > 0.0) {
         const double rx = 1.0 / E.x, rz = 1.0 / E.y;

@@ -32,3 +32,24 @@ def test_paths_that_end_on_a_plate(gpu, thickness, offset):
     ref = oracle.scatter_grid(geo, parts=2, cell=3.0)
     assert ref.max() > 0
     assert np.abs(out.cpu().numpy() - ref).max() <= TOL * ref.max()
+
+
+@pytest.mark.parametrize("exchanged", [False, True])
+def test_level_paths(gpu, exchanged):
+    """Voxels at the depth of the plate's middle: their paths to its cells run level, and are inside the
+    holes whose first cap is the lower one."""
+    cb = geometry._CollimatorBuilder()
+    cb.add_layer(14.0, 0.5, 14.0, 0.0, 0.2, 0.1, 0.1, [(x, z, 0.6) for x in (-3.0, 0.0, 3.0) for z in (-3.0, 0.0, 3.0)])
+    col = cb.build()
+    if exchanged:
+        h = col[100:100 + 9 * 9].reshape(9, 9)
+        h[::2, 1], h[::2, 2] = h[::2, 2].copy(), h[::2, 1].copy()
+    det = geometry._detector([(0.3, 9.0, -0.4), (3.0, 9.0, 1.0)], (1.0, 2.0, 1.0))
+    geo = geometry.Geometry("level", col, det, geometry._image((3, 1, 2), (1.9, 1.0, 2.3), 0.0, shift=(0.2, 0.0, -0.3)),
+                            geometry._physics(lo=40.0))
+    ctx = sysmat.Context(geo)
+    out = gpu.empty((ctx.n_det, ctx.n_vox), dtype=gpu.float32, device="cuda")
+    ctx.scatter_grid(out, parts=sysmat.SCATTER_COLLIMATOR, cell=1.0)
+    ref = oracle.scatter_grid(geo, parts=2, cell=1.0)
+    assert ref.min() > 0
+    assert np.abs(out.cpu().numpy() - ref).max() <= TOL * ref.max()
