@@ -136,11 +136,24 @@ __device__ __forceinline__ int layer_of_hole(const DevGeom& g, int h)
     return m;
 }
 
-// box_chord of the segment voxel -> sub-element through a plate, out of line: few rays need it.
+// box_chord of the segment voxel -> sub-element through a plate, out of line: few rays need it.  Its
+// length decides whether a ray counts at all, so the fused products are written out; they are those of the
+// one-loop kernels, and not the ones of the crystal chord (norm2 with the depth first).
 static __device__ __noinline__ float plate_chord(float xi, float yi, float zi, float xo, float yo, float zo,
                                                  float x1, float y1, float z1, float x2, float y2, float z2)
 {
-    return box_chord(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2);
+    const float dx = xo - xi, dy = yo - yi, dz = zo - zi;
+    if (fabsf(dx) < kEps || fabsf(dy) < kEps || fabsf(dz) < kEps)
+        return box_chord_parallel(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2, 0);
+    const float tio = sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
+    const float ix = tio / dx, iy = tio / dy, iz = tio / dz;
+    const float ax = __fmul_rn(x1 - xi, ix), bx = __fmul_rn(x2 - xi, ix);
+    const float ay = __fmul_rn(y1 - yi, iy), by = __fmul_rn(y2 - yi, iy);
+    const float az = __fmul_rn(z1 - zi, iz), bz = __fmul_rn(z2 - zi, iz);
+    const float tmin = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
+    const float tmax = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
+    const bool out = (tmax - tmin) < kEps || tmin >= tio || tmax >= tio || tmin <= kEps || tmax <= kEps;
+    return out ? 0.0f : tmax - tmin;
 }
 
 // Plate penalty (:1240-1254); true if any layer fired.

@@ -1,6 +1,8 @@
 // The reference's element of a crystal that stands alone (PESysMatGen.cu:1207-1231, :1329-1359: self
-// attenuation, absorption, solid angle; unrotated) one rounding at a time, one thread per voxel.  Arguments:
-// crystal x y z (y with the FOV offset), width thickness height, mu, mu_pe, then x y z of each voxel.
+// attenuation, absorption, solid angle; unrotated) behind a plate without holes or attenuation (:1240-1254: a
+// ray whose chord in it is below 0.1 mm does not count), one rounding at a time, one thread per voxel.
+// Arguments: crystal x y z (y with the FOV offset), width thickness height, mu, mu_pe, the plate's box x1 y1 z1
+// x2 y2 z2 (x1 > x2: none), then x y z of each voxel.
 // Prints the bits of each element.
 #include <cstdint>
 #include <cstdio>
@@ -16,7 +18,7 @@
 #define FMA __fmaf_rn
 
 struct Crystal {
-    float pos[3], size[3], mu, mu_pe;
+    float pos[3], size[3], mu, mu_pe, plate[6];
 };
 
 // centre, centre - voxel, lower and upper face - voxel of part i of n along an axis
@@ -64,6 +66,15 @@ __global__ void elements(Crystal c, const float* voxel, int n, float* out)
             clip(a[k][2], a[k][3], inv, u0, u1);
             world[k] = SUB(ADD(c.pos[k], a[k][0]), voxel[3 * v + k]);
         }
+        if (c.plate[0] <= c.plate[3]) {
+            float d[3], q0 = -INFINITY, q1 = INFINITY;
+            for (int k = 0; k < 3; ++k) d[k] = SUB(ADD(c.pos[k], a[k][0]), voxel[3 * v + k]);
+            const float len = __fsqrt_rn(norm(d[0], d[1], d[2]));
+            for (int k = 0; k < 3; ++k)
+                clip(SUB(c.plate[k], voxel[3 * v + k]), SUB(c.plate[3 + k], voxel[3 * v + k]), DIV(len, d[k]), q0, q1);
+            const bool none = SUB(q1, q0) < 0.001f || q0 >= len || q1 >= len || q0 <= 0.001f || q1 <= 0.001f;
+            if (none || SUB(q1, q0) < 0.1f) continue;
+        }
         const float self = SUB(inside(t0, t1, tio), inside(u0, u1, tio));
         const float dsq = norm(world[0], world[1], world[2]), sq = __fsqrt_rn(dsq);
         for (int k = 0; k < 3; ++k) {
@@ -90,13 +101,13 @@ int main(int argc, char** argv)
 {
     std::vector<float> a;
     for (int i = 1; i < argc; ++i) a.push_back((float)std::atof(argv[i]));
-    const int n = ((int)a.size() - 8) / 3;
+    const int n = ((int)a.size() - 14) / 3;
     if (n < 1) return 1;
-    const Crystal c{{a[0], a[1], a[2]}, {a[3], a[4], a[5]}, a[6], a[7]};
+    const Crystal c{{a[0], a[1], a[2]}, {a[3], a[4], a[5]}, a[6], a[7], {a[8], a[9], a[10], a[11], a[12], a[13]}};
     float *voxel, *out;
     cudaMalloc(&voxel, 3 * n * sizeof(float));
     cudaMalloc(&out, n * sizeof(float));
-    cudaMemcpy(voxel, &a[8], 3 * n * sizeof(float), cudaMemcpyHostToDevice);
+    cudaMemcpy(voxel, &a[14], 3 * n * sizeof(float), cudaMemcpyHostToDevice);
     elements<<<(n + 31) / 32, 32>>>(c, voxel, n, out);
     std::vector<uint32_t> bits(n);
     if (cudaMemcpy(bits.data(), out, n * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
