@@ -146,14 +146,21 @@ static __device__ __noinline__ float plate_chord(float xi, float yi, float zi, f
     if (fabsf(dx) < kEps || fabsf(dy) < kEps || fabsf(dz) < kEps)
         return box_chord_parallel(xi, yi, zi, xo, yo, zo, x1, y1, z1, x2, y2, z2, 0);
     const float tio = sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
-    const float ix = tio / dx, iy = tio / dy, iz = tio / dz;
-    const float ax = __fmul_rn(x1 - xi, ix), bx = __fmul_rn(x2 - xi, ix);
-    const float ay = __fmul_rn(y1 - yi, iy), by = __fmul_rn(y2 - yi, iy);
-    const float az = __fmul_rn(z1 - zi, iz), bz = __fmul_rn(z2 - zi, iz);
-    const float tmin = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
-    const float tmax = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
-    const bool out = (tmax - tmin) < kEps || tmin >= tio || tmax >= tio || tmin <= kEps || tmax <= kEps;
-    return out ? 0.0f : tmax - tmin;
+    float tmin, tmax, a0, a1;
+    slab_interval(xi, x1, x2, tio / dx, tmin, tmax);
+    slab_interval(yi, y1, y2, tio / dy, a0, a1);
+    if (tmin > a1 || a0 > tmax) return 0.0f;
+    tmin = (a0 > tmin) ? a0 : tmin;
+    tmax = (a1 < tmax) ? a1 : tmax;
+    slab_interval(zi, z1, z2, tio / dz, a0, a1);
+    if (tmin > a1 || a0 > tmax) return 0.0f;
+    tmin = (a0 > tmin) ? a0 : tmin;
+    tmax = (a1 < tmax) ? a1 : tmax;
+    const float len = __fsub_rn(tmax, tmin);
+    if (len < kEps) return 0.0f;
+    if (tmin >= tio || tmax >= tio) return 0.0f;
+    if (tmin <= kEps || tmax <= kEps) return 0.0f;
+    return len;
 }
 
 // Plate penalty (:1240-1254); true if any layer fired.
