@@ -366,7 +366,7 @@ PeLaunch pe_block(sysmat_ctx* ctx, float rotation, int det_begin, int det_count,
 }
 
 // Zero the counter and status word, launch (launch(L) returns non-zero on a launch error),
-// then wait for the status word: SYSMAT_ERR_CAPACITY if an element overflowed a list.
+// then wait for the status word: the call is synchronous.
 template <class Launch>
 int run_pe_block(sysmat_ctx* ctx, const PeLaunch& L, cudaStream_t s, Launch&& launch)
 {

@@ -5,8 +5,10 @@
 // as the reference kernel photodetectorCudaMe defines it
 // (PEGen_RayTracing_CircularHole/PESysMatGen.cu:951-1364), with a different execution plan:
 //
-//  * a block owns one crystal d and a brick of up to 16 voxels (choose_bricks; work items handed
-//    out by an atomic counter over a persistent grid); one warp per matrix element;
+//  * a block owns one crystal d and a brick of voxels: up to 16 in a launch of its own
+//    (choose_bricks), what the plan says in a batched one (4 x 4 x 2 unless set or tuned, 512 at
+//    most), 4 x 4 x 2 in a projection; work items are handed out by an atomic counter over a
+//    persistent grid; one warp per matrix element;
 //  * the block builds a conservative superset of the reference's cone test (:1105-1186) for
 //    every voxel of the brick, from the brick's centre and radius, in the reference's object
 //    order.  Each warp keeps the objects of its element that pass the reference cone test and
@@ -257,7 +259,7 @@ __device__ __forceinline__ int block_append(Superset& bs, bool in, unsigned shor
 // extent: |u_o - u_d| <= (rho + r_o)/(L_o - rho) + (rho + r_d)/(L_d - rho) + 1e-4 at the centre (each
 // direction moves by at most rho/(L - rho) in chord length, each angular radius r/L grows to at most
 // r/(L - rho)).  Each warp scans its own run of objects, a lane keeping a group's ballot, so the block
-// meets twice and not twice per 256 objects.  On a production plane the slope test leaves 60 of the
+// meets twice and not twice per 256 objects.  On a production plane the slope test leaves 73 of the
 // 435 objects that pass the cone test, and the elements' own filters scan that much less: 128
 // crystals x that plane, 77.4 -> 74.1 ms.
 __device__ void build_superset(const DevGeom& g, Superset& bs, int d, float cx, float cy, float cz, float rho,

@@ -7,7 +7,8 @@
 
 namespace sysmat {
 
-// Bits of the device status word.
+// Bits of the device status word.  No kernel sets one: an element whose lists overflow takes them in
+// pieces.  The callers read the word all the same, which is what they wait on.
 constexpr int kStatusCapacity = 1;
 
 // Sampled form of the photoelectric element (no reference counterpart): crystal sub-elements
@@ -55,7 +56,9 @@ struct PeLaunch {
     int* status;                           // zeroed before the launch
     // optional work counters (nullptr in timed runs): [0] sub-elements evaluated,
     // [1] non-zero hole chords, [2] non-zero crystal chords, [3] elements, [4] plate-blocked
-    // sub-elements, [5] cone-test candidates (holes + crystals)
+    // sub-elements, [5] elements whose kept objects fill several record arrays, [6] kept objects (of
+    // the last array), [7] entries over all rounds, [8] elements without a superset, [9] superset
+    // objects, [10] hole chords, [11] crystal chords formed
     unsigned long long* counters;
     Sampling smp;                          // read by the sampled instances only
     // local sampled instance only (optional): per-sub-element contributions, written at

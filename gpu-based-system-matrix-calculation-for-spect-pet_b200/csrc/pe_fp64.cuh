@@ -8,10 +8,10 @@
 // float moves cap planes and plate faces by an ulp of ~60 mm, and T/cos(theta) - sum L cancels.
 // In double those errors are ~1e-15.
 //
-// The culling machinery is the float kernel's: block superset, slope rectangles, round
-// capsules and per-lane rectangles are geometric filters with margins far above float
-// rounding, so every object they skip has a zero chord in double too.  The kept list's cone
-// test, which is part of the reference's model rather than a filter, is evaluated in double.
+// The culling machinery is the float kernel's: block superset, slope rectangles and the rounds'
+// masks (Shadow) are geometric filters with margins far above float rounding, so every object they
+// skip has a zero chord in double too.  The kept list's cone test, which is part of the reference's
+// model rather than a filter, is evaluated in double.
 
 // Per-element constants in double.
 struct Elem64 {
@@ -163,7 +163,7 @@ struct Mode64 {
             ++s.lay;
         }
     }
-    // The chord of ray_cyl64_chord (chord64.cuh) as selects.
+    // The cylinder chord (chord64.cuh says which of its forms) as selects.
     static __device__ __forceinline__ void hole(const DevGeom& g, const Warp& ws, Ray& q, int, int id, State& s)
     {
         const Elem64& E = ws.c.e64;

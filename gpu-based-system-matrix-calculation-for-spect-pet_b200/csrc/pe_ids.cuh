@@ -1,10 +1,9 @@
 // Phases of the element modes that read their own geometry tables (pe_fp64.cuh, pe_local.cuh),
 // included by pe.cu inside its anonymous namespace: kept objects as ids, round masks, and the walk
 // over rounds, as pe_ref.cuh does for the float program (why phases: see there).  The mode supplies
-// its constants, its ray and its chords:
+// its constants, which lane 0 fills in before the phases, its ray and its chords:
 //
 //   Consts                        the element's constants, in shared memory
-//   init(g, ws, d, v, ...)        called by lane 0
 //   Ray ray(ws, ix, iy, iz)       what the holes need of a ray
 //   records(g, ws, count, nh)     per-object terms of the element, kUnitBytes a hole, two units a crystal
 //   State                         a ray's attenuation and its open layer (att, open, lay)

@@ -21,7 +21,7 @@
 //     chords from the sub-element centre in crystal d's frame;
 //   - the 1024 contributions are summed with Neumaier's compensated summation, per lane and
 //     across the warp.
-// The culling (superset, slope rectangles, capsules) is the float kernel's; its margins are far
+// The culling (superset, slope rectangles, masks) is the float kernel's; its margins are far
 // above float rounding, and the kept list's cone test is the double one of the FP64 mode.
 
 struct ElemL {

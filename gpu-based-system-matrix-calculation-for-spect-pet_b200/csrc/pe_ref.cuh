@@ -14,8 +14,8 @@
 //   6. the sum.
 // Why phases: a warp scheduler's instruction cache holds about 8 KB (512 instructions; measured
 // on B200 with straight-line multiply-add loops: 0.93-0.98 issues per cycle up to there, 0.5-0.65
-// beyond).  One loop over rounds with the whole body in it (about 1300 instructions) ran at
-// that second rate whatever was shortened in it; every phase's loop fits the first.
+// beyond).  One loop over rounds with the whole body in it ran at that second rate whatever was
+// shortened in it; every phase's loop fits the first.
 // The walks take two rounds at a time, for two independent chains per lane, and a block's warps start
 // each element together, which keeps the warps of a scheduler in the same phase.
 // Bound by instruction issue (DRAM moves a few MB per launch).  Crystals 1984..2015 x one plane of
@@ -1033,7 +1033,7 @@ __device__ double pe_element_ref(const DevGeom& g, const Superset& sup, RefWarp&
 // sub-elements (x, depth, z), every contribution summed in FP64.  Each source point has its own
 // cone test and kept objects, drawn from one list per voxel of the objects near the ray bundle of
 // any source point (a few percent of the block's superset).  The configuration-2 sampling, 96
-// crystals x 4608 voxels: 38.0 -> 18.8 ms, bound by instruction issue.  With 8 x 16 x 8 and 1 x 1 x 1 it runs
+// crystals x 4608 voxels: 38.0 -> 16.7 ms, bound by instruction issue.  With 8 x 16 x 8 and 1 x 1 x 1 it runs
 // pe_element_ref<1>'s float program, summed in another order.
 template <bool ELL>
 __device__ double pe_element_sampled(const DevGeom& g, const Superset& sup, RefWarp& ws, int d, long long v, float cr,

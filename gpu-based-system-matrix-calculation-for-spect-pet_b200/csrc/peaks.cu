@@ -1,5 +1,5 @@
 // Measured FP32 and MUFU peaks of the current device, for the roofline of the
-// system-matrix kernels (which are FP32/MUFU bound, not HBM or tensor-core bound).
+// system-matrix kernels (bound by the issue of FP32 and MUFU work, not by HBM or tensor cores).
 //
 // fp32: each thread runs 8 independent FMA chains; one FMA = 2 flops.
 // mufu: each thread runs 8 independent ex2.approx chains (one MUFU op each).

@@ -46,7 +46,7 @@ constexpr int kPairChunk = 256;
 // ---- reference helper formulas (scatter.cu:961-1038) ----
 
 // Scattering angle at the point a between the directions s -> a and a -> d; mb = |a -> d|, the
-// pair's distance (the same float).
+// pair's distance (within an ulp of what the three differences here give: another product is fused).
 __device__ __forceinline__ float cone_angle(float xs, float ys, float zs, float xa, float ya, float za,
                                             float xd, float yd, float zd, float mb)
 {
@@ -125,7 +125,7 @@ __device__ __forceinline__ bool cone_meets(const float4& k, const float4& j)
 // unless the distance and the radii's sum are within the error of both forms: reciprocal roots to
 // 2^-22 put a unit vector's components within 4e-7, a distance of two within 3e-6 with the reference
 // form's own rounding, and the radii's sum within 1e-6 of itself.  Configuration 3, the crystal bitmap:
-// 4.04 -> 2.15 ms.
+// 4.04 -> 2.18 ms.
 __device__ __forceinline__ bool cone_meets_from(float x, float y, float z, float xk, float yk, float zk, float rk,
                                                 float xi, float yi, float zi, float ri)
 {
@@ -980,7 +980,8 @@ static int build_pairs(const DevGeom& g, int parts, const uint32_t* bm_cry, cons
 {
     const int ns = g.n_det + (NATIVE ? g.n_holes : g.n_holes0);
     const long long np = (long long)g.n_det * ns;
-    // layout: [counts (np+1)][64-bit offsets (np+1)][cub temp][pairs][native][att]
+    // layout: [counts (np+1)][64-bit offsets (np+1)][cub temp][pairs][native]; the lists have a buffer of
+    // their own, sized once they are counted
     size_t temp_bytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, (long long*)nullptr, (long long*)nullptr, np + 1, s);
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };

@@ -72,7 +72,7 @@ struct ScatterLaunch {
     const PairNative* native;   // hole_model 2 only
     const AttEntry* att;
     const long long* att_offsets;   // 64-bit list offset of pair p; row d starts at [d * ns]
-    const double* kn_tab;  // Klein-Nishina table (kn_table_build), kKnTable + 1 nodes on [0, pi]
+    const double* kn_tab;  // Klein-Nishina tables (kn_table_build), kKnDoubles in all
     float* out;
 };
 

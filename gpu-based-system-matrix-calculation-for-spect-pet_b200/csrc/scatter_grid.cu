@@ -57,7 +57,7 @@ namespace {
 
 constexpr int kGridThreads = 256;
 constexpr int kGridChunk = 256;          // points per chunk (one per thread)
-constexpr int kGridMaxVox = 48;          // voxels per pass
+constexpr int kGridMaxVox = 48;          // voxels per pass (three blocks fit an SM up to 33, two beyond)
 constexpr int kGridDetTile = 32;         // detectors per block
 constexpr int kGridChunksPerBlock = 8;   // chunks per block at most
 
@@ -685,10 +685,11 @@ __host__ __device__ constexpr size_t grid_smem_bytes(int nv)
            (size_t)nv * (sizeof(float4) + sizeof(double) * kGridDetTile + sizeof(float) * kGridChunk);
 }
 
-// Three blocks to an SM: a block's phases (candidates, terms in double, items) each leave issue slots
-// idle (38 % used with at most two at 128 registers), which other blocks fill.  Configuration 3 at 0.5 mm
-// cells, 64 detectors x 24 voxels: 38.3 ms with two blocks, 27.0 with three (80 registers, 176 B of
-// spills), 28.1 with four.
+// Three blocks to an SM, in passes of up to 33 voxels (a block's shared memory is 34 KB and 1.3 KB a
+// voxel): a block's phases (candidates, terms in double, items) each leave issue slots idle (38 % used with
+// at most two at 128 registers), which other blocks fill.  Configuration 3 at 0.5 mm cells, 64 detectors x
+// 24 voxels: 38.3 ms with two blocks, 27.0 with three (80 registers, 176 B of spills), 28.1 with four.
+// Larger passes run two blocks with the registers of three: 31.1 ms at 33 voxels, 37.2 at 34, 42 to 46 at 48.
 __global__ void __launch_bounds__(kGridThreads, 3) grid_sum_kernel(DevGeom g, GridGeom G, GridSum S, int chunks_per_block)
 {
     extern __shared__ __align__(16) unsigned char grid_smem_raw[];
